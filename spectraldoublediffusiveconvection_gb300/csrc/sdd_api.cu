@@ -11,6 +11,7 @@
 #include <mutex>
 #include <vector>
 
+#include "sdd_fixed.cuh"
 #include "sdd_internal.cuh"
 #include "sdd_krylov.cuh"
 
@@ -58,27 +59,34 @@ const FftPlan* get_fft_plan(int L) {
   FftPlan* fp = new FftPlan();
   fp->L = L;
   if (L < 1 || !factor_length(L, fp->rad, &fp->nst)) { delete fp; return nullptr; }
-  std::vector<double2> w(L), e(L);
+  std::vector<int4> w(L), e(L);
   std::vector<float2> wf(L), ef(L);
-  const double pi = 3.14159265358979323846264338327950288;
+  const long double pi = 3.14159265358979323846264338327950288L;
+  auto digits = [](long double c, long double sn) {   // round(. 2^62) in two signed 32-bit digits each
+    int4 d;
+    fx_split_host(llroundl(ldexpl(c, 62)), &d.x, &d.y);
+    fx_split_host(llroundl(ldexpl(sn, 62)), &d.z, &d.w);
+    return d;
+  };
   for (int k = 0; k < L; ++k) {
-    const double a = 2.0 * pi * (double)k / (double)L;
-    w[k] = make_double2(std::cos(a), -std::sin(a));
-    const double b = pi * (double)k / (2.0 * (double)L);
-    e[k] = make_double2(0.5 * std::cos(b), 0.5 * std::sin(b));
-    wf[k] = make_float2((float)w[k].x, (float)w[k].y);
-    ef[k] = make_float2((float)e[k].x, (float)e[k].y);
+    const long double a = 2.0L * pi * (long double)k / (long double)L;
+    const long double b = pi * (long double)k / (2.0L * (long double)L);
+    w[k] = digits(cosl(a), -sinl(a));
+    e[k] = digits(0.5L * cosl(b), 0.5L * sinl(b));
+    const double ad = 2.0 * (double)pi * (double)k / (double)L, bd = (double)pi * (double)k / (2.0 * (double)L);
+    wf[k] = make_float2((float)std::cos(ad), (float)-std::sin(ad));
+    ef[k] = make_float2((float)(0.5 * std::cos(bd)), (float)(0.5 * std::sin(bd)));
   }
-  bool ok = cudaMalloc(&fp->w64, L * sizeof(double2)) == cudaSuccess &&
-            cudaMalloc(&fp->e64, L * sizeof(double2)) == cudaSuccess &&
+  bool ok = cudaMalloc(&fp->wfx, L * sizeof(int4)) == cudaSuccess &&
+            cudaMalloc(&fp->efx, L * sizeof(int4)) == cudaSuccess &&
             cudaMalloc(&fp->w32, L * sizeof(float2)) == cudaSuccess &&
             cudaMalloc(&fp->e32, L * sizeof(float2)) == cudaSuccess;
-  ok = ok && cudaMemcpy(fp->w64, w.data(), L * sizeof(double2), cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(fp->e64, e.data(), L * sizeof(double2), cudaMemcpyHostToDevice) == cudaSuccess &&
+  ok = ok && cudaMemcpy(fp->wfx, w.data(), L * sizeof(int4), cudaMemcpyHostToDevice) == cudaSuccess &&
+       cudaMemcpy(fp->efx, e.data(), L * sizeof(int4), cudaMemcpyHostToDevice) == cudaSuccess &&
        cudaMemcpy(fp->w32, wf.data(), L * sizeof(float2), cudaMemcpyHostToDevice) == cudaSuccess &&
        cudaMemcpy(fp->e32, ef.data(), L * sizeof(float2), cudaMemcpyHostToDevice) == cudaSuccess;
   if (!ok) {
-    cudaFree(fp->w64); cudaFree(fp->e64); cudaFree(fp->w32); cudaFree(fp->e32);
+    cudaFree(fp->wfx); cudaFree(fp->efx); cudaFree(fp->w32); cudaFree(fp->e32);
     delete fp;
     return nullptr;
   }
@@ -238,7 +246,7 @@ int sdd_transform(int kind, int rows, int n_in, int n_out, const double* in, dou
   const int L = inverse ? n_out : n_in;
   const FftPlan* fp = get_fft_plan(L);
   if (!fp) return SDD_ERR_UNSUPPORTED;
-  const size_t smem = 6 * (size_t)L * sizeof(double2) + (4 * 32 + 8) * sizeof(double);
+  const size_t smem = 6 * (size_t)L * sizeof(int4) + (4 * 32 + 8) * sizeof(double);
   if (smem > 227 * 1024) return SDD_ERR_UNSUPPORTED;
   cudaError_t e = launch_transform(kind, rows, n_in, n_out, fp, in, out, (cudaStream_t)stream);
   SDD_CUDA(e);
@@ -884,7 +892,7 @@ static FxArgs fx_args(const sdd_plan* p, int prec, const double* X, void* base, 
     a.ops.w = p->fft->w32; a.ops.e = p->fft->e32;
   } else {
     a.ops.Dr = p->Dr; a.ops.D2r2 = p->D2r2; a.ops.ir4r2 = p->ir4r2;
-    a.ops.w = p->fft->w64; a.ops.e = p->fft->e64;
+    a.ops.w = p->fft->wfx; a.ops.e = p->fft->efx;
   }
   a.X = X; a.x_stride = shell_elems(p);
   a.base = base; a.base_stride = sdd_plan_base_cache_elems(p);
@@ -1914,7 +1922,7 @@ static DiagArgs diag_args(const sdd_plan* p, const double* X, double* out) {
   std::memset(&a, 0, sizeof(a));
   a.M = p->M; a.nr = p->nr; a.sym = p->sym; a.L = p->dfft->L;
   a.st = stage_args(p->dfft);
-  a.w = p->dfft->w64; a.e = p->dfft->e64;
+  a.w = p->dfft->wfx; a.e = p->dfft->efx;
   a.Dr = p->Dr; a.ir = p->dg_ir; a.tw = p->dg_tw; a.wr = p->dg_wr; a.nuw = p->dg_nuw;
   a.ke_scale = p->ke_scale;
   a.X = X; a.x_stride = shell_elems(p);

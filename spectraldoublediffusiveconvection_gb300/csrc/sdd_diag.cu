@@ -8,7 +8,7 @@
 // integrates |.|^2 by the trapezoidal rule over r (x = R interior) and then over theta with sin(theta).
 // Both rules are weighted sums, so KE = (1/2V) sum_n wr_n sum_i wt_i sin(theta_i) (J^2 + D^2)(r_n, theta_i):
 // k_diag_rows computes the inner sum of one radius (the two transforms ride in one complex FFT of length
-// 3 N_fm, power-of-two balanced as in the other transforms) and k_diag_final the outer sums.
+// 3 N_fm, in fixed point like the other FP64 transforms) and k_diag_final the outer sums.
 //
 // Nusselt.  Nu - 1 at r = R[0] is (R[0]^2/A_T) sum_{k even} (D TT_k)[0]/(1 - k^2), TT_k the zero-padded
 // radial profile of mode k: a fixed weighted sum of the even-mode coefficients (weights from the plan).
@@ -44,22 +44,22 @@ size_t diag_rows_smem_bytes(int M, int L) { return (4 * (size_t)L * 2 + 5 * (siz
 
 // One CTA per (interior radius n, shell).
 __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
-  using C = double2;
+  using C = longlong2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, L = a.L;
   const int n = blockIdx.x, b = blockIdx.y;
   const int tid = threadIdx.x, bd = blockDim.x;
   C* RA = reinterpret_cast<C*>(smem_raw);
   C* RB = RA + L;
-  C* Wt = RB + L;
-  C* Et = Wt + L;
+  int4* Wt = reinterpret_cast<int4*>(RB + L);
+  int4* Et = Wt + L;
   double* pv = reinterpret_cast<double*>(Et + L);
   double* Sc = pv + M;
   double* dp = Sc + M;
   double* Ar = dp + M;        // cosine row: J_theta_RT(psi)_k(r_n) / r_n
   double* Br = Ar + M;        // sine row: (Dr psi)_{k-1}(r_n), [0] = 0
-  double* scl = Br + M;       // 2 scales + 2 inverses
-  unsigned long long* red = reinterpret_cast<unsigned long long*>(scl + 8);
+  double* scl = Br + M;       // the two rows' exponents
+  unsigned* red = reinterpret_cast<unsigned*>(scl + 8);
   for (int i = tid; i < L; i += bd) {
     Wt[i] = a.w[i];
     Et[i] = a.e[i];
@@ -77,47 +77,42 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
   parity_suffix<double>(pv, Sc, M);   // as J_theta_RT
   __syncthreads();
   const double irn = a.ir[n];
-  unsigned long long mb[2] = {0, 0};
   for (int k = tid; k < M; k += bd) {
     const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;
     double jp = (k == 0) ? 1.0 * s1 : (k + 1.0) * pv[k - 1] + 2.0 * s1;
     if (a.sym && (k % 2 == 1)) jp = 0.0;
-    const double av = irn * jp;
-    const double bv = k >= 1 ? dp[k - 1] : 0.0;
-    Ar[k] = av;
-    Br[k] = bv;
-    const unsigned long long ua = Bits<double>::absbits(av), ub = Bits<double>::absbits(bv);
-    mb[0] = ua > mb[0] ? ua : mb[0];
-    mb[1] = ub > mb[1] ? ub : mb[1];
+    Ar[k] = irn * jp;
+    Br[k] = k >= 1 ? dp[k - 1] : 0.0;
   }
-  block_max_scales<double, 2>(mb, red, scl);   // ends with a barrier
-  const double sa = scl[0], sb = scl[1];
+  __syncthreads();
   // DCT3 inputs with n_in = M on length L (see k_transform): cosine x_k = A_k; sine x_k = B_{L-k}
+  double* XV = reinterpret_cast<double*>(RB);
+  unsigned mx[2] = {0, 0};
   for (int k = tid; k < L; k += bd) {
     const double xa = (k < M) ? Ar[k] : 0.0;
     const double xb = (L - k <= M - 1 && k > 0) ? Br[L - k] : 0.0;
-    if (k == 0) {
-      RA[k] = make_double2(sa * xa, sb * xb);
-    } else {
-      const double xar = (L - k < M) ? Ar[L - k] : 0.0;
-      const double xbr = (k <= M - 1) ? Br[k] : 0.0;
-      const C e = Et[k];
-      const double a1 = fma(e.x, xa, e.y * xar), a2 = fma(e.y, xa, -(e.x * xar));
-      const double b1 = fma(e.x, xb, e.y * xbr), b2 = fma(e.y, xb, -(e.x * xbr));
-      RA[k] = make_double2(fma(sa, a1, -(sb * b2)), fma(sa, a2, sb * b1));
-    }
+    XV[k] = xa;
+    XV[L + k] = xb;
+    mx[0] = max(mx[0], abs_hi(xa));
+    mx[1] = max(mx[1], abs_hi(xb));
   }
+  int* E = reinterpret_cast<int*>(scl);
+  rows_to_fixed<2>(XV, L, 2, mx, red, E);
+  const i64* XA = reinterpret_cast<const i64*>(XV);
+  const i64* XB = XA + L;
+  for (int k = tid; k < L; k += bd)
+    RA[k] = k == 0 ? make_longlong2(XA[0], XB[0]) : dct3_pack_fx(Et[k], XA[k], XA[L - k], XB[k], XB[L - k]);
   __syncthreads();
   C* res = fft_rows<double, true>(RA, RB, 1, a.st, Wt);
+  const bool bad = E[0] == kFxBad || E[1] == kFxBad;
   double s[1] = {0.0};
   for (int i = tid; i < L; i += bd) {
     const int src = (i & 1) ? (L - 1 - (i >> 1)) : (i >> 1);
     const C v = res[src];
-    const double ja = v.x * scl[2];
-    double db = v.y * scl[3];
-    if (i & 1) db = -db;
+    const double ja = bad ? fx_nan() : fx2d(v.x, 60 - E[0]), db = fx2d(v.y, 60 - E[1]);   // (db's sign drops out)
     s[0] = fma(a.tw[i], fma(ja, ja, db * db), s[0]);
   }
+  __syncthreads();                      // (the scales are read before the sums reuse the reduction words)
   block_sum<1>(s, reinterpret_cast<double*>(red));
   if (tid == 0) a.part[(size_t)b * nr + n] = s[0];
 }

@@ -116,11 +116,92 @@ __device__ __forceinline__ void grid_products(int pair, const T* RG, const T* bs
   }
 }
 
+// The scaling of the rows that enter a transform, their packing, and their way out, for FP32 rows (exact
+// power-of-two balance of a pair, pow2_scale) and FP64 rows (64-bit fixed point, rows_to_fixed).  scl: the
+// block's scale words (FP32: K scales then K inverses; FP64: K exponents as ints).
+template <typename T> struct RowTr;
+template <> struct RowTr<float> {
+  static __device__ __forceinline__ unsigned key(float v) { return Bits<float>::absbits(v); }
+  static __device__ __forceinline__ float sign(float v, bool n) { return n ? -v : v; }
+  template <int K>
+  static __device__ __forceinline__ void scale(float*, int, int, unsigned (&mx)[K], void* red, float* scl) {
+    block_max_scales<float, K>(mx, reinterpret_cast<unsigned*>(red), scl);
+  }
+  // W_k of a DCT3 pair (rows A = t, B = t + 1 of XV; hasb: row B is there)
+  template <int K>
+  static __device__ __forceinline__ float2 pack(const float* XV, int P, int t, bool hasb, int k, const float2* Et,
+                                                const float* scl) {
+    const float sa = scl[t], sb = hasb ? scl[t + 1] : 0.0f;
+    const float xa = XV[t * P + k], xb = hasb ? XV[(t + 1) * P + k] : 0.0f;
+    if (k == 0) return cmk<float2>(sa * xa, sb * xb);
+    const float xar = XV[t * P + P - k], xbr = hasb ? XV[(t + 1) * P + P - k] : 0.0f;
+    return dct3_pack<float, float2>(Et[k], xa, xar, xb, xbr, sa, sb);
+  }
+  static __device__ __forceinline__ float2 load(const float* PR, int P, int t, int src, const float* scl) {
+    return cmk<float2>(scl[t] * PR[t * P + src], scl[t + 1] * PR[(t + 1) * P + src]);
+  }
+  // component (h = 0: row A, 1: row B) of a transformed pair whose first row is t of K
+  template <int K>
+  static __device__ __forceinline__ float out(float2 v, int h, int t, const float* scl) {
+    return (h ? v.y : v.x) * scl[K + t + h];
+  }
+  template <int K>
+  static __device__ __forceinline__ void unpack(const float2* Z, int P, int k, int t, const float2* Et, const float* scl,
+                                                float sc, float& ya, float& yb) {
+    dct2_unpack<float, float2>(Z[k], Z[(P - k) % P], Et[k], ya, yb);
+    ya *= sc * scl[K + t];
+    yb *= sc * scl[K + t + 1];
+  }
+};
+template <> struct RowTr<double> {
+  static __device__ __forceinline__ unsigned key(double v) { return abs_hi(v); }
+  static __device__ __forceinline__ double sign(double v, bool n) { return neg_if(v, n); }
+  template <int K>
+  static __device__ __forceinline__ void scale(double* XV, int P, int nrows, unsigned (&mx)[K], void* red, double* scl) {
+    rows_to_fixed<K>(XV, P, nrows, mx, reinterpret_cast<unsigned*>(red), reinterpret_cast<int*>(scl));
+  }
+  template <int K>
+  static __device__ __forceinline__ longlong2 pack(const double* XV, int P, int t, bool hasb, int k, const int4* Et,
+                                                   const double*) {
+    const i64* A = reinterpret_cast<const i64*>(XV) + t * P;
+    const i64* B = A + P;
+    const i64 xa = A[k], xb = hasb ? B[k] : 0;
+    if (k == 0) return make_longlong2(xa, xb);
+    return dct3_pack_fx(Et[k], xa, A[P - k], xb, hasb ? B[P - k] : 0);
+  }
+  static __device__ __forceinline__ longlong2 load(const double* PR, int P, int t, int src, const double*) {
+    const i64* A = reinterpret_cast<const i64*>(PR) + t * P;
+    return make_longlong2(A[src], A[P + src]);
+  }
+  // a row with an infinity or NaN makes both rows of its pair NaN (they share one complex transform)
+  template <int K>
+  static __device__ __forceinline__ bool bad(int t, const double* scl) {
+    const int* E = reinterpret_cast<const int*>(scl);
+    return E[t] == kFxBad || (t + 1 < K && E[t + 1] == kFxBad);
+  }
+  template <int K>
+  static __device__ __forceinline__ double out(longlong2 v, int h, int t, const double* scl) {
+    return bad<K>(t, scl) ? fx_nan() : fx2d(h ? v.y : v.x, 60 - reinterpret_cast<const int*>(scl)[t + h]);
+  }
+  template <int K>
+  static __device__ __forceinline__ void unpack(const longlong2* Z, int P, int k, int t, const int4* Et,
+                                                const double* scl, double sc, double& ya, double& yb) {
+    const int* E = reinterpret_cast<const int*>(scl);
+    i64 a, b;
+    dct2_unpack_fx(Z[k], Z[(P - k) % P], Et[k], a, b);
+    const bool n = bad<K>(t, scl);
+    ya = n ? fx_nan() : sc * fx2d(a, 60 - E[t]);
+    yb = n ? fx_nan() : sc * fx2d(b, 60 - E[t + 1]);
+  }
+};
+
 // MODE 0: NLIN_FX (optionally storing the grid fields); 1: NLIN_DFX with base fields from the cache;
 // 2: grid fields only (fills the cache).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   using C = typename Cplx<T>::type;
+  using W = typename Cplx<T>::tw;
+  using Tr = RowTr<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, P = a.P;
   const int n = blockIdx.x, b = blockIdx.y;
@@ -129,14 +210,13 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
 
   C* RA = reinterpret_cast<C*>(smem_raw);
   C* RB = RA + 5 * P;
-  C* Wt = RB + 5 * P;
-  C* Et = Wt + P;
+  W* Wt = reinterpret_cast<W*>(RB + 5 * P);
+  W* Et = Wt + P;
   T* RG = reinterpret_cast<T*>(Et + P);
   T* kf = RG + 9 * P;          // kf[k] = k, k < P + 2
   T* opr = kf + P + 2;
   T* scl = opr + 2 * kMaxNr;   // 9 scales + 9 inverse scales (inverse transforms), reused for 4+4
-  using U = typename Bits<T>::U;
-  U* red = reinterpret_cast<U*>(scl + 32);   // 9*32 reduction words
+  void* red = scl + 32;        // 9*32 reduction words of 8 bytes
   T* pv = RG;
   T* Tv = pv + M;
   T* Sv = Tv + M;
@@ -146,8 +226,8 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   T* DCv = DTv + M;
   T* JP = DCv + M;
   T* Sc = JP + M;
-  const C* wg = reinterpret_cast<const C*>(a.ops.w);
-  const C* eg = reinterpret_cast<const C*>(a.ops.e);
+  const W* wg = reinterpret_cast<const W*>(a.ops.w);
+  const W* eg = reinterpret_cast<const W*>(a.ops.e);
   for (int i = tid; i < P; i += bd) {
     Wt[i] = wg[i];
     Et[i] = eg[i];
@@ -218,33 +298,21 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   // the nine DCT3 input rows, materialised once (in RB, free until the FFT), with their maxima
   T* XV = reinterpret_cast<T*>(RB);
   {
-    U mb[9];
+    unsigned mb[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
       mb[t] = 0;
       for (int k = tid; k < P; k += bd) {
         const T v = fx_x<T>(t, k, M, P, kf, JP, OM, DP, DTv, DCv, Tv, Sv);
         XV[t * P + k] = v;
-        const U u = Bits<T>::absbits(v);
-        mb[t] = u > mb[t] ? u : mb[t];
+        mb[t] = max(mb[t], Tr::key(v));
       }
     }
-    block_max_scales<T, 9>(mb, red, scl);
+    Tr::template scale<9>(XV, P, 9, mb, red, scl);
   }
-  // W_k = s_A V_A(k) + i s_B V_B(k),  V(k) = 0.5 e^{i pi k/2P} (x_k - i x_{P-k}),  V(0) = x_0;
-  // Et holds 0.5 e^{i pi k/2P}.
   for (int idx = tid; idx < 5 * P; idx += bd) {
     const int p = idx / P;
-    const int k = idx - p * P;
-    const int ta = 2 * p, tb = 2 * p + 1;
-    const T sa = scl[ta], sb = (tb < 9) ? scl[tb] : (T)0;
-    const T xa = XV[ta * P + k], xb = (tb < 9) ? XV[tb * P + k] : (T)0;
-    if (k == 0) {
-      RA[idx] = cmk<C>(sa * xa, sb * xb);
-    } else {
-      const T xar = XV[ta * P + P - k], xbr = (tb < 9) ? XV[tb * P + P - k] : (T)0;
-      RA[idx] = dct3_pack<T, C>(Et[k], xa, xar, xb, xbr, sa, sb);
-    }
+    RA[idx] = Tr::template pack<9>(XV, P, 2 * p, p < 4, idx - p * P, Et, scl);
   }
   __syncthreads();
   C* res = fft_rows<T, true>(RA, RB, 5, a.st, Wt);
@@ -252,10 +320,8 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
     const int t = idx / P;
     const int i = idx - t * P;
     const int src = (i & 1) ? (P - 1 - (i >> 1)) : (i >> 1);
-    const C v = res[(t >> 1) * P + src];
-    T val = ((t & 1) ? v.y : v.x) * scl[9 + t];
-    if (t >= 5 && (i & 1)) val = -val;
-    RG[idx] = val;
+    const T val = Tr::template out<9>(res[(t >> 1) * P + src], t & 1, t & ~1, scl);
+    RG[idx] = Tr::sign(val, t >= 5 && (i & 1));
   }
   __syncthreads();
 
@@ -270,31 +336,23 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   const T* bs = (MODE == 1) ? reinterpret_cast<const T*>(a.base) + (size_t)b * a.base_stride +
                                   (size_t)n * 9 * P
                             : nullptr;
-  U m4[4] = {0, 0, 0, 0};
+  unsigned m4[4] = {0, 0, 0, 0};
   for (int i = tid; i < P; i += bd) {
-    T Q, Rr, NT, NS;
-    grid_products<T, MODE>(0, RG, bs, i, P, Q, Rr);
-    grid_products<T, MODE>(1, RG, bs, i, P, NT, NS);
-    const T sg = (i & 1) ? (T)-1 : (T)1;
-    PR[i] = sg * Q;
-    PR[P + i] = sg * Rr;
-    PR[2 * P + i] = NT;
-    PR[3 * P + i] = NS;
-    const U u0 = Bits<T>::absbits(Q), u1 = Bits<T>::absbits(Rr), u2 = Bits<T>::absbits(NT),
-            u3 = Bits<T>::absbits(NS);
-    m4[0] = u0 > m4[0] ? u0 : m4[0];
-    m4[1] = u1 > m4[1] ? u1 : m4[1];
-    m4[2] = u2 > m4[2] ? u2 : m4[2];
-    m4[3] = u3 > m4[3] ? u3 : m4[3];
+    T v[4];
+    grid_products<T, MODE>(0, RG, bs, i, P, v[0], v[1]);
+    grid_products<T, MODE>(1, RG, bs, i, P, v[2], v[3]);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      PR[t * P + i] = t < 2 ? Tr::sign(v[t], i & 1) : v[t];
+      m4[t] = max(m4[t], Tr::key(v[t]));
+    }
   }
-  block_max_scales<T, 4>(m4, red, scl);   // scl[0..4) scales, scl[4..8) inverses
+  Tr::template scale<4>(PR, P, 4, m4, red, scl);
 
   // ---- 4. four forward transforms as two paired DCT2s (:797-802) ----
   for (int idx = tid; idx < 2 * P; idx += bd) {
     const int p = idx / P;
-    const int nn = idx - p * P;
-    const int src = makhoul_src(nn, P);
-    RB[idx] = cmk<C>(scl[2 * p] * PR[(2 * p) * P + src], scl[2 * p + 1] * PR[(2 * p + 1) * P + src]);
+    RB[idx] = Tr::load(PR, P, 2 * p, makhoul_src(idx - p * P, P), scl);
   }
   __syncthreads();
   C* Z = fft_rows<T, false>(RB, RA, 2, a.st, Wt);
@@ -314,10 +372,7 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
       k = s;
     }
     if (!zero) {
-      dct2_unpack<T, C>(Z[p * P + k], Z[p * P + ((P - k) % P)], Et[k], ya, yb);
-      const T sc = (p == 1 && k == 0) ? one_P : two_P;
-      ya *= sc * scl[4 + 2 * p];
-      yb *= sc * scl[4 + 2 * p + 1];
+      Tr::template unpack<4>(Z + p * P, P, k, 2 * p, Et, scl, (p == 1 && k == 0) ? one_P : two_P, ya, yb);
     }
     const size_t q0 = (size_t)(2 * p) * N + (size_t)s * nr + n;
     o[q0] = (double)ya;
@@ -583,6 +638,8 @@ __global__ void __launch_bounds__(384) k_fx_deriv(FxArgs a, T* deriv, size_t der
 template <typename T>
 __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, size_t grid_stride) {
   using C = typename Cplx<T>::type;
+  using W = typename Cplx<T>::tw;
+  using Tr = RowTr<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, P = a.P;
   const int n = blockIdx.x, pr = blockIdx.y, b = blockIdx.z;
@@ -592,8 +649,8 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
 
   C* RA = reinterpret_cast<C*>(smem_raw);
   C* RB = RA + P;
-  C* Wt = RB + P;
-  C* Et = Wt + P;
+  W* Wt = reinterpret_cast<W*>(RB + P);
+  W* Et = Wt + P;
   T* kf = reinterpret_cast<T*>(Et + P);   // kf[k] = k, k < P + 2
   T* pv = kf + P + 2;
   T* Tv = pv + M;
@@ -605,10 +662,9 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
   T* JP = DCv + M;
   T* Sc = JP + M;
   T* scl = Sc + M;
-  using U = typename Bits<T>::U;
-  U* red = reinterpret_cast<U*>(scl + 32);
-  const C* wg = reinterpret_cast<const C*>(a.ops.w);
-  const C* eg = reinterpret_cast<const C*>(a.ops.e);
+  void* red = scl + 32;
+  const W* wg = reinterpret_cast<const W*>(a.ops.w);
+  const W* eg = reinterpret_cast<const W*>(a.ops.e);
   for (int i = tid; i < P; i += bd) {               // asynchronous: in flight while the row loads
     cp_async_elem(Wt + i, wg + i);
     cp_async_elem(Et + i, eg + i);
@@ -723,10 +779,11 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
     }
     __syncthreads();
   }
-  // the pair's two DCT3 input rows (in RB, free until the FFT) and their maxima
+  // the pair's two DCT3 input rows (in RB, free until the FFT) and their scales
+  const int nt = (tb < 9) ? 2 : 1;
   T* XV = reinterpret_cast<T*>(RB);
   {
-    U mb[2] = {0, 0};
+    unsigned mb[2] = {0, 0};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int t = ta + u;
@@ -734,41 +791,30 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
         for (int k = tid; k < P; k += bd) {
           const T v = fx_x<T>(t, k, M, P, kf, JP, OM, DP, DTv, DCv, Tv, Sv);
           XV[u * P + k] = v;
-          const U w = Bits<T>::absbits(v);
-          mb[u] = w > mb[u] ? w : mb[u];
+          mb[u] = max(mb[u], Tr::key(v));
         }
     }
-    block_max_scales<T, 2>(mb, red, scl);
+    Tr::template scale<2>(XV, P, nt, mb, red, scl);
   }
-  const T sa = scl[0], sb = (tb < 9) ? scl[1] : (T)0;
-  for (int k = tid; k < P; k += bd) {
-    const T xa = XV[k], xb = (tb < 9) ? XV[P + k] : (T)0;
-    if (k == 0) {
-      RA[k] = cmk<C>(sa * xa, sb * xb);
-    } else {
-      const T xar = XV[P - k], xbr = (tb < 9) ? XV[P + P - k] : (T)0;
-      RA[k] = dct3_pack<T, C>(Et[k], xa, xar, xb, xbr, sa, sb);
-    }
-  }
+  for (int k = tid; k < P; k += bd) RA[k] = Tr::template pack<2>(XV, P, 0, nt > 1, k, Et, scl);
   __syncthreads();
   C* res = fft_rows<T, true>(RA, RB, 1, a.st, Wt);
   T* g = grid + (size_t)b * grid_stride + (size_t)n * 9 * P;
-  const int nt = (tb < 9) ? 2 : 1;
   for (int idx = tid; idx < nt * P; idx += bd) {
     const int u = idx / P;
     const int i = idx - u * P;
     const int t = ta + u;
     const int src = (i & 1) ? (P - 1 - (i >> 1)) : (i >> 1);
-    const C v = res[src];
-    T val = (u ? v.y : v.x) * scl[2 + u];
-    if (t >= 5 && (i & 1)) val = -val;
-    g[(size_t)t * P + i] = val;
+    const T val = Tr::template out<2>(res[src], u, 0, scl);
+    g[(size_t)t * P + i] = Tr::sign(val, t >= 5 && (i & 1));
   }
 }
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* grid, size_t grid_stride) {
   using C = typename Cplx<T>::type;
+  using W = typename Cplx<T>::tw;
+  using Tr = RowTr<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, P = a.P;
   const int n = blockIdx.x, p = blockIdx.y, b = blockIdx.z;
@@ -776,14 +822,13 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
   const int tid = threadIdx.x, bd = blockDim.x;
   C* RA = reinterpret_cast<C*>(smem_raw);
   C* RB = RA + P;
-  C* Wt = RB + P;
-  C* Et = Wt + P;
+  W* Wt = reinterpret_cast<W*>(RB + P);
+  W* Et = Wt + P;
   T* PR = reinterpret_cast<T*>(Et + P);
   T* scl = PR + 2 * P;
-  using U = typename Bits<T>::U;
-  U* red = reinterpret_cast<U*>(scl + 32);
-  const C* wg = reinterpret_cast<const C*>(a.ops.w);
-  const C* eg = reinterpret_cast<const C*>(a.ops.e);
+  void* red = scl + 32;
+  const W* wg = reinterpret_cast<const W*>(a.ops.w);
+  const W* eg = reinterpret_cast<const W*>(a.ops.e);
   for (int i = tid; i < P; i += bd) {               // asynchronous: in flight while the products load
     cp_async_elem(Wt + i, wg + i);
     cp_async_elem(Et + i, eg + i);
@@ -791,28 +836,19 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
   const T* RG = grid + (size_t)b * grid_stride + (size_t)n * 9 * P;
   const T* bs = (MODE == 1) ? reinterpret_cast<const T*>(a.base) + (size_t)b * a.base_stride + (size_t)n * 9 * P
                             : nullptr;
-  U m2[2] = {0, 0};
+  unsigned m2[2] = {0, 0};
 #pragma unroll 2
   for (int i = tid; i < P; i += bd) {               // (unrolled: both iterations' grid loads in flight)
-    T v0, v1;
-    grid_products<T, MODE>(p, RG, bs, i, P, v0, v1);
-    if (p == 0) {
-      const T sg = (i & 1) ? (T)-1 : (T)1;
-      PR[i] = sg * v0;
-      PR[P + i] = sg * v1;
-    } else {
-      PR[i] = v0;
-      PR[P + i] = v1;
+    T v[2];
+    grid_products<T, MODE>(p, RG, bs, i, P, v[0], v[1]);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      PR[t * P + i] = p == 0 ? Tr::sign(v[t], i & 1) : v[t];
+      m2[t] = max(m2[t], Tr::key(v[t]));
     }
-    const U u0 = Bits<T>::absbits(v0), u1 = Bits<T>::absbits(v1);
-    m2[0] = u0 > m2[0] ? u0 : m2[0];
-    m2[1] = u1 > m2[1] ? u1 : m2[1];
   }
-  block_max_scales<T, 2>(m2, red, scl);   // scl[0..2) scales, scl[2..4) inverses
-  for (int nn = tid; nn < P; nn += bd) {
-    const int src = makhoul_src(nn, P);
-    RB[nn] = cmk<C>(scl[0] * PR[src], scl[1] * PR[P + src]);
-  }
+  Tr::template scale<2>(PR, P, 2, m2, red, scl);
+  for (int nn = tid; nn < P; nn += bd) RB[nn] = Tr::load(PR, P, 0, makhoul_src(nn, P), scl);
   cp_async_all_done();
   __syncthreads();
   C* Z = fft_rows<T, false>(RB, RA, 1, a.st, Wt);
@@ -831,10 +867,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
       k = s;
     }
     if (!zero) {
-      dct2_unpack<T, C>(Z[k], Z[(P - k) % P], Et[k], ya, yb);
-      const T sc = (p == 1 && k == 0) ? one_P : two_P;
-      ya *= sc * scl[2];
-      yb *= sc * scl[3];
+      Tr::template unpack<2>(Z, P, k, 0, Et, scl, (p == 1 && k == 0) ? one_P : two_P, ya, yb);
     }
     const size_t q0 = (size_t)(2 * p) * N + (size_t)s * nr + n;
     o[q0] = (double)ya;
@@ -1092,8 +1125,8 @@ __global__ void __launch_bounds__(kFxThreads) k_theta_op(ThetaArgs a) {
 struct TrArgs {
   int kind, rows, n_in, n_out, L;
   StageArgs st;
-  const double2* w;
-  const double2* e;
+  const int4* w;
+  const int4* e;
   const double* in;
   double* out;
 };
@@ -1101,123 +1134,82 @@ struct TrArgs {
 constexpr int kTrPairs = 2;
 
 __global__ void __launch_bounds__(kFxThreads) k_transform(TrArgs a) {
-  using C = double2;
+  using C = longlong2;
+  using Tr = RowTr<double>;
+  constexpr int kRows = 2 * kTrPairs;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int L = a.L;
   C* RA = reinterpret_cast<C*>(smem_raw);
   C* RB = RA + kTrPairs * L;
-  C* Wt = RB + kTrPairs * L;
-  C* Et = Wt + L;
-  double* scl = reinterpret_cast<double*>(Et + L);   // 4 scales + 4 inverses
-  unsigned long long* red = reinterpret_cast<unsigned long long*>(scl + 8);   // 4*32
+  int4* Wt = reinterpret_cast<int4*>(RB + kTrPairs * L);
+  int4* Et = Wt + L;
+  double* scl = reinterpret_cast<double*>(Et + L);   // the rows' exponents
+  void* red = scl + 8;                               // 4*32 reduction words of 8 bytes
   const int tid = threadIdx.x, bd = blockDim.x;
   for (int i = tid; i < L; i += bd) {
     Wt[i] = a.w[i];
     Et[i] = a.e[i];
   }
-  const int r0 = blockIdx.x * 2 * kTrPairs;
+  const int r0 = blockIdx.x * kRows;
   const bool inverse = (a.kind == SDD_IDCT || a.kind == SDD_IDST);
   const bool sine = (a.kind == SDD_IDST || a.kind == SDD_DST);
   const int n_in = a.n_in, n_out = a.n_out;
-  {  // per-row power-of-two balance of the pairs (see pow2_scale)
-    unsigned long long m[4] = {0, 0, 0, 0};
+  // the rows as they enter the transforms (DCT3: x_k, a sine row by its mirrored wavenumbers; DCT2: f_i with
+  // the alternating sign of a sine row), in RB, free until the FFT
+  double* XV = reinterpret_cast<double*>(RB);
+  unsigned mx[kRows];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const int r = r0 + h;
-      if (r < a.rows)
-        for (int i = tid; i < n_in; i += bd) {
-          const unsigned long long u = Bits<double>::absbits(a.in[(size_t)r * n_in + i]);
-          m[h] = u > m[h] ? u : m[h];
-        }
+  for (int t = 0; t < kRows; ++t) {
+    mx[t] = 0;
+    const int r = r0 + t;
+    const double* src = a.in + (size_t)r * n_in;
+    for (int k = tid; k < L; k += bd) {
+      double v = 0.0;
+      if (r < a.rows) {
+        if (!inverse) v = neg_if(src[k], sine && (k & 1));
+        else if (!sine) v = (k < n_in) ? src[k] : 0.0;
+        else if (k == 0) v = (L < n_in) ? 0.5 * src[L] : 0.0;
+        else v = (L - k <= n_in - 1) ? src[L - k] : 0.0;
+      }
+      XV[t * L + k] = v;
+      mx[t] = max(mx[t], abs_hi(v));
     }
-    block_max_scales<double, 4>(m, red, scl);
   }
+  rows_to_fixed<kRows>(XV, L, kRows, mx, reinterpret_cast<unsigned*>(red), reinterpret_cast<int*>(scl));
   if (inverse) {
     for (int idx = tid; idx < kTrPairs * L; idx += bd) {
       const int p = idx / L;
-      const int k = idx - p * L;
-      C V[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = r0 + 2 * p + h;
-        double x = 0, xr = 0;
-        if (r < a.rows) {
-          const double* src = a.in + (size_t)r * n_in;
-          for (int pass = 0; pass < 2; ++pass) {
-            const int kk = pass == 0 ? k : L - k;
-            double v = 0;
-            if (pass == 1 && k == 0) break;
-            if (!sine) {
-              v = (kk < n_in) ? src[kk] : 0.0;
-            } else if (kk == 0) {
-              v = (L < n_in) ? 0.5 * src[L] : 0.0;
-            } else {
-              const int w = L - kk;
-              v = (w <= n_in - 1) ? src[w] : 0.0;
-            }
-            if (pass == 0) x = v; else xr = v;
-          }
-          x *= scl[2 * p + h];
-          xr *= scl[2 * p + h];
-        }
-        if (k == 0) {
-          V[h] = make_double2(x, 0.0);
-        } else {
-          const C e = Et[k];
-          V[h] = make_double2(fma(e.x, x, e.y * xr), fma(e.y, x, -(e.x * xr)));
-        }
-      }
-      RA[idx] = make_double2(V[0].x - V[1].y, V[0].y + V[1].x);
+      RA[idx] = Tr::template pack<kRows>(XV, L, 2 * p, true, idx - p * L, Et, scl);
     }
     __syncthreads();
     C* res = fft_rows<double, true>(RA, RB, kTrPairs, a.st, Wt);
-    for (int idx = tid; idx < 2 * kTrPairs * L; idx += bd) {
+    for (int idx = tid; idx < kRows * L; idx += bd) {
       const int t = idx / L;
       const int i = idx - t * L;
       const int r = r0 + t;
       if (r >= a.rows) continue;
       const int src = (i & 1) ? (L - 1 - (i >> 1)) : (i >> 1);
-      const C v = res[(t >> 1) * L + src];
-      double val = ((t & 1) ? v.y : v.x) * scl[4 + t];
-      if (sine && (i & 1)) val = -val;
-      a.out[(size_t)r * n_out + i] = val;
+      const double val = Tr::template out<kRows>(res[(t >> 1) * L + src], t & 1, t & ~1, scl);
+      a.out[(size_t)r * n_out + i] = neg_if(val, sine && (i & 1));
     }
   } else {
     for (int idx = tid; idx < kTrPairs * L; idx += bd) {
       const int p = idx / L;
-      const int nn = idx - p * L;
-      const int src = makhoul_src(nn, L);
-      double v[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = r0 + 2 * p + h;
-        double x = (r < a.rows) ? a.in[(size_t)r * n_in + src] * scl[2 * p + h] : 0.0;
-        if (sine && (src & 1)) x = -x;
-        v[h] = x;
-      }
-      RA[idx] = make_double2(v[0], v[1]);
+      RA[idx] = Tr::load(XV, L, 2 * p, makhoul_src(idx - p * L, L), scl);
     }
     __syncthreads();
     C* Z = fft_rows<double, false>(RA, RB, kTrPairs, a.st, Wt);
-    for (int idx = tid; idx < 2 * kTrPairs * n_out; idx += bd) {
-      const int t = idx / n_out;
-      const int s = idx - t * n_out;
-      const int r = r0 + t;
-      if (r >= a.rows) continue;
-      double y = 0;
+    for (int idx = tid; idx < kTrPairs * n_out; idx += bd) {
+      const int p = idx / n_out;
+      const int s = idx - p * n_out;
+      const int r = r0 + 2 * p;
+      double ya = 0.0, yb = 0.0;
       if (!(sine && s == 0)) {
         const int k = sine ? L - s : s;
-        const int p = t >> 1;
-        const C Zk = Z[p * L + k];
-        const C Zm = Z[p * L + ((L - k) % L)];
-        const C e = Et[k];
-        if ((t & 1) == 0)
-          y = fma(e.x, Zk.x + Zm.x, e.y * (Zk.y - Zm.y));
-        else
-          y = fma(e.x, Zk.y + Zm.y, -(e.y * (Zk.x - Zm.x)));
-        y *= ((!sine && k == 0) ? 1.0 / L : 2.0 / L) * scl[4 + t];
+        Tr::template unpack<kRows>(Z + p * L, L, k, 2 * p, Et, scl, (!sine && k == 0) ? 1.0 / L : 2.0 / L, ya, yb);
       }
-      a.out[(size_t)r * n_out + s] = y;
+      if (r < a.rows) a.out[(size_t)r * n_out + s] = ya;
+      if (r + 1 < a.rows) a.out[(size_t)(r + 1) * n_out + s] = yb;
     }
   }
 }
@@ -1450,11 +1442,11 @@ cudaError_t launch_transform(int kind, int rows, int n_in, int n_out, const FftP
   a.n_out = n_out;
   a.L = fp->L;
   a.st = stage_args(fp);
-  a.w = fp->w64;
-  a.e = fp->e64;
+  a.w = fp->wfx;
+  a.e = fp->efx;
   a.in = in;
   a.out = out;
-  const size_t smem = (2 * kTrPairs + 2) * (size_t)fp->L * sizeof(double2) + (4 * 32 + 8) * 8;
+  const size_t smem = (2 * kTrPairs + 2) * (size_t)fp->L * sizeof(longlong2) + (4 * 32 + 8) * 8;
   static unsigned long long done = 0;
   cudaError_t e = ensure_smem_attr(k_transform, &done);
   if (e != cudaSuccess) return e;

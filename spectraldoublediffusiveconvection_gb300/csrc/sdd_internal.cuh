@@ -78,8 +78,8 @@ struct FftPlan {
   int L = 0;
   int nst = 0;
   int rad[kMaxStages] = {0};
-  double2* w64 = nullptr;   // exp(-2 pi i k / L), k < L
-  double2* e64 = nullptr;   // 0.5 exp(+i pi k / (2L)), k < L
+  int4* wfx = nullptr;      // exp(-2 pi i k / L), k < L, in 32-bit digits (re hi, lo, im hi, lo) of 2^62
+  int4* efx = nullptr;      // 0.5 exp(+i pi k / (2L)), k < L, the same
   float2* w32 = nullptr;
   float2* e32 = nullptr;
 };
@@ -136,8 +136,8 @@ struct FxOps {               // FP64 or FP32 copies of the operators the nonline
   const void* Dr;            // nr*nr
   const void* D2r2;          // nr*nr
   const void* ir4r2;         // nr
-  const void* w;             // FFT twiddles (complex, P)
-  const void* e;             // DCT twiddles (complex, P)
+  const void* w;             // FFT twiddles (P): FP32 complex, or fixed-point digits (FP64)
+  const void* e;             // DCT twiddles (P), the same
 };
 
 struct RhsArgs {
@@ -323,8 +323,8 @@ struct ChainArgs {
 struct DiagArgs {
   int M, nr, sym, L;         // L = 3 M: the kinetic-energy grid
   StageArgs st;              // FFT of length L
-  const double2* w;          // FFT twiddles of length L
-  const double2* e;          // DCT twiddles of length L
+  const int4* w;             // FFT twiddles of length L (fixed-point digits)
+  const int4* e;             // DCT twiddles of length L
   const double* Dr;          // nr*nr interior D
   const double* ir;          // nr  1/R interior
   const double* tw;          // L   trapezoid weight * sin(theta_i) on the L-point midpoint grid
