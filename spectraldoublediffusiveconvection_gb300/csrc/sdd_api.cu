@@ -132,9 +132,9 @@ struct sdd_plan {
   double dt, Pr, Tau;
   const FftPlan* fft;
   // FP64 operators
-  double *Dr, *D2r2, *ir4r2, *D2s, *ir2s, *D2A4, *ir2A4, *ir4A4, *rsq, *dT0, *gr;
-  double *LinvA4, *LinvT, *LinvS;
-  double *ABA4;                     // transposed [A_j B_j] of the psi chain
+  double *Dr, *D2r2, *ir4r2, *D2s, *ir2s, *rsq, *dT0, *gr;
+  const i64 *LinvA4, *LinvT, *LinvS;   // fixed-point blocks (sdd_fixed.cuh), one per mode
+  const i64* ABA4;                  // [A_j B_j] of the psi chain, two blocks per mode
   double *coefA4, *coefT, *coefS;   // per-step scalars of the chains
   // chunked chains: cs[0] the chunking of layout 2 (sequential carry), cs[1] of layout 3 (parallel
   // carry); leading dimensions; workspaces sized for the larger chunk and product counts
@@ -266,19 +266,41 @@ static int upload32(float** dst, const double* src, size_t n) {
   SDD_CUDA(cudaMemcpy(*dst, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
   return SDD_OK;
 }
-// Linv blocks (and D2_A4 with M = 1) go to the device transposed, column c of a block contiguous with
-// leading dimension ldl (even, so every block starts on a 16-byte boundary for cp.async).
-static int upload_linv(double** dst, const double* src, int M, int nr, int ldl) {
-  if (!src) return SDD_ERR_ARG;
-  std::vector<double> h((size_t)M * nr * ldl, 0.0);
-  for (int m = 0; m < M; ++m)
-    for (int i = 0; i < nr; ++i)
-      for (int c = 0; c < nr; ++c) h[((size_t)m * nr + c) * ldl + i] = src[((size_t)m * nr + i) * nr + c];
-  SDD_CUDA(cudaMalloc(dst, h.size() * sizeof(double)));
-  SDD_CUDA(cudaMemcpy(*dst, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+// Matrices as fixed-point blocks (sdd_fixed.cuh): nmat host matrices of nrg nr x nseg nr, column-major with
+// leading dimension ld (stride cols ld), become nrg nseg blocks each, row halves outermost.
+// On the plan's private non-blocking stream: another host thread may be capturing a graph meanwhile, which
+// rules out the default stream's launches and device-wide waits.
+static int upload_fixed(sdd_plan* p, const i64** dst, const double* src, int nmat, int cols, int ld, int nr, int ldl,
+                        int nrg, int nseg) {
+  if (!p->cap_stream) SDD_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
+  cudaStream_t s = p->cap_stream;
+  const size_t n = (size_t)nmat * cols * ld, bw = fx_block_words(ldl), per = (size_t)nrg * nseg * bw;
+  double* tmp = nullptr;
+  i64* out = nullptr;
+  cudaError_t e = cudaMalloc(&tmp, n * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&out, nmat * per * sizeof(i64));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, src, n * sizeof(double), cudaMemcpyHostToDevice, s);
+  for (int q = 0; q < nrg * nseg && e == cudaSuccess; ++q)
+    e = launch_to_fixed(tmp, (size_t)cols * ld, ld, nrg * nr, q / nseg * nr, q % nseg * nr, nr, ldl, out + q * bw, per,
+                        nmat, s);
+  const cudaError_t ew = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = ew;
+  cudaFree(tmp);
+  if (e != cudaSuccess) cudaFree(out);
+  SDD_CUDA(e);
+  *dst = out;
   return SDD_OK;
 }
-// The same transposed layout rounded to FP32.
+// Linv blocks (row-major on the host).
+static int upload_linv(sdd_plan* p, const i64** dst, const double* src, int M, int nr, int ldl) {
+  if (!src) return SDD_ERR_ARG;
+  std::vector<double> h((size_t)M * nr * nr);
+  for (int m = 0; m < M; ++m)
+    for (int i = 0; i < nr; ++i)
+      for (int c = 0; c < nr; ++c) h[((size_t)m * nr + c) * nr + i] = src[((size_t)m * nr + i) * nr + c];
+  return upload_fixed(p, dst, h.data(), M, nr, nr, nr, ldl, 1, 1);
+}
+// Linv blocks transposed (column c contiguous, leading dimension ldl) and rounded to FP32.
 static int upload_linv32(float** dst, const double* src, int M, int nr, int ldl) {
   if (!src) return SDD_ERR_ARG;
   std::vector<float> h((size_t)M * nr * ldl, 0.0f);
@@ -339,8 +361,8 @@ static void clear_step_graphs(sdd_plan* p) {
 }
 
 static void free_chunk_set(ChunkSet& c) {
-  const double* t[] = {c.GA4, c.GT, c.GS, c.PhiA4, c.PhiT, c.PhiS, c.PA4, c.PT, c.PS};
-  for (const double* x : t) cudaFree(const_cast<double*>(x));
+  const i64* t[] = {c.GA4, c.GT, c.GS, c.PhiA4, c.PhiT, c.PhiS, c.PA4, c.PT, c.PS};
+  for (const i64* x : t) cudaFree(const_cast<i64*>(x));
   c = ChunkSet{};
 }
 
@@ -353,11 +375,12 @@ static void free_plan(sdd_plan* p) {
   if (p->branch_stream) cudaStreamDestroy(p->branch_stream);
   for (cudaEvent_t e : p->branch_ev)
     if (e) cudaEventDestroy(e);
-  double* d[] = {p->Dr, p->D2r2, p->ir4r2, p->D2s, p->ir2s, p->D2A4, p->ir2A4, p->ir4A4, p->rsq, p->dT0,
-                 p->gr, p->LinvA4, p->LinvT, p->LinvS, p->out4, p->rhs, p->xtmp, p->coefA4, p->coefT, p->coefS, p->ABA4, p->hbuf,
+  double* d[] = {p->Dr, p->D2r2, p->ir4r2, p->D2s, p->ir2s, p->rsq, p->dT0,
+                 p->gr, p->out4, p->rhs, p->xtmp, p->coefA4, p->coefT, p->coefS, p->hbuf,
                  p->dbuf, p->cbuf, p->pbuf,
                  p->dg_ir, p->dg_tw, p->dg_wr, p->dg_nuw, p->dg_part, p->dg_out};
   for (double* x : d) cudaFree(x);
+  for (const i64* x : {p->LinvA4, p->LinvT, p->LinvS, p->ABA4}) cudaFree(const_cast<i64*>(x));
   for (ChunkSet& c : p->cs) free_chunk_set(c);
   cudaFree(p->Dr32); cudaFree(p->D2r232); cudaFree(p->ir4r232); cudaFree(p->D2s32);
   cudaFree(p->tcB); cudaFree(p->tc_err);
@@ -377,8 +400,8 @@ static void free_plan(sdd_plan* p) {
 //     Psi_{k+1} = [[I, 0], [bjt I, I]] Psi_k + [I; bj I] G_k   (f_e += f, bf_e += bj f + bjt f_e)
 //   T/S (s = b, m = nr):  G_k = -w_k Linv_k Psi_k,  Psi_{k+1} = Psi_k + k_{k+1} G_k   (b += k f before
 //     the next step, k = 2 dt (j+2) of that step, w = 0.5 for j = 0 else 1)
-// with Psi = I at the chunk start, and Phi_c = Psi after the chunk's last step.  G is stored transposed
-// per mode ([jj][m cols][ldl]) and Phi per (parity, chunk) ([m cols][ldm]).
+// with Psi = I at the chunk start, and Phi_c = Psi after the chunk's last step.  Formed in FP64 (transposed, G
+// per mode [jj][m cols][ldl], Phi per (parity, chunk) [m cols][ldm]), uploaded as fixed-point blocks.
 static void matmul_rows(const double* A, const double* B, double* C, int n, int k, int m) {  // C = A B
   for (int i = 0; i < n; ++i) {
     double* c = C + (size_t)i * m;
@@ -464,18 +487,10 @@ static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB,
               Phi[(((size_t)par * nch + c) * m + col) * ldm + i] = Psi[(size_t)i * m + col];
       }
     int st;
-    double* g = nullptr;
-    double* t = nullptr;
-    if ((st = upload(&g, G.data(), G.size()))) return st;
-    cs->GA4 = g;
-    if (products) {
-      carry_products(Phi, nch, m, ldm, Pr);
-      if ((st = upload(&t, Pr.data(), Pr.size()))) return st;
-      cs->PA4 = t;
-    } else {
-      if ((st = upload(&t, Phi.data(), Phi.size()))) return st;
-      cs->PhiA4 = t;
-    }
+    if ((st = upload_fixed(p, &cs->GA4, G.data(), M, m, ldl, nr, ldl, 1, 2))) return st;
+    if (products) carry_products(Phi, nch, m, ldm, Pr);
+    if (products && cs->np > 0 && (st = upload_fixed(p, &cs->PA4, Pr.data(), 2 * cs->np, m, ldm, nr, ldl, 2, 2))) return st;
+    if (!products && (st = upload_fixed(p, &cs->PhiA4, Phi.data(), 2 * nch, m, ldm, nr, ldl, 2, 2))) return st;
   }
   for (int fld = 1; fld <= 2; ++fld) {  // T, S
     const int m = nr, ldm = p->ldmT;
@@ -503,18 +518,13 @@ static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB,
               Phi[(((size_t)par * nch + c) * m + col) * ldm + i] = Psi[(size_t)i * m + col];
       }
     int st;
-    double* g = nullptr;
-    double* t = nullptr;
-    if ((st = upload(&g, G.data(), G.size()))) return st;
-    (fld == 1 ? cs->GT : cs->GS) = g;
-    if (products) {
-      carry_products(Phi, nch, m, ldm, Pr);
-      if ((st = upload(&t, Pr.data(), Pr.size()))) return st;
-      (fld == 1 ? cs->PT : cs->PS) = t;
-    } else {
-      if ((st = upload(&t, Phi.data(), Phi.size()))) return st;
-      (fld == 1 ? cs->PhiT : cs->PhiS) = t;
-    }
+    if ((st = upload_fixed(p, fld == 1 ? &cs->GT : &cs->GS, G.data(), M, m, ldl, nr, ldl, 1, 1))) return st;
+    if (products) carry_products(Phi, nch, m, ldm, Pr);
+    if (products && cs->np > 0 &&
+        (st = upload_fixed(p, fld == 1 ? &cs->PT : &cs->PS, Pr.data(), 2 * cs->np, m, ldm, nr, ldl, 1, 1)))
+      return st;
+    if (!products && (st = upload_fixed(p, fld == 1 ? &cs->PhiT : &cs->PhiS, Phi.data(), 2 * nch, m, ldm, nr, ldl, 1, 1)))
+      return st;
   }
   return SDD_OK;
 }
@@ -597,7 +607,7 @@ int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
   if (!fp) return SDD_ERR_UNSUPPORTED;
   sdd_plan* p = new sdd_plan();
   std::memset(p, 0, sizeof(*p));
-  p->M = M; p->nr = nr; p->P = P; p->ldl = nr + (nr & 1); p->sym = d->symmetric ? 1 : 0;
+  p->M = M; p->nr = nr; p->P = P; p->ldl = fx_ld(nr); p->sym = d->symmetric ? 1 : 0;
   p->prec = d->precision; p->device = dev;
   p->reorth_eta = kReorthEta;
   p->dt = d->dt; p->Pr = d->Pr; p->Tau = d->Tau;
@@ -606,12 +616,10 @@ int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
   int st = SDD_OK;
   if ((st = upload(&p->Dr, d->Dr, nn)) || (st = upload(&p->D2r2, d->D2_r2, nn)) ||
       (st = upload(&p->ir4r2, d->ir4_r2, nr)) || (st = upload(&p->D2s, d->D2_sine, nn)) ||
-      (st = upload(&p->ir2s, d->ir2_sine, nr)) || (st = upload_linv(&p->D2A4, d->D2_A4, 1, nr, p->ldl)) ||
-      (st = upload(&p->ir2A4, d->ir2_A4, nr)) || (st = upload(&p->ir4A4, d->ir4_A4, nr)) ||
-      (st = upload(&p->rsq, d->rsq, nr)) || (st = upload(&p->dT0, d->dT0, nr)) ||
-      (st = upload(&p->gr, d->gr, nr)) || (st = upload_linv(&p->LinvA4, d->Linv_A4, M, nr, p->ldl)) ||
-      (st = upload_linv(&p->LinvT, d->Linv_T, M, nr, p->ldl)) ||
-      (st = upload_linv(&p->LinvS, d->Linv_S, M, nr, p->ldl)) ||
+      (st = upload(&p->ir2s, d->ir2_sine, nr)) || (st = upload(&p->rsq, d->rsq, nr)) || (st = upload(&p->dT0, d->dT0, nr)) ||
+      (st = upload(&p->gr, d->gr, nr)) || (st = upload_linv(p, &p->LinvA4, d->Linv_A4, M, nr, p->ldl)) ||
+      (st = upload_linv(p, &p->LinvT, d->Linv_T, M, nr, p->ldl)) ||
+      (st = upload_linv(p, &p->LinvS, d->Linv_S, M, nr, p->ldl)) ||
       (st = upload32(&p->Dr32, d->Dr, nn)) || (st = upload32(&p->D2r232, d->D2_r2, nn)) ||
       (st = upload32(&p->ir4r232, d->ir4_r2, nr))) {
     free_plan(p);
@@ -687,7 +695,7 @@ int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
         }
       }
     }
-    if ((st = upload(&p->ABA4, AB.data(), AB.size())) ||
+    if ((st = upload_fixed(p, &p->ABA4, AB.data(), M, 2 * nr, ldl, nr, ldl, 1, 2)) ||
         (st = build_chunk_tables(p, AB.data(), d->Linv_T, d->Linv_S, cA.data(), cT.data(), cS.data())) ||
         (st = build_diag_tables(p, d))) {
       free_plan(p);
@@ -934,12 +942,12 @@ static ChainArgs chain_args(const sdd_plan* p, const double* g, double* f, const
   a.f = f; a.f_stride = shell_elems(p);
   a.sub = sub; a.sub_stride = shell_elems(p);
   a.LinvA4 = p->LinvA4; a.LinvT = p->LinvT; a.LinvS = p->LinvS;
-  a.ABA4 = p->ABA4; a.D2A4 = p->D2A4; a.ir2A4 = p->ir2A4; a.ir4A4 = p->ir4A4;
+  a.ABA4 = p->ABA4;
   a.h = p->hbuf;
   a.h_stride = shell_elems(p);
   a.coefA4 = p->coefA4; a.coefT = p->coefT; a.coefS = p->coefS;
   a.dtA4 = p->Pr * p->dt; a.dtT = p->dt; a.dtS = p->Tau * p->dt;
-  a.ldmA = p->ldmA; a.ldmT = p->ldmT; a.ldd = p->ldd;
+  a.ldd = p->ldd;
   a.cset[0] = p->cs[0];
   a.cset[1] = p->cs[1];
   a.dbuf = p->dbuf; a.cbuf = p->cbuf; a.counter = p->dcnt;

@@ -4,10 +4,10 @@
 // a 32 x 32 + 64-bit integer multiply-add (IMAD.WIDE) every 2.1, a 64-bit add every 2-3.  The transforms and
 // the block matvecs of the implicit solves are sums of products with known operators over a row or a vector
 // whose largest entry is easy to find, so they run on integers: a vector is scaled by one power of two to a
-// 64-bit integer each, an operator by one per row (on the host), both are split into two signed 32-bit digits
-// (value = hi 2^32 + lo, lo in [-2^31, 2^31)), and a product keeps three of its four digit products in two
-// 64-bit accumulators (hi hi, and hi lo + lo hi; lo lo is below the last bit kept).  The sums are exact, so
-// they do not depend on their order.  Rounding to 57-60 bits below a bound on the vector replaces FP64's 53
+// 64-bit integer each, an operator by one per row and one per column, both are split into two signed digits
+// (transforms: value = hi 2^32 + lo; matvecs: hi 2^27 + lo with 30 bits of hi, so that no sum of products of 64
+// columns overflows), and a product keeps three of its four digit products in 64-bit accumulators (hi hi, hi lo
+// and lo hi; lo lo is below the last bit kept).  The sums are exact, so they do not depend on their order.  Rounding to 57-60 bits below a bound on the vector replaces FP64's 53
 // bits per operation: against extended precision the errors are below FP64's (transforms: the bound is the
 // row's 1-norm, which no intermediate value exceeds; matvecs: 1e-18 to 1e-17 of the result's norm against
 // 1.5e-16 to 1e-15 on states of the time step).
@@ -55,6 +55,16 @@ __device__ __forceinline__ double fx2d(i64 v, int s) {
   if (e >= 2047) bits = 0x7ff0000000000000ull;
   if (v == 0 || e <= 0) bits = 0;
   return __longlong_as_double((i64)(bits | ((u64)v & 0x8000000000000000ull)));
+}
+
+// The same by the FP64 pipe's conversion: half the latency (66 against 107 cycles), as many cycles of issue;
+// for a lone dependent value.
+__device__ __forceinline__ double fx2d_lat(i64 v, int s) {
+  const double d = __ll2double_rn(v);
+  const int hi = __double2hiint(d), e = ((hi >> 20) & 0x7ff) - s;
+  const double r = __hiloint2double(hi - (s << 20), __double2loint(d));
+  if (v == 0 || e <= 0) return 0.0;
+  return e >= 2047 ? __longlong_as_double((v < 0 ? 0xfff0000000000000ll : 0x7ff0000000000000ll)) : r;
 }
 
 __device__ __forceinline__ double fx_nan() { return __longlong_as_double(0x7ff8000000000000ll); }
@@ -138,5 +148,174 @@ __device__ __forceinline__ void rows_to_fixed(double* XV, int P, int nrows, cons
   }
   __syncthreads();
 }
+
+// ---- block matvecs -------------------------------------------------------------------------------
+// An nr x nr block A in global memory, padded with zeros to L x L (L = fx_ld(nr), so that the inner loops have
+// no remainder) and its columns scaled to a = A 2^-cx with |a| < 1: word [col][row] = the two digits of
+// round(a 2^(57 - ea)) (lo in the low half), then the L rows' exponents ea as ints, sum over a row of
+// |a| < 2^ea (kFxBad: a row with an infinity or NaN), and the L columns' exponents cx.  Operands are scaled by
+// 2^cx before their largest entry sets their fixed point: so the bits kept are relative to the largest product
+// A_kc x_c, not to the largest x_c (the Chebyshev operators' columns differ by N^2 to N^4, and so do a state's
+// derivatives against them).  Blocks start on 16 bytes.
+__host__ __device__ inline int fx_ld(int nr) { return nr <= 32 ? (nr + 7) / 8 * 8 : (nr + 15) / 16 * 16; }
+__host__ __device__ constexpr size_t fx_block_words(int ld) { return (size_t)(ld + 1) * ld; }
+__device__ __forceinline__ const int* fx_row_exp(const i64* blk, int ld) {
+  return reinterpret_cast<const int*>(blk + (size_t)ld * ld);
+}
+__device__ __forceinline__ const int* fx_col_exp(const i64* blk, int ld) { return fx_row_exp(blk, ld) + ld; }
+
+// A matvec's digits: v = hi 2^27 + lo, lo in [-2^26, 2^26), |v| <= 2^57.
+__device__ __forceinline__ int2 mv_digits(i64 v) {
+  return make_int2(((int)v << 5) >> 5, (int)((v + (1ll << 26)) >> 27));
+}
+__device__ __forceinline__ i64 mv_value(int2 d) { return ((i64)d.y << 27) + d.x; }
+
+// An operand's exponent (biased, after its column scale): x = 0 counts below every number, an infinity above
+// (kFxInf), a NaN above that (kFxBad).
+constexpr int kFxInf = kFxBad - 1;
+__device__ __forceinline__ int fx_key(double x, int cx) {
+  const unsigned h = abs_hi(x);
+  const int e = (int)(h >> 20);
+  if (e == 0x7ff) return ((h & 0xfffffu) | (unsigned)__double2loint(x)) ? kFxBad : kFxInf;
+  return e ? e + cx : -0x10000;
+}
+// The operand's digits, 57 bits below the largest exponent em; with em = kFxInf its raw bits.
+__device__ __forceinline__ int2 fx_digits(double x, int cx, int em) {
+  const i64 X = em >= kFxInf ? __double_as_longlong(x) : d2fx(x, 5 + em - cx);
+  return em >= kFxInf ? make_int2((int)X, (int)(X >> 32)) : mv_digits(X);
+}
+
+// A product's unit: fx_dot's integer is the product times 2^(kFxMvExp - ea - em).
+constexpr int kFxMvExp = 1022 + 61;
+
+// A value v 2^e (|v| <= 2^61), or with e = kFxBad the bits of a double.
+struct FxVal {
+  i64 v;
+  int e;
+};
+__device__ __forceinline__ i64 fx_shr(i64 v, int n) { return v >> min(n, 63); }
+__device__ __forceinline__ double fx_val(FxVal p) { return p.e == kFxBad ? __longlong_as_double(p.v) : fx2d(p.v, -p.e); }
+
+// h + p and h + p + q, summed in fixed point 59 bits below the largest and rounded once (LAT: the conversion
+// with the lower latency, for the chains).
+template <bool LAT = false>
+__device__ __forceinline__ double fx_sum(double h, FxVal p) {
+  const int eh = (int)(abs_hi(h) >> 20);
+  if (p.e == kFxBad || eh == 0x7ff) return h + fx_val(p);
+  const int em = max(eh - 1081, p.e);
+  const i64 v = fx_shr(p.v, em - p.e) + d2fx(h, 1084 + em);
+  return LAT ? fx2d_lat(v, -em) : fx2d(v, -em);
+}
+template <bool LAT = false>
+__device__ __forceinline__ double fx_sum(double h, FxVal p, FxVal q) {
+  const int eh = (int)(abs_hi(h) >> 20);
+  if (p.e == kFxBad || q.e == kFxBad || eh == 0x7ff) return (h + fx_val(p)) + fx_val(q);
+  const int em = max(max(eh - 1081, p.e), q.e);
+  const i64 v = fx_shr(p.v, em - p.e) + fx_shr(q.v, em - q.e) + d2fx(h, 1084 + em);
+  return LAT ? fx2d_lat(v, -em) : fx2d(v, -em);
+}
+
+// Row A of a block in shared memory (column stride LD words) times NC operand digits xs, in units of 2^53 of the
+// operands' units.
+template <int NC, int LD>
+__device__ __forceinline__ i64 fx_dot(const int2* A, const int2* xs) {
+  const int4* x4 = reinterpret_cast<const int4*>(xs);
+  i64 t2 = 0, t1 = 1ll << 25, t0 = 0;
+#pragma unroll
+  for (int c = 0; c < NC; c += 2) {
+    const int4 v = x4[c >> 1];
+    const int2 a = A[c * LD], b = A[(c + 1) * LD];
+    t2 = fx_mad(a.y, v.y, t2);
+    t1 = fx_mad(a.y, v.x, t1);
+    t0 = fx_mad(a.x, v.y, t0);
+    t2 = fx_mad(b.y, v.w, t2);
+    t1 = fx_mad(b.y, v.z, t1);
+    t0 = fx_mad(b.x, v.w, t0);
+  }
+  return (t2 << 1) + ((t1 + t0) >> 26);
+}
+
+// The same product in FP64 over columns [c0, c1) of row r, for an operand with an infinity (em = kFxInf: raw
+// doubles in xs): the infinities and NaNs that FP64 gives.
+static __device__ __noinline__ double fx_dot_slow(const i64* blk, int ld, int r, const int2* xs, int c0, int c1, int em) {
+  const int2* A = reinterpret_cast<const int2*>(blk) + r;
+  const int ea = fx_row_exp(blk, ld)[r];
+  const int* cx = fx_col_exp(blk, ld);
+  double acc = 0.0;
+  for (int c = c0; c < c1; ++c) {
+    const int2 a = A[(size_t)c * ld], x = xs[c];
+    const double av = ea == kFxBad ? fx_nan() : ldexp(__ll2double_rn(mv_value(a)), ea - 57 + cx[c]);
+    const double xv = em >= kFxInf ? __hiloint2double(x.y, x.x)
+                                   : ldexp(__ll2double_rn(mv_value(x)), em - (1022 + 57) - cx[c]);
+    acc = fma(av, xv, acc);
+  }
+  return acc;
+}
+
+// A vector of nr <= 32 NP elements (x[p] = element 32 p + lane) as operand digits in xs for a block with column
+// exponents cx; returns its exponent em.
+template <int NP>
+__device__ __forceinline__ int publish_regs(const double (&x)[NP], const int (&cx)[NP], int nr, int lane, int2* xs) {
+  int m = -0x10000;
+#pragma unroll
+  for (int p = 0; p < NP; ++p)
+    if (p * 32 + lane < nr) m = max(m, fx_key(x[p], cx[p]));
+  const int em = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll
+  for (int p = 0; p < NP; ++p)
+    if (p * 32 + lane < nr) xs[p * 32 + lane] = fx_digits(x[p], cx[p], em);
+  __syncwarp();
+  return em;
+}
+// A lane's row of a block in registers (its loads all in flight at once), and its product with a published
+// operand: the arithmetic of fx_dot.  LD <= 32 NP.
+template <int LD, int NP>
+struct FxRow {
+  int2 m[LD];
+  int ea, cx[NP];            // the row's exponent; the column exponents of the lane's operand elements
+  __device__ __forceinline__ void load(const i64* blk, int r) {
+    const int2* A = reinterpret_cast<const int2*>(blk) + r;
+#pragma unroll
+    for (int c = 0; c < LD; ++c) m[c] = __ldg(A + c * LD);
+    ea = __ldg(fx_row_exp(blk, LD) + r);
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) cx[p] = 32 * p + lane < LD ? __ldg(fx_col_exp(blk, LD) + 32 * p + lane) : 0;
+  }
+  __device__ __forceinline__ FxVal times(const i64* blk, int nr, int r, const int2* xs, int em) const {
+    FxVal p;
+    i64 t2 = 0, t1 = 1ll << 25, t0 = 0;
+#pragma unroll
+    for (int c = 0; c < LD; c += 2) {
+      const int4 v = reinterpret_cast<const int4*>(xs)[c >> 1];
+      t2 = fx_mad(m[c].y, v.y, t2);
+      t1 = fx_mad(m[c].y, v.x, t1);
+      t0 = fx_mad(m[c].x, v.y, t0);
+      t2 = fx_mad(m[c + 1].y, v.w, t2);
+      t1 = fx_mad(m[c + 1].y, v.z, t1);
+      t0 = fx_mad(m[c + 1].x, v.w, t0);
+    }
+    p.v = (t2 << 1) + ((t1 + t0) >> 26);
+    p.e = ea + em - kFxMvExp;
+    if (em >= kFxInf || ea == kFxBad) {                // (after the registers of the row are done with)
+      p.v = __double_as_longlong(em == kFxInf ? fx_dot_slow(blk, LD, r, xs, 0, nr, em) : fx_nan());
+      p.e = kFxBad;
+    }
+    return p;
+  }
+};
+
+// ---- asynchronous copies -------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 }  // namespace sdd

@@ -391,7 +391,6 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
 //     sine-type Q, R; p = 1: the cosine-type NT, NS) and runs their paired forward transform into out4.
 // Per element the operations and their order are those of k_fx_rows, so the results are identical.
 constexpr int kFxSplitThreads = 256;
-constexpr size_t kFxDerivStageMaxBytes = 110 * 1024;   // two derivative CTAs per SM
 
 // FP32 grid kernels of the fused right-hand side keep FP64 copies of the row's psi, T, S and psi's parity
 // suffix sums (4 M doubles) for the linear parts, after the T-typed arrays.
@@ -412,14 +411,6 @@ size_t fx_prod_smem_bytes(int P, int prec) {
 // columns in the order of the fused kernel's (so both paths round identically).  With the fused
 // right-hand side a fifth block, D2s psi_k in FP64, follows the four T-typed blocks (per shell:
 // 4 M nr T then M nr doubles).
-// sum over the TPR lanes of a row group (the order of the chains' group_sum)
-template <int TPR>
-__device__ __forceinline__ double lane_group_sum(double v) {
-#pragma unroll
-  for (int off = 1; off < TPR; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
-}
-
 // One asynchronous global -> shared copy of an element of 4, 8 or 16 bytes (the issuing thread does not
 // wait for the data: a loop of such copies has all its loads in flight at once).
 template <int BYTES>
@@ -438,35 +429,25 @@ __device__ __forceinline__ void cp_async_all_done() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_all;\n" ::: "memory");
 }
 
-// Shared memory for a staged pending correction (FixArgs::stage): the G blocks of the mode's three chains
-// (2 nr + nr + nr columns of ldl) and, per chain, d_{c-1} and the carry terms of its chunk c (at most
-// nch - 1 vectors of 2 nr / nr / nr doubles).
-__host__ __device__ inline size_t fix_stage_doubles(int nr, int ldl, int nch) {
-  return (size_t)4 * nr * ldl + (size_t)(nch > 1 ? nch - 1 : 0) * 4 * nr;
-}
+// The terms d_{c-1}, part_{c,0}, ..., part_{c,c-2} of the carried states of a pending correction of mode k, by
+// asynchronous copies (the caller commits and waits): per chain f, from st + c o_f (o = 0, 2 nr, 3 nr), c
+// vectors of m_f = 2 nr, nr, nr doubles.
+__host__ __device__ inline size_t fix_term_doubles(int nr, int nch) { return (size_t)(nch > 1 ? nch - 1 : 0) * 4 * nr; }
 
-// The asynchronous copies of a staged correction of mode k into st (16-byte aligned): the G blocks of the
-// three chains at st, st + 2 nr ldl, st + 3 nr ldl; then per chain f, from st + 4 nr ldl + c o_f
-// (o = 0, 2 nr, 3 nr), the c vectors d_{c-1}, part_{c,0}, ..., part_{c,c-2} of m_f doubles each.  The
-// caller commits and waits.
-__device__ __forceinline__ void stage_pending_fix(const FxArgs& a, int b, int k, double* st) {
+__device__ __forceinline__ void stage_fix_terms(const FxArgs& a, int b, int k, double* st) {
   const FixArgs& x = a.fix;
-  const int M = a.M, nr = a.nr, ldl = x.ldl;
-  const int jj = M - 1 - k, par = jj & 1, c = (jj >> 1) / x.kc;
+  const int nr = a.nr;
+  const int jj = a.M - 1 - k, par = jj & 1, c = (jj >> 1) / x.kc;
   if (c < 1) return;
   for (int f = 0; f < 3; ++f) {
     const bool a4 = f == 0;
     if (a.sym && !(a4 ? par == 0 : par == 1)) continue;
     const int m = a4 ? 2 * nr : nr;
     const int o = a4 ? 0 : (f == 1 ? 2 * nr : 3 * nr);
-    const double* G = (a4 ? x.GA4 : (f == 1 ? x.GT : x.GS)) + (size_t)jj * m * ldl;
-    double* Gs = st + (size_t)o * ldl;
-    for (int e = threadIdx.x; e < m * ldl / 2; e += blockDim.x)   // m ldl is even (ldl even)
-      cp_async_bytes<16>(Gs + 2 * e, G + 2 * e);
     const size_t chain = (size_t)(f * 2 + par);
     const double* d = x.dbuf + (size_t)b * x.d_stride + chain * x.nch * x.ldd + (size_t)(c - 1) * x.ldd;
     const double* prow = x.pbuf + (size_t)b * x.p_stride + (chain * x.np + (size_t)(c - 1) * (c - 2) / 2) * x.ldd;
-    double* Ts = st + (size_t)4 * nr * ldl + (size_t)c * o;
+    double* Ts = st + (size_t)c * o;
     for (int e = threadIdx.x; e < c * m; e += blockDim.x) {
       const int v = e / m, i = e - v * m;
       cp_async_bytes<8>(Ts + e, v == 0 ? d + i : prow + (size_t)(v - 1) * x.ldd + i);
@@ -474,93 +455,79 @@ __device__ __forceinline__ void stage_pending_fix(const FxArgs& a, int b, int k,
   }
 }
 
-// The pending correction of mode k (see FixArgs) on xd (the mode's FP64 psi, T, S rows, in shared memory),
-// the three fields at once, each by its own 128 threads (threads 128 f .. 128 f + 127; the CTA has 384):
-// s_c = d_{c-1} + part_{c,0} + ... in index order, then xd += G_jj s_c with rows split over TPR lanes as
-// k_mode_mv<TPR, true> (the same bits); the corrected rows are written back to the state (and its FP32
-// copy).  sc holds the three carried states (4 nr doubles).  st: the staged G blocks and terms
-// (stage_pending_fix, landed), or null to read them from global memory.
-template <int TPR>
+// The pending correction of mode k (see FixArgs) on xd (the mode's FP64 psi, T, S rows, in shared memory; xd
+// and the terms `st` still in flight).  Four tasks of NP warps each (psi's two operand halves, T, S): a warp's
+// rows of G load into registers while the terms arrive; s_c = d_{c-1} + part_{c,0} + ... in index order; then
+// xd += G_jj s_c in the arithmetic of k_mode_mv (the same bits).  The corrected rows are written back to the
+// state (and its FP32 copy).  sc: 4 nr doubles.
+template <int LD>
 __device__ void apply_pending_fix(const FxArgs& a, int b, int k, double* xd, double* sc, const double* st) {
+  constexpr int NP = (LD + 31) / 32;
+  constexpr int bw = (int)fx_block_words(LD);
+  __shared__ __align__(16) int2 s_x[4 * NP][32 * NP];
+  __shared__ i64 s_v[4][32 * NP];
+  __shared__ int s_e[4][32 * NP];
   const FixArgs& x = a.fix;
-  const int M = a.M, nr = a.nr, ldl = x.ldl;
+  const int M = a.M, nr = a.nr;
   const int jj = M - 1 - k, par = jj & 1, c = (jj >> 1) / x.kc;
+  const bool psi_on = !a.sym || par == 0, ts_on = !a.sym || par == 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = warp / NP, r = (warp % NP) * 32 + lane, rr = min(r, nr - 1);
+  const bool on = c >= 1 && warp < 4 * NP && (task < 2 ? psi_on : ts_on);   // uniform over the warp
+  const i64* blk = task < 2 ? x.GA4 + ((size_t)jj * 2 + task) * bw : (task == 2 ? x.GT : x.GS) + (size_t)jj * bw;
+  FxRow<LD, NP> G;
+  if (on) G.load(blk, rr);
+  cp_async_all_done();
+  __syncthreads();
   if (c < 1) return;                                   // uniform over the CTA
-  const size_t N = (size_t)M * nr;
-  const int f = threadIdx.x >> 7, t = threadIdx.x & 127;
-  const bool a4 = f == 0;
-  const bool on = f < 3 && !(a.sym && !(a4 ? par == 0 : par == 1));
-  const int m = a4 ? 2 * nr : nr;
-  const int o = a4 ? 0 : (f == 1 ? 2 * nr : 3 * nr);
-  double* s = sc + o;
-  if (on) {
-    const size_t chain = (size_t)(f * 2 + par);
-    const int nt = c - 1;
-    if (st) {
-      const double* Ts = st + (size_t)4 * nr * ldl + (size_t)c * o;
-      for (int e = t; e < m; e += 128) {
-        double v = Ts[e];                              // d_{c-1} + part_0 + ... + part_{c-2} in index order
-        for (int u = 0; u < nt; ++u) v += Ts[(size_t)(u + 1) * m + e];
-        s[e] = v;
-      }
-    } else {
-      const double* d = x.dbuf + (size_t)b * x.d_stride + chain * x.nch * x.ldd;
-      const double* prow = x.pbuf + (size_t)b * x.p_stride + (chain * x.np + (size_t)(c - 1) * (c - 2) / 2) * x.ldd;
-      for (int e = t; e < m; e += 128) {
-        // d_{c-1} + part_0 + ... + part_{c-2} in index order, the terms loaded eight at a time (a load
-        // after each addition would wait out one L2 round trip per term)
-        double v = d[(size_t)(c - 1) * x.ldd + e];
-        for (int u0 = 0; u0 < nt; u0 += 8) {
-          double tv[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) tv[k] = (u0 + k < nt) ? prow[(size_t)(u0 + k) * x.ldd + e] : 0.0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (u0 + k < nt) v += tv[k];
-        }
-        s[e] = v;
-      }
-    }
+  for (int e = threadIdx.x; e < 4 * nr; e += blockDim.x) {
+    if (!(e < 2 * nr ? psi_on : ts_on)) continue;
+    const int o = e < 2 * nr ? 0 : (e < 3 * nr ? 2 * nr : 3 * nr), m = e < 2 * nr ? 2 * nr : nr;
+    const double* Ts = st + (size_t)c * o + (e - o);
+    double v = Ts[0];                                  // d_{c-1} + part_0 + ... + part_{c-2} in index order
+    for (int u = 1; u < c; ++u) v += Ts[(size_t)u * m];
+    sc[e] = v;
   }
   __syncthreads();
   if (on) {
-    const double* G = st ? st + (size_t)o * ldl : (a4 ? x.GA4 : (f == 1 ? x.GT : x.GS)) + (size_t)jj * m * ldl;
-    const int i = t / TPR, q = t % TPR;
-    for (int r0 = 0; r0 < nr; r0 += 128 / TPR) {
-      const int r = r0 + i;
-      const int rr = r < nr ? r : 0;
-      double acc = 0.0;
-#pragma unroll 16
-      for (int col = q; col < m; col += TPR) acc = fma(G[(size_t)col * ldl + rr], s[col], acc);
-      acc = lane_group_sum<TPR>(acc);
-      if (r < nr && q == 0) {
-        const double v = xd[f * nr + r] + acc;
-        xd[f * nr + r] = v;
-        const size_t o = (size_t)b * a.x_stride + (size_t)f * N + (size_t)k * nr + r;
-        x.X[o] = v;
-        if (x.X32) x.X32[(size_t)b * a.x32_stride + (size_t)f * N + (size_t)k * nr + r] = (float)v;
-      }
-    }
+    double xv[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) xv[p] = 32 * p + lane < nr ? sc[task * nr + 32 * p + lane] : 0.0;
+    const int em = publish_regs<NP>(xv, G.cx, nr, lane, s_x[warp]);
+    const FxVal p = G.times(blk, nr, rr, s_x[warp], em);
+    s_v[task][r] = p.v;
+    s_e[task][r] = p.e;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 3 * nr; e += blockDim.x) {
+    const int f = e / nr, i = e - f * nr;
+    if (!(f == 0 ? psi_on : ts_on)) continue;
+    const FxVal p{s_v[f == 0 ? 0 : f + 1][i], s_e[f == 0 ? 0 : f + 1][i]}, q{s_v[1][i], s_e[1][i]};
+    const double v = f == 0 ? fx_sum(xd[e], p, q) : fx_sum(xd[e], p);
+    xd[e] = v;
+    const size_t o = (size_t)f * M * nr + (size_t)k * nr + i;
+    x.X[(size_t)b * a.x_stride + o] = v;
+    if (x.X32) x.X32[(size_t)b * a.x32_stride + o] = (float)v;
   }
   __syncthreads();
 }
 
 // T-typed Dr, D2r2 and the mode's rows; then (FP64) the corrected rows and carried states of a pending fix
 // (7 nr); then the fused right-hand side's D2s (nr^2) and the mode's FP64 psi row (nr); then, 16-byte
-// aligned, the staged correction (stage_doubles, fix_stage_doubles, or 0)
+// aligned, the correction's terms (fix_term_doubles)
 __host__ __device__ inline size_t fx_deriv_stage_offset(int nr, int prec, bool fix, bool fuse) {
   const size_t es = prec == SDD_PREC_MIXED ? sizeof(float) : sizeof(double);
   const size_t t = ((2 * (size_t)nr * nr + 3 * (size_t)nr) * es + 15) / 16 * 16;
   return (t + (fix ? 7 * (size_t)nr * sizeof(double) : 0) + (fuse ? ((size_t)nr * nr + nr) * sizeof(double) : 0) +
           15) / 16 * 16;
 }
-size_t fx_deriv_smem_bytes(int nr, int prec, bool fix, bool fuse, size_t stage_doubles) {
-  return fx_deriv_stage_offset(nr, prec, fix, fuse) + stage_doubles * sizeof(double);
+size_t fx_deriv_smem_bytes(int nr, int prec, bool fix, bool fuse, int nch) {
+  return fx_deriv_stage_offset(nr, prec, fix, fuse) + (fix ? fix_term_doubles(nr, nch) : 0) * sizeof(double);
 }
 
 
-template <typename T>
-__global__ void __launch_bounds__(384) k_fx_deriv(FxArgs a, T* deriv, size_t deriv_stride) {
+template <typename T, int LD>
+__global__ void __launch_bounds__(256, LD <= 32 ? 2 : 1) k_fx_deriv(FxArgs a, T* deriv, size_t deriv_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr;
   const int k = blockIdx.x, b = blockIdx.y;
@@ -573,14 +540,11 @@ __global__ void __launch_bounds__(384) k_fx_deriv(FxArgs a, T* deriv, size_t der
   double* D2sm = xd + (a.fix.on ? 7 * nr : 0);        // fused right-hand side: A2_SINE's D2 (FP64)
   const T* Drg = reinterpret_cast<const T*>(a.ops.Dr);
   const T* D2g = reinterpret_cast<const T*>(a.ops.D2r2);
-  double* stg = (a.fix.on && a.fix.stage)
-                    ? reinterpret_cast<double*>(smem_raw + fx_deriv_stage_offset(nr, sizeof(T) == 4 ? SDD_PREC_MIXED
-                                                                                                    : SDD_PREC_FP64,
-                                                                                 true, a.fuse_rhs != 0))
-                    : nullptr;
-  // the operators (and the rows, G blocks and carry terms of a pending fix) stream in asynchronously: one
-  // L2 round trip, not one per element each thread copies
-  if (stg) stage_pending_fix(a, b, k, stg);
+  // the operators (and the rows and carry terms of a pending fix) stream in asynchronously: one L2 round
+  // trip, not one per element each thread copies
+  double* terms = reinterpret_cast<double*>(
+      smem_raw + fx_deriv_stage_offset(nr, sizeof(T) == 4 ? SDD_PREC_MIXED : SDD_PREC_FP64, true, a.fuse_rhs != 0));
+  if (a.fix.on) stage_fix_terms(a, b, k, terms);
   for (int e = threadIdx.x; e < nr * nr; e += blockDim.x) {
     cp_async_elem(ops + e, Drg + e);
     cp_async_elem(ops + nr * nr + e, D2g + e);
@@ -592,10 +556,7 @@ __global__ void __launch_bounds__(384) k_fx_deriv(FxArgs a, T* deriv, size_t der
       const int f = e / nr, m = e - f * nr;
       cp_async_elem(xd + e, a.fix.X + (size_t)b * a.x_stride + (size_t)f * N + (size_t)k * nr + m);
     }
-    cp_async_all_done();
-    __syncthreads();
-    if (nr <= 32) apply_pending_fix<4>(a, b, k, xd, sc, stg);
-    else apply_pending_fix<2>(a, b, k, xd, sc, stg);
+    apply_pending_fix<LD>(a, b, k, xd, sc, terms);
     for (int e = threadIdx.x; e < 3 * nr; e += blockDim.x) xv[e] = (T)xd[e];
   } else {
     with_x<T>(a, b, [&](auto xr) {
@@ -1306,22 +1267,21 @@ static cudaError_t launch_fx_split_t(const FxArgs& a, int batch, cudaStream_t s)
   T* grid = reinterpret_cast<T*>((MODE != 1 && a.base) ? a.base : a.grid);
   const size_t gs = (MODE != 1 && a.base) ? a.base_stride : a.grid_stride;
   cudaError_t e;
+  using Deriv = void (*)(FxArgs, T*, size_t);
+  static const Deriv derivs[6] = {k_fx_deriv<T, 8>,  k_fx_deriv<T, 16>, k_fx_deriv<T, 24>,
+                                  k_fx_deriv<T, 32>, k_fx_deriv<T, 48>, k_fx_deriv<T, 64>};
+  const int ldi = a.nr <= 32 ? (a.nr - 1) / 8 : (a.nr <= 48 ? 4 : 5);   // fx_ld(nr)
+  const Deriv deriv = derivs[ldi];
   {
-    static unsigned long long done = 0;   // large nr with a pending correction can pass 48 KB
-    if ((e = ensure_smem_attr(k_fx_deriv<T>, &done)) != cudaSuccess) return e;
+    static unsigned long long done[6] = {};   // large nr with a pending correction can pass 48 KB
+    if ((e = ensure_smem_attr(deriv, &done[ldi])) != cudaSuccess) return e;
   }
   // with tensor cores the per-mode kernel only applies a pending chain correction and forms the fused
   // right-hand side's FP64 block; the contractions follow on the corrected state
   const bool tc = sizeof(T) == 4 && a.deriv_t;
   if (!tc || a.fix.on || a.fuse_rhs) {
-    // a pending correction's G blocks and terms are staged with the operators while the CTA still fits
-    // twice on an SM (the per-mode CTAs of one shell outnumber the SMs)
-    FxArgs ad = a;
-    size_t sd = a.fix.on ? fix_stage_doubles(a.nr, a.fix.ldl, a.fix.nch) : 0;
-    if (fx_deriv_smem_bytes(a.nr, prec, a.fix.on != 0, a.fuse_rhs != 0, sd) > kFxDerivStageMaxBytes) sd = 0;
-    ad.fix.stage = sd > 0 ? 1 : 0;
-    e = launch_kernel(k_fx_deriv<T>, dim3(a.M, batch), dim3(a.fix.on ? 384 : 256),
-                      fx_deriv_smem_bytes(a.nr, prec, a.fix.on != 0, a.fuse_rhs != 0, sd), s, ad,
+    e = launch_kernel(deriv, dim3(a.M, batch), dim3(256),
+                      fx_deriv_smem_bytes(a.nr, prec, a.fix.on != 0, a.fuse_rhs != 0, a.fix.nch), s, a,
                       reinterpret_cast<T*>(a.deriv), a.deriv_stride);
     ktimer_mark(SDD_K_FX_DERIV, s);
     if (e != cudaSuccess) return e;

@@ -5,6 +5,7 @@
 #include <stddef.h>
 
 #include "../../include/sdd_gb300.h"
+#include "sdd_fixed.cuh"
 
 namespace sdd {
 
@@ -176,19 +177,17 @@ struct RhsArgs {
 
 // A chunk correction of the state left pending by the previous time step (layouts 3 / 11, sdd_step): the split
 // nonlinear term's k_fx_deriv applies X[jj] += G_jj s_c(jj) to its mode before using it, with the
-// arithmetic of k_mode_mv<TPR, true> (the same bits), and writes the corrected rows back (and their FP32
+// arithmetic of k_mode_mv (the same bits), and writes the corrected rows back (and their FP32
 // copy).  The previous step's chunk end states and carry products are still in dbuf / pbuf: this step's
 // chains overwrite them only after the nonlinear term.
 struct FixArgs {
   int on;
   int kc, nch, np, ldd, ldl;
-  const double* GA4, *GT, *GS;
+  const i64* GA4, *GT, *GS;
   const double* dbuf, *pbuf;
   size_t d_stride, p_stride;
   double* X;                 // the state being corrected in place (the nonlinear term's input)
   float* X32;                // nullable: its FP32 copy
-  int stage;                 // set by the launcher: the mode's G blocks and carried-state terms are staged
-                             // in shared memory when they fit (fix_stage_doubles)
 };
 
 struct FxArgs {
@@ -254,16 +253,16 @@ struct TcArgs {
 // row j after row j-1; the parallel carry of layout 3).
 struct ChunkSet {
   int kc, nch, np;
-  const double* GA4, *GT, *GS;        // [M][m cols][ldl] transposed G_jj (m = 2 nr for psi, nr for T/S)
-  const double* PhiA4, *PhiT, *PhiS;  // [2 parity][nch][m cols][ldm] transposed Phi_c
-  const double* PA4, *PT, *PS;        // [2 parity][np][m cols][ldm] transposed P_{j,i}
+  const i64* GA4, *GT, *GS;           // G_jj: [M][2] blocks (psi: f_e, bf_e half), [M] blocks (T, S)
+  const i64* PhiA4, *PhiT, *PhiS;     // Phi_c: [2 parity][nch] x 4 blocks (row half, operand half) or 1
+  const i64* PA4, *PT, *PS;           // P_{j,i}: [2 parity][np] x 4 blocks or 1
 };
 
 struct ChainArgs {
   int M, nr, ldl, sym;
   int field0;                // first field handled (blockIdx.x/2 + field0)
-  int layout;                // 1 one lane per row, 4 rows split over 4 warps, 2/3 chunked, 6/7 the reference's
-                             // order (resolved by the host)
+  int layout;                // the requested layout (0 automatic; resolve_chain_layout)
+  int type0, fmask;          // set by launch_chain: first chain type (0 psi, 1 T and S), fields to solve
   size_t field_off;          // doubles between field blocks (N_fm*nr, or 0 when g/f point at one block)
   const double* g;           // rhs [shell][3][M][nr]
   size_t g_stride;
@@ -273,12 +272,10 @@ struct ChainArgs {
   size_t f32_stride;
   const double* sub;         // nullable: f -= sub (Newton residual), same layout
   size_t sub_stride;
-  const double* LinvA4, *LinvT, *LinvS;  // [M][nr cols][ldl] transposed blocks
-  const double* ABA4;        // [M][2 nr cols][ldl]: transposed [A_j B_j] of the psi chain
-  const double* D2A4;        // [nr cols][ldl]: transposed D2 of the psi operator (layouts 6 and 7)
+  // fixed-point blocks (sdd_fixed.cuh): Linv of every mode, and the psi step matrices [A_j B_j] as two
+  const i64* LinvA4, *LinvT, *LinvS, *ABA4;
   double* h;                 // [shell][3][M][nr] h = Linv g
   size_t h_stride;           // doubles between shells in h
-  const double* ir2A4, *ir4A4;
   const double* coefA4;      // [M][4] per jj: (dt bjt, dt bjt bj, bj, bjt), dt = Pr*dt, j = M - jj
   const double* coefT, *coefS;  // [M][4] per jj: (2 dt (j+2), 0.5 if j == 0 else 1, 0, 0), j = M-1-jj
   double dtA4, dtT, dtS;     // Pr*dt, dt, Tau*dt
@@ -295,20 +292,19 @@ struct ChainArgs {
   // of kc steps.  Chunk c runs from a zero carried state (f_local, end state d_c); the carried states
   // s_c at the chunk starts follow s_{c+1} = Phi_c s_c + d_c; then f += G_jj s_c for the chunk's modes.
   int kc, nch;               // chunk length (steps) and chunks per chain
-  int ldmA, ldmT;            // leading dimensions of Phi for the psi (m = 2 nr) and T/S (m = nr) states
   int ldd;                   // doubles per (field, parity, chunk) slot of dbuf / cbuf (>= 2 nr, even)
-  const double* GA4, *GT, *GS;        // [M][m cols][ldl] transposed G_jj (m = 2 nr for psi, nr for T/S)
-  const double* PhiA4, *PhiT, *PhiS;  // [2 parity][nch][m cols][ldm] transposed Phi_c
+  const i64* GA4, *GT, *GS;           // G_jj: [M][2] blocks (psi: f_e, bf_e half), [M] blocks (T, S)
+  const i64* PhiA4, *PhiT, *PhiS;     // Phi_c: [2 parity][nch] x 4 blocks (row half, operand half) or 1
   double* dbuf;              // [shell][3][2][nch][ldd] chunk end states from a zero start
   double* cbuf;              // [shell][3][2][nch][ldd] carried states at the chunk starts (c >= 1)
   size_t d_stride;           // doubles per shell in dbuf / cbuf
   int* counter;              // [shell][6] chunks finished per chain (the last one runs the carry), zeroed
-  // layouts 3 / 11 (parallel carry): the chunks only write their end states; k_carry_par forms
+  // layouts 3 / 11 (parallel carry): the chunks only write their end states; k_carry_fx forms
   // part_{j,i} = P_{j,i} d_i for every product in parallel and the corrections sum
   // s_j = d_{j-1} + sum_i part_{j,i} (index order)
   int carry_seq;             // 1: the last-finishing chunk CTA runs the sequential carry (layouts 2 / 10)
   int np;                    // products per chain
-  const double* PA4, *PT, *PS;
+  const i64* PA4, *PT, *PS;
   double* pbuf;              // [shell][6][np][ldd] products P_{j,i} d_i
   size_t p_stride;           // doubles per shell in pbuf
   ChunkSet cset[2];          // the chunkings of layouts 2 and 3 (launch_chain copies one into the fields above)
@@ -355,8 +351,11 @@ size_t fx_rows_max_dynamic_smem(int prec);
 bool fx_split_rule(int split, int nr, int batch);
 cudaError_t launch_rhs(const RhsArgs& a, int batch, cudaStream_t s);
 cudaError_t launch_chain(const ChainArgs& a, int batch, int nfields, cudaStream_t s);
-// the chain layout (1, 2, 3 or 4) launch_chain runs for a.layout (0 = automatic) and this launch size
+// the chain layout launch_chain runs for a.layout (0 = automatic) and this launch size
 int resolve_chain_layout(const ChainArgs& a, int batch, int nfields);
+// fixed-point blocks from FP64 matrices on the device (setup)
+cudaError_t launch_to_fixed(const double* src, size_t src_stride, int ld, int nrows, int r0, int c0, int nr, int ldl,
+                            i64* out, size_t out_stride, int nblk, cudaStream_t s);
 cudaError_t launch_chunk_fix(const ChainArgs& a, int batch, int nfields, cudaStream_t s);
 cudaError_t launch_theta_op(int op, int M, int nr, int sym, const double* D2, const double* ir,
                             const double* dT0, const double* g, double* f, int batch,

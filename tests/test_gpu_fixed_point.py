@@ -67,3 +67,101 @@ def test_non_finite_rows_stay_in_their_pair(cuda):
     assert np.isnan(y[2]).all() and np.isnan(y[5]).all()
     for r in (0, 1, 6, 7):
         assert np.array_equal(y[r], good[r])
+
+
+# ---- block matvecs of the implicit solves ----------------------------------------------------------
+
+
+def _solve_ld(ops, G, field, sym):
+    """The oracle's chains (Matrix_Operators.py:1033-1194) in extended precision on the same FP64 blocks."""
+    M, nr, h = ops.N_fm, ops.nr, LD(ops.Pr * ops.dt if field == 0 else (ops.dt if field == 1 else ops.Tau * ops.dt))
+    F = np.zeros((M, nr), LD)
+    G = G.reshape(M, nr).astype(LD)
+    L = (ops.Linv_A4, ops.Linv_T, ops.Linv_S)[field].astype(LD)
+    D2, i4, i2 = ops.D2_A4.astype(LD), ops.IR4_A4.astype(LD), ops.IR2_A4.astype(LD)
+    for p in ((0 if field == 0 else 1,) if sym else (0, 1)):
+        fe, bf = np.zeros(nr, LD), np.zeros(nr, LD)
+        for jj in range(p, M, 2):
+            row = M - 1 - jj
+            if field == 0:
+                j = M - jj
+                bj, bt, g = -j * (j + 1), -2 * j, G[row]
+                if jj > p:
+                    fe = fe + F[row + 2]
+                    g = g + h * bt * (D2 @ fe + bj * i4 * fe + i4 * bf) - bt * i2 * fe
+                F[row] = L[jj] @ g
+                bf = bf + bj * F[row] + (bt * fe if jj > p else 0)
+            else:
+                if jj > p:
+                    fe = fe + 2 * h * (row + 2) * F[row + 2]
+                F[row] = L[jj] @ (G[row] - (LD(1) / 2 if row == 0 else 1) * fe)
+    return F.ravel()
+
+
+def _run(p, G, field, torch):
+    t = torch.from_numpy(np.ascontiguousarray(G)).cuda()
+    return (p.a4_bsub(t) if field == 0 else p.nab2_bsub(field, t)).cpu().numpy()
+
+
+@pytest.mark.parametrize("nr", [1, 7, 8, 9, 16, 17, 24, 25, 31, 32, 33, 47, 48, 49, 63, 64])
+def test_chains_are_no_less_exact_than_fp64(cuda, nr):
+    """Whole and chunked chains at the edges of the padded block sizes (8, 16, 24, 32, 48, 64) and of one and two
+    warps a group, against extended precision: at most twice the error of the same chains in FP64 (numpy; two
+    samples of rounding noise) plus four roundings of the result.  Scaling the right-hand side by a power of
+    two scales every bit of the result: operands have no range of their own."""
+    from oracle import sdd_oracle as O
+    from spectraldoublediffusiveconvection_gb300.plan import Plan
+    M, dt = 24, 1e-3
+    ops = O.Operators(M, nr + 1, 2.0, dt, 1.0, 0.01)
+    p = Plan(M, nr + 1, 2.0, dt, 1.0, 0.01)
+    rng = np.random.default_rng(nr)
+    s = np.sin(np.pi * np.arange(1, nr + 1) / (nr + 1)) ** 2
+    G = (rng.standard_normal((M, nr)) * s * np.exp(-np.arange(M) / 6.0)[:, None]).ravel()
+    for field in range(3):
+        ref = _solve_ld(ops, G, field, False)
+        n = float(np.linalg.norm(ref.astype(float)))
+        if field == 0:
+            o = O.A4_BSub_TSTEP_V2(G, ops.Linv_A4, ops.D2_A4, ops.IR4_A4, ops.IR2_A4, M, nr, dt, False)
+        else:
+            o = O.NAB2_BSub_TSTEP_V2(G, ops.Linv_T if field == 1 else ops.Linv_S, M, nr, dt if field == 1 else 0.01 * dt,
+                                     False)
+        e64 = float(np.linalg.norm((o - ref).astype(float))) / n
+        for layout in (1, 2, 3):
+            p.set_chain_layout(layout)
+            y = _run(p, G, field, cuda)
+            assert float(np.linalg.norm((y - ref).astype(float))) / n <= 2 * e64 + 4 * 2.0 ** -53, (field, layout)
+            for k in (-300, 200):
+                assert np.array_equal(_run(p, np.ldexp(G, k), field, cuda), np.ldexp(y, k))
+
+
+@pytest.mark.parametrize("N_r", [20, 48])
+@pytest.mark.parametrize("layout", [1, 2, 3])
+def test_non_finite_operands_follow_fp64(cuda, N_r, layout):
+    """An infinity or a NaN in the right-hand side reaches the modes it reaches in FP64 (the modes below it of
+    its parity), with whole chains the same infinities; the others are untouched."""
+    from oracle import sdd_oracle as O
+    from spectraldoublediffusiveconvection_gb300.plan import Plan
+    M, nr, dt = 32, N_r - 1, 1e-3
+    ops = O.Operators(M, N_r, 2.0, dt, 1.0, 0.01)
+    p = Plan(M, N_r, 2.0, dt, 1.0, 0.01)
+    p.set_chain_layout(layout)
+    G = np.random.default_rng(1).standard_normal((M, nr))
+    for field in range(3):
+        clean = _run(p, G.ravel(), field, cuda).reshape(M, nr)
+        for bad in (np.nan, np.inf, -np.inf):
+            H = G.copy()
+            H[20, 5] = bad
+            with np.errstate(all="ignore"):
+                if field == 0:
+                    ref = O.A4_BSub_TSTEP_V2(H.ravel(), ops.Linv_A4, ops.D2_A4, ops.IR4_A4, ops.IR2_A4, M, nr, dt, False)
+                else:
+                    ref = O.NAB2_BSub_TSTEP_V2(H.ravel(), ops.Linv_T if field == 1 else ops.Linv_S, M, nr,
+                                               dt if field == 1 else 0.01 * dt, False)
+            ref = ref.reshape(M, nr)
+            y = _run(p, H.ravel(), field, cuda).reshape(M, nr)
+            touched = np.zeros(M, bool)
+            touched[20::-2] = True
+            assert np.array_equal(y[~touched], clean[~touched])
+            assert not np.isfinite(y[touched]).any()
+            if layout == 1:
+                assert np.array_equal(y[20], ref[20], equal_nan=True)
