@@ -135,6 +135,8 @@ struct sdd_plan {
   double *Dr, *D2r2, *ir4r2, *D2s, *ir2s, *rsq, *dT0, *gr;
   const i64 *LinvA4, *LinvT, *LinvS;   // fixed-point blocks (sdd_fixed.cuh), one per mode
   const i64* ABA4;                  // [A_j B_j] of the psi chain, two blocks per mode
+  const i64* fxDr;                  // Dr as a two-digit block
+  int* opwx[3];                     // D^2/r^2, A2_SINE's D2, Dr as three-digit blocks
   double *coefA4, *coefT, *coefS;   // per-step scalars of the chains
   // chunked chains: cs[0] the chunking of layout 2 (sequential carry), cs[1] of layout 3 (parallel
   // carry); leading dimensions; workspaces sized for the larger chunk and product counts
@@ -291,7 +293,26 @@ static int upload_fixed(sdd_plan* p, const i64** dst, const double* src, int nma
   *dst = out;
   return SDD_OK;
 }
-// Linv blocks (row-major on the host).
+// A radial operator (row-major on the host) as a three-digit block.
+static int upload_wide(sdd_plan* p, int** dst, const double* src, int nr, int ld) {
+  if (!src) return SDD_ERR_ARG;
+  if (!p->cap_stream) SDD_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
+  const size_t n = (size_t)nr * nr * sizeof(double);
+  double* tmp = nullptr;
+  int* out = nullptr;
+  cudaError_t e = cudaMalloc(&tmp, n);
+  if (e == cudaSuccess) e = cudaMalloc(&out, wx_block_ints(ld) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, src, n, cudaMemcpyHostToDevice, p->cap_stream);
+  if (e == cudaSuccess) e = launch_to_wide(tmp, nr, ld, out, p->cap_stream);
+  const cudaError_t ew = cudaStreamSynchronize(p->cap_stream);
+  if (e == cudaSuccess) e = ew;
+  cudaFree(tmp);
+  if (e != cudaSuccess) cudaFree(out);
+  SDD_CUDA(e);
+  *dst = out;
+  return SDD_OK;
+}
+// Linv blocks and Dr (row-major on the host).
 static int upload_linv(sdd_plan* p, const i64** dst, const double* src, int M, int nr, int ldl) {
   if (!src) return SDD_ERR_ARG;
   std::vector<double> h((size_t)M * nr * nr);
@@ -380,7 +401,8 @@ static void free_plan(sdd_plan* p) {
                  p->dbuf, p->cbuf, p->pbuf,
                  p->dg_ir, p->dg_tw, p->dg_wr, p->dg_nuw, p->dg_part, p->dg_out};
   for (double* x : d) cudaFree(x);
-  for (const i64* x : {p->LinvA4, p->LinvT, p->LinvS, p->ABA4}) cudaFree(const_cast<i64*>(x));
+  for (const i64* x : {p->LinvA4, p->LinvT, p->LinvS, p->ABA4, p->fxDr}) cudaFree(const_cast<i64*>(x));
+  for (int* x : p->opwx) cudaFree(x);
   for (ChunkSet& c : p->cs) free_chunk_set(c);
   cudaFree(p->Dr32); cudaFree(p->D2r232); cudaFree(p->ir4r232); cudaFree(p->D2s32);
   cudaFree(p->tcB); cudaFree(p->tc_err);
@@ -619,6 +641,10 @@ int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
       (st = upload(&p->ir2s, d->ir2_sine, nr)) || (st = upload(&p->rsq, d->rsq, nr)) || (st = upload(&p->dT0, d->dT0, nr)) ||
       (st = upload(&p->gr, d->gr, nr)) || (st = upload_linv(p, &p->LinvA4, d->Linv_A4, M, nr, p->ldl)) ||
       (st = upload_linv(p, &p->LinvT, d->Linv_T, M, nr, p->ldl)) ||
+      (st = upload_linv(p, &p->fxDr, d->Dr, 1, nr, p->ldl)) ||
+      (st = upload_wide(p, &p->opwx[0], d->D2_r2, nr, p->ldl)) ||
+      (st = upload_wide(p, &p->opwx[1], d->D2_sine, nr, p->ldl)) ||
+      (st = upload_wide(p, &p->opwx[2], d->Dr, nr, p->ldl)) ||
       (st = upload_linv(p, &p->LinvS, d->Linv_S, M, nr, p->ldl)) ||
       (st = upload32(&p->Dr32, d->Dr, nn)) || (st = upload32(&p->D2r232, d->D2_r2, nn)) ||
       (st = upload32(&p->ir4r232, d->ir4_r2, nr))) {
@@ -902,6 +928,8 @@ static FxArgs fx_args(const sdd_plan* p, int prec, const double* X, void* base, 
     a.ops.Dr = p->Dr; a.ops.D2r2 = p->D2r2; a.ops.ir4r2 = p->ir4r2;
     a.ops.w = p->fft->wfx; a.ops.e = p->fft->efx;
   }
+  a.ops.fxDr = p->fxDr;
+  for (int q = 0; q < 2; ++q) a.ops.wx[q] = p->opwx[q];
   a.X = X; a.x_stride = shell_elems(p);
   a.base = base; a.base_stride = sdd_plan_base_cache_elems(p);
   a.out4 = out4; a.out_stride = (size_t)4 * p->M * p->nr;
@@ -968,9 +996,9 @@ static int check_plan(sdd_plan* p, int batch) {
 // One application of Phi (the step map) or its Jacobian to X (or dv), into out.
 // mode 0: FX (nonlinear term of X); 1: DFX about the base in `base`; 2: linear only.
 // Same as apply_step with explicit strides (doubles between shells) of the input X, the output and sub.
-// With the split nonlinear term, the right-hand sides are not assembled by k_rhs: the grid kernel writes
-// their linear parts (FP64 in both precisions) and the chains' h kernel adds the nonlinear parts (same
-// roundings).
+// The right-hand sides are not assembled by k_rhs: the grid kernel (split nonlinear term) or k_rhs_lin writes
+// their linear parts (FP64 in both precisions) and the chains' h kernel adds the nonlinear parts (the roundings
+// of k_rhs).
 // ev (nullable): four events recorded around the nonlinear term, the rhs and the chains.
 // The pending correction of layouts 3 / 11 (chunk set 1) of a state X (and its FP32 copy x32, nullable),
 // for FixArgs.
@@ -1008,7 +1036,9 @@ static int apply_step_ld(sdd_plan* p, int batch, const double* Ra, const double*
     ra.q32 = p->q32;
     ra.Dr32 = p->Dr32;
   }
-  bool fuse = false;
+  bool fuse = false, split = false, rhs32 = false;
+  const double* d2psi = nullptr;
+  size_t d2_stride = 0;
   if (ev) SDD_CUDA(cudaEventRecord(ev[0], s));
   if (mode != 2) {
     FxArgs fa = fx_args(p, prec, X, base, p->out4);
@@ -1024,9 +1054,11 @@ static int apply_step_ld(sdd_plan* p, int batch, const double* Ra, const double*
     }
     if (prec == SDD_PREC_MIXED) fa.q32 = p->q32;
     const int fm = mode == 1 ? 1 : 0;
-    fuse = fx_uses_split(fa, batch, fm);
+    split = fx_uses_split(fa, batch, fm);
+    rhs32 = v32 && v32_rhs && mode == 1 && prec == SDD_PREC_MIXED && !split && p->g32 && ra.q32;
+    fuse = !rhs32;
     if (fix_in) {
-      if (!fuse || mode != 0) return SDD_ERR_ARG;   // only the split path's derivative kernel applies it
+      if (!fuse || mode != 0) return SDD_ERR_ARG;   // the derivative kernel applies it
       fa.fix = fix_args(p, X, x32_in);
     }
     if (fuse) {
@@ -1034,15 +1066,17 @@ static int apply_step_ld(sdd_plan* p, int batch, const double* Ra, const double*
       fa.rl = ra;
     }
     SDD_CUDA(launch_fx(fa, batch, fm, prec, s));
+    d2psi = reinterpret_cast<const double*>(fa.deriv) + (size_t)4 * p->M * p->nr * (prec == SDD_PREC_MIXED ? 4 : 8) / 8;
+    d2_stride = fa.deriv_stride * (prec == SDD_PREC_MIXED ? 4 : 8) / 8;
   }
   if (ev) SDD_CUDA(cudaEventRecord(ev[1], s));
-  const bool rhs32 = v32 && v32_rhs && mode == 1 && prec == SDD_PREC_MIXED && !fuse && p->g32 && ra.q32;
   if (rhs32) {
     ra.X32 = v32;
     ra.x32_stride = ldx;
     ra.rhs32 = p->g32;
     ra.D2s32 = p->D2s32;
   }
+  if (fuse && !split) SDD_CUDA(launch_rhs_lin(ra, d2psi, d2_stride, batch, s));   // (split: the grid kernel's)
   if (!fuse) SDD_CUDA(launch_rhs(ra, batch, s));
   if (ev) SDD_CUDA(cudaEventRecord(ev[2], s));
   ChainArgs ca = chain_args(p, p->rhs, out, sub);
@@ -1063,7 +1097,8 @@ static int apply_step_ld(sdd_plan* p, int batch, const double* Ra, const double*
     ca.lin = p->rhs;
     ca.out4 = p->out4;
     ca.out_stride = (size_t)4 * p->M * p->nr;
-    ca.Dr = p->Dr;
+    ca.split_fx = split;
+    ca.wxDr = p->opwx[2];
     ca.q32 = ra.q32;
     ca.Dr32 = ra.Dr32;
     ca.dt = p->dt;
@@ -1087,17 +1122,17 @@ static int apply_step(sdd_plan* p, int batch, const double* Ra, const double* Ra
 // so the rule is applied as if they were there.
 static ChainArgs step_chain_args(const sdd_plan* p, int batch) {
   ChainArgs ca = chain_args(p, nullptr, nullptr, nullptr);
-  ca.fuse_rhs = fx_split_rule(p->fx_split, p->nr, batch) ? 1 : 0;
+  ca.split_fx = fx_split_rule(p->fx_split, p->nr, batch) ? 1 : 0;
   return ca;
 }
 
 // Whether sdd_step's steps leave the chains' correction to the next step's nonlinear term: layout 3 or 11
-// (chunk set 1, parallel carries) with the split nonlinear term, non-linear steps.
+// (chunk set 1, parallel carries), non-linear steps.
 static bool step_defers_fix(sdd_plan* p, int batch, int linear) {
   if (linear || p->cs[1].nch < 2) return false;
   const ChainArgs ca = step_chain_args(p, batch);
   const int layout = resolve_chain_layout(ca, batch, 3);
-  return ca.fuse_rhs && (layout == 3 || layout == 11);
+  return layout == 3 || layout == 11;
 }
 
 // The correction left pending by the last step of a sequence, on the state X (and its FP32 copy).
@@ -1240,7 +1275,7 @@ int sdd_step(sdd_plan* p, int batch, const double* Ra, const double* Ras, const 
   // for the next step's nonlinear term (the caller's X_in has none)
   const double* cur = X_in;
   const float* cur32 = nullptr;
-  // layout 3 or 11 with the split nonlinear term: each step's chain correction is applied by the next step's
+  // layout 3 or 11: each step's chain correction is applied by the next step's
   // first kernel (one launch fewer per step); the last one runs on its own at the end
   const int dfix = step_defers_fix(p, batch, linear) ? 1 : 0;
   cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;

@@ -16,8 +16,8 @@
 // Arithmetic.  An FP64 warp instruction holds its SM sub-partition for 64 cycles on GB300, and a chain is one
 // dependent matvec after another, so with FP64 matvecs a chain step cost (columns per lane) x 64 cycles.  Every
 // block matvec here runs in 64-bit fixed point (sdd_fixed.cuh): blocks as digits scaled per row by its
-// 1-norm, the operand scaled by its largest entry to 57 bits, three IMAD.WIDE (6.4 cycles) a column instead of
-// 64.  The carried states (f_e, bf_e, b) stay FP64; h, the matvec and its parts are summed in fixed point and
+// 1-norm, the operand scaled by its largest entry to 57 bits, three IMAD.WIDE (13 to 15 cycles) a column instead
+// of 64.  The carried states (f_e, bf_e, b) stay FP64; h, the matvec and its parts are summed in fixed point and
 // rounded once.  Error of a matvec against extended precision: 1e-18 to 1e-17 of the result, FP64's 1.5e-16.
 // An operand with an infinity takes an FP64 path with the same blocks (fx_dot_slow); one with a NaN gives NaN.
 //
@@ -46,36 +46,6 @@
 
 namespace sdd {
 
-// g of mode `row` for the fused right-hand side, element n (see ChainArgs::fuse_rhs): the roundings of
-// k_rhs, psi: (-dt (Dr Q - R)) + lin, T: (-dt NT) + lin, S: (-dt NS) + lin.
-// Dr and the Q row may be given in shared memory (Drs: nr x nr row-major, Qs: nr); nullptr reads global.
-__device__ __forceinline__ double fused_g(const ChainArgs& a, int b, int field, int row, int n,
-                                         const double* Drs = nullptr, const double* Qs = nullptr) {
-  const int M = a.M, nr = a.nr;
-  const size_t N = (size_t)M * nr;
-  const double* o4 = a.out4 + (size_t)b * a.out_stride;
-  double nl;
-  if (field == 0) {
-    double dq = 0.0;
-    if (a.q32) {            // FP32 nonlinear term: Dr Q in FP32, the order of k_rhs
-      const float* qs = a.q32 + (size_t)b * M * nr + (size_t)row * nr;
-      const float* drn = a.Dr32 + (size_t)n * nr;
-      float d = 0.0f;
-      for (int c = 0; c < nr; ++c) d = fmaf(__ldg(drn + c), __ldg(qs + c), d);
-      dq = (double)d;
-    } else {
-      const double* qs = Qs ? Qs : o4 + (size_t)row * nr;
-      const double* drn = (Drs ? Drs : a.Dr) + (size_t)n * nr;
-      for (int c = 0; c < nr; ++c) dq = fma(drn[c], qs[c], dq);
-    }
-    nl = __dmul_rn(-a.dt, __dsub_rn(dq, o4[N + (size_t)row * nr + n]));
-  } else {
-    nl = __dmul_rn(-a.dt, o4[(size_t)(field + 1) * N + (size_t)row * nr + n]);
-  }
-  return __dadd_rn(nl, a.lin[(size_t)b * a.g_stride + (size_t)field * a.field_off + (size_t)row * nr + n]);
-}
-
-
 // Operand x of one row (ignored where !ok) published as digits for column exponent cx; returns the exponent of
 // the warp's rows.
 __device__ __forceinline__ int publish(double x, int cx, bool ok, int2* xs) {
@@ -94,7 +64,7 @@ __device__ __forceinline__ FxVal block_row(const i64* blk, int nr, int r, const 
 #pragma unroll
   for (int w = 0; w < W; ++w) worst = max(worst, em[w]);
   FxVal o;
-  if (W == 1) {
+  if constexpr (W == 1) {
     o.v = fx_dot<LD, LD>(A, xs);
     o.e = ea + em[0] - kFxMvExp;
   } else {
@@ -457,23 +427,35 @@ __device__ __forceinline__ double carried_state(const ChainArgs& a, int b, size_
 //   FIX = true:   f_jj += G_jj s_c(jj) for the modes of chunks c >= 1   (chunked chains' correction)
 constexpr int kMvShells = 4;
 
+// The right-hand side of FIX = false is a.g, or (fuse_rhs) formed here with the roundings of k_rhs:
+//   psi: (-dt (Dr Q - R)) + lin,  T: (-dt NT) + lin,  S: (-dt NS) + lin,
+// Dr Q in fixed point like the other matvecs, or (mixed plans' FP32 nonlinear term) in FP32.
 template <bool FIX, int LD>
 __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int batch, int group) {
   constexpr int NP = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
-  extern __shared__ __align__(16) double msm[];        // fused right-hand side: Dr (nr x nr)
+  extern __shared__ __align__(16) int msm[];           // fused right-hand side: Dr's block, or Dr^T in FP32
+  __shared__ int4 s_w[FIX ? 1 : 4][32 * NP];           // Q's digits
   __shared__ __align__(16) int2 s_x[4][32 * NP];
-  __shared__ double s_q[4][32 * NP];
+  __shared__ float s_q[4][32 * NP];
   __shared__ i64 s_pv[FIX ? 4 : 1][kMvShells][32];     // psi's first half of a correction, per shell
   __shared__ int s_pe[FIX ? 4 : 1][kMvShells][32];
   const int M = a.M, nr = a.nr;
   const int wid = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool stage_dr = !FIX && a.fuse_rhs && a.field0 == 0 && !a.q32;
-  if (stage_dr && blockIdx.x * 4 < M * NP) {           // (a CTA with a psi mode; uniform)
-    for (int e = threadIdx.x; e < nr * nr; e += blockDim.x) cp_async8(msm + e, a.Dr + e);
-    cp_async_commit();
-    cp_async_wait<0>();
+  const bool fuse = !FIX && a.fuse_rhs;
+  if (fuse && a.field0 == 0 && blockIdx.x * 4 < M * NP) {   // (a CTA with a psi mode; uniform)
+    if (a.q32) {
+      float* Dt = reinterpret_cast<float*>(msm);
+      for (int e = threadIdx.x; e < nr * nr; e += blockDim.x) {
+        const int n = e / nr, c = e - n * nr;
+        Dt[c * nr + n] = __ldg(a.Dr32 + e);
+      }
+    } else {
+      for (int e = threadIdx.x; e < (int)wx_block_ints(LD) / 4; e += blockDim.x) cp_async16(msm + 4 * e, a.wxDr + 4 * e);
+      cp_async_commit();
+      cp_async_wait<0>();
+    }
     __syncthreads();
   }
   if (wid >= nfields * M * NP) return;
@@ -481,7 +463,8 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
   const int fl = fm / M, jj = fm - fl * M;
   const int field = a.field0 + fl;
   const int row = M - 1 - jj;
-  const size_t foff = (size_t)field * a.field_off + (size_t)row * nr;
+  const size_t N = (size_t)M * nr, ro = (size_t)row * nr;
+  const size_t foff = (size_t)field * a.field_off + ro;
   const bool a4 = field == 0;
   const int rr = min(r, nr - 1);
   const int par = jj & 1;
@@ -505,24 +488,73 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
       const int u = b - b0;
       if (a.active && !a.active[b]) continue;
       double x[NP];
-      if (!FIX && a.fuse_rhs && a4 && !a.q32) {        // the Q row, for fused_g
-        const double* q4 = a.out4 + (size_t)b * a.out_stride + (size_t)row * nr;
-        for (int e = lane; e < nr; e += 32) s_q[wl][e] = q4[e];
-        __syncwarp();
-      }
 #pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        const int e = p * 32 + lane;
-        x[p] = 0.0;
-        if (e < nr) {
-          if (FIX)
+      for (int p = 0; p < NP; ++p) x[p] = 0.0;
+      if (FIX) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const int e = p * 32 + lane;
+          if (e < nr)
             x[p] = a.carry_seq ? a.cbuf[(size_t)b * a.d_stride + (chain * a.nch + c) * a.ldd + sg * nr + e]
                                : carried_state(a, b, chain, c, sg * nr + e);
-          else if (a.fuse_rhs)
-            x[p] = fused_g(a, b, field, row, e, stage_dr ? msm : nullptr, stage_dr ? s_q[wl] : nullptr);
-          else
-            x[p] = a.g[(size_t)b * a.g_stride + foff + e];
         }
+      } else if (!fuse) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          if (p * 32 + lane < nr) x[p] = a.g[(size_t)b * a.g_stride + foff + p * 32 + lane];
+      } else {
+        const double* o4 = a.out4 + (size_t)b * a.out_stride + ro;
+        const double* lin = a.lin + (size_t)b * a.g_stride + foff;
+        double nl[NP], ln[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const int e = p * 32 + lane;
+          nl[p] = e < nr ? o4[(size_t)(field + 1) * N + e] : 0.0;   // psi: R
+          ln[p] = e < nr ? lin[e] : 0.0;
+        }
+        if (a4) {
+          double dq[NP];
+          if (a.q32) {
+            const float* qs = a.q32 + (size_t)b * N + ro;
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+              if (p * 32 + lane < nr) s_q[wl][p * 32 + lane] = __ldg(qs + p * 32 + lane);
+            __syncwarp();
+            const float* Dt = reinterpret_cast<const float*>(msm);
+            float d[NP];
+#pragma unroll
+            for (int p = 0; p < NP; ++p) d[p] = 0.0f;
+            for (int cc = 0; cc < nr; ++cc) {
+              const float qv = s_q[wl][cc];
+#pragma unroll
+              for (int p = 0; p < NP; ++p) d[p] = fmaf(Dt[cc * nr + min(p * 32 + lane, nr - 1)], qv, d[p]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int p = 0; p < NP; ++p) dq[p] = (double)d[p];
+          } else {
+            double q[NP];
+            int cx[NP];
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+              const int e = p * 32 + lane;
+              q[p] = e < nr ? o4[e] : 0.0;
+              cx[p] = e < nr ? msm[3 * LD * LD + LD + e] : 0;
+            }
+            const int em = publish_wide<NP>(q, cx, nr, lane, s_w[wl]);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+              const int e = min(p * 32 + lane, nr - 1);
+              dq[p] = fx_val(wx_dot<LD>(msm, nr, e, s_w[wl], em));
+            }
+            __syncwarp();                              // the digits are read before the next shell's replace them
+          }
+#pragma unroll
+          for (int p = 0; p < NP; ++p) nl[p] = __dsub_rn(dq[p], nl[p]);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          if (p * 32 + lane < nr) x[p] = __dadd_rn(__dmul_rn(-a.dt, nl[p]), ln[p]);
       }
       const int em = publish_regs<NP>(x, m.cx, nr, lane, xs);
       const FxVal p = m.times(B, nr, rr, xs, em);
@@ -538,7 +570,7 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
           if (a.f32) a.f32[(size_t)b * a.f32_stride + foff + r] = (float)v;
         }
       } else if (r < nr) {
-        a.h[(size_t)b * a.h_stride + foff + r] = fx_sum(0.0, p);
+        a.h[(size_t)b * a.h_stride + foff + r] = fx_val(p);
       }
     }
   }
@@ -631,9 +663,15 @@ static cudaError_t launch_mode_mv(const ChainArgs& a, int batch, int nfields, cu
   int group = 1;
   while (group < kMvShells && warps * batch / (2 * group) >= 32l * sm_count()) group *= 2;
   const dim3 grid((unsigned)((warps + 3) / 4), (batch + group - 1) / group);
-  const size_t smem = !FIX && a.fuse_rhs && a.field0 == 0 && !a.q32 ? (size_t)a.nr * a.nr * sizeof(double) : 0;
+  const size_t smem = FIX || !a.fuse_rhs || a.field0 != 0 ? 0
+                      : a.q32                            ? (size_t)a.nr * a.nr * sizeof(float)
+                                                         : wx_block_ints(a.ldl) * sizeof(int);
   const cudaError_t e = with_ld(a.ldl, [&](auto ld) {
-    return launch_kernel(k_mode_mv<FIX, decltype(ld)::value>, grid, dim3(128), smem, s, a, nfields, batch, group);
+    constexpr int LD = decltype(ld)::value;
+    static unsigned long long done = 0;
+    const cudaError_t er = smem > 40 * 1024 ? ensure_smem_attr(k_mode_mv<FIX, LD>, &done) : cudaSuccess;
+    if (er != cudaSuccess) return er;
+    return launch_kernel(k_mode_mv<FIX, LD>, grid, dim3(128), smem, s, a, nfields, batch, group);
   });
   ktimer_mark(FIX ? SDD_K_MODE_FIX : SDD_K_MODE_H, s);
   return e;
@@ -718,7 +756,7 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   const ChunkSet& c2 = a.cset[0];
   const ChunkSet& c3 = a.cset[1];
   // layout 8 needs all three fields of a step with full right-hand sides, and its three rings in one CTA
-  if (layout == 8 && (nfields != 3 || a.field0 != 0 || a.fuse_rhs || a.g32 ||
+  if (layout == 8 && (nfields != 3 || a.field0 != 0 || a.split_fx || a.g32 ||
                       layout_bytes(8, a.M, a.nr, a.ldl) > (size_t)optin))
     layout = 6;
   // layout 9 needs all three fields and its three rings in one CTA
@@ -729,9 +767,9 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   if (layout == 0 && c3.nch > 1 && c3.GA4 && 2 * nfields * batch * c3.nch <= 2 * sms) layout = 3;
   if (layout == 0 && c2.nch > 1 && c2.GA4 && 2 * nfields * batch * c2.nch <= 2 * sms) layout = 2;
   // chosen chunks run in the reference's order where the full FP64 right-hand side is there (no pre-pass)
-  if (a.layout == 0 && (layout == 2 || layout == 3) && !a.fuse_rhs && !a.g32) layout += 8;
+  if (a.layout == 0 && (layout == 2 || layout == 3) && !a.split_fx && !a.g32) layout += 8;
   // layouts 6 / 7 need the full right-hand side in FP64: with the fused or the FP32 one, the pre-pass form
-  if ((layout == 6 || layout == 7) && (a.fuse_rhs || a.g32)) layout = 5;
+  if ((layout == 6 || layout == 7) && (a.split_fx || a.g32)) layout = 5;
   if ((layout == 6 || layout == 7) && layout_bytes(6, a.M, a.nr, a.ldl) > (size_t)optin) layout = 2;
   if (layout != 2 && layout != 3 && layout < 6 && layout_bytes(4, a.M, a.nr, a.ldl) > (size_t)optin)
     layout = 2;   // whole chain too long for shared memory
@@ -739,7 +777,7 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   // step's three chains per CTA where they fit (64 shells N_r=30 N_theta=256: 287 us against 301 us)
   if (layout == 0) {
     if (2 * nfields * batch <= sms) layout = 4;
-    else if (a.fuse_rhs || a.g32) layout = 5;
+    else if (a.split_fx || a.g32) layout = 5;
     else if (nfields == 3 && a.field0 == 0 && layout_bytes(8, a.M, a.nr, a.ldl) <= (size_t)optin) layout = 8;
     else layout = 6;
   }
@@ -806,6 +844,44 @@ __global__ void __launch_bounds__(64) k_to_fixed(const double* src, size_t src_s
     }
     rexp[r] = ea;
   }
+}
+
+// A radial operator (row-major nr x nr on the device) as a three-digit block; one thread per column, then row.
+__global__ void __launch_bounds__(64) k_to_wide(const double* src, int nr, int ld, int* out) {
+  __shared__ int cx[kMaxNr];
+  int* rexp = out + 3 * ld * ld;
+  for (int c = threadIdx.x; c < ld; c += blockDim.x) {
+    unsigned m = 0;
+    if (c < nr)
+      for (int r = 0; r < nr; ++r) m = max(m, abs_hi(src[r * nr + c]));
+    const int e = m >> 20 && m < 0x7ff00000u ? (int)(m >> 20) - 1022 : 0;
+    cx[c] = e;
+    rexp[ld + c] = e;
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < ld; r += blockDim.x) {
+    double l1 = 0.0;
+    if (r < nr)
+      for (int c = 0; c < nr; ++c) l1 += fabs(ldexp(src[r * nr + c], -cx[c]));
+    const unsigned h = abs_hi(l1 * (1.0 + 1e-13)) >> 20;
+    const int ea = h == 0x7ff ? kFxBad : (int)h - 1022;
+    for (int c = 0; c < ld; ++c) {
+      int d2 = 0, d1 = 0, d0 = 0;
+      if (r < nr && c < nr && ea != kFxBad) {
+        const double x = src[r * nr + c];
+        wx_split(x, 1022 + cx[c] + ea - (int)(abs_hi(x) >> 20), d2, d1, d0);
+      }
+      out[c * ld + r] = d2;
+      out[(ld + c) * ld + r] = d1;
+      out[(2 * ld + c) * ld + r] = d0;
+    }
+    rexp[r] = ea;
+  }
+}
+
+cudaError_t launch_to_wide(const double* src, int nr, int ld, int* out, cudaStream_t s) {
+  k_to_wide<<<1, 64, 0, s>>>(src, nr, ld, out);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_to_fixed(const double* src, size_t src_stride, int ld, int nrows, int r0, int c0, int nr, int ldl,

@@ -60,12 +60,14 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
   double* Br = Ar + M;        // sine row: (Dr psi)_{k-1}(r_n), [0] = 0
   double* scl = Br + M;       // the two rows' exponents
   unsigned* red = reinterpret_cast<unsigned*>(scl + 8);
+#pragma unroll 1
   for (int i = tid; i < L; i += bd) {
     Wt[i] = a.w[i];
     Et[i] = a.e[i];
   }
   const double* ps = a.X + (size_t)b * a.x_stride;
   const double* drn = a.Dr + (size_t)n * nr;
+#pragma unroll 1
   for (int k = tid; k < M; k += bd) {
     const double* pk = ps + (size_t)k * nr;
     double acc = 0.0;
@@ -77,6 +79,7 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
   parity_suffix<double>(pv, Sc, M);   // as J_theta_RT
   __syncthreads();
   const double irn = a.ir[n];
+#pragma unroll 1
   for (int k = tid; k < M; k += bd) {
     const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;
     double jp = (k == 0) ? 1.0 * s1 : (k + 1.0) * pv[k - 1] + 2.0 * s1;
@@ -87,29 +90,29 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
   __syncthreads();
   // DCT3 inputs with n_in = M on length L (see k_transform): cosine x_k = A_k; sine x_k = B_{L-k}
   double* XV = reinterpret_cast<double*>(RB);
-  unsigned mx[2] = {0, 0};
+#pragma unroll 1
   for (int k = tid; k < L; k += bd) {
     const double xa = (k < M) ? Ar[k] : 0.0;
     const double xb = (L - k <= M - 1 && k > 0) ? Br[L - k] : 0.0;
     XV[k] = xa;
     XV[L + k] = xb;
-    mx[0] = max(mx[0], abs_hi(xa));
-    mx[1] = max(mx[1], abs_hi(xb));
   }
   int* E = reinterpret_cast<int*>(scl);
-  rows_to_fixed<2>(XV, L, 2, mx, red, E);
+  rows_to_fixed(XV, L, 2, red, E);
   const i64* XA = reinterpret_cast<const i64*>(XV);
   const i64* XB = XA + L;
+#pragma unroll 1
   for (int k = tid; k < L; k += bd)
-    RA[k] = k == 0 ? make_longlong2(XA[0], XB[0]) : dct3_pack_fx(Et[k], XA[k], XA[L - k], XB[k], XB[L - k]);
+    RA[k] = k == 0 ? make_longlong2(XB[0], XA[0]) : dct3_pack_fx(Et[k], XA[k], XA[L - k], XB[k], XB[L - k]);
   __syncthreads();
-  C* res = fft_rows<double, true>(RA, RB, 1, a.st, Wt);
+  C* res = fft_rows<double, false>(RA, RB, 1, a.st, Wt);
   const bool bad = E[0] == kFxBad || E[1] == kFxBad;
   double s[1] = {0.0};
+#pragma unroll 1
   for (int i = tid; i < L; i += bd) {
     const int src = (i & 1) ? (L - 1 - (i >> 1)) : (i >> 1);
     const C v = res[src];
-    const double ja = bad ? fx_nan() : fx2d(v.x, 60 - E[0]), db = fx2d(v.y, 60 - E[1]);   // (db's sign drops out)
+    const double ja = bad ? fx_nan() : fx2d(v.y, 60 - E[0]), db = fx2d(v.x, 60 - E[1]);   // (db's sign drops out)
     s[0] = fma(a.tw[i], fma(ja, ja, db * db), s[0]);
   }
   __syncthreads();                      // (the scales are read before the sums reuse the reduction words)

@@ -18,9 +18,8 @@
 // the host.
 //
 // FP32 transforms run in FP32.  FP64 transforms run in 64-bit fixed point on the integer pipe (sdd_fixed.cuh):
-// each row scaled by a power of two above its 1-norm, which bounds every value inside its transform, with 60
-// bits below it; one radix-4 butterfly (3 complex products, 8 complex additions) is 36 IMAD.WIDE (2.1 cycles
-// each) and 16 64-bit additions where it was 28 FP64 instructions of 64 cycles.  N_r=30, N_theta=256: grid kernel
+// each row scaled by a power of two above its 1-norm, which bounds every value inside its transform, 36 wide multiply-adds (4.5 to 5
+// cycles each)  N_r=30, N_theta=256: grid kernel
 // 18.9 -> 14.6 us, product kernel 14.4 -> 10.2 us, row kernel of 64 shells 712 -> 492 us.
 #pragma once
 #include <cuda_runtime.h>
@@ -154,31 +153,79 @@ __device__ __forceinline__ void fft_pass_r(const typename Cplx<T>::type* __restr
   }
 }
 
-template <typename T, bool INV>
-__device__ __forceinline__ void fft_pass(const typename Cplx<T>::type* __restrict__ in,
-                                         typename Cplx<T>::type* __restrict__ out, int L, int nf, int R, int Ns,
-                                         const typename Cplx<T>::tw* w, FastDiv fnb, FastDiv fns, int tws) {
-  switch (R) {
-    case 4: fft_pass_r<T, INV, 4>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
-    case 2: fft_pass_r<T, INV, 2>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
-    case 3: fft_pass_r<T, INV, 3>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
-    case 5: fft_pass_r<T, INV, 5>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
-    default: fft_pass_r<T, INV, 7>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
+// The same pass in fixed point, out of line: the buffers and the table by their byte offsets in the block's
+// dynamic shared memory (a generic pointer would cost the shared-memory loads).  Kept small: the row kernel
+// once had 200 KB of inlined and unrolled code, and its warps waited for instructions more than for anything
+// else.
+template <int R>
+static __device__ __noinline__ void fft_pass_fx(int in, int out, int w, int L, int nf, int Ns, FastDiv fnb, FastDiv fns,
+                                                int tws) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const longlong2* I = reinterpret_cast<const longlong2*>(smem_raw + in);
+  longlong2* O = reinterpret_cast<longlong2*>(smem_raw + out);
+  const int4* W = reinterpret_cast<const int4*>(smem_raw + w);
+  const int nb = L / R;
+  const int total = nf * nb;
+#pragma unroll 1
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    const int f = (int)fast_div((unsigned)t, fnb);
+    const int j = t - f * nb;
+    const int jq = (int)fast_div((unsigned)j, fns);
+    const int k = j - jq * Ns;
+    longlong2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = I[f * L + j + r * nb];
+    if (Ns > 1) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = fx_cmul<false>(v[r], W[k * r * tws]);
+    }
+    butterfly<double, false, R>(v, W, L);
+    const int d = f * L + jq * Ns * R + k;
+#pragma unroll
+    for (int r = 0; r < R; ++r) O[d + r * Ns] = v[r];
+  }
+}
+
+template <typename T, bool INV, bool OUTLINE>
+__device__ __forceinline__ void fft_pass(typename Cplx<T>::type* in, typename Cplx<T>::type* out, int L, int nf, int R,
+                                         int Ns, const typename Cplx<T>::tw* w, FastDiv fnb, FastDiv fns, int tws) {
+  if constexpr (sizeof(T) == 8 && OUTLINE) {
+    static_assert(!INV, "FP64 inverse transforms are forward ones of swapped pairs (dct3_pack_fx)");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto off = [&](const void* p) { return (int)(reinterpret_cast<const unsigned char*>(p) - smem_raw); };
+    const int i = off(in), o = off(out), wo = off(w);
+    switch (R) {
+      case 4: fft_pass_fx<4>(i, o, wo, L, nf, Ns, fnb, fns, tws); break;
+      case 2: fft_pass_fx<2>(i, o, wo, L, nf, Ns, fnb, fns, tws); break;
+      case 3: fft_pass_fx<3>(i, o, wo, L, nf, Ns, fnb, fns, tws); break;
+      case 5: fft_pass_fx<5>(i, o, wo, L, nf, Ns, fnb, fns, tws); break;
+      default: fft_pass_fx<7>(i, o, wo, L, nf, Ns, fnb, fns, tws); break;
+    }
+  } else {
+    switch (R) {
+      case 4: fft_pass_r<T, INV, 4>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
+      case 2: fft_pass_r<T, INV, 2>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
+      case 3: fft_pass_r<T, INV, 3>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
+      case 5: fft_pass_r<T, INV, 5>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
+      default: fft_pass_r<T, INV, 7>(in, out, L, nf, Ns, w, fnb, fns, tws); break;
+    }
   }
 }
 
 // Full FFT of nf rows in buffer a (b is scratch of the same size).  Returns the buffer holding the
-// result.  Must be called by all threads of the block; ends with a __syncthreads().
-template <typename T, bool INV>
+// result.  OUTLINE: FP64 passes out of line, for kernels with many rows per CTA and more than one transform; the
+// split path's one-transform kernels inline them (10.2 against 12.2 us for the product kernel).  Must be called by all threads of the block; ends with a __syncthreads().
+template <typename T, bool INV, bool OUTLINE = true>
 __device__ typename Cplx<T>::type* fft_rows(typename Cplx<T>::type* a, typename Cplx<T>::type* b, int nf,
                                             const StageArgs& st, const typename Cplx<T>::tw* w) {
   using C = typename Cplx<T>::type;
   C* in = a;
   C* out = b;
   int Ns = 1;
+#pragma unroll 1
   for (int s = 0; s < st.nst; ++s) {
     const int R = st.rad[s];
-    fft_pass<T, INV>(in, out, st.L, nf, R, Ns, w, st.nb[s], st.ns[s], st.tws[s]);
+    fft_pass<T, INV, OUTLINE>(in, out, st.L, nf, R, Ns, w, st.nb[s], st.ns[s], st.tws[s]);
     __syncthreads();
     Ns *= R;
     C* tmp = in; in = out; out = tmp;
@@ -192,7 +239,8 @@ __device__ __forceinline__ longlong2 dct3_pack_fx(int4 e, i64 xa, i64 xar, i64 x
   longlong2 z;
   z.x = xa + xbr;
   z.y = xb - xar;
-  return fx_cmul<false>(z, e);
+  z = fx_cmul<false>(z, e);
+  return make_longlong2(z.y, z.x);                     // swapped: the inverse transform is a forward one
 }
 // y_A, y_B of a DCT2 pair in fixed point from Z_k, Z_{-k} and e_k = 0.5 (cos, sin)(pi k/2P).
 __device__ __forceinline__ void dct2_unpack_fx(longlong2 Zk, longlong2 Zm, int4 e, i64& ya, i64& yb) {

@@ -1,7 +1,7 @@
 // FP64 data in 64-bit fixed point on the integer pipe.
 //
 // GB300 issues one FP64 warp instruction per SM sub-partition every 64 cycles (measured: DFMA 64.1, DADD 64-76),
-// a 32 x 32 + 64-bit integer multiply-add (IMAD.WIDE) every 2.1, a 64-bit add every 2-3.  The transforms and
+// a 32 x 32 + 64-bit integer multiply-add every 4.5 to 5, a 64-bit add every 2.2.  The transforms and
 // the block matvecs of the implicit solves are sums of products with known operators over a row or a vector
 // whose largest entry is easy to find, so they run on integers: a vector is scaled by one power of two to a
 // 64-bit integer each, an operator by one per row and one per column, both are split into two signed digits
@@ -67,6 +67,13 @@ __device__ __forceinline__ double fx2d_lat(i64 v, int s) {
   return e >= 2047 ? __longlong_as_double((v < 0 ? 0xfff0000000000000ll : 0x7ff0000000000000ll)) : r;
 }
 
+// n < 2^31 as a double by its bits (the conversion takes the FP64 pipe)
+__device__ __forceinline__ double fx_int(unsigned n) {
+  if (n == 0) return 0.0;
+  const int lz = __clz((int)n);
+  return __longlong_as_double((i64)(((u64)(1054 - lz) << 52) + (((u64)(n << lz) << 21) & 0xfffffffffffffull)));
+}
+
 __device__ __forceinline__ double fx_nan() { return __longlong_as_double(0x7ff8000000000000ll); }
 
 // |x|'s high word: its unsigned order is the order of magnitudes (to 20 mantissa bits)
@@ -100,53 +107,64 @@ __device__ __forceinline__ i64 fx_rmul(i64 x, int h1, int h0) {
   return (((i64)x1 * h1) << 2) + (fx_mad(x1, h0, fx_mad(x0, h1, 1ll << 29)) >> 30);
 }
 
-// Scales of K rows by their 1-norms and their conversion in place.  Row t holds P doubles at XV + t P; mx[t]
-// is the calling thread's maximum of abs_hi over its elements k = tid, tid + blockDim, ... (only those were
-// written by it: no barrier is needed before the call).  Afterwards the row holds round(x 2^(60 - E[t])) as
-// 64-bit integers with sum |x| < 2^E[t]: the row's transform and everything inside it stays below 2^61 (two
-// rows of a pair).  E[t] = kFxBad marks a row with an infinity or NaN (left as zeros).  red: 2 K 32 words.
-// Ends with a barrier.
+// Scales of rows by their 1-norms and their conversion in place.  Row t holds P doubles at XV + t P, of which the
+// calling thread wrote the elements k = tid, tid + blockDim, ... (no barrier is needed before the call).
+// Afterwards the row holds round(x 2^(60 - E[t])) as 64-bit integers with sum |x| < 2^E[t]: the row's transform
+// and everything inside it stays below 2^61 (two rows of a pair).  E[t] = kFxBad marks a row with an infinity
+// or NaN (left as zeros); E of the row after an odd last one is a zero row's.  red: 2 nrows 32 words.  Ends with
+// a barrier.
 constexpr int kFxBad = 0x7fffffff;
-template <int K>
-__device__ __forceinline__ void rows_to_fixed(double* XV, int P, int nrows, const unsigned (&mx)[K], unsigned* red,
-                                              int* E) {
+// (Out of line, with byte offsets into the dynamic shared memory, like the transforms' passes.)
+static __device__ __noinline__ void rows_to_fixed_at(int xv, int P, int nrows, int redo, int eo) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* XV = reinterpret_cast<double*>(smem_raw + xv);
+  unsigned* red = reinterpret_cast<unsigned*>(smem_raw + redo);
+  int* E = reinterpret_cast<int*>(smem_raw + eo);
   const int tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = bd >> 5;
-#pragma unroll
-  for (int t = 0; t < K; ++t) {
-    if (t < nrows) {
-      const int ew = (int)(__reduce_max_sync(0xffffffffu, mx[t]) >> 20);
-      unsigned s = 0;
-      for (int k = tid; k < P; k += bd) {
-        const unsigned h = abs_hi(XV[t * P + k]);
-        const int e = (int)(h >> 20);
-        if (e) s += (((h & 0xfffffu) | 0x100000u) >> min(ew - e, 31)) + 1;
-      }
-      s = __reduce_add_sync(0xffffffffu, s);
-      if (lane == 0) {
-        red[t * 32 + warp] = (unsigned)ew;
-        red[(K + t) * 32 + warp] = s;
-      }
+#pragma unroll 1
+  for (int t = 0; t < nrows; ++t) {
+    const double* x = XV + t * P;
+    unsigned m = 0, s = 0;
+#pragma unroll 1
+    for (int k = tid; k < P; k += bd) m = max(m, abs_hi(x[k]));
+    const int ew = (int)(__reduce_max_sync(0xffffffffu, m) >> 20);
+#pragma unroll 1
+    for (int k = tid; k < P; k += bd) {
+      const unsigned h = abs_hi(x[k]);
+      const int e = (int)(h >> 20);
+      if (e) s += (((h & 0xfffffu) | 0x100000u) >> min(ew - e, 31)) + 1;
+    }
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) {
+      red[t * 32 + warp] = (unsigned)ew;
+      red[(nrows + t) * 32 + warp] = s;
     }
   }
   __syncthreads();
-  for (int t = warp; t < K; t += nw) {                 // (a row that is not there gets a zero row's scale)
+#pragma unroll 1
+  for (int t = warp; t < ((nrows + 1) & ~1); t += nw) {
     const bool on = t < nrows && lane < nw;
     const unsigned e = on ? red[t * 32 + lane] : 0u;
-    const unsigned s = on ? red[(K + t) * 32 + lane] : 0u;
+    const unsigned s = on ? red[(nrows + t) * 32 + lane] : 0u;
     const unsigned em = __reduce_max_sync(0xffffffffu, e);
     const unsigned tot = __reduce_add_sync(0xffffffffu, s ? ((s >> 3) >> min(em - e, 31u)) + 1 : 0u);
     if (lane == 0) E[t] = em >= 0x7ffu ? kFxBad : (int)em - 1040 + (32 - __clz((int)tot));
   }
   __syncthreads();
-#pragma unroll
-  for (int t = 0; t < K; ++t) {
-    if (t < nrows) {
-      const int et = E[t];
-      for (int k = tid; k < P; k += bd)
-        reinterpret_cast<i64*>(XV)[t * P + k] = et == kFxBad ? 0 : d2fx(XV[t * P + k], 1024 + et);
-    }
+#pragma unroll 1
+  for (int t = 0; t < nrows; ++t) {
+    const int et = E[t];
+#pragma unroll 1
+    for (int k = tid; k < P; k += bd)
+      reinterpret_cast<i64*>(XV)[t * P + k] = et == kFxBad ? 0 : d2fx(XV[t * P + k], 1024 + et);
   }
   __syncthreads();
+}
+
+__device__ __forceinline__ void rows_to_fixed(double* XV, int P, int nrows, void* red, int* E) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto off = [&](const void* p) { return (int)(reinterpret_cast<const unsigned char*>(p) - smem_raw); };
+  rows_to_fixed_at(off(XV), P, nrows, off(red), off(E));
 }
 
 // ---- block matvecs -------------------------------------------------------------------------------
@@ -267,26 +285,42 @@ __device__ __forceinline__ int publish_regs(const double (&x)[NP], const int (&c
   __syncwarp();
   return em;
 }
-// A lane's row of a block in registers (its loads all in flight at once), and its product with a published
-// operand: the arithmetic of fx_dot.  LD <= 32 NP.
-template <int LD, int NP>
+// Row r of a block in shared memory times an operand of one exponent.
+template <int LD>
+__device__ __forceinline__ FxVal block_vec(const i64* blk, int nr, int r, const int2* xs, int em) {
+  const int ea = fx_row_exp(blk, LD)[r];
+  FxVal p;
+  p.v = fx_dot<LD, LD>(reinterpret_cast<const int2*>(blk) + r, xs);
+  p.e = ea + em - kFxMvExp;
+  if (em >= kFxInf || ea == kFxBad) {
+    p.v = __double_as_longlong(em == kFxInf ? fx_dot_slow(blk, LD, r, xs, 0, nr, em) : fx_nan());
+    p.e = kFxBad;
+  }
+  return p;
+}
+
+// Columns [c0, c0 + NC) of a lane's row of a block in registers (its loads all in flight at once), and their
+// product with a published operand: the arithmetic of fx_dot.  LD <= 32 NP; sums of ranges add up to a row's.
+struct FxPart {
+  i64 t2, t1;                // the product is t2 2 + (t1 + 2^25 >> 26)
+};
+template <int LD, int NP, int NC = LD>
 struct FxRow {
-  int2 m[LD];
+  int2 m[NC];
   int ea, cx[NP];            // the row's exponent; the column exponents of the lane's operand elements
-  __device__ __forceinline__ void load(const i64* blk, int r) {
+  __device__ __forceinline__ void load(const i64* blk, int r, int c0 = 0) {
     const int2* A = reinterpret_cast<const int2*>(blk) + r;
 #pragma unroll
-    for (int c = 0; c < LD; ++c) m[c] = __ldg(A + c * LD);
+    for (int c = 0; c < NC; ++c) m[c] = __ldg(A + (c0 + c) * LD);
     ea = __ldg(fx_row_exp(blk, LD) + r);
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int p = 0; p < NP; ++p) cx[p] = 32 * p + lane < LD ? __ldg(fx_col_exp(blk, LD) + 32 * p + lane) : 0;
   }
-  __device__ __forceinline__ FxVal times(const i64* blk, int nr, int r, const int2* xs, int em) const {
-    FxVal p;
-    i64 t2 = 0, t1 = 1ll << 25, t0 = 0;
+  __device__ __forceinline__ FxPart part(const int2* xs) const {   // xs: from column c0 (even)
+    i64 t2 = 0, t1 = 0, t0 = 0;
 #pragma unroll
-    for (int c = 0; c < LD; c += 2) {
+    for (int c = 0; c < NC; c += 2) {
       const int4 v = reinterpret_cast<const int4*>(xs)[c >> 1];
       t2 = fx_mad(m[c].y, v.y, t2);
       t1 = fx_mad(m[c].y, v.x, t1);
@@ -295,7 +329,11 @@ struct FxRow {
       t1 = fx_mad(m[c + 1].y, v.z, t1);
       t0 = fx_mad(m[c + 1].x, v.w, t0);
     }
-    p.v = (t2 << 1) + ((t1 + t0) >> 26);
+    return {t2, t1 + t0};
+  }
+  __device__ __forceinline__ FxVal value(FxPart t, const i64* blk, int nr, int r, const int2* xs, int em) const {
+    FxVal p;
+    p.v = (t.t2 << 1) + ((t.t1 + (1ll << 25)) >> 26);
     p.e = ea + em - kFxMvExp;
     if (em >= kFxInf || ea == kFxBad) {                // (after the registers of the row are done with)
       p.v = __double_as_longlong(em == kFxInf ? fx_dot_slow(blk, LD, r, xs, 0, nr, em) : fx_nan());
@@ -303,7 +341,106 @@ struct FxRow {
     }
     return p;
   }
+  __device__ __forceinline__ FxVal times(const i64* blk, int nr, int r, const int2* xs, int em) const {
+    return value(part(xs), blk, nr, r, xs, em);
+  }
 };
+
+// ---- second derivatives --------------------------------------------------------------------------
+// The second-derivative matrices take three digits of 27 bits (80 bits; sign and magnitude) on both sides: applied
+// to a state that is not smooth at the walls their products' range within one row is N^4, of which the implicit
+// solves then keep the small end, so two digits would lose what FP64 keeps (psi of a step at N_r = 65 and dt = 1:
+// 1e-11 instead of 3e-13).  Six IMAD.WIDE a column: the digit products down to 2^-80 of the largest product.
+// A block: planes of the high, middle and low digits ([col][row], L x L ints each), then the rows' and the
+// columns' exponents (as in the two-digit blocks).
+__host__ __device__ constexpr size_t wx_block_ints(int ld) { return (size_t)(3 * ld + 2) * ld; }
+
+// The digits of m 2^27 >> sh (m the 53-bit significand of x), with x's sign; x = 0 (or subnormal) gives 0.
+__device__ __forceinline__ void wx_split(double x, int sh, int& d2, int& d1, int& d0) {
+  const unsigned hi = (unsigned)__double2hiint(x), mask = 0x7ffffffu;
+  const u64 m = ((hi >> 20) & 0x7ffu) ? ((u64)((hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x) : 0;
+  const unsigned a2 = (unsigned)(m >> min(27 + sh, 63)), a1 = (unsigned)(m >> min(sh, 63)) & mask;
+  const unsigned a0 = (unsigned)(sh <= 27 ? m << (27 - sh) : m >> min(sh - 27, 63)) & mask;
+  const int s = (int)hi >> 31;
+  d2 = ((int)a2 ^ s) - s;
+  d1 = ((int)a1 ^ s) - s;
+  d0 = ((int)a0 ^ s) - s;
+}
+struct WxAcc {
+  i64 s4 = 0, s3 = 0, s2 = 0;
+  __device__ __forceinline__ void add(int a2, int a1, int a0, int4 x) {   // x = (high, middle, low, -)
+    s4 = fx_mad(a2, x.x, s4);
+    s3 = fx_mad(a1, x.x, fx_mad(a2, x.y, s3));
+    s2 = fx_mad(a0, x.x, fx_mad(a1, x.y, fx_mad(a2, x.z, s2)));
+  }
+  // (s4 2^54 + s3 2^27 + s2) 2^e as a value of at most 61 bits
+  __device__ __forceinline__ FxVal value(int e) const {
+    const __int128 t = ((__int128)s4 << 54) + ((__int128)s3 << 27) + s2;
+    const i64 hi = (i64)(t >> 64);
+    const u64 lo = (u64)t;
+    const i64 h = hi ^ (hi >> 63);
+    const u64 l = lo ^ (u64)(hi >> 63);
+    const int nb = h ? 128 - __clzll(h) : 64 - __clzll((i64)l);
+    const int n = max(nb - 61, 0);
+    FxVal p;
+    p.v = n == 0 ? (i64)lo : (n < 64 ? (i64)((u64)hi << (64 - n) | lo >> n) : hi >> (n - 64));
+    p.e = e + n;
+    return p;
+  }
+};
+// A product's exponent: (ea + em) - kWxExp.
+constexpr int kWxExp = 1022 + 106;
+
+// A vector as an operand for column exponents cx; returns its exponent (publish_regs); with an infinity in it the
+// raw doubles.
+template <int NP>
+__device__ __forceinline__ int publish_wide(const double (&x)[NP], const int (&cx)[NP], int nr, int lane, int4* xs) {
+  int m = -0x10000;
+#pragma unroll
+  for (int p = 0; p < NP; ++p)
+    if (p * 32 + lane < nr) m = max(m, fx_key(x[p], cx[p]));
+  const int em = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    int4 d = make_int4(0, 0, 0, 0);
+    if (em >= kFxInf) {
+      d.x = __double2loint(x[p]);
+      d.y = __double2hiint(x[p]);
+    } else {
+      wx_split(x[p], em - fx_key(x[p], cx[p]), d.x, d.y, d.z);
+    }
+    xs[p * 32 + lane] = d;                             // (32 NP entries: the block's padding meets zeros)
+  }
+  __syncwarp();
+  return em;
+}
+// Row r of a block times an operand with an infinity (raw doubles), as FP64 gives it.
+static __device__ __noinline__ double wx_dot_slow(const int* blk, int ld, int nr, int r, const int4* xs) {
+  const int ea = blk[3 * ld * ld + r];
+  const int* cx = blk + 3 * ld * ld + ld;
+  double acc = 0.0;
+  for (int c = 0; c < nr; ++c) {
+    const int o = c * ld + r;
+    const double a = __ll2double_rn(((i64)blk[o] << 27) + blk[ld * ld + o]);   // (its sign and zeros matter)
+    acc = fma(ldexp(a, ea + cx[c] - 53), __hiloint2double(xs[c].y, xs[c].x), acc);
+  }
+  return acc;
+}
+// Row r of a block (in shared memory) times a published operand.
+template <int LD>
+__device__ __forceinline__ FxVal wx_dot(const int* blk, int nr, int r, const int4* xs, int em) {
+  const int* A = blk + r;
+  WxAcc acc;
+#pragma unroll 8
+  for (int c = 0; c < LD; ++c) acc.add(A[c * LD], A[(LD + c) * LD], A[(2 * LD + c) * LD], xs[c]);
+  const int ea = blk[3 * LD * LD + r];
+  FxVal p = acc.value(ea + em - kWxExp);
+  if (em >= kFxInf || ea == kFxBad) {
+    p.v = __double_as_longlong(em == kFxInf ? wx_dot_slow(blk, LD, nr, r, xs) : fx_nan());
+    p.e = kFxBad;
+  }
+  return p;
+}
 
 // ---- asynchronous copies -------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {

@@ -121,14 +121,9 @@ __device__ __forceinline__ void grid_products(int pair, const T* RG, const T* bs
 // block's scale words (FP32: K scales then K inverses; FP64: K exponents as ints).
 template <typename T> struct RowTr;
 template <> struct RowTr<float> {
-  static __device__ __forceinline__ unsigned key(float v) { return Bits<float>::absbits(v); }
+  static constexpr bool kInv = true;                   // inverse transforms with conjugated twiddles
   static __device__ __forceinline__ float sign(float v, bool n) { return n ? -v : v; }
-  template <int K>
-  static __device__ __forceinline__ void scale(float*, int, int, unsigned (&mx)[K], void* red, float* scl) {
-    block_max_scales<float, K>(mx, reinterpret_cast<unsigned*>(red), scl);
-  }
   // W_k of a DCT3 pair (rows A = t, B = t + 1 of XV; hasb: row B is there)
-  template <int K>
   static __device__ __forceinline__ float2 pack(const float* XV, int P, int t, bool hasb, int k, const float2* Et,
                                                 const float* scl) {
     const float sa = scl[t], sb = hasb ? scl[t + 1] : 0.0f;
@@ -140,33 +135,26 @@ template <> struct RowTr<float> {
   static __device__ __forceinline__ float2 load(const float* PR, int P, int t, int src, const float* scl) {
     return cmk<float2>(scl[t] * PR[t * P + src], scl[t + 1] * PR[(t + 1) * P + src]);
   }
-  // component (h = 0: row A, 1: row B) of a transformed pair whose first row is t of K
-  template <int K>
-  static __device__ __forceinline__ float out(float2 v, int h, int t, const float* scl) {
-    return (h ? v.y : v.x) * scl[K + t + h];
+  // row t + h (h = 0: A, 1: B) of a transformed pair, nrows rows in all
+  static __device__ __forceinline__ float out(float2 v, int h, int t, int nrows, const float* scl) {
+    return (h ? v.y : v.x) * scl[nrows + t + h];
   }
-  template <int K>
-  static __device__ __forceinline__ void unpack(const float2* Z, int P, int k, int t, const float2* Et, const float* scl,
-                                                float sc, float& ya, float& yb) {
+  static __device__ __forceinline__ void unpack(const float2* Z, int P, int k, int t, int nrows, const float2* Et,
+                                                const float* scl, float sc, float& ya, float& yb) {
     dct2_unpack<float, float2>(Z[k], Z[(P - k) % P], Et[k], ya, yb);
-    ya *= sc * scl[K + t];
-    yb *= sc * scl[K + t + 1];
+    ya *= sc * scl[nrows + t];
+    yb *= sc * scl[nrows + t + 1];
   }
 };
 template <> struct RowTr<double> {
-  static __device__ __forceinline__ unsigned key(double v) { return abs_hi(v); }
+  static constexpr bool kInv = false;                  // inverse transforms as forward ones of swapped pairs
   static __device__ __forceinline__ double sign(double v, bool n) { return neg_if(v, n); }
-  template <int K>
-  static __device__ __forceinline__ void scale(double* XV, int P, int nrows, unsigned (&mx)[K], void* red, double* scl) {
-    rows_to_fixed<K>(XV, P, nrows, mx, reinterpret_cast<unsigned*>(red), reinterpret_cast<int*>(scl));
-  }
-  template <int K>
   static __device__ __forceinline__ longlong2 pack(const double* XV, int P, int t, bool hasb, int k, const int4* Et,
                                                    const double*) {
     const i64* A = reinterpret_cast<const i64*>(XV) + t * P;
     const i64* B = A + P;
     const i64 xa = A[k], xb = hasb ? B[k] : 0;
-    if (k == 0) return make_longlong2(xa, xb);
+    if (k == 0) return make_longlong2(xb, xa);
     return dct3_pack_fx(Et[k], xa, A[P - k], xb, hasb ? B[P - k] : 0);
   }
   static __device__ __forceinline__ longlong2 load(const double* PR, int P, int t, int src, const double*) {
@@ -174,26 +162,69 @@ template <> struct RowTr<double> {
     return make_longlong2(A[src], A[P + src]);
   }
   // a row with an infinity or NaN makes both rows of its pair NaN (they share one complex transform)
-  template <int K>
   static __device__ __forceinline__ bool bad(int t, const double* scl) {
     const int* E = reinterpret_cast<const int*>(scl);
-    return E[t] == kFxBad || (t + 1 < K && E[t + 1] == kFxBad);
+    return E[t] == kFxBad || E[t + 1] == kFxBad;
   }
-  template <int K>
-  static __device__ __forceinline__ double out(longlong2 v, int h, int t, const double* scl) {
-    return bad<K>(t, scl) ? fx_nan() : fx2d(h ? v.y : v.x, 60 - reinterpret_cast<const int*>(scl)[t + h]);
+  static __device__ __forceinline__ double out(longlong2 v, int h, int t, int, const double* scl) {
+    return bad(t, scl) ? fx_nan() : fx2d(h ? v.x : v.y, 60 - reinterpret_cast<const int*>(scl)[t + h]);
   }
-  template <int K>
-  static __device__ __forceinline__ void unpack(const longlong2* Z, int P, int k, int t, const int4* Et,
+  static __device__ __forceinline__ void unpack(const longlong2* Z, int P, int k, int t, int, const int4* Et,
                                                 const double* scl, double sc, double& ya, double& yb) {
     const int* E = reinterpret_cast<const int*>(scl);
     i64 a, b;
     dct2_unpack_fx(Z[k], Z[(P - k) % P], Et[k], a, b);
-    const bool n = bad<K>(t, scl);
+    const bool n = bad(t, scl);
     ya = n ? fx_nan() : sc * fx2d(a, 60 - E[t]);
     yb = n ? fx_nan() : sc * fx2d(b, 60 - E[t + 1]);
   }
 };
+
+// f(i) for the calling thread's elements i < n of a row loop: left to the compiler to unroll in FP32, rolled up in
+// FP64 (the fixed-point bodies are long: unrolled, a kernel's code outgrows the instruction cache).
+template <typename T, typename F>
+__device__ __forceinline__ void for_elems(int n, F&& f) {
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < n; i += blockDim.x) f(i);
+  } else {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) f(i);
+  }
+}
+
+// Forms NR rows (or `nrows` of them) of P elements, row(t, k), in XV and their scales.  FP32: unrolled, the maxima
+// tracked as the rows are formed; FP64: rolled up (code size), rows_to_fixed reads them back.
+template <typename T, int NR, typename F>
+__device__ __forceinline__ void form_rows(T* XV, int P, int nrows, void* red, T* scl, F&& row) {
+  const int tid = threadIdx.x, bd = blockDim.x;
+  if constexpr (sizeof(T) == 4) {
+    unsigned mb[NR];
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      mb[t] = 0;
+      if (t < nrows)
+        for (int k = tid; k < P; k += bd) {
+          const T v = row(t, k);
+          XV[t * P + k] = v;
+          mb[t] = max(mb[t], Bits<float>::absbits(v));
+        }
+    }
+    block_max_scales<T, NR>(mb, reinterpret_cast<unsigned*>(red), scl);
+  } else {
+#pragma unroll 1
+    for (int t = 0; t < nrows; ++t)
+#pragma unroll 1
+      for (int k = tid; k < P; k += bd) XV[t * P + k] = row(t, k);
+    rows_to_fixed(XV, P, nrows, red, reinterpret_cast<int*>(scl));
+  }
+}
+
+// The scales of K formed rows (mx: FP32, the calling thread's maxima).
+template <typename T, int K>
+__device__ __forceinline__ void scale_rows(T* PR, int P, unsigned (&mx)[K], void* red, T* scl) {
+  if constexpr (sizeof(T) == 4) block_max_scales<T, K>(mx, reinterpret_cast<unsigned*>(red), scl);
+  else rows_to_fixed(PR, P, K, red, reinterpret_cast<int*>(scl));
+}
 
 // MODE 0: NLIN_FX (optionally storing the grid fields); 1: NLIN_DFX with base fields from the cache;
 // 2: grid fields only (fills the cache).
@@ -228,10 +259,12 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   T* Sc = JP + M;
   const W* wg = reinterpret_cast<const W*>(a.ops.w);
   const W* eg = reinterpret_cast<const W*>(a.ops.e);
+#pragma unroll 1
   for (int i = tid; i < P; i += bd) {
     Wt[i] = wg[i];
     Et[i] = eg[i];
   }
+#pragma unroll 1
   for (int i = tid; i < P + 2; i += bd) kf[i] = (T)i;
   const T* Drg = reinterpret_cast<const T*>(a.ops.Dr);
   const T* D2g = reinterpret_cast<const T*>(a.ops.D2r2);
@@ -244,10 +277,14 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
 
   // ---- 1. radial contractions of row n (Derivatives, :698-729) and the row values ----
   const int N = M * nr;
-  // mixed plans with tensor cores: the four contractions were formed by k_deriv_tc ([op][n][k] blocks)
-  const T* Dt = (sizeof(T) == 4 && a.deriv_t) ? reinterpret_cast<const T*>(a.deriv) + (size_t)b * a.deriv_stride
-                                              : nullptr;
+  // the four contractions were formed by k_fx_deriv ([op][k][n], FP64) or k_deriv_tc ([op][n][k], mixed plans
+  // with tensor cores); without their scratch (and in FP32 on the CUDA cores) here
+  const T* Dt = (a.deriv && (sizeof(T) == 8 || a.deriv_t))
+                    ? reinterpret_cast<const T*>(a.deriv) + (size_t)b * a.deriv_stride
+                    : nullptr;
+  const size_t dk = a.deriv_t ? 1 : nr, d0 = a.deriv_t ? (size_t)n * M : n;
   with_x<T>(a, b, [&](auto xr) {
+#pragma unroll 1
   for (int k = tid; k < M; k += bd) {
     const size_t ps = (size_t)k * nr, ts = N + (size_t)k * nr, ss = 2 * (size_t)N + (size_t)k * nr;
     const bool psi_on = !(a.sym && (k % 2 == 0));
@@ -255,8 +292,8 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
     T dp = 0, d2 = 0, dtv = 0, dcv = 0, pn = 0, tn = 0, sn = 0;
     if (psi_on) {
       if (Dt) {
-        dp = Dt[(size_t)n * M + k];
-        d2 = Dt[((size_t)nr + n) * M + k];
+        dp = Dt[d0 + k * dk];
+        d2 = Dt[(size_t)N + d0 + k * dk];
       } else {
         for (int m = 0; m < nr; ++m) {
           const T x = xr(ps + m);
@@ -268,8 +305,8 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
     }
     if (ts_on) {
       if (Dt) {
-        dtv = Dt[((size_t)2 * nr + n) * M + k];
-        dcv = Dt[((size_t)3 * nr + n) * M + k];
+        dtv = Dt[2 * (size_t)N + d0 + k * dk];
+        dcv = Dt[3 * (size_t)N + d0 + k * dk];
       } else {
         for (int m = 0; m < nr; ++m) {
           dtv = fma(opr[m], xr(ts + m), dtv);
@@ -292,37 +329,27 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   parity_suffix<T>(pv, Sc, M);
   __syncthreads();
   // J_theta_RT (:437-472) and A2_SINE_R2 (:476-526) along the row
+#pragma unroll 1
   for (int k = tid; k < M; k += bd) jp_om<T>(k, M, kf, pv, Sc, ir4n, JP[k], OM[k]);
   __syncthreads();
   // ---- 2. nine inverse transforms as five paired DCT3s (:776-786) ----
   // the nine DCT3 input rows, materialised once (in RB, free until the FFT), with their maxima
   T* XV = reinterpret_cast<T*>(RB);
-  {
-    unsigned mb[9];
-#pragma unroll
-    for (int t = 0; t < 9; ++t) {
-      mb[t] = 0;
-      for (int k = tid; k < P; k += bd) {
-        const T v = fx_x<T>(t, k, M, P, kf, JP, OM, DP, DTv, DCv, Tv, Sv);
-        XV[t * P + k] = v;
-        mb[t] = max(mb[t], Tr::key(v));
-      }
-    }
-    Tr::template scale<9>(XV, P, 9, mb, red, scl);
-  }
-  for (int idx = tid; idx < 5 * P; idx += bd) {
+  form_rows<T, 9>(XV, P, 9, red, scl,
+                  [&](int t, int k) { return fx_x<T>(t, k, M, P, kf, JP, OM, DP, DTv, DCv, Tv, Sv); });
+  for_elems<T>(5 * P, [&](int idx) {
     const int p = idx / P;
-    RA[idx] = Tr::template pack<9>(XV, P, 2 * p, p < 4, idx - p * P, Et, scl);
-  }
+    RA[idx] = Tr::pack(XV, P, 2 * p, p < 4, idx - p * P, Et, scl);
+  });
   __syncthreads();
-  C* res = fft_rows<T, true>(RA, RB, 5, a.st, Wt);
-  for (int idx = tid; idx < 9 * P; idx += bd) {
+  C* res = fft_rows<T, Tr::kInv>(RA, RB, 5, a.st, Wt);
+  for_elems<T>(9 * P, [&](int idx) {
     const int t = idx / P;
     const int i = idx - t * P;
     const int src = (i & 1) ? (P - 1 - (i >> 1)) : (i >> 1);
-    const T val = Tr::template out<9>(res[(t >> 1) * P + src], t & 1, t & ~1, scl);
+    const T val = Tr::out(res[(t >> 1) * P + src], t & 1, t & ~1, 9, scl);
     RG[idx] = Tr::sign(val, t >= 5 && (i & 1));
-  }
+  });
   __syncthreads();
 
   if (MODE != 1 && a.base != nullptr) {
@@ -337,29 +364,30 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
                                   (size_t)n * 9 * P
                             : nullptr;
   unsigned m4[4] = {0, 0, 0, 0};
-  for (int i = tid; i < P; i += bd) {
+  for_elems<T>(P, [&](int i) {
     T v[4];
     grid_products<T, MODE>(0, RG, bs, i, P, v[0], v[1]);
     grid_products<T, MODE>(1, RG, bs, i, P, v[2], v[3]);
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       PR[t * P + i] = t < 2 ? Tr::sign(v[t], i & 1) : v[t];
-      m4[t] = max(m4[t], Tr::key(v[t]));
+      if constexpr (sizeof(T) == 4) m4[t] = max(m4[t], Bits<T>::absbits(v[t]));
     }
-  }
-  Tr::template scale<4>(PR, P, 4, m4, red, scl);
+  });
+  scale_rows<T, 4>(PR, P, m4, red, scl);
 
   // ---- 4. four forward transforms as two paired DCT2s (:797-802) ----
-  for (int idx = tid; idx < 2 * P; idx += bd) {
-    const int p = idx / P;
+  for_elems<T>(2 * P, [&](int idx) {
+    const int p = idx >= P ? 1 : 0;
     RB[idx] = Tr::load(PR, P, 2 * p, makhoul_src(idx - p * P, P), scl);
-  }
+  });
   __syncthreads();
   C* Z = fft_rows<T, false>(RB, RA, 2, a.st, Wt);
   double* o = a.out4 + (size_t)b * a.out_stride;
   const T two_P = (T)2 / (T)P, one_P = (T)1 / (T)P;
+#pragma unroll 1
   for (int idx = tid; idx < 2 * M; idx += bd) {
-    const int p = idx / M;
+    const int p = idx >= M;
     const int s = idx - p * M;
     T ya = 0, yb = 0;
     bool zero = false;
@@ -372,7 +400,7 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
       k = s;
     }
     if (!zero) {
-      Tr::template unpack<4>(Z + p * P, P, k, 2 * p, Et, scl, (p == 1 && k == 0) ? one_P : two_P, ya, yb);
+      Tr::unpack(Z + p * P, P, k, 2 * p, 4, Et, scl, (p == 1 && k == 0) ? one_P : two_P, ya, yb);
     }
     const size_t q0 = (size_t)(2 * p) * N + (size_t)s * nr + n;
     o[q0] = (double)ya;
@@ -406,11 +434,6 @@ size_t fx_prod_smem_bytes(int P, int prec) {
   return (8 * (size_t)P + 2 * (size_t)P + 32) * es + 2 * 32 * 8;
 }
 
-// Radial contractions of the split path (Derivatives, Matrix_Operators.py:698-729), one CTA per (mode,
-// shell): Dr psi_k, D2r2 psi_k, Dr T_k, Dr S_k for every radial row n, each a sequential fma chain over the
-// columns in the order of the fused kernel's (so both paths round identically).  With the fused
-// right-hand side a fifth block, D2s psi_k in FP64, follows the four T-typed blocks (per shell:
-// 4 M nr T then M nr doubles).
 // One asynchronous global -> shared copy of an element of 4, 8 or 16 bytes (the issuing thread does not
 // wait for the data: a loop of such copies has all its loads in flight at once).
 template <int BYTES>
@@ -429,169 +452,227 @@ __device__ __forceinline__ void cp_async_all_done() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_all;\n" ::: "memory");
 }
 
-// The terms d_{c-1}, part_{c,0}, ..., part_{c,c-2} of the carried states of a pending correction of mode k, by
-// asynchronous copies (the caller commits and waits): per chain f, from st + c o_f (o = 0, 2 nr, 3 nr), c
-// vectors of m_f = 2 nr, nr, nr doubles.
-__host__ __device__ inline size_t fix_term_doubles(int nr, int nch) { return (size_t)(nch > 1 ? nch - 1 : 0) * 4 * nr; }
+// The pending correction of modes k0 .. k0 + kn - 1 (see FixArgs) on xd (the modes' FP64 psi, T, S rows, in
+// shared memory, still in flight but for one group of copies).  s_c = d_{c-1} + part_{c,0} + ... in index order
+// (per chain f vectors of 2 nr, nr, nr doubles) while the rows of G load; then xd += G_jj s_c in the arithmetic
+// of k_mode_mv (the same bits).  Four tasks of NP^2 warps (32 rows and the columns, or half of them) per mode:
+// psi's two operand halves, T, S; 8 warps take two modes at once, 16 warps one.  The corrected rows are written
+// back to the state (and its FP32 copy).  sc: 4 nr doubles a mode.
+constexpr int deriv_warps(int ld) { return ld <= 32 ? 8 : 16; }
 
-__device__ __forceinline__ void stage_fix_terms(const FxArgs& a, int b, int k, double* st) {
-  const FixArgs& x = a.fix;
-  const int nr = a.nr;
-  const int jj = a.M - 1 - k, par = jj & 1, c = (jj >> 1) / x.kc;
-  if (c < 1) return;
-  for (int f = 0; f < 3; ++f) {
-    const bool a4 = f == 0;
-    if (a.sym && !(a4 ? par == 0 : par == 1)) continue;
-    const int m = a4 ? 2 * nr : nr;
-    const int o = a4 ? 0 : (f == 1 ? 2 * nr : 3 * nr);
-    const size_t chain = (size_t)(f * 2 + par);
-    const double* d = x.dbuf + (size_t)b * x.d_stride + chain * x.nch * x.ldd + (size_t)(c - 1) * x.ldd;
-    const double* prow = x.pbuf + (size_t)b * x.p_stride + (chain * x.np + (size_t)(c - 1) * (c - 2) / 2) * x.ldd;
-    double* Ts = st + (size_t)c * o;
-    for (int e = threadIdx.x; e < c * m; e += blockDim.x) {
-      const int v = e / m, i = e - v * m;
-      cp_async_bytes<8>(Ts + e, v == 0 ? d + i : prow + (size_t)(v - 1) * x.ldd + i);
-    }
-  }
-}
-
-// The pending correction of mode k (see FixArgs) on xd (the mode's FP64 psi, T, S rows, in shared memory; xd
-// and the terms `st` still in flight).  Four tasks of NP warps each (psi's two operand halves, T, S): a warp's
-// rows of G load into registers while the terms arrive; s_c = d_{c-1} + part_{c,0} + ... in index order; then
-// xd += G_jj s_c in the arithmetic of k_mode_mv (the same bits).  The corrected rows are written back to the
-// state (and its FP32 copy).  sc: 4 nr doubles.
-template <int LD>
-__device__ void apply_pending_fix(const FxArgs& a, int b, int k, double* xd, double* sc, const double* st) {
-  constexpr int NP = (LD + 31) / 32;
-  constexpr int bw = (int)fx_block_words(LD);
-  __shared__ __align__(16) int2 s_x[4 * NP][32 * NP];
-  __shared__ i64 s_v[4][32 * NP];
-  __shared__ int s_e[4][32 * NP];
-  const FixArgs& x = a.fix;
-  const int M = a.M, nr = a.nr;
-  const int jj = M - 1 - k, par = jj & 1, c = (jj >> 1) / x.kc;
-  const bool psi_on = !a.sym || par == 0, ts_on = !a.sym || par == 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = warp / NP, r = (warp % NP) * 32 + lane, rr = min(r, nr - 1);
-  const bool on = c >= 1 && warp < 4 * NP && (task < 2 ? psi_on : ts_on);   // uniform over the warp
-  const i64* blk = task < 2 ? x.GA4 + ((size_t)jj * 2 + task) * bw : (task == 2 ? x.GT : x.GS) + (size_t)jj * bw;
-  FxRow<LD, NP> G;
-  if (on) G.load(blk, rr);
-  cp_async_all_done();
-  __syncthreads();
-  if (c < 1) return;                                   // uniform over the CTA
-  for (int e = threadIdx.x; e < 4 * nr; e += blockDim.x) {
-    if (!(e < 2 * nr ? psi_on : ts_on)) continue;
-    const int o = e < 2 * nr ? 0 : (e < 3 * nr ? 2 * nr : 3 * nr), m = e < 2 * nr ? 2 * nr : nr;
-    const double* Ts = st + (size_t)c * o + (e - o);
-    double v = Ts[0];                                  // d_{c-1} + part_0 + ... + part_{c-2} in index order
-    for (int u = 1; u < c; ++u) v += Ts[(size_t)u * m];
-    sc[e] = v;
-  }
-  __syncthreads();
-  if (on) {
-    double xv[NP];
+__device__ __forceinline__ double carried_term(const FixArgs& x, int b, int par, int c, int e, int nr) {
+  const int f = e < 2 * nr ? 0 : (e < 3 * nr ? 1 : 2), i = e - (f == 0 ? 0 : (f + 1) * nr);
+  const size_t chain = (size_t)(f * 2 + par);
+  const double* d = x.dbuf + (size_t)b * x.d_stride + (chain * x.nch + (c - 1)) * x.ldd;
+  const double* row = x.pbuf + (size_t)b * x.p_stride + (chain * x.np + (size_t)(c - 1) * (c - 2) / 2) * x.ldd;
+  const int nt = c - 1;
+  double v = __ldcg(d + i);
+  for (int u0 = 0; u0 < nt; u0 += 8) {                 // eight loads in flight
+    double tv[8];
 #pragma unroll
-    for (int p = 0; p < NP; ++p) xv[p] = 32 * p + lane < nr ? sc[task * nr + 32 * p + lane] : 0.0;
-    const int em = publish_regs<NP>(xv, G.cx, nr, lane, s_x[warp]);
-    const FxVal p = G.times(blk, nr, rr, s_x[warp], em);
-    s_v[task][r] = p.v;
-    s_e[task][r] = p.e;
+    for (int k = 0; k < 8; ++k) tv[k] = u0 + k < nt ? __ldcg(row + (size_t)(u0 + k) * x.ldd + i) : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (u0 + k < nt) v += tv[k];
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 3 * nr; e += blockDim.x) {
-    const int f = e / nr, i = e - f * nr;
-    if (!(f == 0 ? psi_on : ts_on)) continue;
-    const FxVal p{s_v[f == 0 ? 0 : f + 1][i], s_e[f == 0 ? 0 : f + 1][i]}, q{s_v[1][i], s_e[1][i]};
-    const double v = f == 0 ? fx_sum(xd[e], p, q) : fx_sum(xd[e], p);
-    xd[e] = v;
-    const size_t o = (size_t)f * M * nr + (size_t)k * nr + i;
-    x.X[(size_t)b * a.x_stride + o] = v;
-    if (x.X32) x.X32[(size_t)b * a.x32_stride + o] = (float)v;
-  }
-  __syncthreads();
+  return v;
 }
 
-// T-typed Dr, D2r2 and the mode's rows; then (FP64) the corrected rows and carried states of a pending fix
-// (7 nr); then the fused right-hand side's D2s (nr^2) and the mode's FP64 psi row (nr); then, 16-byte
-// aligned, the correction's terms (fix_term_doubles)
-__host__ __device__ inline size_t fx_deriv_stage_offset(int nr, int prec, bool fix, bool fuse) {
-  const size_t es = prec == SDD_PREC_MIXED ? sizeof(float) : sizeof(double);
-  const size_t t = ((2 * (size_t)nr * nr + 3 * (size_t)nr) * es + 15) / 16 * 16;
-  return (t + (fix ? 7 * (size_t)nr * sizeof(double) : 0) + (fuse ? ((size_t)nr * nr + nr) * sizeof(double) : 0) +
-          15) / 16 * 16;
-}
-size_t fx_deriv_smem_bytes(int nr, int prec, bool fix, bool fuse, int nch) {
-  return fx_deriv_stage_offset(nr, prec, fix, fuse) + (fix ? fix_term_doubles(nr, nch) : 0) * sizeof(double);
-}
-
-
-template <typename T, int LD>
-__global__ void __launch_bounds__(256, LD <= 32 ? 2 : 1) k_fx_deriv(FxArgs a, T* deriv, size_t deriv_stride) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+template <int LD>
+__device__ void apply_pending_fix(const FxArgs& a, int b, int k0, int kn, double* xd, double* sc) {
+  constexpr int NP = (LD + 31) / 32, NC = LD / NP, kMw = 4 * NP * NP, kG = deriv_warps(LD) / kMw;
+  constexpr int bw = (int)fx_block_words(LD);
+  __shared__ __align__(16) int2 s_x[deriv_warps(LD)][32 * NP];
+  __shared__ i64 s_v[kG][4][32 * NP];
+  __shared__ int s_e[kG][4][32 * NP];
+  __shared__ FxPart s_p[NP > 1 ? 8 : 1][32];           // the second column half's sums, per task and row slab
+  const FixArgs& x = a.fix;
   const int M = a.M, nr = a.nr;
-  const int k = blockIdx.x, b = blockIdx.y;
-  if (a.active && !a.active[b]) return;
-  T* ops = reinterpret_cast<T*>(smem_raw);     // Dr, D2r2 (nr x nr each, row-major)
-  T* xv = ops + 2 * nr * nr;                  // psi_k, T_k, S_k
-  // with a pending correction: the mode's FP64 rows (corrected here) and a carried state
-  double* xd = reinterpret_cast<double*>(smem_raw + ((2 * (size_t)nr * nr + 3 * (size_t)nr) * sizeof(T) + 15) / 16 * 16);
-  double* sc = xd + 3 * nr;
-  double* D2sm = xd + (a.fix.on ? 7 * nr : 0);        // fused right-hand side: A2_SINE's D2 (FP64)
-  const T* Drg = reinterpret_cast<const T*>(a.ops.Dr);
-  const T* D2g = reinterpret_cast<const T*>(a.ops.D2r2);
-  // the operators (and the rows and carry terms of a pending fix) stream in asynchronously: one L2 round
-  // trip, not one per element each thread copies
-  double* terms = reinterpret_cast<double*>(
-      smem_raw + fx_deriv_stage_offset(nr, sizeof(T) == 4 ? SDD_PREC_MIXED : SDD_PREC_FP64, true, a.fuse_rhs != 0));
-  if (a.fix.on) stage_fix_terms(a, b, k, terms);
-  for (int e = threadIdx.x; e < nr * nr; e += blockDim.x) {
-    cp_async_elem(ops + e, Drg + e);
-    cp_async_elem(ops + nr * nr + e, D2g + e);
-    if (a.fuse_rhs) cp_async_elem(D2sm + e, a.rl.D2s + e);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto chunk_of = [&](int k) { return ((M - 1 - k) >> 1) / x.kc; };
+  auto on = [&](int k, bool psi) { return chunk_of(k) >= 1 && (!a.sym || ((M - 1 - k) & 1) == (psi ? 0 : 1)); };
+  const int task = warp % kMw / (NP * NP), sl = warp / NP % NP, h = warp % NP;
+  const int r = sl * 32 + lane, rr = min(r, nr - 1);
+  FxRow<LD, NP, NC> G;
+  auto block = [&](int m) {
+    const size_t jj = M - 1 - (k0 + m);
+    return task < 2 ? x.GA4 + (jj * 2 + task) * bw : (task == 2 ? x.GT : x.GS) + jj * bw;
+  };
+  auto mine = [&](int m) { return m < kn && on(k0 + m, task < 2); };   // uniform over the warp
+  int m = warp / kMw;
+  if (mine(m)) G.load(block(m), rr, h * NC);
+  for (int q = threadIdx.x; q < kn * 4 * nr; q += blockDim.x) {
+    const int mm = q / (4 * nr), e = q - mm * 4 * nr;
+    if (on(k0 + mm, e < 2 * nr)) sc[q] = carried_term(x, b, (M - 1 - k0 - mm) & 1, chunk_of(k0 + mm), e, nr);
   }
-  const int N = M * nr;
-  if (a.fix.on) {
-    for (int e = threadIdx.x; e < 3 * nr; e += blockDim.x) {
-      const int f = e / nr, m = e - f * nr;
-      cp_async_elem(xd + e, a.fix.X + (size_t)b * a.x_stride + (size_t)f * N + (size_t)k * nr + m);
-    }
-    apply_pending_fix<LD>(a, b, k, xd, sc, terms);
-    for (int e = threadIdx.x; e < 3 * nr; e += blockDim.x) xv[e] = (T)xd[e];
-  } else {
-    with_x<T>(a, b, [&](auto xr) {
-      for (int e = threadIdx.x; e < 3 * nr; e += blockDim.x) {
-        const int f = e / nr, m = e - f * nr;
-        xv[e] = xr((size_t)f * N + (size_t)k * nr + m);
-      }
-    });
-    if (a.fuse_rhs)
-      for (int e = threadIdx.x; e < nr; e += blockDim.x)
-        cp_async_elem(D2sm + nr * nr + e, a.X + (size_t)b * a.x_stride + (size_t)k * nr + e);
-    cp_async_all_done();
-  }
+  cp_async_wait<1>();
   __syncthreads();
-  T* D = deriv + (size_t)b * deriv_stride;
-  const int nops = a.fuse_rhs ? 5 : 4;
-  const int op0 = a.deriv_t ? 4 : 0;    // tensor cores: only the pending correction and the FP64 block here
-  for (int e = threadIdx.x + op0 * nr; e < nops * nr; e += blockDim.x) {
-    const int op = e / nr, n = e - op * nr;
-    if (op < 4) {
-      const T* row = ops + (op == 1 ? nr * nr : 0) + (size_t)n * nr;
-      const T* x = xv + (op < 2 ? 0 : (op - 1) * nr);
-      T acc = 0;
-      for (int m = 0; m < nr; ++m) acc = fma(row[m], x[m], acc);
-      D[((size_t)op * M + k) * nr + n] = acc;
-    } else {   // A2_SINE's D2 psi for the fused right-hand side (FP64; the order of k_rhs's dot)
-      const double* row = D2sm + (size_t)n * nr;
-      double acc = 0;
-      if (a.fix.on) {          // the corrected rows (this kernel wrote them: not through the read-only path)
-        for (int m = 0; m < nr; ++m) acc = fma(row[m], xd[m], acc);
-      } else {
-        const double* ps = D2sm + nr * nr;     // the mode's FP64 psi row
-        for (int m = 0; m < nr; ++m) acc = fma(row[m], ps[m], acc);
+#pragma unroll 1
+  for (int g = 0; g < kn; g += kG, m += kG) {
+    const int mg = m - g;
+    FxPart t;
+    int em;
+    const bool act = mine(m);
+    if (act) {
+      double xv[NP];
+#pragma unroll
+      for (int p = 0; p < NP; ++p) xv[p] = 32 * p + lane < nr ? sc[(m * 4 + task) * nr + 32 * p + lane] : 0.0;
+      em = publish_regs<NP>(xv, G.cx, nr, lane, s_x[warp]);
+      t = G.part(s_x[warp] + h * NC);
+      if (NP > 1 && h == 1) s_p[task * NP + sl][lane] = t;
+    }
+    if (NP > 1) __syncthreads();
+    if (act && h == 0) {
+      if (NP > 1) {
+        const FxPart u = s_p[task * NP + sl][lane];
+        t.t2 += u.t2;
+        t.t1 += u.t1;
       }
-      reinterpret_cast<double*>(D)[(size_t)4 * M * nr * sizeof(T) / 8 + (size_t)k * nr + n] = acc;
+      const FxVal p = G.value(t, block(m), nr, rr, s_x[warp], em);
+      s_v[mg][task][r] = p.v;
+      s_e[mg][task][r] = p.e;
+    }
+    if (mine(m + kG)) G.load(block(m + kG), rr, h * NC);
+    __syncthreads();
+    const int gn = min(kG, kn - g);
+    for (int q = threadIdx.x; q < gn * 3 * nr; q += blockDim.x) {
+      const int mm = q / (3 * nr), e = q - mm * 3 * nr, f = e / nr, i = e - f * nr, k = k0 + g + mm;
+      if (!on(k, f == 0)) continue;
+      double* xp = xd + (size_t)(g + mm) * 3 * nr + e;
+      const FxVal p{s_v[mm][f == 0 ? 0 : f + 1][i], s_e[mm][f == 0 ? 0 : f + 1][i]}, u{s_v[mm][1][i], s_e[mm][1][i]};
+      const double v = f == 0 ? fx_sum(*xp, p, u) : fx_sum(*xp, p);
+      *xp = v;
+      const size_t o = (size_t)f * M * nr + (size_t)k * nr + i;
+      x.X[(size_t)b * a.x_stride + o] = v;
+      if (x.X32) x.X32[(size_t)b * a.x32_stride + o] = (float)v;
+    }
+    __syncthreads();
+  }
+}
+
+// Shared memory of k_fx_deriv: the fixed-point operators (FP64: D2r2, Dr and with the fused right-hand side
+// A2_SINE's D2; FP32: the latter alone), the modes' FP64 rows (3 nr each), with a pending correction the carried
+// states (4 nr); FP32 contractions on the CUDA cores: Dr, D2r2 and the modes' rows in FP32.
+template <typename T>
+__host__ __device__ inline size_t deriv_op_bytes(int ld, bool d2s) {
+  return (sizeof(T) == 8 ? wx_block_ints(ld) * sizeof(int) + fx_block_words(ld) * sizeof(i64) : 0) +
+         (d2s ? wx_block_ints(ld) * sizeof(int) : 0);
+}
+template <typename T>
+static size_t fx_deriv_smem_bytes(int nr, bool d2s, bool fix, int km, bool f32) {
+  return deriv_op_bytes<T>(fx_ld(nr), d2s) + (size_t)km * (fix ? 7 : 3) * nr * sizeof(double) +
+         (f32 ? (2 * (size_t)nr * nr + (size_t)km * 3 * nr) * sizeof(float) : 0);
+}
+
+// Radial contractions (Derivatives, Matrix_Operators.py:698-729) of km modes of one shell per CTA: Dr psi_k,
+// D2r2 psi_k, Dr T_k, Dr S_k for every radial row n, and with the fused right-hand side A2_SINE's D2 psi in
+// FP64 as a fifth block (per shell: 4 M nr T, [op][k][n], then M nr doubles).  FP64 contractions run in fixed
+// point (sdd_fixed.cuh), a warp per operator, 32 rows and mode, the operators in shared memory; FP32 ones
+// (contract: not already on the tensor cores) as sequential FP32 chains in the order of the fused kernel's.  Inside sdd_step a pending chain correction is applied to the rows first.
+// Dr takes two digits here: its products with psi, T and S go into pointwise products, which no operator
+// differentiates again on the way to the result (the h kernel's Dr Q and D2 psi meet the implicit solves, which
+// cancel their large parts, and take three).
+// Bound: 64 shells of 256 x 30, the integer pipe (a D2 product is about 1500 warp cycles, a Dr product 800): 79 us,
+// 146 us with every operator in three digits.  One shell, the L2 round trips of the rows, the correction's blocks
+// and the operators: 14 us; 540 x 65: 37 us (64 us with the operators' rows in registers, loaded for every mode).
+template <typename T, int LD>
+__global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
+    k_fx_deriv(FxArgs a, T* deriv, size_t deriv_stride, int km, int contract) {
+  constexpr int NP = (LD + 31) / 32, kW = deriv_warps(LD);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int4 s_x[kW][32 * NP];
+  const int M = a.M, nr = a.nr;
+  const int k0 = blockIdx.x * km, kn = min(km, M - k0), b = blockIdx.y;
+  if (a.active && !a.active[b]) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t N = (size_t)M * nr;
+  const bool d2s = a.fuse_rhs;
+  int* opw = reinterpret_cast<int*>(smem_raw);         // the wide blocks, then Dr
+  i64* opd = reinterpret_cast<i64*>(opw + ((sizeof(T) == 8) + d2s) * wx_block_ints(LD));
+  double* xd = reinterpret_cast<double*>(smem_raw + deriv_op_bytes<T>(LD, d2s));   // [mode][field][nr]
+  double* sc = xd + (size_t)km * 3 * nr;
+  // FP32 on the CUDA cores: the operators and rows in FP32, behind the doubles
+  float* ops = reinterpret_cast<float*>(xd + (size_t)km * (a.fix.on ? 7 : 3) * nr);
+  const double* Xs = (a.fix.on ? a.fix.X : a.X) + (size_t)b * a.x_stride;
+  for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) {
+    const int m = q / (3 * nr), e = q - m * 3 * nr, f = e / nr;
+    cp_async_elem(xd + q, Xs + f * N + (size_t)(k0 + m) * nr + (e - f * nr));
+  }
+  cp_async_commit();
+  constexpr int wq = (int)wx_block_ints(LD) / 4, dq = (int)fx_block_words(LD) / 2;
+  if (sizeof(T) == 8) {
+    for (int e = threadIdx.x; e < wq; e += blockDim.x) cp_async16(opw + 4 * e, a.ops.wx[0] + 4 * e);
+    for (int e = threadIdx.x; e < dq; e += blockDim.x) cp_async16(opd + 2 * e, a.ops.fxDr + 2 * e);
+  }
+  if (d2s) {
+    int* dst = opw + (sizeof(T) == 8 ? 4 * wq : 0);
+    for (int e = threadIdx.x; e < wq; e += blockDim.x) cp_async16(dst + 4 * e, a.ops.wx[1] + 4 * e);
+  }
+  if (contract) {
+    const float* Drg = reinterpret_cast<const float*>(a.ops.Dr);
+    const float* D2g = reinterpret_cast<const float*>(a.ops.D2r2);
+    for (int e = threadIdx.x; e < nr * nr; e += blockDim.x) {
+      cp_async_elem(ops + e, Drg + e);
+      cp_async_elem(ops + nr * nr + e, D2g + e);
+    }
+  }
+  cp_async_commit();
+  T* D = deriv + (size_t)b * deriv_stride;
+  double* D5 = reinterpret_cast<double*>(D) + 4 * N * sizeof(T) / 8;
+  if (a.fix.on) apply_pending_fix<LD>(a, b, k0, kn, xd, sc);
+  cp_async_wait<0>();
+  __syncthreads();
+  // the fixed-point contractions, as items (operator, row slab, mode): D2 first, whose products cost twice Dr's
+  // (FP64: D2r2 psi, A2_SINE's D2 psi where it is asked for, then Dr psi, Dr T, Dr S; FP32: A2_SINE's D2 psi)
+  const int nd2 = (sizeof(T) == 8) + d2s, nit = (nd2 + (sizeof(T) == 8 ? 3 : 0)) * NP * kn;
+#pragma unroll 1
+  for (int it = warp; it < nit; it += kW) {
+    const int oi = it / (NP * kn), m = it / NP % kn;
+    const int r = (it % NP) * 32 + lane, rr = min(r, nr - 1);
+    const size_t o = (size_t)(k0 + m) * nr + r;
+    const int f = oi < nd2 ? 0 : oi - nd2;
+    const double* xr = xd + (m * 3 + f) * nr;
+    const int* ce = oi < nd2 ? opw + oi * (4 * wq) + 3 * LD * LD + LD : fx_col_exp(opd, LD);
+    double x[NP];
+    int cx[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      x[p] = 32 * p + lane < nr ? xr[32 * p + lane] : 0.0;
+      cx[p] = 32 * p + lane < nr ? ce[32 * p + lane] : 0;
+    }
+    if (oi < nd2) {
+      const int em = publish_wide<NP>(x, cx, nr, lane, s_x[warp]);
+      const double v = fx_val(wx_dot<LD>(opw + oi * (4 * wq), nr, rr, s_x[warp], em));
+      if (r < nr) {
+        if (sizeof(T) == 4 || oi == 1) D5[o] = v;
+        else D[N + o] = (T)v;
+      }
+    } else {
+      int2* xs = reinterpret_cast<int2*>(s_x[warp]);
+      const int em = publish_regs<NP>(x, cx, nr, lane, xs);
+      const double v = fx_val(block_vec<LD>(opd, nr, rr, xs, em));
+      if (r < nr) D[(f == 0 ? 0 : f + 1) * N + o] = (T)v;   // Dr of psi, T, S: blocks 0, 2, 3
+    }
+    __syncwarp();                                      // the digits are read before the next item's replace them
+  }
+  if (contract) {
+    float* xv = ops + 2 * nr * nr;
+    if (a.X32 && !a.fix.on) {                          // the caller's FP32 copy (the same values)
+      for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) {
+        const int m = q / (3 * nr), e = q - m * 3 * nr, f = e / nr;
+        xv[q] = __ldg(a.X32 + (size_t)b * a.x32_stride + f * N + (size_t)(k0 + m) * nr + (e - f * nr));
+      }
+    } else {
+      for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) xv[q] = (float)xd[q];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < kn * 4 * nr; q += blockDim.x) {
+      const int m = q / (4 * nr), e = q - m * 4 * nr, o = e / nr, n = e - o * nr;
+      const float* row = ops + (o == 1 ? nr * nr : 0) + (size_t)n * nr;
+      const float* x = xv + m * 3 * nr + (o < 2 ? 0 : (o - 1) * nr);
+      float acc = 0.0f;
+      for (int c = 0; c < nr; ++c) acc = fmaf(row[c], x[c], acc);
+      D[o * N + (size_t)(k0 + m) * nr + n] = (T)acc;
     }
   }
 }
@@ -626,10 +707,12 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
   void* red = scl + 32;
   const W* wg = reinterpret_cast<const W*>(a.ops.w);
   const W* eg = reinterpret_cast<const W*>(a.ops.e);
+#pragma unroll 1
   for (int i = tid; i < P; i += bd) {               // asynchronous: in flight while the row loads
     cp_async_elem(Wt + i, wg + i);
     cp_async_elem(Et + i, eg + i);
   }
+#pragma unroll 1
   for (int i = tid; i < P + 2; i += bd) kf[i] = (T)i;
   const T ir4n = reinterpret_cast<const T*>(a.ops.ir4r2)[n];
   // (no barrier: the row loads below do not read the tables; the one after them covers both)
@@ -715,6 +798,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
     const double Ra = lRa, Ras = lRas;
     const double ir2 = lir2, rsq = lrsq, dT0 = ldT0, gr = lgr;
     double* R = lin ? r.rhs + (size_t)b * r.rhs_stride : nullptr;
+#pragma unroll 1
     for (int k = tid; k < M; k += bd) {
       if (need_psi) jp_om<T>(k, M, kf, pv, Sc, ir4n, JP[k], OM[k]);
       if (lin) {
@@ -743,32 +827,20 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
   // the pair's two DCT3 input rows (in RB, free until the FFT) and their scales
   const int nt = (tb < 9) ? 2 : 1;
   T* XV = reinterpret_cast<T*>(RB);
-  {
-    unsigned mb[2] = {0, 0};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int t = ta + u;
-      if (t < 9)
-        for (int k = tid; k < P; k += bd) {
-          const T v = fx_x<T>(t, k, M, P, kf, JP, OM, DP, DTv, DCv, Tv, Sv);
-          XV[u * P + k] = v;
-          mb[u] = max(mb[u], Tr::key(v));
-        }
-    }
-    Tr::template scale<2>(XV, P, nt, mb, red, scl);
-  }
-  for (int k = tid; k < P; k += bd) RA[k] = Tr::template pack<2>(XV, P, 0, nt > 1, k, Et, scl);
+  form_rows<T, 2>(XV, P, nt, red, scl,
+                  [&](int u, int k) { return fx_x<T>(ta + u, k, M, P, kf, JP, OM, DP, DTv, DCv, Tv, Sv); });
+  for_elems<T>(P, [&](int k) { RA[k] = Tr::pack(XV, P, 0, nt > 1, k, Et, scl); });
   __syncthreads();
-  C* res = fft_rows<T, true>(RA, RB, 1, a.st, Wt);
+  C* res = fft_rows<T, Tr::kInv, false>(RA, RB, 1, a.st, Wt);
   T* g = grid + (size_t)b * grid_stride + (size_t)n * 9 * P;
-  for (int idx = tid; idx < nt * P; idx += bd) {
-    const int u = idx / P;
+  for_elems<T>(nt * P, [&](int idx) {
+    const int u = idx >= P ? 1 : 0;
     const int i = idx - u * P;
     const int t = ta + u;
     const int src = (i & 1) ? (P - 1 - (i >> 1)) : (i >> 1);
-    const T val = Tr::template out<2>(res[src], u, 0, scl);
+    const T val = Tr::out(res[src], u, 0, 2, scl);
     g[(size_t)t * P + i] = Tr::sign(val, t >= 5 && (i & 1));
-  }
+  });
 }
 
 template <typename T, int MODE>
@@ -790,6 +862,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
   void* red = scl + 32;
   const W* wg = reinterpret_cast<const W*>(a.ops.w);
   const W* eg = reinterpret_cast<const W*>(a.ops.e);
+#pragma unroll 1
   for (int i = tid; i < P; i += bd) {               // asynchronous: in flight while the products load
     cp_async_elem(Wt + i, wg + i);
     cp_async_elem(Et + i, eg + i);
@@ -805,17 +878,18 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       PR[t * P + i] = p == 0 ? Tr::sign(v[t], i & 1) : v[t];
-      m2[t] = max(m2[t], Tr::key(v[t]));
+      if constexpr (sizeof(T) == 4) m2[t] = max(m2[t], Bits<T>::absbits(v[t]));
     }
   }
-  Tr::template scale<2>(PR, P, 2, m2, red, scl);
-  for (int nn = tid; nn < P; nn += bd) RB[nn] = Tr::load(PR, P, 0, makhoul_src(nn, P), scl);
+  scale_rows<T, 2>(PR, P, m2, red, scl);
+  for_elems<T>(P, [&](int nn) { RB[nn] = Tr::load(PR, P, 0, makhoul_src(nn, P), scl); });
   cp_async_all_done();
   __syncthreads();
-  C* Z = fft_rows<T, false>(RB, RA, 1, a.st, Wt);
+  C* Z = fft_rows<T, false, false>(RB, RA, 1, a.st, Wt);
   const int N = M * nr;
   double* o = a.out4 + (size_t)b * a.out_stride;
   const T two_P = (T)2 / (T)P, one_P = (T)1 / (T)P;
+#pragma unroll 1
   for (int s = tid; s < M; s += bd) {
     T ya = 0, yb = 0;
     bool zero;
@@ -828,7 +902,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
       k = s;
     }
     if (!zero) {
-      Tr::template unpack<2>(Z, P, k, 0, Et, scl, (p == 1 && k == 0) ? one_P : two_P, ya, yb);
+      Tr::unpack(Z, P, k, 0, 2, Et, scl, (p == 1 && k == 0) ? one_P : two_P, ya, yb);
     }
     const size_t q0 = (size_t)(2 * p) * N + (size_t)s * nr + n;
     o[q0] = (double)ya;
@@ -936,6 +1010,53 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
     R[o] = nxp + (Om + dtPr * grv);
     R[N + o] = nxt + (rsq * Tv[k] - dt * psiT0);
     R[2 * N + o] = nxs + (rsq * Sv[k] - dt * psiT0);
+  }
+}
+
+// The linear parts alone (fuse_rhs with the fused row kernel; k_fx_grid forms the same expressions in the split
+// path), with A2_SINE's D2 psi formed by k_fx_deriv.  One CTA per (row, shell).  Bound by the FP64 pipe (about 20
+// operations an element) and its column-strided loads: 39 us at 64 shells of 256 x 30, 76 us as k_rhs with D2 psi.
+__global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double* d2psi, size_t d2_stride) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int M = a.M, nr = a.nr;
+  const int n = blockIdx.x, b = blockIdx.y;
+  if (a.active && !a.active[b]) return;
+  const int tid = threadIdx.x, bd = blockDim.x;
+  double* pv = reinterpret_cast<double*>(smem_raw);
+  double* Sc = pv + M;
+  double* D2p = Sc + M;
+  double* Tv = D2p + M;
+  double* Sv = Tv + M;
+  const size_t N = (size_t)M * nr;
+  const double* Xs = a.X + (size_t)b * a.x_stride;
+  const double* d2 = d2psi + (size_t)b * d2_stride;
+  for (int k = tid; k < M; k += bd) {
+    const bool psi_on = !(a.sym && (k % 2 == 0));
+    const bool ts_on = !(a.sym && (k % 2 == 1));
+    const size_t o = (size_t)k * nr + n;
+    pv[k] = psi_on ? __ldg(Xs + o) : 0.0;
+    D2p[k] = psi_on ? __ldg(d2 + o) : 0.0;
+    Tv[k] = ts_on ? __ldg(Xs + N + o) : 0.0;
+    Sv[k] = ts_on ? __ldg(Xs + 2 * N + o) : 0.0;
+  }
+  const double dt = a.dt, dtPr = a.dt * a.Pr;
+  const double Ra = a.Ra[b], Ras = a.Ra_s[b];
+  const double ir2 = a.ir2s[n], rsq = a.rsq[n], dT0 = a.dT0[n], gr = a.gr[n];
+  __syncthreads();
+  parity_suffix<double>(pv, Sc, M);
+  double* R = a.rhs + (size_t)b * a.rhs_stride;
+  for (int k = tid; k < M; k += bd) {
+    const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;
+    const double k1 = fx_int(k + 1), k2 = fx_int(k + 2);
+    const double JP = (k == 0) ? 1.0 * s1 : k1 * pv[k - 1] + 2.0 * s1;    // J_theta_RT
+    const double s2 = (k + 2 < M) ? Sc[k + 2] : 0.0;
+    const double Om = D2p[k] - k1 * ir2 * (k2 * pv[k] + 2.0 * s2);       // A2_SINE
+    const double grv = (k < M - 1) ? (-k1 * gr) * (Ra * Tv[k + 1] - Ras * Sv[k + 1]) : 0.0;
+    const double psiT0 = dT0 * JP;                                              // DT0_theta
+    const size_t o = (size_t)k * nr + n;
+    R[o] = Om + dtPr * grv;
+    R[N + o] = rsq * Tv[k] - dt * psiT0;
+    R[2 * N + o] = rsq * Sv[k] - dt * psiT0;
   }
 }
 
@@ -1107,6 +1228,7 @@ __global__ void __launch_bounds__(kFxThreads) k_transform(TrArgs a) {
   double* scl = reinterpret_cast<double*>(Et + L);   // the rows' exponents
   void* red = scl + 8;                               // 4*32 reduction words of 8 bytes
   const int tid = threadIdx.x, bd = blockDim.x;
+#pragma unroll 1
   for (int i = tid; i < L; i += bd) {
     Wt[i] = a.w[i];
     Et[i] = a.e[i];
@@ -1118,12 +1240,11 @@ __global__ void __launch_bounds__(kFxThreads) k_transform(TrArgs a) {
   // the rows as they enter the transforms (DCT3: x_k, a sine row by its mirrored wavenumbers; DCT2: f_i with
   // the alternating sign of a sine row), in RB, free until the FFT
   double* XV = reinterpret_cast<double*>(RB);
-  unsigned mx[kRows];
-#pragma unroll
+#pragma unroll 1
   for (int t = 0; t < kRows; ++t) {
-    mx[t] = 0;
     const int r = r0 + t;
     const double* src = a.in + (size_t)r * n_in;
+#pragma unroll 1
     for (int k = tid; k < L; k += bd) {
       double v = 0.0;
       if (r < a.rows) {
@@ -1133,33 +1254,36 @@ __global__ void __launch_bounds__(kFxThreads) k_transform(TrArgs a) {
         else v = (L - k <= n_in - 1) ? src[L - k] : 0.0;
       }
       XV[t * L + k] = v;
-      mx[t] = max(mx[t], abs_hi(v));
     }
   }
-  rows_to_fixed<kRows>(XV, L, kRows, mx, reinterpret_cast<unsigned*>(red), reinterpret_cast<int*>(scl));
+  rows_to_fixed(XV, L, kRows, red, reinterpret_cast<int*>(scl));
   if (inverse) {
+#pragma unroll 1
     for (int idx = tid; idx < kTrPairs * L; idx += bd) {
       const int p = idx / L;
-      RA[idx] = Tr::template pack<kRows>(XV, L, 2 * p, true, idx - p * L, Et, scl);
+      RA[idx] = Tr::pack(XV, L, 2 * p, true, idx - p * L, Et, scl);
     }
     __syncthreads();
-    C* res = fft_rows<double, true>(RA, RB, kTrPairs, a.st, Wt);
+    C* res = fft_rows<double, false>(RA, RB, kTrPairs, a.st, Wt);
+#pragma unroll 1
     for (int idx = tid; idx < kRows * L; idx += bd) {
       const int t = idx / L;
       const int i = idx - t * L;
       const int r = r0 + t;
       if (r >= a.rows) continue;
       const int src = (i & 1) ? (L - 1 - (i >> 1)) : (i >> 1);
-      const double val = Tr::template out<kRows>(res[(t >> 1) * L + src], t & 1, t & ~1, scl);
+      const double val = Tr::out(res[(t >> 1) * L + src], t & 1, t & ~1, kRows, scl);
       a.out[(size_t)r * n_out + i] = neg_if(val, sine && (i & 1));
     }
   } else {
+#pragma unroll 1
     for (int idx = tid; idx < kTrPairs * L; idx += bd) {
       const int p = idx / L;
       RA[idx] = Tr::load(XV, L, 2 * p, makhoul_src(idx - p * L, L), scl);
     }
     __syncthreads();
     C* Z = fft_rows<double, false>(RA, RB, kTrPairs, a.st, Wt);
+#pragma unroll 1
     for (int idx = tid; idx < kTrPairs * n_out; idx += bd) {
       const int p = idx / n_out;
       const int s = idx - p * n_out;
@@ -1167,7 +1291,7 @@ __global__ void __launch_bounds__(kFxThreads) k_transform(TrArgs a) {
       double ya = 0.0, yb = 0.0;
       if (!(sine && s == 0)) {
         const int k = sine ? L - s : s;
-        Tr::template unpack<kRows>(Z + p * L, L, k, 2 * p, Et, scl, (!sine && k == 0) ? 1.0 / L : 2.0 / L, ya, yb);
+        Tr::unpack(Z + p * L, L, k, 2 * p, kRows, Et, scl, (!sine && k == 0) ? 1.0 / L : 2.0 / L, ya, yb);
       }
       if (r < a.rows) a.out[(size_t)r * n_out + s] = ya;
       if (r + 1 < a.rows) a.out[(size_t)(r + 1) * n_out + s] = yb;
@@ -1203,6 +1327,16 @@ __global__ void __launch_bounds__(kFxThreads) k_fx_finish(FinishArgs a) {
     F[N + o] = O4[2 * N + o];
     F[2 * N + o] = O4[3 * N + o];
   }
+}
+
+static int fx_sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 1;
+  }();
+  return sms;
 }
 
 // ---- launchers ---------------------------------------------------------------------------------
@@ -1248,12 +1382,41 @@ size_t fx_rows_max_dynamic_smem(int prec) {
   return (size_t)optin > stat ? (size_t)optin - stat : 0;
 }
 
+// k_fx_deriv where it has something to do: FP64 contractions, FP32 ones of the split path that are not on the
+// tensor cores, the fused right-hand side's D2 psi, a pending correction.  Modes per CTA: with nr > 32 (one CTA an
+// SM: 130 KB of operators) as many as make one wave, up to 8 (540 x 65: 37 us with 4, 64 us with 1); otherwise two
+// (a pending correction takes two at once), and more as the batch grows, the operators loaded once for them.
+template <typename T>
+static cudaError_t launch_deriv(const FxArgs& a, int batch, bool split, cudaStream_t s) {
+  const bool f32 = sizeof(T) == 4 && split && !a.deriv_t;
+  if (sizeof(T) == 4 && !f32 && !a.fuse_rhs && !a.fix.on) return cudaSuccess;
+  using Deriv = void (*)(FxArgs, T*, size_t, int, int);
+  static const Deriv derivs[6] = {k_fx_deriv<T, 8>,  k_fx_deriv<T, 16>, k_fx_deriv<T, 24>,
+                                  k_fx_deriv<T, 32>, k_fx_deriv<T, 48>, k_fx_deriv<T, 64>};
+  static unsigned long long done[6] = {};
+  const int ldi = a.nr <= 32 ? (a.nr - 1) / 8 : (a.nr <= 48 ? 4 : 5);   // fx_ld(nr)
+  cudaError_t e;
+  if ((e = ensure_smem_attr(derivs[ldi], &done[ldi])) != cudaSuccess) return e;
+  const bool d2s = a.fuse_rhs != 0;
+  int km = 2;
+  if (a.nr > 32)
+    km = min(8, max(1, (int)(((long)a.M * batch + fx_sm_count() - 1) / fx_sm_count())));
+  else if (!a.fix.on)
+    while (km < 16 && (long)a.M * batch >= 8l * km * fx_sm_count()) km *= 2;
+  e = launch_kernel(derivs[ldi], dim3((a.M + km - 1) / km, batch), dim3(32 * deriv_warps(fx_ld(a.nr))),
+                    fx_deriv_smem_bytes<T>(a.nr, d2s, a.fix.on != 0, km, f32), s, a, reinterpret_cast<T*>(a.deriv),
+                    a.deriv_stride, km, f32 ? 1 : 0);
+  ktimer_mark(SDD_K_FX_DERIV, s);
+  return e;
+}
+
 template <typename T, int MODE>
 static cudaError_t launch_fx_t(const FxArgs& a, int batch, cudaStream_t s) {
   const size_t smem = fx_smem_bytes(a.M, a.P, sizeof(T) == 4 ? SDD_PREC_MIXED : SDD_PREC_FP64);
   static unsigned long long done = 0;
   cudaError_t e = ensure_smem_attr(k_fx_rows<T, MODE>, &done);
   if (e != cudaSuccess) return e;
+  if (a.deriv && (e = launch_deriv<T>(a, batch, false, s)) != cudaSuccess) return e;
   if (sizeof(T) == 4 && a.deriv_t && (e = launch_tc_for(a, batch, s)) != cudaSuccess) return e;
   e = launch_kernel(k_fx_rows<T, MODE>, dim3(a.nr, batch), dim3(kFxRowThreads), smem, s, a);
   ktimer_mark(SDD_K_FX_ROWS, s);
@@ -1267,26 +1430,9 @@ static cudaError_t launch_fx_split_t(const FxArgs& a, int batch, cudaStream_t s)
   T* grid = reinterpret_cast<T*>((MODE != 1 && a.base) ? a.base : a.grid);
   const size_t gs = (MODE != 1 && a.base) ? a.base_stride : a.grid_stride;
   cudaError_t e;
-  using Deriv = void (*)(FxArgs, T*, size_t);
-  static const Deriv derivs[6] = {k_fx_deriv<T, 8>,  k_fx_deriv<T, 16>, k_fx_deriv<T, 24>,
-                                  k_fx_deriv<T, 32>, k_fx_deriv<T, 48>, k_fx_deriv<T, 64>};
-  const int ldi = a.nr <= 32 ? (a.nr - 1) / 8 : (a.nr <= 48 ? 4 : 5);   // fx_ld(nr)
-  const Deriv deriv = derivs[ldi];
-  {
-    static unsigned long long done[6] = {};   // large nr with a pending correction can pass 48 KB
-    if ((e = ensure_smem_attr(deriv, &done[ldi])) != cudaSuccess) return e;
-  }
-  // with tensor cores the per-mode kernel only applies a pending chain correction and forms the fused
-  // right-hand side's FP64 block; the contractions follow on the corrected state
-  const bool tc = sizeof(T) == 4 && a.deriv_t;
-  if (!tc || a.fix.on || a.fuse_rhs) {
-    e = launch_kernel(deriv, dim3(a.M, batch), dim3(256),
-                      fx_deriv_smem_bytes(a.nr, prec, a.fix.on != 0, a.fuse_rhs != 0, a.fix.nch), s, a,
-                      reinterpret_cast<T*>(a.deriv), a.deriv_stride);
-    ktimer_mark(SDD_K_FX_DERIV, s);
-    if (e != cudaSuccess) return e;
-  }
-  if (tc && (e = launch_tc_for(a, batch, s)) != cudaSuccess) return e;
+  if ((e = launch_deriv<T>(a, batch, true, s)) != cudaSuccess) return e;
+  // (the tensor cores' contractions follow on the corrected state)
+  if (sizeof(T) == 4 && a.deriv_t && (e = launch_tc_for(a, batch, s)) != cudaSuccess) return e;
   {
     static unsigned long long done = 0;
     if ((e = ensure_smem_attr(k_fx_grid<T>, &done)) != cudaSuccess) return e;
@@ -1302,16 +1448,6 @@ static cudaError_t launch_fx_split_t(const FxArgs& a, int batch, cudaStream_t s)
                  a, (const T*)grid, gs);
   ktimer_mark(SDD_K_FX_PROD, s);
   return e;
-}
-
-static int fx_sm_count() {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 1;
-  }();
-  return sms;
 }
 
 // The split path is taken when forced (split = 2) or, automatically, while the fused kernel would leave
@@ -1373,6 +1509,13 @@ cudaError_t launch_rhs(const RhsArgs& a, int batch, cudaStream_t s) {
   ktimer_mark(SDD_K_RHS, s);
   if (er != cudaSuccess) return er;
   return cudaGetLastError();
+}
+
+cudaError_t launch_rhs_lin(const RhsArgs& a, const double* d2psi, size_t d2_stride, int batch, cudaStream_t s) {
+  const cudaError_t e = launch_kernel(k_rhs_lin, dim3(a.nr, batch), dim3(kFxThreads), 5 * (size_t)a.M * sizeof(double), s,
+                                      a, d2psi, d2_stride);
+  ktimer_mark(SDD_K_RHS, s);
+  return e;
 }
 
 cudaError_t launch_theta_op(int op, int M, int nr, int sym, const double* D2, const double* ir,

@@ -137,6 +137,8 @@ struct FxOps {               // FP64 or FP32 copies of the operators the nonline
   const void* Dr;            // nr*nr
   const void* D2r2;          // nr*nr
   const void* ir4r2;         // nr
+  const i64* fxDr;           // Dr as a two-digit block, D^2/r^2 and A2_SINE's D2 as three-digit blocks
+  const int* wx[2];          // (sdd_fixed.cuh)
   const void* w;             // FFT twiddles (P): FP32 complex, or fixed-point digits (FP64)
   const void* e;             // DCT twiddles (P), the same
 };
@@ -213,9 +215,10 @@ struct FxArgs {
   void* deriv;               // split path: radial derivatives [shell][5][M][nr] (T): Dr psi, D2r2 psi, Dr T, Dr S
                              // (and, with fuse_rhs, D2s psi in FP64 as the fifth block)
   size_t deriv_stride;       // elements between shells in deriv
-  // fuse_rhs (FP64 split path): k_fx_grid writes the linear parts of the three right-hand sides into
-  // rl.rhs (the terms of k_rhs that do not involve the nonlinear term); the chains' h kernel adds the
-  // nonlinear parts from out4.  rl carries the operators, parameters and the rhs buffer.
+  // fuse_rhs: the right-hand sides' linear parts (the terms of k_rhs that do not involve the nonlinear term)
+  // are written into rl.rhs, by k_fx_grid (split path) or k_rhs_lin; the chains' h kernel adds the nonlinear
+  // parts from out4.  rl carries the operators, parameters and the rhs buffer; deriv's fifth block the FP64
+  // D2 psi that they need.
   int fuse_rhs;
   RhsArgs rl;
   FixArgs fix;               // split path: a pending correction of X (see FixArgs)
@@ -285,8 +288,9 @@ struct ChainArgs {
   const double* lin;         // [shell][3][M][nr] linear parts (k_fx_grid), stride g_stride
   const double* out4;        // [shell][4][M][nr]
   size_t out_stride;
-  const double* Dr;          // nr*nr (FP64)
+  const int* wxDr;           // Dr as a three-digit block (sdd_fixed.cuh)
   const float* q32, *Dr32;   // mixed plans: Dr Q in FP32 (see RhsArgs)
+  int split_fx;              // the nonlinear term runs split over CTAs (one small batch): resolve_chain_layout
   double dt;                 // the step's dt
   // chunked (parallel-in-modes) chains, layout 2: every chain of S = N_fm/2 steps is cut into nch chunks
   // of kc steps.  Chunk c runs from a zero carried state (f_local, end state d_c); the carried states
@@ -350,12 +354,15 @@ size_t fx_rows_max_dynamic_smem(int prec);
 // reserved
 bool fx_split_rule(int split, int nr, int batch);
 cudaError_t launch_rhs(const RhsArgs& a, int batch, cudaStream_t s);
+// the linear parts alone, with D2 psi formed ([shell][M][nr], stride d2_stride)
+cudaError_t launch_rhs_lin(const RhsArgs& a, const double* d2psi, size_t d2_stride, int batch, cudaStream_t s);
 cudaError_t launch_chain(const ChainArgs& a, int batch, int nfields, cudaStream_t s);
 // the chain layout launch_chain runs for a.layout (0 = automatic) and this launch size
 int resolve_chain_layout(const ChainArgs& a, int batch, int nfields);
 // fixed-point blocks from FP64 matrices on the device (setup)
 cudaError_t launch_to_fixed(const double* src, size_t src_stride, int ld, int nrows, int r0, int c0, int nr, int ldl,
                             i64* out, size_t out_stride, int nblk, cudaStream_t s);
+cudaError_t launch_to_wide(const double* src, int nr, int ld, int* out, cudaStream_t s);
 cudaError_t launch_chunk_fix(const ChainArgs& a, int batch, int nfields, cudaStream_t s);
 cudaError_t launch_theta_op(int op, int M, int nr, int sym, const double* D2, const double* ir,
                             const double* dT0, const double* g, double* f, int batch,

@@ -165,3 +165,53 @@ def test_non_finite_operands_follow_fp64(cuda, N_r, layout):
             assert not np.isfinite(y[touched]).any()
             if layout == 1:
                 assert np.array_equal(y[20], ref[20], equal_nan=True)
+
+
+# ---- radial contractions and the whole step --------------------------------------------------------
+
+
+def _oracle_ld():
+    """The oracle's functions in extended precision: its source with every array of type float one of long
+    doubles."""
+    import types
+    from oracle import sdd_oracle as O
+    with open(O.__file__) as f:
+        src = f.read()
+    m = types.ModuleType("sdd_oracle_ld")
+    m.__dict__["__file__"] = O.__file__
+    exec(compile(src.replace("dtype=float", "dtype=np.longdouble"), O.__file__, "exec"), m.__dict__)
+    m.Vecs_to_X = lambda psi, t, c, M, nr, sym: np.concatenate([a.T.ravel() for a in (psi, t, c)])   # (sym off)
+    return m
+
+
+@pytest.mark.parametrize("nr", [1, 7, 8, 9, 16, 17, 24, 25, 31, 32, 33, 48, 49, 64])
+def test_steps_are_no_less_exact_than_fp64(cuda, nr):
+    """The nonlinear term and whole steps (radial derivatives, linear terms, chains) at the edges of the padded
+    block sizes, on a smooth state and on one that is not smooth at the walls, against the oracle in extended
+    precision: each field at most twice the error of the FP64 oracle (two samples of rounding noise) plus four
+    roundings of the result; in the two launch forms of the nonlinear term."""
+    from oracle import sdd_oracle as O
+    from spectraldoublediffusiveconvection_gb300.plan import Plan
+    M, dt, N = 24, 1e-3, 24 * nr
+    Q = _oracle_ld()
+    ops, opl = O.Operators(M, nr + 1, 2.0, dt, 1.0, 0.01), O.Operators(M, nr + 1, 2.0, dt, 1.0, 0.01)
+    for k in ("D", "R", "Dr", "rsq", "gr", "DT0", "Linv_A4", "Linv_T", "Linv_S", "D2_A4", "IR2_A4", "IR4_A4"):
+        setattr(opl, k, getattr(ops, k).astype(LD))
+    p = Plan(M, nr + 1, 2.0, dt, 1.0, 0.01)
+    s = np.sin(np.pi * np.arange(1, nr + 1) / (nr + 1)) ** 4
+    X = O.seeded_state(M, nr, nr)
+    for X in (X, (X.reshape(3, M, nr) * s).ravel()):
+        Xd = cuda.from_numpy(X).cuda().reshape(1, -1)
+        XL = X.astype(LD)
+        want = ((p.nlin_fx, Q.NLIN_FX(XL, opl.D, opl.R, M, nr, False), O.NLIN_FX(X, ops.D, ops.R, M, nr, False)),
+                (lambda x: p.step(x, 8000.0, 500.0), Q.step(opl, XL, 8000.0, 500.0, False),
+                 O.step(ops, X, 8000.0, 500.0, False)))
+        for split in (1, 2):
+            p.set_fx_split(split)
+            for fn, ref, o in want:
+                y = fn(Xd).cpu().numpy().ravel()
+                for f in range(3):
+                    r = ref[f * N:(f + 1) * N]
+                    n = float(np.linalg.norm(r.astype(float)))
+                    e = [float(np.linalg.norm((v[f * N:(f + 1) * N] - r).astype(float))) for v in (y, o)]
+                    assert e[0] <= 2 * e[1] + 4 * 2.0 ** -53 * n, (split, f, e, n)
