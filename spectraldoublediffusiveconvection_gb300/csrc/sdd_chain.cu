@@ -764,8 +764,16 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
     layout = 5;
   // layouts 10 / 11 (chunks in the reference's order) need an FP64 right-hand side (full or fused): else 2 / 3
   if ((layout == 10 || layout == 11) && a.g32) layout -= 8;
-  if (layout == 0 && c3.nch > 1 && c3.GA4 && 2 * nfields * batch * c3.nch <= 2 * sms) layout = 3;
-  if (layout == 0 && c2.nch > 1 && c2.GA4 && 2 * nfields * batch * c2.nch <= 2 * sms) layout = 2;
+  // Chunks shorten the chains' critical path and add a correction matvec per mode (nr > 32: two, or their columns
+  // in halves), so what decides is the batch.  Parallel carry while its chunks and products fit the chip (us a
+  // step, parallel / sequential carry: 256 x 30, 4 shells 77 / 82, 8: 128 / 123; 64 x 20, 8 shells 44 / 48; 192 x 36,
+  // 2 shells 68 / 78, 4: 100 / 90); sequential carry against whole chains: 256 x 30, 8 shells 123 / 206, 32: 343 /
+  // 384, 64: 605 / 608; 64 x 20, 32 shells 114 / 119, 64: 195 / 192; 192 x 36, 8 shells 137 / 174, 16: 203 / 206, 32:
+  // 361 / 278; 540 x 65, 8 shells 610 / 752, 16: 1072 / 1077.  Short chains gain nothing (16 x 8: 27.0 parallel, 25.9
+  // whole; 24 x 20, 24 shells 69 sequential, 67 whole).
+  const bool wide = a.nr > 32;
+  if (layout == 0 && a.M > 16 && c3.nch > 1 && c3.GA4 && 4 * nfields * batch * c3.nch <= (wide ? 3 : 7) * sms) layout = 3;
+  if (layout == 0 && a.M >= 40 && c2.nch > 1 && c2.GA4 && (wide ? 4 : 1) * nfields * batch <= sms) layout = 2;
   // chosen chunks run in the reference's order where the full FP64 right-hand side is there (no pre-pass)
   if (a.layout == 0 && (layout == 2 || layout == 3) && !a.split_fx && !a.g32) layout += 8;
   // layouts 6 / 7 need the full right-hand side in FP64: with the fused or the FP32 one, the pre-pass form
@@ -773,8 +781,7 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   if ((layout == 6 || layout == 7) && layout_bytes(6, a.M, a.nr, a.ldl) > (size_t)optin) layout = 2;
   if (layout != 2 && layout != 3 && layout < 6 && layout_bytes(4, a.M, a.nr, a.ldl) > (size_t)optin)
     layout = 2;   // whole chain too long for shared memory
-  // a launch that fills the SMs: the reference-order chains (4 nr^2 multiply-adds per mode instead of 7), a
-  // step's three chains per CTA where they fit (64 shells N_r=30 N_theta=256: 287 us against 301 us)
+  // a launch that fills the SMs (one kernel; the number as in layout_bytes)
   if (layout == 0) {
     if (2 * nfields * batch <= sms) layout = 4;
     else if (a.split_fx || a.g32) layout = 5;

@@ -215,3 +215,24 @@ def test_steps_are_no_less_exact_than_fp64(cuda, nr):
                     n = float(np.linalg.norm(r.astype(float)))
                     e = [float(np.linalg.norm((v[f * N:(f + 1) * N] - r).astype(float))) for v in (y, o)]
                     assert e[0] <= 2 * e[1] + 4 * 2.0 ** -53 * n, (split, f, e, n)
+
+
+@pytest.mark.parametrize("N_fm,N_r,batch,layouts", [(16, 8, 1, (4,)), (40, 20, 40, (10,)), (64, 24, 8, (3, 11)),
+                                                    (64, 24, 32, (10,)), (64, 40, 12, (10,)), (64, 40, 13, (4,)),
+                                                    (24, 20, 24, (4,))])
+def test_batches_take_the_faster_chains(cuda, N_fm, N_r, batch, layouts):
+    """The automatic layout on both sides of its lines (on 152 SMs), and the same steps as whole chains: the
+    layouts differ in the order of FP64 sums of a few terms per mode, far below the 1e-12 that any layout keeps to
+    the oracle."""
+    from oracle import sdd_oracle as O
+    from spectraldoublediffusiveconvection_gb300.plan import Plan
+    if cuda.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the lines are in units of SMs")
+    p = Plan(N_fm, N_r, 2.0, 5e-4, 1.0, 0.01)
+    X = cuda.from_numpy(np.stack([O.seeded_state(N_fm, N_r - 1, k) for k in range(batch)])).cuda()
+    assert p.chain_choice(batch)[0] in layouts
+    y = p.step(X, 8000.0, 500.0, nsteps=3)
+    p.set_chain_layout(1)
+    z = p.step(X, 8000.0, 500.0, nsteps=3)
+    for k in range(batch):
+        assert float((y[k] - z[k]).norm() / z[k].norm()) <= 1e-12
