@@ -1576,6 +1576,14 @@ static int gmres_solve(sdd_plan* p, const MatVec& A, const MvSpec& spec, const d
     return basis32 ? krylov_scale(src, G.inv, V32 + (size_t)col * vs, nu, ld, B, s, p->kv_v32, p->kv_vin)
                    : krylov_scale(src, G.inv, p->kv_V + (size_t)col * vs, nu, ld, B, s, p->kv_v32, p->kv_vin);
   };
+  const bool one_launch = krylov_orth_takes(nu, basis32);
+  auto orth = [&](int j, int* flags) {
+    const size_t next = (size_t)(j + 1) * vs;
+    return basis32 ? krylov_orth(V32, vs, p->kv_w, nu, ld, j, B, G, p->reorth_eta, j + 1 < m ? V32 + next : nullptr,
+                                 p->kv_v32, p->kv_vin, flags, s)
+                   : krylov_orth(p->kv_V, vs, p->kv_w, nu, ld, j, B, G, p->reorth_eta,
+                                 j + 1 < m ? p->kv_V + next : nullptr, p->kv_v32, p->kv_vin, flags, s);
+  };
   int st;
   resid.assign(B, 0.0);
   SDD_CUDA(cudaMemcpyAsync(G.target, target.data(), B * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -1597,19 +1605,23 @@ static int gmres_solve(sdd_plan* p, const MatVec& A, const MvSpec& spec, const d
       // kv_vin (and kv_v32 in FP32) hold V_j: a fixed address, so one captured graph serves every column
       if ((st = run_mv(p, A, spec, B, p->kv_vin, p->kv_w, G.active, p->kv_v32, s))) return st;
       ++*matvecs;
-      // shells whose Arnoldi process has stopped skip the Gram-Schmidt work (krylov_arnoldi_finish ignores them);
-      // each pass is two launches: the projections, then the update with the new norm (and after the first
-      // pass the flag of the shells that repeat it: those whose first pass cancelled w below reorth_eta of
-      // its norm; the others get zero second projections)
-      SDD_CUDA(dots(G.hcol, j + 1, G.active));
-      SDD_CUDA(sub_norm(G.hcol, j + 1, G.active, &G, j));
-      SDD_CUDA(dots(G.h2, j + 1, G.reo));
-      SDD_CUDA(sub_norm(G.h2, j + 1, G.reo, nullptr, j));
-      SDD_CUDA(krylov_arnoldi_finish(G, p->kv_nrm2, j, B, s));
-      if (j + 1 < m) SDD_CUDA(to_basis(p->kv_w, j + 1));
       // the flags after column j go to slot j; the host reads those of column j - kFlagLag
       const int slot = j % (kFlagLag + 1);
-      SDD_CUDA(cudaMemcpyAsync(p->h_int + (size_t)slot * B, G.active, B * sizeof(int), cudaMemcpyDeviceToHost, s));
+      // shells whose Arnoldi process has stopped skip the Gram-Schmidt work (krylov_arnoldi_finish ignores them);
+      // short vectors take one launch, otherwise each pass is two: the projections, then the update with the new
+      // norm (and after the first pass the flag of the shells that repeat it: those whose first pass cancelled w
+      // below reorth_eta of its norm; the others get zero second projections)
+      if (one_launch) {
+        SDD_CUDA(orth(j, p->h_int + (size_t)slot * B));   // (pinned: the kernel leaves the flags there itself)
+      } else {
+        SDD_CUDA(dots(G.hcol, j + 1, G.active));
+        SDD_CUDA(sub_norm(G.hcol, j + 1, G.active, &G, j));
+        SDD_CUDA(dots(G.h2, j + 1, G.reo));
+        SDD_CUDA(sub_norm(G.h2, j + 1, G.reo, nullptr, j));
+        SDD_CUDA(krylov_arnoldi_finish(G, p->kv_nrm2, j, B, s));
+        if (j + 1 < m) SDD_CUDA(to_basis(p->kv_w, j + 1));
+        SDD_CUDA(cudaMemcpyAsync(p->h_int + (size_t)slot * B, G.active, B * sizeof(int), cudaMemcpyDeviceToHost, s));
+      }
       SDD_CUDA(cudaEventRecord(p->flag_ev[slot], s));
       if (j >= kFlagLag) {
         const int old = (j - kFlagLag) % (kFlagLag + 1);

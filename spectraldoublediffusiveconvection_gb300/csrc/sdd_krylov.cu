@@ -16,10 +16,14 @@
 // solves whose tolerance (relative 1e-4 in Newton) is far above FP32 rounding: the outer residual is FP64,
 // so the converged state is unchanged in accuracy.  The FP64 products are bound by the FP64 multiply-add
 // rate (one per element of V), the FP32 ones by the bytes of V, half as many.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
+#include "sdd_fixed.cuh"
+#include "sdd_internal.cuh"
 #include "sdd_krylov.cuh"
 
 namespace sdd {
@@ -132,11 +136,15 @@ __global__ void __launch_bounds__(kDotThreads) k_dot_partials(const VT* __restri
         sp[u] = (VT)0;
         if (i0 + u < ie) {
           const VT* vb = V + (size_t)(i0 + u) * vstride_i + (size_t)b * ld;
+          VT x[kDotPer];                               // (all loads in flight before the first multiply-add)
 #pragma unroll
           for (int k = 0; k < kDotPer; ++k) {
             const int e = e0 + threadIdx.x + k * kDotThreads;
-            if (e < n) sp[u] = fma(vb[e], wr[k], sp[u]);
+            x[k] = e < n ? vb[e] : (VT)0;
           }
+#pragma unroll
+          for (int k = 0; k < kDotPer; ++k)
+            if (e0 + k * kDotThreads + (int)threadIdx.x < n) sp[u] = fma(x[k], wr[k], sp[u]);
         }
       }
       static_assert(kDotVecs == 4, "warp_sum4 reduces four vectors");
@@ -340,80 +348,331 @@ __global__ void k_cycle_start(GmresState s, const double* __restrict__ nrm2, int
   s.resid[b] = beta;
 }
 
+// One warp: column col[0 .. j] through the previous rotations (csv, snv) into out[0 .. j - 1]; returns the entry a of
+// row j that the new rotation takes.  a_{i+1} = -sn_i a_i + cs_i col_{i+1} is a linear recurrence, scanned 32 rows at
+// a time (each step of a serial chain would hold the SM sub-partition for four FP64 instructions of 64 cycles).
+__device__ __forceinline__ double rotate_rows(const double* col, const double* csv, const double* snv, int j, int lane,
+                                              double* out) {
+  double a0 = col[0];
+  for (int i0 = 0; i0 < j; i0 += 32) {
+    const int i = i0 + lane;
+    const bool ok = i < j;
+    const double c = ok ? csv[i] : 0.0, s = ok ? snv[i] : 0.0, x = ok ? col[i + 1] : 0.0;
+    double mul = ok ? -s : 1.0, add = c * x;           // rows past j: the identity
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double m1 = __shfl_up_sync(0xffffffffu, mul, o), q1 = __shfl_up_sync(0xffffffffu, add, o);
+      if (lane >= o) {
+        add = fma(mul, q1, add);
+        mul *= m1;
+      }
+    }
+    const double an = fma(mul, a0, add);               // a_{i+1}
+    double ai = __shfl_up_sync(0xffffffffu, an, 1);
+    if (lane == 0) ai = a0;
+    if (ok) out[i] = fma(c, ai, s * x);
+    a0 = __shfl_sync(0xffffffffu, an, 31);
+  }
+  return a0;
+}
+
+// One warp: the new rotation of column j from a and |w|^2, and whether the shell goes on.  The square roots and
+// the divisions run in lanes side by side.
+struct ArnoldiColumn {
+  double cj, sj, r, gj, res, inv;
+  int act;
+};
+__device__ __forceinline__ ArnoldiColumn new_rotation(double a, double nrm2, double gj, double beta, double target, int j,
+                                                      int m, int lane) {
+  ArnoldiColumn o;
+  const double root = sqrt(lane == 0 ? nrm2 : fma(a, a, nrm2));
+  const double hnext = __shfl_sync(0xffffffffu, root, 0);
+  o.r = __shfl_sync(0xffffffffu, root, 1);
+  const double q = (lane == 0 ? a : (lane == 1 ? hnext : 1.0)) / (lane < 2 ? o.r : hnext);
+  o.cj = __shfl_sync(0xffffffffu, q, 0);
+  o.sj = __shfl_sync(0xffffffffu, q, 1);
+  o.inv = __shfl_sync(0xffffffffu, q, 2);
+  if (!(o.r > 0.0)) {
+    o.cj = 1.0;
+    o.sj = 0.0;
+  }
+  o.gj = gj;
+  o.res = fabs(-o.sj * gj);
+  const bool breakdown = !(hnext > 1e-300 * beta);
+  o.act = !(o.res <= target || breakdown || j + 1 == m);
+  if (!o.act || !(hnext > 0.0)) o.inv = 0.0;
+  return o;
+}
+__device__ __forceinline__ void store_column(const GmresState& s, int b, int j, const ArnoldiColumn& o) {
+  const int m = s.m;
+  double* H = s.H + (size_t)b * (m + 1) * m;
+  double* g = s.g + (size_t)b * (m + 1);
+  s.cs[(size_t)b * m + j] = o.cj;
+  s.sn[(size_t)b * m + j] = o.sj;
+  H[j * m + j] = o.r;
+  H[(j + 1) * m + j] = 0.0;
+  g[j + 1] = -o.sj * o.gj;
+  g[j] = o.cj * o.gj;
+  s.resid[b] = o.res;
+  s.kb[b] = j + 1;
+  s.active[b] = o.act;
+  s.inv[b] = o.inv;
+}
+
 // After Gram-Schmidt for column j: hcol + h2 [b][0..j] hold the projections, nrm2[b] = ||w||^2.  Stores the
 // column in H, applies the previous Givens rotations, makes the new one, updates g and the residual estimate.
 __global__ void __launch_bounds__(32) k_arnoldi_finish(GmresState s, const double* __restrict__ nrm2, int j,
                                                         int B) {
-  // one warp per shell: the lanes stage the column (hcol + h2) and the previous rotations in shared memory,
-  // lane 0 applies the rotations (the rotated entry of row i + 1 carried in a register, the only dependent
-  // chain) and makes the new one, the lanes write the column back
-  __shared__ double col[kMaxRestart + 1], csv[kMaxRestart], snv[kMaxRestart];
+  // one warp per shell: the column (hcol + h2) and the previous rotations in shared memory
+  __shared__ double col[kMaxRestart + 1], csv[kMaxRestart], snv[kMaxRestart], out[kMaxRestart];
   const int b = blockIdx.x, lane = threadIdx.x;
   if (b >= B) return;
   const int m = s.m;
-  double* H = s.H + (size_t)b * (m + 1) * m;   // H[row*m + col]
   const double* hc = s.hcol + (size_t)b * (m + 1);
   const double* hd = s.h2 + (size_t)b * (m + 1);
-  double* cs = s.cs + (size_t)b * m;
-  double* sn = s.sn + (size_t)b * m;
-  double* g = s.g + (size_t)b * (m + 1);
   if (!s.active[b]) {
     if (lane == 0) s.inv[b] = 0.0;
     return;
   }
   for (int i = lane; i <= j; i += 32) col[i] = hc[i] + hd[i];
   for (int i = lane; i < j; i += 32) {
-    csv[i] = cs[i];
-    snv[i] = sn[i];
+    csv[i] = s.cs[(size_t)b * m + i];
+    snv[i] = s.sn[(size_t)b * m + i];
   }
+  const double gj = s.g[(size_t)b * (m + 1) + j], beta = s.beta[b], target = s.target[b];
   __syncwarp();
-  if (lane == 0) {
-    const double hnext = sqrt(nrm2[b]);
-    double a = col[0];
-    for (int i = 0; i < j; ++i) {
-      const double c = col[i + 1];
-      col[i] = fma(csv[i], a, snv[i] * c);
-      a = fma(-snv[i], a, csv[i] * c);
-    }
-    const double c = hnext;
-    const double r = hypot(a, c);
-    double cj = 1.0, sj = 0.0;
-    if (r > 0.0) {
-      cj = a / r;
-      sj = c / r;
-    }
-    cs[j] = cj;
-    sn[j] = sj;
-    H[j * m + j] = r;
-    H[(j + 1) * m + j] = 0.0;
-    g[j + 1] = -sj * g[j];
-    g[j] = cj * g[j];
-    const double res = fabs(g[j + 1]);
-    s.resid[b] = res;
-    s.kb[b] = j + 1;
-    const bool breakdown = !(hnext > 1e-300 * s.beta[b]);
-    int act = 1;
-    if (res <= s.target[b] || breakdown || j + 1 == m) act = 0;
-    s.active[b] = act;
-    s.inv[b] = (act && hnext > 0.0) ? 1.0 / hnext : 0.0;
-  }
+  const double a = rotate_rows(col, csv, snv, j, lane, out);
+  const ArnoldiColumn o = new_rotation(a, nrm2[b], gj, beta, target, j, m, lane);
+  if (lane == 0) store_column(s, b, j, o);
   __syncwarp();
-  for (int i = lane; i < j; i += 32) H[i * m + j] = col[i];
+  double* H = s.H + (size_t)b * (m + 1) * m;           // H[row*m + col]
+  for (int i = lane; i < j; i += 32) H[i * m + j] = out[i];
 }
 
-// Back substitution R y = g over the first kb[b] columns.
-__global__ void k_solve_y(GmresState s, int B) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
+template <typename E>
+__device__ __forceinline__ void cp_async_one(E* smem, const E* gmem) {
+  static_assert(sizeof(E) == 4 || sizeof(E) == 8, "element size");
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (sizeof(E) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem));
+}
+
+// Everything of column j after the product in one launch, for short vectors: w = A V_j is orthogonalised against
+// V_0 .. V_j (the second pass where the first cancelled w below eta of its norm), the column of H rotated,
+// V_{j+1} = w / |w| written (out; out2 and out32: its FP64 and FP32 copies).  A cluster of kOrthCtas CTAs per shell,
+// each with a slice of w in shared memory; the partial projections and norms meet in distributed shared memory,
+// every CTA sums them in rank order, so that all of a cluster hold the same column and the same 1 / |w|.
+// As separate launches (two passes of two, the rotations, the scaling) each step pays a launch, a global reduction
+// and a ticket.  This kernel is bound by about 14 dependent FP64 sums and five cluster barriers (11 us), then by its
+// multiply-adds, which run on kOrthCtas SMs a shell only: longer vectors keep the launches.  us a column with its
+// product, launches / one launch: FP64, n = 3648 104 / 67, 7488 114 / 83, 11808 120 / 109, 15744 128 / 132; FP32 basis,
+// 8 shells, n = 4416 113 / 80, 15744 182 / 180.
+// Projections: a warp takes four vectors and (few vectors) a quarter or a half of the slice; FP64 sums, or with an
+// FP32 basis FP32 sums of at most 256 products, as in k_dot_partials.
+// STAGE: the slice's part of V_0 .. V_j waits in shared memory (both passes read it twice), where it fits.
+template <typename VT, bool STAGE>
+__global__ void __launch_bounds__(kDotThreads + 32) k_orth(const VT* __restrict__ V, size_t vstride_i, const double* w, int n,
+                                                     int ld, int j, GmresState s, double eta2, VT* out, float* out32,
+                                                     double* out2, int* flags) {
+  extern __shared__ __align__(16) unsigned char orth_smem[];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ double sw[kOrthSlice];
+  __shared__ double ps[4][kMaxRestart], pd[2][kMaxRestart], pn[2];
+  __shared__ double hcol[kMaxRestart], hrot[kMaxRestart], h[kMaxRestart], csv[kMaxRestart], snv[kMaxRestart];
+  __shared__ VT hv[kMaxRestart];
+  __shared__ double red[kDotThreads / 32], s_nrm, s_h2, s_inv, s_a;
+  const int rank = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nv = j + 1, m = s.m;
+  const int ne = (n + kOrthCtas * 32 - 1) / (kOrthCtas * 32) * 32;   // the slice, at most kOrthSlice
+  const int e0 = rank * ne, cnt = max(0, min(ne, n - e0));
+  const double* wb = w + (size_t)b * ld + e0;
+  const VT* Vg = V + (size_t)b * ld + e0;
+  VT* Vs = reinterpret_cast<VT*>(orth_smem);           // [vector][ne]
+  const VT* Vb = STAGE ? Vs : Vg;
+  const size_t vstr = STAGE ? (size_t)ne : vstride_i;
+  const size_t ob = (size_t)b * ld + e0;
+  const int act = s.active[b];                         // (in flight with the copies below)
+  if (STAGE) {
+    for (int i = warp; i < nv; i += kDotThreads / 32 + 1)
+      for (int e = lane; e < cnt; e += 32) cp_async_one(Vs + (size_t)i * ne + e, Vg + (size_t)i * vstride_i + e);
+    cp_async_commit();
+  }
+  if (!act) {                                          // (the whole cluster) a shell that has stopped
+    cp_async_wait<0>();
+    if (rank == 0 && tid == 0) {
+      s.inv[b] = 0.0;
+      if (flags) flags[b] = 0;
+    }
+    if (out)
+      for (int e = tid; e < cnt; e += blockDim.x) {
+        const double v = wb[e] * 0.0;
+        out[ob + e] = (VT)v;
+        if (out32) out32[ob + e] = (float)v;
+        if (out2) out2[ob + e] = (double)(VT)v;
+      }
+    return;
+  }
+  const bool rot = warp == kDotThreads / 32;           // the last warp only rotates the column
+  for (int e = tid; e < ne; e += blockDim.x) sw[e] = e < cnt ? wb[e] : 0.0;
+  if (tid < j) {                                       // (j < kMaxRestart threads)
+    csv[tid] = s.cs[(size_t)b * m + tid];
+    snv[tid] = s.sn[(size_t)b * m + tid];
+  }
+  const double gj = s.g[(size_t)b * (m + 1) + j], beta = s.beta[b], target = s.target[b];
+  const int ng = (nv + 3) / 4, nseg = ng == 1 ? 4 : (ng == 2 ? 2 : 1);
+  const int seg = (ne / nseg + 31) / 32 * 32;          // elements of a segment, whole warps of them
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    if (STAGE && pass == 0) cp_async_wait<0>();
+    __syncthreads();                                   // sw, the slice of V
+    for (int t = rot ? ng * nseg : warp; t < ng * nseg; t += kDotThreads / 32) {
+      const int i0 = t / nseg * 4, q = t % nseg, a0 = q * seg, a1 = min(cnt, a0 + seg);
+      double sum = 0.0;
+      VT sp[4] = {(VT)0, (VT)0, (VT)0, (VT)0};
+      const VT* vb = Vb + (size_t)i0 * vstr + lane;
+      const int nu = min(4, nv - i0);
+      for (int c0 = a0; c0 < a1; c0 += 256) {
+        const int c1 = min(a1, c0 + 256);
+#pragma unroll 4
+        for (int c = c0; c < c1; c += 32) {
+          const bool in = c + lane < c1;
+          const VT x = in ? (VT)sw[c + lane] : (VT)0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (u < nu) sp[u] = fma(in ? vb[(size_t)u * vstr + c] : (VT)0, x, sp[u]);
+        }
+        if constexpr (sizeof(VT) == 4) {
+          sum += (double)warp_sum4f(sp, lane);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) sp[u] = (VT)0;
+        }
+      }
+      if constexpr (sizeof(VT) == 8) sum = warp_sum4(sp, lane);
+      if ((lane & 7) == 0) ps[q][i0 + (lane >> 3)] = sum;
+    }
+    __syncthreads();
+    if (tid < nv) {
+      double t = ps[0][tid];
+      for (int q = 1; q < nseg; ++q) t += ps[q][tid];
+      pd[pass][tid] = t;
+    }
+    cluster.sync();
+    if (tid < 4 * kMaxRestart) {                       // h_i over the ranks, four of them a thread
+      const int i = tid >> 2, q = tid & 3;
+      double t = 0.0;
+      if (i < nv) {
+        double v[kOrthCtas / 4];
+#pragma unroll
+        for (int r = 0; r < kOrthCtas / 4; ++r) v[r] = *cluster.map_shared_rank(&pd[pass][i], q * (kOrthCtas / 4) + r);
+        t = v[0];
+#pragma unroll
+        for (int r = 1; r < kOrthCtas / 4; ++r) t += v[r];
+      }
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      if (q == 0 && i < nv) {
+        h[i] = t;
+        hv[i] = (VT)t;
+        hcol[i] = pass ? hcol[i] + t : t;
+      }
+    }
+    __syncthreads();
+    if (rot) {                                         // beside the update: the rotations so far, and |h|^2
+      const double a = rotate_rows(hcol, csv, snv, j, lane, hrot);
+      double t = lane < nv ? h[lane] * h[lane] : 0.0;
+      for (int i = lane + 32; i < nv; i += 32) t = fma(h[i], h[i], t);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) {
+        s_a = a;
+        if (pass == 0) s_h2 = t;
+      }
+    }
+    double nn = 0.0;
+    for (int e = rot ? cnt : tid; e < cnt; e += kDotThreads) {
+      VT t = (VT)0;
+      const VT* vb = Vb + e;
+#pragma unroll 8
+      for (int i = 0; i < nv; ++i) t += vb[(size_t)i * vstr] * hv[i];
+      const double x = sw[e] - (double)t;
+      sw[e] = x;
+      nn = fma(x, x, nn);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
+    if (lane == 0 && !rot) red[warp] = nn;
+    __syncthreads();
+    if (warp == 0) {
+      double t = lane < kDotThreads / 32 ? red[lane] : 0.0;
+#pragma unroll
+      for (int o = kDotThreads / 64; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) pn[pass] = t;
+    }
+    cluster.sync();
+    if (warp == 0) {
+      double t = lane < kOrthCtas ? *cluster.map_shared_rank(&pn[pass], lane) : 0.0;
+#pragma unroll
+      for (int o = kOrthCtas / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) s_nrm = t;
+    }
+    __syncthreads();
+    const double t = s_nrm;
+    if (pass == 0 && !(t < eta2 * (t + s_h2))) break;  // (the same numbers in every CTA of the cluster)
+  }
+  ArnoldiColumn col;
+  if (warp == 0) {
+    col = new_rotation(s_a, s_nrm, gj, beta, target, j, m, lane);
+    if (lane == 0) s_inv = col.inv;
+  }
+  cluster.sync();                                      // all have read the shell's state; remote reads are done
+  if (rank == 0) {
+    if (tid == 0) {
+      store_column(s, b, j, col);
+      if (flags) flags[b] = col.act;
+    }
+    double* H = s.H + (size_t)b * (m + 1) * m;
+    for (int i = tid; i < j; i += blockDim.x) H[i * m + j] = hrot[i];
+  }
+  if (out) {
+    const double inv = s_inv;
+    for (int e = tid; e < cnt; e += blockDim.x) {
+      const double v = sw[e] * inv;
+      out[ob + e] = (VT)v;
+      if (out32) out32[ob + e] = (float)v;
+      if (out2) out2[ob + e] = (double)(VT)v;
+    }
+  }
+}
+
+// Back substitution R y = g over the first kb[b] columns, one warp per shell: R in shared memory, lane l the rows l
+// and l + 32; y_i = t_i (1 / R_ii) goes to all lanes, which take its column off their rows (one thread for a whole
+// shell, a division a row: 37 us at 50 columns; now 9 us).
+__global__ void __launch_bounds__(32) k_solve_y(GmresState s) {
+  extern __shared__ __align__(16) double R[];
+  const int b = blockIdx.x, lane = threadIdx.x;
   const int m = s.m, k = s.kb[b];
   const double* H = s.H + (size_t)b * (m + 1) * m;
   const double* g = s.g + (size_t)b * (m + 1);
   double* y = s.y + (size_t)b * m;
+#pragma unroll 8
+  for (int q = lane; q < k * m; q += 32) R[q] = H[q];
+  __syncwarp();
+  double t[2], inv[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int r = lane + 32 * u;
+    t[u] = r < k ? g[r] : 0.0;
+    const double d = r < k ? R[r * m + r] : 0.0;
+    inv[u] = d != 0.0 ? 1.0 / d : 0.0;
+  }
   for (int i = k - 1; i >= 0; --i) {
-    double t = g[i];
-    for (int c = i + 1; c < k; ++c) t -= H[i * m + c] * y[c];
-    const double d = H[i * m + i];
-    y[i] = d != 0.0 ? t / d : 0.0;
+    const int u = i >> 5;
+    const double yi = __shfl_sync(0xffffffffu, u ? t[1] * inv[1] : t[0] * inv[0], i & 31);
+    if (lane == 0) y[i] = yi;
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+      if (lane + 32 * v < i) t[v] -= R[(lane + 32 * v) * m + i] * yi;
   }
 }
 
@@ -586,6 +845,71 @@ cudaError_t krylov_arnoldi_finish(const GmresState& s, const double* nrm2, int j
   return cudaGetLastError();
 }
 
+constexpr int kOrthStage = 160 * 1024;                 // bytes of V's slice in shared memory at most
+
+static cudaLaunchConfig_t orth_config(int B, size_t smem, cudaLaunchAttribute* at, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kOrthCtas, B);
+  cfg.blockDim = dim3(kDotThreads + 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = kOrthCtas;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+// Clusters of 16 CTAs are above the portable 8: whether this device takes them (asked once).
+template <typename VT, bool STAGE>
+static bool orth_fits() {
+  cudaLaunchAttribute at = {};
+  const size_t smem = STAGE ? kOrthStage : 0;
+  const cudaLaunchConfig_t cfg = orth_config(1, smem, &at, nullptr);
+  const auto k = k_orth<VT, STAGE>;
+  int n = 0;
+  const bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+bool krylov_orth_takes(int n, bool basis32) {
+  if (n > (basis32 ? kOrthMax : kOrthMax / 4 * 3)) return false;
+  static std::atomic<int> state[64][2];                // per device and basis: 0 not asked, 1 yes, 2 no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::atomic<int>& q = state[dev & 63][basis32];
+  if (q.load() == 0)
+    q.store((basis32 ? orth_fits<float, false>() && orth_fits<float, true>()
+                     : orth_fits<double, false>() && orth_fits<double, true>()) ? 1 : 2);
+  return q.load() == 1;
+}
+
+template <typename VT>
+static cudaError_t krylov_orth_t(const VT* V, size_t vstride_i, const double* w, int n, int ld, int j, int B,
+                                 const GmresState& s, double eta, VT* out, float* out32, double* out2, int* flags,
+                                 cudaStream_t st) {
+  if (n > kOrthMax || s.m > kMaxRestart || j >= s.m) return cudaErrorInvalidValue;
+  const int ne = (n + kOrthCtas * 32 - 1) / (kOrthCtas * 32) * 32;
+  const size_t slice = (size_t)(j + 1) * ne * sizeof(VT);
+  const bool stage = slice <= kOrthStage;
+  cudaLaunchAttribute at = {};
+  const cudaLaunchConfig_t cfg = orth_config(B, stage ? slice : 0, &at, st);
+  return cudaLaunchKernelEx(&cfg, stage ? k_orth<VT, true> : k_orth<VT, false>, V, vstride_i, w, n, ld, j, s, eta * eta,
+                            out, out32, out2, flags);
+}
+cudaError_t krylov_orth(const double* V, size_t vstride_i, const double* w, int n, int ld, int j, int B,
+                        const GmresState& s, double eta, double* out, float* out32, double* out2, int* flags,
+                        cudaStream_t st) {
+  return krylov_orth_t(V, vstride_i, w, n, ld, j, B, s, eta, out, out32, out2, flags, st);
+}
+cudaError_t krylov_orth(const float* V, size_t vstride_i, const double* w, int n, int ld, int j, int B,
+                        const GmresState& s, double eta, float* out, float* out32, double* out2, int* flags,
+                        cudaStream_t st) {
+  return krylov_orth_t(V, vstride_i, w, n, ld, j, B, s, eta, out, out32, out2, flags, st);
+}
+
 cudaError_t contin_grk_T(const double* X, int ldx, double* g, int M, int nr, const double* gr, double dtPr, int sym,
                          int B, cudaStream_t st) {
   k_grk_T<<<dim3(grid_x(3 * M * nr), B), 256, 0, st>>>(X, ldx, g, M, nr, gr, dtPr, sym);
@@ -611,7 +935,8 @@ cudaError_t krylov_axpy_shell(const double* x0, int ldx0, const double* d, int l
 }
 
 cudaError_t krylov_solve_y(const GmresState& s, int B, cudaStream_t st) {
-  k_solve_y<<<(B + 63) / 64, 64, 0, st>>>(s, B);
+  if (s.m > kMaxRestart) return cudaErrorInvalidValue;
+  k_solve_y<<<B, 32, (size_t)s.m * s.m * sizeof(double), st>>>(s);   // (at most 32 KB)
   return cudaGetLastError();
 }
 

@@ -7,6 +7,9 @@ namespace sdd {
 
 constexpr int kDotChunk = 2048;   // elements per CTA in the two-level dot products
 constexpr int kSubChunk = 512;    // elements per CTA of the fused Gram-Schmidt update and norm
+constexpr int kOrthCtas = 16;     // krylov_orth: CTAs of a cluster, elements of a CTA's slice of w at most
+constexpr int kOrthSlice = 1024;
+constexpr int kOrthMax = kOrthCtas * kOrthSlice;
 constexpr int kMaxRestart = 64;   // GMRES restart length limit (Newton and continuation check it)
 
 struct GmresState {
@@ -65,6 +68,16 @@ cudaError_t krylov_add_combination(const double* V, size_t vstride_i, double* x,
 // out = a * scale[b]; out32 / out2 (nullable, same strides): the result also rounded to FP32 / copied
 cudaError_t krylov_scale(const double* a, const double* scale, double* out, int n, int ld, int B, cudaStream_t st,
                          float* out32 = nullptr, double* out2 = nullptr);
+bool krylov_orth_takes(int n, bool basis32);   // vectors short enough, and the device takes its clusters
+// One launch for all of column j after its product w (krylov_orth_takes): both Gram-Schmidt passes, the rotations, the
+// next basis vector (out; nullable) with its copies out32 / out2 (nullable), the shells' new flags (nullable; B ints that the host may
+// read).  Skips shells with !s.active.
+cudaError_t krylov_orth(const double* V, size_t vstride_i, const double* w, int n, int ld, int j, int B,
+                        const GmresState& s, double eta, double* out, float* out32, double* out2, int* flags,
+                        cudaStream_t st);
+cudaError_t krylov_orth(const float* V, size_t vstride_i, const double* w, int n, int ld, int j, int B,
+                        const GmresState& s, double eta, float* out, float* out32, double* out2, int* flags,
+                        cudaStream_t st);
 cudaError_t krylov_sub(const double* a, const double* b, double* out, size_t n, cudaStream_t st);
 cudaError_t krylov_widen(const float* in, double* out, size_t n, cudaStream_t st);   // out = (double)in
 cudaError_t krylov_masked_sub(double* X, const double* dx, const int* mask, int n, int ldx, int ld, int B,
