@@ -186,7 +186,7 @@ struct sdd_plan {
   double *sv_F, *sv_x, *sv_X0, *sv_Xd, *sv_t, *sv_G, *sv_Jmu, *sv_g, *sv_base64, *sv_dev;
   float* sv_base32;
   float* kv_v32;      // mixed plans: [B][ld] FP32 copy of the Krylov vector the next product is applied to
-  // diagnostics (sdd_diagnostics): FFT plan of length 3M and weight tables; part = per-radius sums
+  // diagnostics (sdd_diagnostics): FFT plan of length 3M and weight tables; part = partial sums
   const FftPlan* dfft;
   double *dg_ir, *dg_tw, *dg_wr, *dg_nuw, *dg_part, *dg_out;
   double ke_scale;
@@ -896,7 +896,7 @@ int sdd_plan_reserve(sdd_plan* p, int max_batch) {
   SDD_CUDA(ws_malloc(&p->base_tmp, (size_t)max_batch * be * sizeof(double)));
   SDD_CUDA(ws_malloc(&p->gridbuf, (size_t)max_batch * be * sizeof(double)));
   SDD_CUDA(ws_malloc(&p->derivbuf, (size_t)max_batch * 5 * p->M * p->nr * sizeof(double)));
-  SDD_CUDA(ws_malloc(&p->dg_part, (size_t)max_batch * p->nr * sizeof(double)));
+  SDD_CUDA(ws_malloc(&p->dg_part, (size_t)max_batch * p->nr * 4 * sizeof(double)));
   SDD_CUDA(ws_malloc(&p->dg_out, (size_t)max_batch * 4 * sizeof(double)));
   SDD_CUDA(ws_malloc(&p->dcnt, (size_t)max_batch * 6 * sizeof(int)));
   SDD_CUDA(cudaMemset(p->dcnt, 0, (size_t)max_batch * 6 * sizeof(int)));
@@ -1981,7 +1981,7 @@ static DiagArgs diag_args(const sdd_plan* p, const double* X, double* out) {
   a.Dr = p->Dr; a.ir = p->dg_ir; a.tw = p->dg_tw; a.wr = p->dg_wr; a.nuw = p->dg_nuw;
   a.ke_scale = p->ke_scale;
   a.X = X; a.x_stride = shell_elems(p);
-  a.part = p->dg_part; a.out = out;
+  a.part = p->dg_part; a.ticket = p->dcnt; a.out = out;
   return a;
 }
 

@@ -7,8 +7,8 @@
 // sinusoid convention), transforms both to the 3 N_fm midpoint grid (IDCT / IDST with n = 3 N_fm) and
 // integrates |.|^2 by the trapezoidal rule over r (x = R interior) and then over theta with sin(theta).
 // Both rules are weighted sums, so KE = (1/2V) sum_n wr_n sum_i wt_i sin(theta_i) (J^2 + D^2)(r_n, theta_i):
-// k_diag_rows computes the inner sum of one radius (the two transforms ride in one complex FFT of length
-// 3 N_fm, in fixed point like the other FP64 transforms) and k_diag_final the outer sums.
+// a CTA computes the inner sum of one radius (the two transforms ride in one complex FFT of length 3 N_fm, in
+// fixed point like the other FP64 transforms) and the last one of a shell the outer sums.
 //
 // Nusselt.  Nu - 1 at r = R[0] is (R[0]^2/A_T) sum_{k even} (D TT_k)[0]/(1 - k^2), TT_k the zero-padded
 // radial profile of mode k: a fixed weighted sum of the even-mode coefficients (weights from the plan).
@@ -20,30 +20,15 @@
 
 namespace sdd {
 
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int t = 0; t < K; ++t) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v[t] += __shfl_xor_sync(0xffffffffu, v[t], off);
-    if (lane == 0) red[t * 32 + warp] = v[t];
-  }
-  __syncthreads();
-  if (threadIdx.x < K) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += red[threadIdx.x * 32 + w];
-    red[32 * K + threadIdx.x] = s;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int t = 0; t < K; ++t) v[t] = red[32 * K + t];
+size_t diag_rows_smem_bytes(int M, int L) {
+  return (4 * (size_t)L * 2 + 5 * (size_t)M + 8) * sizeof(double) + 4 * 32 * 8;
 }
 
-size_t diag_rows_smem_bytes(int M, int L) { return (4 * (size_t)L * 2 + 5 * (size_t)M + 8) * sizeof(double) + 4 * 32 * 8; }
-
-// One CTA per (interior radius n, shell).
-__global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
+// One CTA per (interior radius n, shell): the inner kinetic-energy sum of its radius, and a slice of the sums over the
+// state (|X|^2, Nu_T, Nu_S); the shell's last CTA adds the partial sums in order.  (As a kernel of one CTA a shell
+// the outer sums took longer than the rows: 12.0 + 17.5 us at 90 x 23, now 15 us, most of it the latency of the
+// transform's passes and of a few dozen dependent FP64 operations.)
+__global__ void __launch_bounds__(256) k_diag(DiagArgs a) {
   using C = longlong2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, L = a.L;
@@ -62,23 +47,45 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
   unsigned* red = reinterpret_cast<unsigned*>(scl + 8);
 #pragma unroll 1
   for (int i = tid; i < L; i += bd) {
-    Wt[i] = a.w[i];
-    Et[i] = a.e[i];
+    cp_async16(Wt + i, a.w + i);
+    cp_async16(Et + i, a.e + i);
   }
+  cp_async_commit();
   const double* ps = a.X + (size_t)b * a.x_stride;
-  const double* drn = a.Dr + (size_t)n * nr;
 #pragma unroll 1
-  for (int k = tid; k < M; k += bd) {
+  for (int k = tid; k < M; k += bd) pv[k] = (a.sym && (k % 2 == 0)) ? 0.0 : ps[(size_t)k * nr + n];
+  // the slice of the state's sums: 3 M elements, (M + 1) / 2 Nusselt weights
+  double v[4] = {0.0, 0.0, 0.0, 0.0};                  // |X|^2, KE, NuT, NuS
+  {
+    const size_t N = (size_t)M * nr;
+    const double* xs = ps + (size_t)n * 3 * M;
+#pragma unroll 4
+    for (int q = tid; q < 3 * M; q += bd) v[0] = fma(xs[q], xs[q], v[0]);
+    const int ne = (M + 1) / 2;
+    for (int q = tid; q < ne; q += bd) {
+      const int e = n * ne + q, kk = e / nr, m = e - kk * nr;
+      const size_t o = (size_t)(2 * kk) * nr + m;
+      const double w = a.nuw[e];
+      v[2] = fma(w, ps[N + o], v[2]);
+      v[3] = fma(w, ps[2 * N + o], v[3]);
+    }
+  }
+  const double* drn = a.Dr + (size_t)n * nr;
+  const int half = (nr + 1) / 2;
+#pragma unroll 1
+  for (int i = tid; i < (2 * M + 31) / 32 * 32; i += bd) {   // two lanes a mode (whole warps)
+    const int k = min(i >> 1, M - 1), m0 = (i & 1) * half, m1 = min(nr, m0 + half);
     const double* pk = ps + (size_t)k * nr;
     double acc = 0.0;
-    for (int m = 0; m < nr; ++m) acc = fma(drn[m], pk[m], acc);
-    dp[k] = acc;
-    pv[k] = (a.sym && (k % 2 == 0)) ? 0.0 : pk[n];
+#pragma unroll 8
+    for (int m = m0; m < m1; ++m) acc = fma(__ldg(drn + m), pk[m], acc);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    if (i < 2 * M && (i & 1) == 0) dp[k] = acc;
   }
   __syncthreads();
   parity_suffix<double>(pv, Sc, M);   // as J_theta_RT
   __syncthreads();
-  const double irn = a.ir[n];
+  const double irn = a.ir[n], wrn = a.wr[n];
 #pragma unroll 1
   for (int k = tid; k < M; k += bd) {
     const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;
@@ -87,6 +94,7 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
     Ar[k] = irn * jp;
     Br[k] = k >= 1 ? dp[k - 1] : 0.0;
   }
+  cp_async_wait<0>();                                  // the twiddles
   __syncthreads();
   // DCT3 inputs with n_in = M on length L (see k_transform): cosine x_k = A_k; sine x_k = B_{L-k}
   double* XV = reinterpret_cast<double*>(RB);
@@ -107,53 +115,53 @@ __global__ void __launch_bounds__(256) k_diag_rows(DiagArgs a) {
   __syncthreads();
   C* res = fft_rows<double, false>(RA, RB, 1, a.st, Wt);
   const bool bad = E[0] == kFxBad || E[1] == kFxBad;
-  double s[1] = {0.0};
-#pragma unroll 1
+  double ke = 0.0;
+#pragma unroll 2
   for (int i = tid; i < L; i += bd) {
     const int src = (i & 1) ? (L - 1 - (i >> 1)) : (i >> 1);
-    const C v = res[src];
-    const double ja = bad ? fx_nan() : fx2d(v.y, 60 - E[0]), db = fx2d(v.x, 60 - E[1]);   // (db's sign drops out)
-    s[0] = fma(a.tw[i], fma(ja, ja, db * db), s[0]);
+    const C c = res[src];
+    const double ja = bad ? fx_nan() : fx2d(c.y, 60 - E[0]), db = fx2d(c.x, 60 - E[1]);   // (db's sign drops out)
+    ke = fma(a.tw[i], fma(ja, ja, db * db), ke);
   }
-  __syncthreads();                      // (the scales are read before the sums reuse the reduction words)
-  block_sum<1>(s, reinterpret_cast<double*>(red));
-  if (tid == 0) a.part[(size_t)b * nr + n] = s[0];
-}
-
-// One CTA per shell: |X|_2, KE from the per-radius sums, Nu_T and Nu_S.
-__global__ void __launch_bounds__(256) k_diag_final(DiagArgs a) {
-  __shared__ double red[32 * 4 + 4];
-  const int M = a.M, nr = a.nr, b = blockIdx.x;
-  const size_t N = (size_t)M * nr;
-  const double* X = a.X + (size_t)b * a.x_stride;
-  double v[4] = {0.0, 0.0, 0.0, 0.0};   // |X|^2, KE, NuT, NuS
-  for (size_t e = threadIdx.x; e < 3 * N; e += blockDim.x) v[0] = fma(X[e], X[e], v[0]);
-  for (int n = threadIdx.x; n < nr; n += blockDim.x) v[1] = fma(a.wr[n], a.part[(size_t)b * nr + n], v[1]);
-  const int ne = (M + 1) / 2;
-  for (int e = threadIdx.x; e < ne * nr; e += blockDim.x) {
-    const int kk = e / nr, m = e - kk * nr;
-    const size_t o = (size_t)(2 * kk) * nr + m;
-    v[2] = fma(a.nuw[e], X[N + o], v[2]);
-    v[3] = fma(a.nuw[e], X[2 * N + o], v[3]);
+  v[1] = wrn * ke;
+  const int lane = tid & 31, warp = tid >> 5;
+  const double t4 = warp_sum4(v, lane);
+  double* rd = reinterpret_cast<double*>(red);
+  __syncthreads();                      // (the exponents are read before the sums reuse the reduction words)
+  if ((lane & 7) == 0) rd[(lane >> 3) * 8 + warp] = t4;
+  __syncthreads();
+  __shared__ int s_last;
+  if (warp == 0) {                      // lane 8 q + w: warp w's sum of value q
+    double t = rd[lane];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 7) == 0) a.part[((size_t)b * nr + n) * 4 + (lane >> 3)] = t;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) {
+      int* cnt = a.ticket + (size_t)b * 6 + 5;
+      const int last = atomicAdd(cnt, 1) == nr - 1;
+      if (last) *cnt = 0;               // ready for the next launch
+      s_last = last;
+    }
   }
-  block_sum<4>(v, red);
-  if (threadIdx.x == 0) {
-    double* o = a.out + (size_t)b * 4;
-    o[0] = sqrt(v[0]);
-    o[1] = a.ke_scale * v[1];
-    o[2] = v[2];
-    o[3] = v[3];
-  }
+  __syncthreads();
+  if (!s_last || warp >= 4) return;
+  __threadfence();
+  // warp q adds value q over the radii
+  const double* p = a.part + (size_t)b * nr * 4 + warp;
+  double t = lane < nr ? __ldcg(p + 4 * lane) : 0.0;
+  if (lane + 32 < nr) t += __ldcg(p + 4 * (lane + 32));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) a.out[(size_t)b * 4 + warp] = warp == 0 ? sqrt(t) : (warp == 1 ? a.ke_scale * t : t);
 }
 
 cudaError_t launch_diag(const DiagArgs& a, int batch, cudaStream_t s) {
   static unsigned long long done = 0;
-  cudaError_t e = ensure_smem_attr(k_diag_rows, &done);
+  const cudaError_t e = ensure_smem_attr(k_diag, &done);
   if (e != cudaSuccess) return e;
-  if ((e = launch_kernel(k_diag_rows, dim3(a.nr, batch), dim3(256), diag_rows_smem_bytes(a.M, a.L), s, a)) !=
-      cudaSuccess)
-    return e;
-  return launch_kernel(k_diag_final, dim3(batch), dim3(256), 0, s, a);
+  return launch_kernel(k_diag, dim3(a.nr, batch), dim3(256), diag_rows_smem_bytes(a.M, a.L), s, a);
 }
 
 }  // namespace sdd

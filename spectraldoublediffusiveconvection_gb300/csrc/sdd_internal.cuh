@@ -333,7 +333,8 @@ struct DiagArgs {
   double ke_scale;           // 1/(2V), V = (2/3)(r_o^3 - r_i^3)
   const double* X;           // states [shell][3][M][nr]
   size_t x_stride;
-  double* part;              // [shell][nr] per-radius kinetic-energy sums
+  double* part;              // [shell][nr][4] partial sums of |X|^2, KE, Nu_T, Nu_S
+  int* ticket;               // six counters a shell of which the last one counts its CTAs (zero between launches)
   double* out;               // [shell][4]
 };
 

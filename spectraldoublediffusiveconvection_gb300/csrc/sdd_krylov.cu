@@ -25,6 +25,7 @@
 #include "sdd_fixed.cuh"
 #include "sdd_internal.cuh"
 #include "sdd_krylov.cuh"
+#include "sdd_rowops.cuh"
 
 namespace sdd {
 
@@ -41,24 +42,6 @@ constexpr int kSubPer = kSubChunk / kDotThreads;
 static_assert(kSubChunk % kDotThreads == 0, "update chunk must be a multiple of the block");
 constexpr int kDotVecs = 4;
 static_assert(kDotChunk % kDotThreads == 0, "dot chunk must be a multiple of the block");
-
-// Warp sums of four values per lane in 6 FP64 additions per lane instead of 4 x 5: the first two shuffle
-// levels exchange halves of the set (lanes with bit 4 set keep vectors 2-3, then lanes with bit 3 set
-// keep the odd one), the last three are a plain tree.  Lanes 8v..8v+7 return the sum of vector v.
-__device__ __forceinline__ double warp_sum4(const double (&sv)[4], int lane) {
-  const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
-  double k0 = h16 ? sv[2] : sv[0], k1 = h16 ? sv[3] : sv[1];
-  const double s0 = h16 ? sv[0] : sv[2], s1 = h16 ? sv[1] : sv[3];
-  k0 += __shfl_xor_sync(0xffffffffu, s0, 16);
-  k1 += __shfl_xor_sync(0xffffffffu, s1, 16);
-  double k = h8 ? k1 : k0;
-  const double t = h8 ? k0 : k1;
-  k += __shfl_xor_sync(0xffffffffu, t, 8);
-  k += __shfl_xor_sync(0xffffffffu, k, 4);
-  k += __shfl_xor_sync(0xffffffffu, k, 2);
-  k += __shfl_xor_sync(0xffffffffu, k, 1);
-  return k;
-}
 
 // warp_sum4 in FP32 (the FP32 basis's projections: conversions and FP64 additions hold the FP64 pipe, the
 // FP32 ones do not); the same lane pattern.

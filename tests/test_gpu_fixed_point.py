@@ -236,3 +236,30 @@ def test_batches_take_the_faster_chains(cuda, N_fm, N_r, batch, layouts):
     z = p.step(X, 8000.0, 500.0, nsteps=3)
     for k in range(batch):
         assert float((y[k] - z[k]).norm() / z[k].norm()) <= 1e-12
+
+
+@pytest.mark.parametrize("N_fm,N_r,sym", [(2, 3, False), (6, 34, True), (30, 8, False), (90, 23, True), (128, 65, False)])
+def test_diagnostics_of_a_batch(cuda, N_fm, N_r, sym):
+    """The per-shell sums over the CTAs of the radii (the last one adds them), at ragged sizes and twice in a row
+    (the counters start again), against the oracle: the norm and the kinetic energy are sums of non-negative
+    terms, (3 N_fm nr + 8) roundings at most; the Nusselt numbers N_fm nr roundings of their largest term's sum."""
+    from oracle import sdd_oracle as O
+    from spectraldoublediffusiveconvection_gb300.plan import Plan
+    nr = N_r - 1
+    p = Plan(N_fm, N_r, 2.0, 1e-3, 1.0, 0.01, symmetric=sym)
+    ops = O.Operators(N_fm, N_r, 2.0, 1e-3, 1.0, 0.01)
+    X = np.stack([O.seeded_state(N_fm, nr, k, sym) for k in range(3)])
+    Xd = cuda.from_numpy(X).cuda()
+    N, u = N_fm * nr, 2.0 ** -53
+    for _ in range(2):
+        y = p.diagnostics(Xd).cpu().numpy()
+        for b in range(3):
+            assert abs(y[b, 0] - np.linalg.norm(X[b])) <= (3 * N + 8) * u * y[b, 0]
+            ke = O.Kinetic_Energy(X[b], ops.R, ops.D, N_fm, nr, sym)
+            # (its terms: squares of transforms of N_fm products of nr)
+            assert abs(y[b, 1] - ke) <= 4 * (3 * N + 8) * u * ke + 1e-300
+            for f in (1, 2):
+                T = X[b, f * N:(f + 1) * N]
+                nu = O.Nusselt(T, 2.0, ops.R, ops.D, N_fm, nr)
+                w = sum(np.abs(ops.D[0, 1:-1]) @ np.abs(T[k * nr:(k + 1) * nr]) for k in range(0, N_fm, 2))
+                assert abs(y[b, 1 + f] - nu) <= 4 * (N + 8) * u * (1 + w * ops.R[0] ** 2 / abs(O.base_state_AT(2.0)))
