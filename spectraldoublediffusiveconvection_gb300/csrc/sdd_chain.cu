@@ -103,6 +103,7 @@ __device__ __forceinline__ void compute_sync(int nt) { asm volatile("bar.sync 1,
 // h = Linv g, which the FP64 form for batches did without) for 64 shells' whole chains.
 template <int LD, bool CHUNK, int D>
 __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batch) {
+  after_previous_kernel();
   constexpr int W = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
   extern __shared__ __align__(16) i64 csm[];
@@ -339,6 +340,7 @@ static size_t chain_fx_smem_bytes(int nsteps, int ld, int D) {
 // the exact algebra of s_{c+1} = Phi_c s_c + d_c.
 template <int LD>
 __global__ void __launch_bounds__(LD > 32 ? 256 : 128) k_carry_fx(ChainArgs a) {
+  after_previous_kernel();
   constexpr int W = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
   extern __shared__ __align__(16) i64 psm[];
@@ -432,6 +434,7 @@ constexpr int kMvShells = 4;
 // Dr Q in fixed point like the other matvecs, or (mixed plans' FP32 nonlinear term) in FP32.
 template <bool FIX, int LD>
 __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int batch, int group) {
+  after_previous_kernel();
   constexpr int NP = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
   extern __shared__ __align__(16) int msm[];           // fused right-hand side: Dr's block, or Dr^T in FP32
@@ -585,6 +588,7 @@ constexpr int kMv32Shells = 16;
 
 template <int NP>
 __global__ void __launch_bounds__(128) k_mode_mv32(ChainArgs a, int nfields, int batch) {
+  after_previous_kernel();
   const int M = a.M, nr = a.nr, ldl = a.ldl;
   const int wid = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;

@@ -29,6 +29,7 @@ size_t diag_rows_smem_bytes(int M, int L) {
 // the outer sums took longer than the rows: 12.0 + 17.5 us at 90 x 23, now 15 us, most of it the latency of the
 // transform's passes and of a few dozen dependent FP64 operations.)
 __global__ void __launch_bounds__(256) k_diag(DiagArgs a) {
+  after_previous_kernel();
   using C = longlong2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, L = a.L;

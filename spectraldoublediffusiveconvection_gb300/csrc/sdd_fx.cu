@@ -230,6 +230,7 @@ __device__ __forceinline__ void scale_rows(T* PR, int P, unsigned (&mx)[K], void
 // 2: grid fields only (fills the cache).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
+  after_previous_kernel();
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
@@ -578,6 +579,7 @@ static size_t fx_deriv_smem_bytes(int nr, bool d2s, bool fix, int km, bool f32) 
 template <typename T, int LD>
 __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
     k_fx_deriv(FxArgs a, T* deriv, size_t deriv_stride, int km, int contract) {
+  after_previous_kernel();
   constexpr int NP = (LD + 31) / 32, kW = deriv_warps(LD);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int4 s_x[kW][32 * NP];
@@ -679,6 +681,7 @@ __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
 
 template <typename T>
 __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, size_t grid_stride) {
+  after_previous_kernel();
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
@@ -845,6 +848,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* grid, size_t grid_stride) {
+  after_previous_kernel();
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
@@ -913,6 +917,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
 
 // ---- right-hand sides of the three implicit solves (Main.py:262-280) ---------------------------
 __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
+  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr;
   const int n = blockIdx.x, b = blockIdx.y;
@@ -1017,6 +1022,7 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
 // path), with A2_SINE's D2 psi formed by k_fx_deriv.  One CTA per (row, shell).  Bound by the FP64 pipe (about 20
 // operations an element) and its column-strided loads: 39 us at 64 shells of 256 x 30, 76 us as k_rhs with D2 psi.
 __global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double* d2psi, size_t d2_stride) {
+  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr;
   const int n = blockIdx.x, b = blockIdx.y;
@@ -1067,6 +1073,7 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double*
 // psi and Q rows in shared memory was measured slower: the 66 KB per CTA cut the resident CTAs that hide
 // the latency of these row reads.)
 __global__ void __launch_bounds__(kFxThreads) k_rhs32(RhsArgs a) {
+  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float scal[8];
   const int M = a.M, nr = a.nr;

@@ -122,6 +122,7 @@ static __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[1
 }
 
 __global__ void __launch_bounds__(kTcThreads, 1) k_deriv_tc(TcArgs a) {
+  after_previous_kernel();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const int KP = a.KP, NP = a.NP, N = 2 * NP, M = a.M, nr = a.nr;
   const int tid = threadIdx.x, warp = tid >> 5;
