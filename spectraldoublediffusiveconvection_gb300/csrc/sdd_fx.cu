@@ -9,6 +9,9 @@
 // the kernel outputs DST(JT_psi*omega) and the rhs kernel applies Dr to it in spectral space, so the
 // row kernel has no cross-row dependency.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+
 #include "sdd_internal.cuh"
 #include "sdd_fft.cuh"
 #include "sdd_rowops.cuh"
@@ -1417,6 +1420,26 @@ static cudaError_t launch_deriv(const FxArgs& a, int batch, bool split, cudaStre
   return e;
 }
 
+// Threads of a k_fx_rows CTA.  A row's transforms leave most of an SM's issue slots empty behind their barriers, so
+// several small CTAs serve it better than a large one: the SM's threads (512 at the FP64 kernel's 128 registers,
+// 1024 FP32) are shared among the CTAs that shared memory lets in and the launch has.  us, 512 threads against the
+// rule: FP64 64 shells of 256 x 30 (2 CTAs of 256) 321 / 248, 16 of 128 x 28 (3 of 160) 54 / 35, 32 of 64 x 20 (4 of 128) 63 /
+// 26; FP32 64 shells of 256 x 30 (4 of 256) 107 / 82; 540 x 65 FP64 (one CTA fits) 113 with 512, 132 with 256.
+template <typename T>
+static int fx_row_threads(size_t smem, long ctas) {
+  static const int sm_smem = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    return n;
+  }();
+  const long fit = (long)(sm_smem / (smem + 1024 + 512));   // (a CTA's reserved and static shared memory)
+  const long want = (ctas + fx_sm_count() - 1) / fx_sm_count();
+  const int n = (int)std::max(1l, std::min({fit, want, 8l}));
+  const int total = sizeof(T) == 8 ? 512 : 1024;
+  return std::max(128, std::min(kFxRowThreads, total / n / 32 * 32));
+}
+
 template <typename T, int MODE>
 static cudaError_t launch_fx_t(const FxArgs& a, int batch, cudaStream_t s) {
   const size_t smem = fx_smem_bytes(a.M, a.P, sizeof(T) == 4 ? SDD_PREC_MIXED : SDD_PREC_FP64);
@@ -1425,7 +1448,7 @@ static cudaError_t launch_fx_t(const FxArgs& a, int batch, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   if (a.deriv && (e = launch_deriv<T>(a, batch, false, s)) != cudaSuccess) return e;
   if (sizeof(T) == 4 && a.deriv_t && (e = launch_tc_for(a, batch, s)) != cudaSuccess) return e;
-  e = launch_kernel(k_fx_rows<T, MODE>, dim3(a.nr, batch), dim3(kFxRowThreads), smem, s, a);
+  e = launch_kernel(k_fx_rows<T, MODE>, dim3(a.nr, batch), dim3(fx_row_threads<T>(smem, (long)a.nr * batch)), smem, s, a);
   ktimer_mark(SDD_K_FX_ROWS, s);
   return e;
 }
