@@ -553,9 +553,12 @@ static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB,
 
 // Chunk lengths.  Layout 2 (sequential carry: kc local steps, then nch - 2 carried matvecs of twice the
 // width, on one SM per chain): kc ~ sqrt(2S).  Layout 3 (parallel carry: kc local steps, then all
-// (nch-1)(nch-2)/2 products at once, spread over the GPU): kc ~ sqrt(S/2), shorter chunks.
-static int chunk_len(int S, int layout) {
-  const double k = layout == 3 ? std::sqrt(0.5 * S) : std::sqrt(2.0 * S);
+// (nch-1)(nch-2)/2 products at once, spread over the GPU): kc ~ sqrt(S/2), shorter chunks; with nr > 32, where the
+// products' blocks are 33 KB each and reading them is what the carry costs, 0.85 sqrt(S) (us a step with 0.71 / 0.85:
+// 540 x 65 149 / 145, 384 x 50 106 / 100, 256 x 50 77 / 73, 384 x 36 81 / 74, 192 x 36 54.8 / 55.2, 128 x 36 43.4 / 42.8;
+// 256 x 30 with 8 / 10 steps 42.9 / 43.6).
+static int chunk_len(int S, int layout, int nr) {
+  const double k = layout == 3 ? std::sqrt((nr > 32 ? 0.72 : 0.5) * S) : std::sqrt(2.0 * S);
   return std::max(layout == 3 ? 2 : 4, std::min(layout == 3 ? 16 : 32, (int)std::lround(k)));
 }
 
@@ -566,8 +569,8 @@ static int build_chunk_tables(sdd_plan* p, const double* AB, const double* LinvT
   p->ldmT = nr + (nr & 1);
   p->ldd = 2 * nr;
   int st;
-  if ((st = build_chunk_set(p, chunk_len(S, 2), false, AB, LinvT, LinvS, cA, cT, cS, &p->cs[0])) ||
-      (st = build_chunk_set(p, chunk_len(S, 3), true, AB, LinvT, LinvS, cA, cT, cS, &p->cs[1])))
+  if ((st = build_chunk_set(p, chunk_len(S, 2, nr), false, AB, LinvT, LinvS, cA, cT, cS, &p->cs[0])) ||
+      (st = build_chunk_set(p, chunk_len(S, 3, nr), true, AB, LinvT, LinvS, cA, cT, cS, &p->cs[1])))
     return st;
   p->nch_alloc = std::max(p->cs[0].nch, p->cs[1].nch);
   p->np_alloc = std::max(p->cs[1].np, 1);
@@ -755,7 +758,7 @@ int sdd_plan_destroy(sdd_plan* p) {
 int sdd_plan_set_chunk_length(sdd_plan* p, int set, int kc) {
   if (!p || set < 0 || set > 1 || kc < 0 || !p->h_AB) return SDD_ERR_ARG;
   const int S = p->M / 2;
-  if (kc == 0) kc = chunk_len(S, set == 1 ? 3 : 2);
+  if (kc == 0) kc = chunk_len(S, set == 1 ? 3 : 2, p->nr);
   const int nch = (S + kc - 1) / kc;
   // at least two steps per chunk; the parallel carry's products grow as nch^2 / 2: at most 32 chunks
   if (kc < 2 || kc > S || (set == 1 && nch > 32) || nch > 64) return SDD_ERR_ARG;

@@ -424,7 +424,9 @@ __device__ __forceinline__ double carried_state(const ChainArgs& a, int b, size_
 
 // Independent per-mode matvecs, one warp per (field, mode, 32 rows) and up to kMvShells shells, one lane per
 // row; the lane's row of the block sits in registers for all shells of the group (the block is read once per
-// group, its loads all in flight at once):
+// group, its loads all in flight at once), the next shell's inputs load beside a shell's product (corrections of 8
+// shells of 384 x 36: 41 us without, 31 with; h of batches is bound by the integer pipe, 61 us at 64 shells of
+// 256 x 30, 21 of it the three-digit Dr Q):
 //   FIX = false:  h_jj = Linv_jj g_jj                          (the chains' right-hand sides)
 //   FIX = true:   f_jj += G_jj s_c(jj) for the modes of chunks c >= 1   (chunked chains' correction)
 constexpr int kMvShells = 4;
@@ -441,6 +443,7 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
   __shared__ int4 s_w[FIX ? 1 : 4][32 * NP];           // Q's digits
   __shared__ __align__(16) int2 s_x[4][32 * NP];
   __shared__ float s_q[4][32 * NP];
+  __shared__ double s_dq[FIX || NP == 1 ? 1 : 2][4][32];   // [buffer][warp] Dr Q of the warp's rows
   __shared__ i64 s_pv[FIX ? 4 : 1][kMvShells][32];     // psi's first half of a correction, per shell
   __shared__ int s_pe[FIX ? 4 : 1][kMvShells][32];
   const int M = a.M, nr = a.nr;
@@ -486,78 +489,83 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
     const i64* B = blk + (size_t)sg * bw;
     FxRow<LD, NP> m;
     m.load(B, rr);
+    // a shell's inputs, loaded one shell ahead of their use
+    struct In {
+      double x[NP], ln[NP], q[NP];
+    };
+    auto load = [&](int b) {
+      In v;
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int e = p * 32 + lane;
+        v.x[p] = v.ln[p] = v.q[p] = 0.0;
+        if (FIX) {
+          if (e < nr)
+            v.x[p] = a.carry_seq ? a.cbuf[(size_t)b * a.d_stride + (chain * a.nch + c) * a.ldd + sg * nr + e]
+                                 : carried_state(a, b, chain, c, sg * nr + e);
+        } else if (!fuse) {
+          if (e < nr) v.x[p] = a.g[(size_t)b * a.g_stride + foff + e];
+        } else if (e < nr) {
+          const double* o4 = a.out4 + (size_t)b * a.out_stride + ro;
+          v.x[p] = o4[(size_t)(field + 1) * N + e];      // psi: R
+          v.ln[p] = a.lin[(size_t)b * a.g_stride + foff + e];
+          if (a4) v.q[p] = a.q32 ? (double)__ldg(a.q32 + (size_t)b * N + ro + e) : o4[e];
+        }
+      }
+      if (FIX && sg + 1 == nseg && r < nr) v.ln[0] = a.f[(size_t)b * a.f_stride + foff + r];
+      return v;
+    };
+    In in = load(b0);
+    int turn = 0;                                      // s_dq's buffer: alternates over the shells that are not skipped
 #pragma unroll 1
     for (int b = b0; b < b1; ++b) {
       const int u = b - b0;
+      const In cur = in;
+      if (b + 1 < b1) in = load(b + 1);
       if (a.active && !a.active[b]) continue;
       double x[NP];
 #pragma unroll
-      for (int p = 0; p < NP; ++p) x[p] = 0.0;
-      if (FIX) {
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const int e = p * 32 + lane;
-          if (e < nr)
-            x[p] = a.carry_seq ? a.cbuf[(size_t)b * a.d_stride + (chain * a.nch + c) * a.ldd + sg * nr + e]
-                               : carried_state(a, b, chain, c, sg * nr + e);
-        }
-      } else if (!fuse) {
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-          if (p * 32 + lane < nr) x[p] = a.g[(size_t)b * a.g_stride + foff + p * 32 + lane];
-      } else {
-        const double* o4 = a.out4 + (size_t)b * a.out_stride + ro;
-        const double* lin = a.lin + (size_t)b * a.g_stride + foff;
-        double nl[NP], ln[NP];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const int e = p * 32 + lane;
-          nl[p] = e < nr ? o4[(size_t)(field + 1) * N + e] : 0.0;   // psi: R
-          ln[p] = e < nr ? lin[e] : 0.0;
-        }
+      for (int p = 0; p < NP; ++p) x[p] = cur.x[p];
+      if (fuse) {
         if (a4) {
           double dq[NP];
+          // (nr > 32: the two warps of a mode form Dr Q's rows of their own and swap them)
+          constexpr int P1 = NP == 1 ? 1 : 2;
+          const int own = NP == 1 ? 0 : wl & 1;
+          const int e = min(own * 32 + lane, nr - 1);
+          double d;
           if (a.q32) {
-            const float* qs = a.q32 + (size_t)b * N + ro;
 #pragma unroll
             for (int p = 0; p < NP; ++p)
-              if (p * 32 + lane < nr) s_q[wl][p * 32 + lane] = __ldg(qs + p * 32 + lane);
+              if (p * 32 + lane < nr) s_q[wl][p * 32 + lane] = (float)cur.q[p];
             __syncwarp();
-            const float* Dt = reinterpret_cast<const float*>(msm);
-            float d[NP];
-#pragma unroll
-            for (int p = 0; p < NP; ++p) d[p] = 0.0f;
-            for (int cc = 0; cc < nr; ++cc) {
-              const float qv = s_q[wl][cc];
-#pragma unroll
-              for (int p = 0; p < NP; ++p) d[p] = fmaf(Dt[cc * nr + min(p * 32 + lane, nr - 1)], qv, d[p]);
-            }
+            const float* Dt = reinterpret_cast<const float*>(msm) + e;
+            float acc = 0.0f;
+            for (int cc = 0; cc < nr; ++cc) acc = fmaf(Dt[cc * nr], s_q[wl][cc], acc);
             __syncwarp();
-#pragma unroll
-            for (int p = 0; p < NP; ++p) dq[p] = (double)d[p];
+            d = (double)acc;
           } else {
-            double q[NP];
             int cx[NP];
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {
-              const int e = p * 32 + lane;
-              q[p] = e < nr ? o4[e] : 0.0;
-              cx[p] = e < nr ? msm[3 * LD * LD + LD + e] : 0;
-            }
-            const int em = publish_wide<NP>(q, cx, nr, lane, s_w[wl]);
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-              const int e = min(p * 32 + lane, nr - 1);
-              dq[p] = fx_val(wx_dot<LD>(msm, nr, e, s_w[wl], em));
-            }
+            for (int p = 0; p < NP; ++p) cx[p] = p * 32 + lane < nr ? msm[3 * LD * LD + LD + p * 32 + lane] : 0;
+            const int em = publish_wide<NP>(cur.q, cx, nr, lane, s_w[wl]);
+            d = fx_val(wx_dot<LD>(msm, nr, e, s_w[wl], em));
             __syncwarp();                              // the digits are read before the next shell's replace them
           }
+          dq[0] = d;
+          if constexpr (NP > 1) {
+            s_dq[turn][wl][lane] = d;
+            asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (wl >> 1)) : "memory");
 #pragma unroll
-          for (int p = 0; p < NP; ++p) nl[p] = __dsub_rn(dq[p], nl[p]);
+            for (int p = 0; p < P1; ++p) dq[p] = s_dq[turn][(wl & 2) + p][lane];
+            turn ^= 1;
+          }
+#pragma unroll
+          for (int p = 0; p < NP; ++p) x[p] = __dsub_rn(dq[p], x[p]);
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p)
-          if (p * 32 + lane < nr) x[p] = __dadd_rn(__dmul_rn(-a.dt, nl[p]), ln[p]);
+          if (p * 32 + lane < nr) x[p] = __dadd_rn(__dmul_rn(-a.dt, x[p]), cur.ln[p]);
       }
       const int em = publish_regs<NP>(x, m.cx, nr, lane, xs);
       const FxVal p = m.times(B, nr, rr, xs, em);
@@ -568,7 +576,8 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
           s_pe[wl][u][lane] = p.e;
         } else if (r < nr) {
           double* y = a.f + (size_t)b * a.f_stride + foff + r;
-          const double v = nseg == 2 ? fx_sum(*y, FxVal{s_pv[wl][u][lane], s_pe[wl][u][lane]}, p) : fx_sum(*y, p);
+          const double v = nseg == 2 ? fx_sum(cur.ln[0], FxVal{s_pv[wl][u][lane], s_pe[wl][u][lane]}, p)
+                                     : fx_sum(cur.ln[0], p);
           *y = v;
           if (a.f32) a.f32[(size_t)b * a.f32_stride + foff + r] = (float)v;
         }
