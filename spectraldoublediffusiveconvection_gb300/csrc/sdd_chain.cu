@@ -103,7 +103,6 @@ __device__ __forceinline__ void compute_sync(int nt) { asm volatile("bar.sync 1,
 // h = Linv g, which the FP64 form for batches did without) for 64 shells' whole chains.
 template <int LD, bool CHUNK, int D>
 __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batch) {
-  after_previous_kernel();
   constexpr int W = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
   extern __shared__ __align__(16) i64 csm[];
@@ -121,7 +120,6 @@ __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batc
   const int b = blockIdx.y * spc + sh;
   const int M = a.M, nr = a.nr;
   const int field = type == 0 ? 0 : 1 + g;
-  const bool on = !loader && b < batch && (a.fmask >> field & 1) && !(a.active && !a.active[b]);
   const int i = 32 * w + lane;
   const bool ok = i < nr;
   const int ir = ok ? i : nr - 1;
@@ -129,14 +127,16 @@ __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batc
   const int chunk = CHUNK ? (int)blockIdx.z : 0;
   const int s0 = CHUNK ? chunk * a.kc : 0;
   const int s1 = CHUNK ? min(S, s0 + a.kc) : S;
-  if (s0 >= S) return;
+  if (s0 >= S) {
+    after_previous_kernel();
+    return;
+  }
   const int nsteps = s1 - s0;
   const size_t foff = (size_t)field * a.field_off;
   const int bs = b < batch ? b : batch - 1;
   const int chain = type == 0 ? par : (1 + g) * 2 + par;
   const size_t dslot = CHUNK ? (size_t)bs * a.d_stride + (size_t)chain * a.nch * a.ldd : 0;
   double* dout = CHUNK ? a.dbuf + dslot + (size_t)chunk * a.ldd : nullptr;
-  const bool wr = on && ok && (type == 1 || g == 0);   // the lanes that write f
   const int e = (type == 0 && g == 1 ? nr : 0) + ir;   // this row's element of the carried state
   // the rows of f (f32, sub, h) of step s: row M - 1 - (par + 2 (s0 + s)), 2 nr apart
   const ptrdiff_t row0 = (ptrdiff_t)(M - 1 - (par + 2 * s0)) * nr + ir, drow = -2 * (ptrdiff_t)nr;
@@ -145,8 +145,40 @@ __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batc
   const double* sub = a.sub ? a.sub + (size_t)bs * a.sub_stride + foff + row0 : nullptr;
   const double* h = a.h + (size_t)bs * a.h_stride + foff + row0;
 
-  // symmetric: only the "evens" loops run (A4 jj = 0,2,..; NAB2 jj = 1,3,..); other rows stay 0.
-  if (a.sym && par != (type == 0 ? 0 : 1)) {
+  i64* ring = csm;                                     // D slots of the two groups' blocks
+  double2* cf = reinterpret_cast<double2*>(ring + 2 * D * bw);   // [group][nsteps + 1] scalars
+  const int jj0 = par + 2 * s0;
+  // psi: (bj, bjt);  T/S: (k, -) with b += k f_{j+2} at the step's start
+  const bool idle = a.sym && par != (type == 0 ? 0 : 1);   // (symmetric: only the "evens" loops run)
+  for (int q = idle ? 2 * (nsteps + 1) : tid; q < 2 * (nsteps + 1); q += blockDim.x) {
+    const int gg = q / (nsteps + 1), jj = jj0 + 2 * (q - gg * (nsteps + 1));
+    const double* c = type == 0 ? a.coefA4 + 2 : (gg == 0 ? a.coefT : a.coefS);
+    cf[q] = jj < M ? make_double2(c[(size_t)jj * 4], c[(size_t)jj * 4 + 1]) : make_double2(0.0, 0.0);
+  }
+
+  auto fetch_step = [&](int s) {                       // the blocks of step s (step 0 needs none: zero state)
+    if (s < nsteps) {
+      const size_t jj = jj0 + 2 * s;
+      i64* dst = ring + (s % D) * 2 * bw;
+      if (type == 0) {
+        copy_words(dst, a.ABA4 + jj * 2 * bw, 2 * bw, lane, 32);
+      } else {
+        copy_words(dst, a.LinvT + jj * bw, bw, lane, 32);
+        copy_words(dst + bw, a.LinvS + jj * bw, bw, lane, 32);
+      }
+    }
+    cp_async_commit();
+  };
+  if (loader && !idle) {                               // (plan tables, as are the scalars)
+#pragma unroll
+    for (int s = 1; s <= D; ++s) fetch_step(s);
+  }
+  after_previous_kernel();
+  const bool on = !loader && b < batch && (a.fmask >> field & 1) && !(a.active && !a.active[b]);
+  const bool wr = on && ok && (type == 1 || g == 0);   // the lanes that write f
+
+  // symmetric: the other parity's rows stay 0
+  if (idle) {
     if (wr)
       for (int s = 0; s < nsteps; ++s) {
         f[s * drow] = 0.0;
@@ -156,38 +188,13 @@ __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batc
     return;
   }
 
-  i64* ring = csm;                                     // D slots of the two groups' blocks
-  double2* cf = reinterpret_cast<double2*>(ring + 2 * D * bw);   // [group][nsteps + 1] scalars
-  const int jj0 = par + 2 * s0;
-  // psi: (bj, bjt);  T/S: (k, -) with b += k f_{j+2} at the step's start
-  for (int q = tid; q < 2 * (nsteps + 1); q += blockDim.x) {
-    const int gg = q / (nsteps + 1), jj = jj0 + 2 * (q - gg * (nsteps + 1));
-    const double* c = type == 0 ? a.coefA4 + 2 : (gg == 0 ? a.coefT : a.coefS);
-    cf[q] = jj < M ? make_double2(c[(size_t)jj * 4], c[(size_t)jj * 4 + 1]) : make_double2(0.0, 0.0);
-  }
-
   if (loader) {
-    auto fetch = [&](int s) {                          // the blocks of step s (step 0 needs none: zero state)
-      if (s < nsteps) {
-        const size_t jj = jj0 + 2 * s;
-        i64* dst = ring + (s % D) * 2 * bw;
-        if (type == 0) {
-          copy_words(dst, a.ABA4 + jj * 2 * bw, 2 * bw, lane, 32);
-        } else {
-          copy_words(dst, a.LinvT + jj * bw, bw, lane, 32);
-          copy_words(dst + bw, a.LinvS + jj * bw, bw, lane, 32);
-        }
-      }
-      cp_async_commit();
-    };
-#pragma unroll
-    for (int s = 1; s <= D; ++s) fetch(s);
     cp_async_wait<D - 1>();
     __syncthreads();
     for (int s = 1; s < nsteps; ++s) {
       cp_async_wait<D - 2>();
       __syncthreads();
-      fetch(s + D);
+      fetch_step(s + D);
     }
     cp_async_wait<0>();
   } else {
@@ -200,6 +207,7 @@ __global__ void __launch_bounds__(160) k_chain_fx(ChainArgs a, int spc, int batc
     double fe = 0.0, bfe = 0.0;                        // psi: f_e, bf_e (group 1 only);  T/S: b in fe
     ptrdiff_t o = 0;                                   // s drow
     for (int s = 0; s < nsteps; ++s, o += drow) {
+      if (s + 2 >= nsteps) next_kernel_may_start();
       const double hi = hn0, si = sn0;
       hn0 = hn1;
       sn0 = sn1;
@@ -340,7 +348,6 @@ static size_t chain_fx_smem_bytes(int nsteps, int ld, int D) {
 // the exact algebra of s_{c+1} = Phi_c s_c + d_c.
 template <int LD>
 __global__ void __launch_bounds__(LD > 32 ? 256 : 128) k_carry_fx(ChainArgs a) {
-  after_previous_kernel();
   constexpr int W = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
   extern __shared__ __align__(16) i64 psm[];
@@ -349,8 +356,10 @@ __global__ void __launch_bounds__(LD > 32 ? 256 : 128) k_carry_fx(ChainArgs a) {
   __shared__ int s_e[4][32 * W];
   const int type = a.type0 + (blockIdx.x >> 1), par = blockIdx.x & 1;
   const int b = blockIdx.y, pidx = blockIdx.z;
-  if (a.sym && par != (type == 0 ? 0 : 1)) return;     // inactive chains: their carried states are not read
-  if (a.active && !a.active[b]) return;
+  if (a.sym && par != (type == 0 ? 0 : 1)) {           // inactive chains: their carried states are not read
+    after_previous_kernel();
+    return;
+  }
   int j = 2;
   while (j * (j - 1) / 2 <= pidx) ++j;                 // row j holds products (j-1)(j-2)/2 .. j(j-1)/2 - 1
   const int ii = pidx - (j - 1) * (j - 2) / 2;
@@ -365,6 +374,11 @@ __global__ void __launch_bounds__(LD > 32 ? 256 : 128) k_carry_fx(ChainArgs a) {
     copy_words(psm + bw, a.PS + m * bw, bw, tid, blockDim.x);
   }
   cp_async_commit();
+  after_previous_kernel();                             // (the blocks are the plan's)
+  if (a.active && !a.active[b]) {
+    cp_async_wait<0>();
+    return;
+  }
   const int chain = type == 0 ? par : (1 + (q >> 1)) * 2 + par;
   const double* d = a.dbuf + (size_t)b * a.d_stride + ((size_t)chain * a.nch + ii) * a.ldd +
                     (type == 0 ? (q & 1) * nr : 0);
@@ -378,6 +392,7 @@ __global__ void __launch_bounds__(LD > 32 ? 256 : 128) k_carry_fx(ChainArgs a) {
   int cx[W];
 #pragma unroll
   for (int p = 0; p < W; ++p) cx[p] = 32 * p + lane < nr ? fx_col_exp(blk, LD)[32 * p + lane] : 0;
+  next_kernel_may_start();
   const int em = publish_regs<W>(x, cx, nr, lane, xs);
   const int ea = fx_row_exp(blk, LD)[ir];
   // psi: all columns of block (row half, operand half); T/S: half the columns of the field's
@@ -436,7 +451,6 @@ constexpr int kMvShells = 4;
 // Dr Q in fixed point like the other matvecs, or (mixed plans' FP32 nonlinear term) in FP32.
 template <bool FIX, int LD>
 __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int batch, int group) {
-  after_previous_kernel();
   constexpr int NP = (LD + 31) / 32;
   constexpr int bw = (int)fx_block_words(LD);
   extern __shared__ __align__(16) int msm[];           // fused right-hand side: Dr's block, or Dr^T in FP32
@@ -460,12 +474,10 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
     } else {
       for (int e = threadIdx.x; e < (int)wx_block_ints(LD) / 4; e += blockDim.x) cp_async16(msm + 4 * e, a.wxDr + 4 * e);
       cp_async_commit();
-      cp_async_wait<0>();
     }
-    __syncthreads();
   }
-  if (wid >= nfields * M * NP) return;
-  const int fm = wid / NP, r = (wid - fm * NP) * 32 + lane;
+  const bool in_range = wid < nfields * M * NP;        // (the last CTA's spare warps: field and mode 0)
+  const int fm = in_range ? wid / NP : 0, r = in_range ? (wid - fm * NP) * 32 + lane : lane;
   const int fl = fm / M, jj = fm - fl * M;
   const int field = a.field0 + fl;
   const int row = M - 1 - jj;
@@ -474,21 +486,25 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
   const bool a4 = field == 0;
   const int rr = min(r, nr - 1);
   const int par = jj & 1;
-  int c = 0;
-  if (FIX) {
-    c = (jj >> 1) / a.kc;
-    if (c == 0 || (a.sym && !(a4 ? par == 0 : par == 1))) return;
-  }
+  const int c = FIX ? (jj >> 1) / a.kc : 0;
+  const bool mine = in_range && !(FIX && (c == 0 || (a.sym && !(a4 ? par == 0 : par == 1))));
   const int nseg = FIX && a4 ? 2 : 1;
   const i64* blk = FIX ? (a4 ? a.GA4 + (size_t)jj * 2 * bw : (field == 1 ? a.GT : a.GS) + (size_t)jj * bw)
                        : (a4 ? a.LinvA4 : (field == 1 ? a.LinvT : a.LinvS)) + (size_t)jj * bw;
   const size_t chain = (size_t)(field * 2 + par);
   const int b0 = blockIdx.y * group, b1 = min(batch, b0 + group);
   int2* xs = s_x[wl];
+  FxRow<LD, NP> m;
+  if (!FIX || mine) m.load(blk, rr);                   // (the plan's, like Dr's block)
+  after_previous_kernel();
+  if (fuse && a.field0 == 0 && blockIdx.x * 4 < M * NP) {
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+  if (!mine) return;
   for (int sg = 0; sg < nseg; ++sg) {
     const i64* B = blk + (size_t)sg * bw;
-    FxRow<LD, NP> m;
-    m.load(B, rr);
+    if (FIX && sg > 0) m.load(B, rr);
     // a shell's inputs, loaded one shell ahead of their use
     struct In {
       double x[NP], ln[NP], q[NP];
@@ -522,6 +538,7 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
       const int u = b - b0;
       const In cur = in;
       if (b + 1 < b1) in = load(b + 1);
+      else next_kernel_may_start();
       if (a.active && !a.active[b]) continue;
       double x[NP];
 #pragma unroll

@@ -29,7 +29,6 @@ size_t diag_rows_smem_bytes(int M, int L) {
 // the outer sums took longer than the rows: 12.0 + 17.5 us at 90 x 23, now 15 us, most of it the latency of the
 // transform's passes and of a few dozen dependent FP64 operations.)
 __global__ void __launch_bounds__(256) k_diag(DiagArgs a) {
-  after_previous_kernel();
   using C = longlong2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, L = a.L;
@@ -52,6 +51,7 @@ __global__ void __launch_bounds__(256) k_diag(DiagArgs a) {
     cp_async16(Et + i, a.e + i);
   }
   cp_async_commit();
+  after_previous_kernel();                             // (the tables are the plan's)
   const double* ps = a.X + (size_t)b * a.x_stride;
 #pragma unroll 1
   for (int k = tid; k < M; k += bd) pv[k] = (a.sym && (k % 2 == 0)) ? 0.0 : ps[(size_t)k * nr + n];
@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(256) k_diag(DiagArgs a) {
     RA[k] = k == 0 ? make_longlong2(XB[0], XA[0]) : dct3_pack_fx(Et[k], XA[k], XA[L - k], XB[k], XB[L - k]);
   __syncthreads();
   C* res = fft_rows<double, false>(RA, RB, 1, a.st, Wt);
+  next_kernel_may_start();
   const bool bad = E[0] == kFxBad || E[1] == kFxBad;
   double ke = 0.0;
 #pragma unroll 2

@@ -233,14 +233,12 @@ __device__ __forceinline__ void scale_rows(T* PR, int P, unsigned (&mx)[K], void
 // 2: grid fields only (fills the cache).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
-  after_previous_kernel();
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, P = a.P;
   const int n = blockIdx.x, b = blockIdx.y;
-  if (a.active && !a.active[b]) return;
   const int tid = threadIdx.x, bd = blockDim.x;
 
   C* RA = reinterpret_cast<C*>(smem_raw);
@@ -277,6 +275,8 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
     opr[nr + m] = D2g[n * nr + m];
   }
   const T ir4n = reinterpret_cast<const T*>(a.ops.ir4r2)[n];
+  after_previous_kernel();     // (the tables and operators are the plan's)
+  if (a.active && !a.active[b]) return;
   __syncthreads();
 
   // ---- 1. radial contractions of row n (Derivatives, :698-729) and the row values ----
@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
   });
   __syncthreads();
   C* Z = fft_rows<T, false>(RB, RA, 2, a.st, Wt);
+  next_kernel_may_start();
   double* o = a.out4 + (size_t)b * a.out_stride;
   const T two_P = (T)2 / (T)P, one_P = (T)1 / (T)P;
 #pragma unroll 1
@@ -457,8 +458,8 @@ __device__ __forceinline__ void cp_async_all_done() {
 }
 
 // The pending correction of modes k0 .. k0 + kn - 1 (see FixArgs) on xd (the modes' FP64 psi, T, S rows, in
-// shared memory, still in flight but for one group of copies).  s_c = d_{c-1} + part_{c,0} + ... in index order
-// (per chain f vectors of 2 nr, nr, nr doubles) while the rows of G load; then xd += G_jj s_c in the arithmetic
+// shared memory, still in flight).  s_c = d_{c-1} + part_{c,0} + ... in index order
+// (per chain f vectors of 2 nr, nr, nr doubles); then xd += G_jj s_c in the arithmetic
 // of k_mode_mv (the same bits).  Four tasks of NP^2 warps (32 rows and the columns, or half of them) per mode:
 // psi's two operand halves, T, S; 8 warps take two modes at once, 16 warps one.  The corrected rows are written
 // back to the state (and its FP32 copy).  sc: 4 nr doubles a mode.
@@ -482,10 +483,40 @@ __device__ __forceinline__ double carried_term(const FixArgs& x, int b, int par,
   return v;
 }
 
+// A warp's task and its rows of G.
 template <int LD>
-__device__ void apply_pending_fix(const FxArgs& a, int b, int k0, int kn, double* xd, double* sc) {
-  constexpr int NP = (LD + 31) / 32, NC = LD / NP, kMw = 4 * NP * NP, kG = deriv_warps(LD) / kMw;
-  constexpr int bw = (int)fx_block_words(LD);
+struct FixRow {
+  static constexpr int NP = (LD + 31) / 32, NC = LD / NP, kMw = 4 * NP * NP, kG = deriv_warps(LD) / kMw;
+  FxRow<LD, NP, NC> G;
+  int task, sl, h;
+  static __device__ __forceinline__ int chunk_of(const FxArgs& a, int k) { return ((a.M - 1 - k) >> 1) / a.fix.kc; }
+  static __device__ __forceinline__ bool on(const FxArgs& a, int k, bool psi) {
+    return chunk_of(a, k) >= 1 && (!a.sym || ((a.M - 1 - k) & 1) == (psi ? 0 : 1));
+  }
+  __device__ __forceinline__ bool mine(const FxArgs& a, int k0, int kn, int m) const {   // uniform over the warp
+    return m < kn && on(a, k0 + m, task < 2);
+  }
+  __device__ __forceinline__ const i64* block(const FxArgs& a, int k) const {
+    constexpr int bw = (int)fx_block_words(LD);
+    const size_t jj = a.M - 1 - k;
+    return task < 2 ? a.fix.GA4 + (jj * 2 + task) * bw : (task == 2 ? a.fix.GT : a.fix.GS) + jj * bw;
+  }
+  __device__ __forceinline__ int row(int nr) const { return min(sl * 32 + (int)(threadIdx.x & 31), nr - 1); }
+  __device__ __forceinline__ void load(const FxArgs& a, int k0, int kn, int m) {
+    if (mine(a, k0, kn, m)) G.load(block(a, k0 + m), row(a.nr), h * NC);
+  }
+  __device__ __forceinline__ void first(const FxArgs& a, int k0, int kn) {
+    const int warp = threadIdx.x >> 5;
+    task = warp % kMw / (NP * NP);
+    sl = warp / NP % NP;
+    h = warp % NP;
+    load(a, k0, kn, warp / kMw);
+  }
+};
+
+template <int LD>
+__device__ void apply_pending_fix(const FxArgs& a, int b, int k0, int kn, double* xd, double* sc, FixRow<LD>& fx) {
+  constexpr int NP = FixRow<LD>::NP, NC = FixRow<LD>::NC, kMw = FixRow<LD>::kMw, kG = FixRow<LD>::kG;
   __shared__ __align__(16) int2 s_x[deriv_warps(LD)][32 * NP];
   __shared__ i64 s_v[kG][4][32 * NP];
   __shared__ int s_e[kG][4][32 * NP];
@@ -493,23 +524,18 @@ __device__ void apply_pending_fix(const FxArgs& a, int b, int k0, int kn, double
   const FixArgs& x = a.fix;
   const int M = a.M, nr = a.nr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto chunk_of = [&](int k) { return ((M - 1 - k) >> 1) / x.kc; };
-  auto on = [&](int k, bool psi) { return chunk_of(k) >= 1 && (!a.sym || ((M - 1 - k) & 1) == (psi ? 0 : 1)); };
-  const int task = warp % kMw / (NP * NP), sl = warp / NP % NP, h = warp % NP;
-  const int r = sl * 32 + lane, rr = min(r, nr - 1);
-  FxRow<LD, NP, NC> G;
-  auto block = [&](int m) {
-    const size_t jj = M - 1 - (k0 + m);
-    return task < 2 ? x.GA4 + (jj * 2 + task) * bw : (task == 2 ? x.GT : x.GS) + jj * bw;
-  };
-  auto mine = [&](int m) { return m < kn && on(k0 + m, task < 2); };   // uniform over the warp
+  auto chunk_of = [&](int k) { return fx.chunk_of(a, k); };
+  auto on = [&](int k, bool psi) { return fx.on(a, k, psi); };
+  auto mine = [&](int m) { return fx.mine(a, k0, kn, m); };
+  const int task = fx.task, sl = fx.sl, h = fx.h;
+  const int r = sl * 32 + lane, rr = fx.row(nr);
+  FxRow<LD, NP, NC>& G = fx.G;
   int m = warp / kMw;
-  if (mine(m)) G.load(block(m), rr, h * NC);
   for (int q = threadIdx.x; q < kn * 4 * nr; q += blockDim.x) {
     const int mm = q / (4 * nr), e = q - mm * 4 * nr;
     if (on(k0 + mm, e < 2 * nr)) sc[q] = carried_term(x, b, (M - 1 - k0 - mm) & 1, chunk_of(k0 + mm), e, nr);
   }
-  cp_async_wait<1>();
+  cp_async_wait<0>();
   __syncthreads();
 #pragma unroll 1
   for (int g = 0; g < kn; g += kG, m += kG) {
@@ -532,11 +558,11 @@ __device__ void apply_pending_fix(const FxArgs& a, int b, int k0, int kn, double
         t.t2 += u.t2;
         t.t1 += u.t1;
       }
-      const FxVal p = G.value(t, block(m), nr, rr, s_x[warp], em);
+      const FxVal p = G.value(t, fx.block(a, k0 + m), nr, rr, s_x[warp], em);
       s_v[mg][task][r] = p.v;
       s_e[mg][task][r] = p.e;
     }
-    if (mine(m + kG)) G.load(block(m + kG), rr, h * NC);
+    fx.load(a, k0, kn, m + kG);
     __syncthreads();
     const int gn = min(kG, kn - g);
     for (int q = threadIdx.x; q < gn * 3 * nr; q += blockDim.x) {
@@ -582,13 +608,11 @@ static size_t fx_deriv_smem_bytes(int nr, bool d2s, bool fix, int km, bool f32) 
 template <typename T, int LD>
 __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
     k_fx_deriv(FxArgs a, T* deriv, size_t deriv_stride, int km, int contract) {
-  after_previous_kernel();
   constexpr int NP = (LD + 31) / 32, kW = deriv_warps(LD);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int4 s_x[kW][32 * NP];
   const int M = a.M, nr = a.nr;
   const int k0 = blockIdx.x * km, kn = min(km, M - k0), b = blockIdx.y;
-  if (a.active && !a.active[b]) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t N = (size_t)M * nr;
   const bool d2s = a.fuse_rhs;
@@ -598,12 +622,6 @@ __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
   double* sc = xd + (size_t)km * 3 * nr;
   // FP32 on the CUDA cores: the operators and rows in FP32, behind the doubles
   float* ops = reinterpret_cast<float*>(xd + (size_t)km * (a.fix.on ? 7 : 3) * nr);
-  const double* Xs = (a.fix.on ? a.fix.X : a.X) + (size_t)b * a.x_stride;
-  for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) {
-    const int m = q / (3 * nr), e = q - m * 3 * nr, f = e / nr;
-    cp_async_elem(xd + q, Xs + f * N + (size_t)(k0 + m) * nr + (e - f * nr));
-  }
-  cp_async_commit();
   constexpr int wq = (int)wx_block_ints(LD) / 4, dq = (int)fx_block_words(LD) / 2;
   if (sizeof(T) == 8) {
     for (int e = threadIdx.x; e < wq; e += blockDim.x) cp_async16(opw + 4 * e, a.ops.wx[0] + 4 * e);
@@ -622,13 +640,27 @@ __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
     }
   }
   cp_async_commit();
+  FixRow<LD> fix;
+  if (a.fix.on) fix.first(a, k0, kn);
+  after_previous_kernel();                             // (the operators and the correction's blocks are the plan's)
+  if (a.active && !a.active[b]) {
+    cp_async_wait<0>();
+    return;
+  }
+  const double* Xs = (a.fix.on ? a.fix.X : a.X) + (size_t)b * a.x_stride;
+  for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) {
+    const int m = q / (3 * nr), e = q - m * 3 * nr, f = e / nr;
+    cp_async_elem(xd + q, Xs + f * N + (size_t)(k0 + m) * nr + (e - f * nr));
+  }
+  cp_async_commit();
   T* D = deriv + (size_t)b * deriv_stride;
   double* D5 = reinterpret_cast<double*>(D) + 4 * N * sizeof(T) / 8;
-  if (a.fix.on) apply_pending_fix<LD>(a, b, k0, kn, xd, sc);
+  if (a.fix.on) apply_pending_fix<LD>(a, b, k0, kn, xd, sc, fix);
   cp_async_wait<0>();
   __syncthreads();
   // the fixed-point contractions, as items (operator, row slab, mode): D2 first, whose products cost twice Dr's
   // (FP64: D2r2 psi, A2_SINE's D2 psi where it is asked for, then Dr psi, Dr T, Dr S; FP32: A2_SINE's D2 psi)
+  next_kernel_may_start();
   const int nd2 = (sizeof(T) == 8) + d2s, nit = (nd2 + (sizeof(T) == 8 ? 3 : 0)) * NP * kn;
 #pragma unroll 1
   for (int it = warp; it < nit; it += kW) {
@@ -684,14 +716,12 @@ __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
 
 template <typename T>
 __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, size_t grid_stride) {
-  after_previous_kernel();
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, P = a.P;
   const int n = blockIdx.x, pr = blockIdx.y, b = blockIdx.z;
-  if (a.active && !a.active[b]) return;
   const int tid = threadIdx.x, bd = blockDim.x;
   const int ta = 2 * pr, tb = 2 * pr + 1;      // tb = 9 (absent) for the last pair
 
@@ -722,6 +752,11 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
   for (int i = tid; i < P + 2; i += bd) kf[i] = (T)i;
   const T ir4n = reinterpret_cast<const T*>(a.ops.ir4r2)[n];
   // (no barrier: the row loads below do not read the tables; the one after them covers both)
+  after_previous_kernel();                          // (the tables are the plan's)
+  if (a.active && !a.active[b]) {
+    cp_async_all_done();
+    return;
+  }
 
   // which row quantities the pair's two fields need (fields: 0 JT_psi, 1 komega, 2 kDpsi, 3 DT, 4 DC,
   // 5 omega, 6 Dpsi, 7 kT, 8 kC)
@@ -838,6 +873,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
   for_elems<T>(P, [&](int k) { RA[k] = Tr::pack(XV, P, 0, nt > 1, k, Et, scl); });
   __syncthreads();
   C* res = fft_rows<T, Tr::kInv, false>(RA, RB, 1, a.st, Wt);
+  next_kernel_may_start();
   T* g = grid + (size_t)b * grid_stride + (size_t)n * 9 * P;
   for_elems<T>(nt * P, [&](int idx) {
     const int u = idx >= P ? 1 : 0;
@@ -851,14 +887,12 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* grid, size_t grid_stride) {
-  after_previous_kernel();
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, P = a.P;
   const int n = blockIdx.x, p = blockIdx.y, b = blockIdx.z;
-  if (a.active && !a.active[b]) return;
   const int tid = threadIdx.x, bd = blockDim.x;
   C* RA = reinterpret_cast<C*>(smem_raw);
   C* RB = RA + P;
@@ -873,6 +907,11 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
   for (int i = tid; i < P; i += bd) {               // asynchronous: in flight while the products load
     cp_async_elem(Wt + i, wg + i);
     cp_async_elem(Et + i, eg + i);
+  }
+  after_previous_kernel();                          // (the tables are the plan's)
+  if (a.active && !a.active[b]) {
+    cp_async_all_done();
+    return;
   }
   const T* RG = grid + (size_t)b * grid_stride + (size_t)n * 9 * P;
   const T* bs = (MODE == 1) ? reinterpret_cast<const T*>(a.base) + (size_t)b * a.base_stride + (size_t)n * 9 * P
@@ -893,6 +932,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
   cp_async_all_done();
   __syncthreads();
   C* Z = fft_rows<T, false, false>(RB, RA, 1, a.st, Wt);
+  next_kernel_may_start();
   const int N = M * nr;
   double* o = a.out4 + (size_t)b * a.out_stride;
   const T two_P = (T)2 / (T)P, one_P = (T)1 / (T)P;
@@ -920,11 +960,9 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* 
 
 // ---- right-hand sides of the three implicit solves (Main.py:262-280) ---------------------------
 __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
-  after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr;
   const int n = blockIdx.x, b = blockIdx.y;
-  if (a.active && !a.active[b]) return;
   const int tid = threadIdx.x, bd = blockDim.x;
   double* sm = reinterpret_cast<double*>(smem_raw);
   double* pv = sm;
@@ -942,6 +980,8 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
     opr[nr + m] = a.D2s[n * nr + m];
   }
   for (int k = tid; k < M + 3; k += bd) kd[k] = (double)k;
+  after_previous_kernel();     // (the operators are the plan's)
+  if (a.active && !a.active[b]) return;
   __syncthreads();
   const int N = M * nr;
   const double* Xs = a.X + (size_t)b * a.x_stride;
@@ -973,6 +1013,7 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
   }
   __syncthreads();
   parity_suffix<double>(pv, Sc, M);
+  next_kernel_may_start();
   __syncthreads();
   const double dt = a.dt, dtPr = a.dt * a.Pr;
   const double Ra = a.Ra[b], Ras = a.Ra_s[b];
@@ -1053,6 +1094,7 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double*
   const double ir2 = a.ir2s[n], rsq = a.rsq[n], dT0 = a.dT0[n], gr = a.gr[n];
   __syncthreads();
   parity_suffix<double>(pv, Sc, M);
+  next_kernel_may_start();
   double* R = a.rhs + (size_t)b * a.rhs_stride;
   for (int k = tid; k < M; k += bd) {
     const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;

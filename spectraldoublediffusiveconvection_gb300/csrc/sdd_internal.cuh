@@ -19,13 +19,20 @@ constexpr int kFxRowThreads = 512;  // threads of the nonlinear-term row kernel
 void set_cuda_error(cudaError_t e);
 
 // Kernel launch through cudaLaunchKernelEx with the launch error returned, as a programmatic dependent of the kernel
-// before it in the stream: it is launched as that kernel's CTAs end, and EVERY kernel launched this way begins with
-// after_previous_kernel(), which waits for the completion (and the writes) of all before it.  Hides most of a
-// launch's latency: single steps of 64 x 20 47.5 -> 31 us, 256 x 30 62.8 -> 46.5, 64 shells 618 -> 606; inside the
-// captured step graphs 44.6 -> 43.4.  Letting the next kernel in earlier (griddepcontrol.launch_dependents at a
-// kernel's start) was slower: its waiting CTAs take the SMs' room (64 shells 667, 256 x 30 in graphs 50).
+// before it in the stream: it is launched once every CTA of that kernel has ended or called next_kernel_may_start().
+// EVERY kernel launched this way calls after_previous_kernel(), which waits for the completion (and the writes) of all
+// kernels before it, ahead of anything it reads that a kernel writes and of every write to global memory.  Before it
+// stand only loads of the plan's tables (operators, twiddles, blocks, chain scalars: written and synchronised when the
+// plan or its chunk tables are made).  Dependents hide most of a launch's latency: single steps of 64 x 20 47.5 -> 31
+// us, 256 x 30 62.8 -> 46.5, 64 shells 618 -> 606; inside the captured step graphs 44.6 -> 43.4.
+// next_kernel_may_start() stands where a kernel's last phase begins: the next kernel's CTAs come up and load their
+// tables beside it (us a step: 256 x 30 43.5 -> 41.5, 540 x 65 146 -> 139, 3 shells of 128 x 28 mixed 44.4 -> 41.7, 90 x
+// 23 with diagnostics 50 -> 45; the tables ahead of the wait alone 42.9, 145, 44.3, 50).  Before the transforms
+// instead of after them it is slower (42.1, 140, 42.8), at a kernel's start far slower (256 x 30 50, 64 shells 606 ->
+// 667): the CTAs that wait then take the room where the next kernel's others would spread over the SMs.
 #ifdef __CUDACC__
 __device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
