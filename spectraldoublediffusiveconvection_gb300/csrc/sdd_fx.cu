@@ -66,6 +66,33 @@ __device__ __forceinline__ void with_x(const FxArgs& a, int b, F&& body) {
   }
 }
 
+// The linear parts of the three right-hand sides (Main.py:262-280) at one row and mode, in the three kernels that form
+// them (k_fx_grid, k_rhs_lin, k_rhs), so that all give the same bits.  An FP64 instruction holds the pipe for 64 cycles
+// and a dependent one waits as long: fused multiply-adds, the row's scalars multiplied once, doublings in the exponent
+// and mode numbers without conversions leave 12 a mode of 22 (k_rhs_lin, 64 shells of 256 x 30: 38.9 -> 28.7 us, in a step 525 -> 516; mixed 315 -> 306;
+// one shell 41.5 -> 41.1).
+__device__ __forceinline__ double twice(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x), e = hi & 0x7ff00000, sgn = hi & (int)0x80000000;
+  if (e == 0x7ff00000) return x;
+  if (e == 0x7fe00000) return __hiloint2double(sgn | 0x7ff00000, 0);
+  const int sh = (int)__funnelshift_l((unsigned)lo, (unsigned)hi, 1) & 0x7fffffff;   // (zero and below the normal range)
+  return e == 0 ? __hiloint2double(sgn | sh, lo << 1) : __hiloint2double(hi + 0x100000, lo);
+}
+// A2_SINE: D2 psi - k1 ir2 (k2 psi_k + 2 s2), k1 = k + 1, k2 = k + 2, s2 = the parity sum from k + 2
+__device__ __forceinline__ double lin_a2(double d2, double k1, double k2, double ir2, double pk, double s2) {
+  return fma(-(k1 * ir2), fma(k2, pk, twice(s2)), d2);
+}
+// psi: A2 psi - dt Pr gr k1 (Ra T_{k+1} - Ra_s S_{k+1}); gd = dt Pr gr
+__device__ __forceinline__ double lin_psi_rhs(double om, double k1, double gd, double Ra, double Ras, double t, double s) {
+  return fma(-(k1 * gd), fma(Ra, t, -(Ras * s)), om);
+}
+// J_theta_RT: k1 psi_{k-1} + 2 s1, k = 0: s1
+__device__ __forceinline__ double lin_jt(int k, double k1, double pkm, double s1) {
+  return k == 0 ? s1 : fma(k1, pkm, twice(s1));
+}
+// T, S: r^2 f - dt dT0 J; dd = dt dT0
+__device__ __forceinline__ double lin_ts_rhs(double rsq, double f, double dd, double jt) { return fma(-dd, jt, rsq * f); }
+
 // Arithmetic shared by the fused and the split nonlinear-term kernels.  This file is compiled without
 // automatic fma contraction and every multiply-add below is an explicit fma, so both kernels round
 // identically.
@@ -267,7 +294,7 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
     Et[i] = eg[i];
   }
 #pragma unroll 1
-  for (int i = tid; i < P + 2; i += bd) kf[i] = (T)i;
+  for (int i = tid; i < P + 2; i += bd) kf[i] = sizeof(T) == 8 ? (T)fx_int(i) : (T)i;
   const T* Drg = reinterpret_cast<const T*>(a.ops.Dr);
   const T* D2g = reinterpret_cast<const T*>(a.ops.D2r2);
   for (int m = tid; m < nr; m += bd) {
@@ -749,7 +776,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
     cp_async_elem(Et + i, eg + i);
   }
 #pragma unroll 1
-  for (int i = tid; i < P + 2; i += bd) kf[i] = (T)i;
+  for (int i = tid; i < P + 2; i += bd) kf[i] = sizeof(T) == 8 ? (T)fx_int(i) : (T)i;
   const T ir4n = reinterpret_cast<const T*>(a.ops.ir4r2)[n];
   // (no barrier: the row loads below do not read the tables; the one after them covers both)
   after_previous_kernel();                          // (the tables are the plan's)
@@ -835,31 +862,32 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
     const double* Tvd = pv64 ? pv64 + 2 * M : reinterpret_cast<const double*>(Tv);
     const double* Svd = pv64 ? pv64 + 3 * M : reinterpret_cast<const double*>(Sv);
     const RhsArgs& r = a.rl;
-    const double dt = r.dt, dtPr = r.dt * r.Pr;
-    const double Ra = lRa, Ras = lRas;
-    const double ir2 = lir2, rsq = lrsq, dT0 = ldT0, gr = lgr;
+    const double gd = r.dt * r.Pr * lgr, dd = r.dt * ldT0;
     double* R = lin ? r.rhs + (size_t)b * r.rhs_stride : nullptr;
 #pragma unroll 1
     for (int k = tid; k < M; k += bd) {
       if (need_psi) jp_om<T>(k, M, kf, pv, Sc, ir4n, JP[k], OM[k]);
       if (lin) {
-        const double pk = pvd[k];
+        double k1, k2;                                 // (conversions would take the FP64 pipe)
+        if constexpr (sizeof(T) == 8) {
+          k1 = kf[k + 1];
+          k2 = kf[k + 2];
+        } else {
+          k1 = fx_int(k + 1);
+          k2 = fx_int(k + 2);
+        }
         const size_t o = (size_t)k * nr + n;
         if (lin_psi && k >= kp0 && k < kp1) {
           const double s2 = (k + 2 < M) ? Scd[k + 2] : 0.0;
           const bool psi_on = !(a.sym && (k % 2 == 0));
           const double d2s = k == tid ? d2s0 : (psi_on ? D2p[(size_t)k * nr + n] : 0.0);
-          const double Om = d2s - (double)(k + 1) * ir2 * ((k + 2.0) * pk + 2.0 * s2);
-          const double grv = (k < M - 1) ? (-(double)(k + 1) * gr) * (Ra * Tvd[k + 1] - Ras * Svd[k + 1]) : 0.0;
-          R[o] = Om + dtPr * grv;
+          const double om = lin_a2(d2s, k1, k2, lir2, pvd[k], s2);
+          R[o] = k < M - 1 ? lin_psi_rhs(om, k1, gd, lRa, lRas, Tvd[k + 1], Svd[k + 1]) : om;
         }
         if (lin_ts) {
-          const double pkm = k > 0 ? pvd[k - 1] : 0.0;
-          const double s1 = (k + 1 < M) ? Scd[k + 1] : 0.0;
-          const double JPk = (k == 0) ? 1.0 * s1 : (k + 1.0) * pkm + 2.0 * s1;
-          const double psiT0 = dT0 * JPk;
-          R[N + o] = rsq * Tvd[k] - dt * psiT0;
-          R[2 * N + o] = rsq * Svd[k] - dt * psiT0;
+          const double jt = lin_jt(k, k1, k > 0 ? pvd[k - 1] : 0.0, (k + 1 < M) ? Scd[k + 1] : 0.0);
+          R[N + o] = lin_ts_rhs(lrsq, Tvd[k], dd, jt);
+          R[2 * N + o] = lin_ts_rhs(lrsq, Svd[k], dd, jt);
         }
       }
     }
@@ -979,7 +1007,7 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
     opr[m] = a.Dr[n * nr + m];
     opr[nr + m] = a.D2s[n * nr + m];
   }
-  for (int k = tid; k < M + 3; k += bd) kd[k] = (double)k;
+  for (int k = tid; k < M + 3; k += bd) kd[k] = fx_int(k);
   after_previous_kernel();     // (the operators are the plan's)
   if (a.active && !a.active[b]) return;
   __syncthreads();
@@ -1019,13 +1047,11 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
   const double Ra = a.Ra[b], Ras = a.Ra_s[b];
   const double ir2 = a.ir2s[n], rsq = a.rsq[n], dT0 = a.dT0[n], gr = a.gr[n];
   double* R = a.rhs + (size_t)b * a.rhs_stride;
+  const double gd = dtPr * gr, dd = dt * dT0;
   for (int k = tid; k < M; k += bd) {
-    const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;
     const double k1 = kd[k + 1], k2 = kd[k + 2];
-    const double JP = (k == 0) ? 1.0 * s1 : k1 * pv[k - 1] + 2.0 * s1;    // J_theta_RT
-    const double s2 = (k + 2 < M) ? Sc[k + 2] : 0.0;
-    const double Om = D2p[k] - k1 * ir2 * (k2 * pv[k] + 2.0 * s2);       // A2_SINE
-    const double grv = (k < M - 1) ? (-k1 * gr) * (Ra * Tv[k + 1] - Ras * Sv[k + 1]) : 0.0;
+    const double JP = lin_jt(k, k1, k > 0 ? pv[k - 1] : 0.0, (k + 1 < M) ? Sc[k + 1] : 0.0);    // J_theta_RT
+    const double Om = lin_a2(D2p[k], k1, k2, ir2, pv[k], (k + 2 < M) ? Sc[k + 2] : 0.0);          // A2_SINE
     double nxp = 0, nxt = 0, nxs = 0;
     if (O4) {
       const size_t o = (size_t)k * nr + n;
@@ -1033,9 +1059,10 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
       nxt = -dt * O4[2 * N + o];
       nxs = -dt * O4[3 * N + o];
     }
-    const double psiT0 = dT0 * JP;                                              // DT0_theta
     const size_t o = (size_t)k * nr + n;
     if (a.cnab2) {
+      const double grv = (k < M - 1) ? (-k1 * gr) * (Ra * Tv[k + 1] - Ras * Sv[k + 1]) : 0.0;
+      const double psiT0 = dT0 * JP;                                            // DT0_theta
       // explicit terms per unit time at this step, and the Adams-Bashforth 2 extrapolation
       const size_t ko = (size_t)k * nr + n;
       const double ep = (O4 ? -(DrQ[k] - O4[N + ko]) : 0.0) + a.Pr * grv;
@@ -1056,15 +1083,16 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
       R[2 * N + o] = fma(dt, xs, 2.0 * (rsq * Sv[k]));
       continue;
     }
-    R[o] = nxp + (Om + dtPr * grv);
-    R[N + o] = nxt + (rsq * Tv[k] - dt * psiT0);
-    R[2 * N + o] = nxs + (rsq * Sv[k] - dt * psiT0);
+    R[o] = nxp + (k < M - 1 ? lin_psi_rhs(Om, k1, gd, Ra, Ras, Tv[k + 1], Sv[k + 1]) : Om);
+    R[N + o] = nxt + lin_ts_rhs(rsq, Tv[k], dd, JP);
+    R[2 * N + o] = nxs + lin_ts_rhs(rsq, Sv[k], dd, JP);
   }
 }
 
 // The linear parts alone (fuse_rhs with the fused row kernel; k_fx_grid forms the same expressions in the split
-// path), with A2_SINE's D2 psi formed by k_fx_deriv.  One CTA per (row, shell).  Bound by the FP64 pipe (about 20
-// operations an element) and its column-strided loads: 39 us at 64 shells of 256 x 30, 76 us as k_rhs with D2 psi.
+// path), with A2_SINE's D2 psi formed by k_fx_deriv.  One CTA per (row, shell).  Bound by the FP64 pipe (about 16
+// operations an element, of them 12 in the loop) and its column-strided loads: 29 us at 64 shells of 256 x 30, 76 us as
+// k_rhs with D2 psi.
 __global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double* d2psi, size_t d2_stride) {
   after_previous_kernel();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1089,25 +1117,20 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double*
     Tv[k] = ts_on ? __ldg(Xs + N + o) : 0.0;
     Sv[k] = ts_on ? __ldg(Xs + 2 * N + o) : 0.0;
   }
-  const double dt = a.dt, dtPr = a.dt * a.Pr;
-  const double Ra = a.Ra[b], Ras = a.Ra_s[b];
-  const double ir2 = a.ir2s[n], rsq = a.rsq[n], dT0 = a.dT0[n], gr = a.gr[n];
+  const double Ra = a.Ra[b], Ras = a.Ra_s[b], ir2 = a.ir2s[n], rsq = a.rsq[n];
+  const double gd = a.dt * a.Pr * a.gr[n], dd = a.dt * a.dT0[n];
   __syncthreads();
   parity_suffix<double>(pv, Sc, M);
   next_kernel_may_start();
   double* R = a.rhs + (size_t)b * a.rhs_stride;
   for (int k = tid; k < M; k += bd) {
-    const double s1 = (k + 1 < M) ? Sc[k + 1] : 0.0;
     const double k1 = fx_int(k + 1), k2 = fx_int(k + 2);
-    const double JP = (k == 0) ? 1.0 * s1 : k1 * pv[k - 1] + 2.0 * s1;    // J_theta_RT
-    const double s2 = (k + 2 < M) ? Sc[k + 2] : 0.0;
-    const double Om = D2p[k] - k1 * ir2 * (k2 * pv[k] + 2.0 * s2);       // A2_SINE
-    const double grv = (k < M - 1) ? (-k1 * gr) * (Ra * Tv[k + 1] - Ras * Sv[k + 1]) : 0.0;
-    const double psiT0 = dT0 * JP;                                              // DT0_theta
+    const double jt = lin_jt(k, k1, k > 0 ? pv[k - 1] : 0.0, (k + 1 < M) ? Sc[k + 1] : 0.0);
+    const double om = lin_a2(D2p[k], k1, k2, ir2, pv[k], (k + 2 < M) ? Sc[k + 2] : 0.0);
     const size_t o = (size_t)k * nr + n;
-    R[o] = Om + dtPr * grv;
-    R[N + o] = rsq * Tv[k] - dt * psiT0;
-    R[2 * N + o] = rsq * Sv[k] - dt * psiT0;
+    R[o] = k < M - 1 ? lin_psi_rhs(om, k1, gd, Ra, Ras, Tv[k + 1], Sv[k + 1]) : om;
+    R[N + o] = lin_ts_rhs(rsq, Tv[k], dd, jt);
+    R[2 * N + o] = lin_ts_rhs(rsq, Sv[k], dd, jt);
   }
 }
 
