@@ -78,20 +78,23 @@ class ShellBatch:
                        priority=-1 if k in high else 0)
             plan.reserve(len(idx))
             self.groups.append(g)
-        # Starting point of the tuning (measured on the 64-shell mixed batch of N_r in {20..36}, N_theta in
-        # {64..384}): the groups' launches share the GPU inside one graph, so the nonlinear term runs as the
-        # fused row kernel once the batch fills the SMs; the chains run in the reference's order of
-        # operations, a shell's three chains of one parity per CTA (layout 8: 4 nr^2 multiply-adds per mode
-        # instead of 7; the library runs layout 5 where the right-hand side is fused or FP32, and layout 6
-        # where the three rings do not fit a CTA), and chunked chains for N_theta >= 256 with the FP32
-        # nonlinear term, where the long chains of the largest shells set the critical path, each chunk in
-        # the reference's order too (layout 10: 96.0k shell-steps/s with it on every group against 88.3k
-        # for the pre-pass chunks of layout 2); in FP64 the nonlinear term dominates and chunking does not
-        # pay.
+        # Starting point of the tuning: the groups' launches share the GPU inside one graph, so the nonlinear term
+        # runs as the fused row kernel once the batch fills the SMs.  Chunked chains shorten the launch while the
+        # batch leaves SMs idle, and cost correction matvecs once it fills them, so the chains go by the whole
+        # batch's shells.  ms a launch of 10 steps on 152 SMs, N_r 20..36, N_theta 64..384 (a second set, N_r 16..48,
+        # N_theta 48..384, has the same lines within 5%):
+        #   shells            8           16           32           40           48           56
+        #   whole (8)    2.21 / 2.35  3.08 / 3.62  2.73 / 3.32  3.56 / 4.64  3.88 / 5.59  4.28 / 6.23   mixed / FP64
+        #   per group    1.00 / 1.21  2.35 / 3.04  2.57 / 3.55  3.77 / 5.30  4.44 / 6.45  5.11 / 7.46
+        #   10, M >= 128 1.09 / 1.28  2.25 / 2.81  2.22 / 3.08  3.34 / 4.75  3.97 / 5.97  4.48 / 6.80
+        #   10, M >= 256 1.26 / 1.28  2.23 / 2.76  2.25 / 3.02  3.21 / 4.58  3.82 / 5.83  4.32 / 6.59
+        # (128 shells, mixed: 6.21 whole, 7.00 with chunks for M >= 256.)
         sms = _torch().cuda.get_device_properties(self.device).multi_processor_count
         total_rows = sum(g.plan.nr * len(g.idx) for g in self.groups)
+        n = len(shells)
+        chunked = 128 if 4 * n <= sms else 256 if precision == "mixed" and 3 * n <= sms else 1 << 30
         for g in self.groups:
-            g.plan.set_chain_layout(10 if (precision == "mixed" and g.plan.N_fm >= 256) else 8)
+            g.plan.set_chain_layout(0 if 15 * n <= sms else 10 if g.plan.N_fm >= chunked else 8)
             g.plan.set_fx_split(1 if 2 * total_rows > sms else 0)
         self.graph = None
         self.steps_per_launch = 0
