@@ -97,31 +97,19 @@ int sdd_plan_create(const sdd_plan_desc* desc, sdd_plan** plan);
 int sdd_plan_destroy(sdd_plan* plan);
 /* Pre-allocates the plan's workspace for up to max_batch shells (otherwise grown on first use). */
 int sdd_plan_reserve(sdd_plan* plan, int max_batch);
-/* Chain-kernel layout of the implicit solves: 0 automatic (chunked while its CTAs fit the GPU at two per
- * SM, layout 3 before 2, else split rows over 4 warps when the launch leaves SMs idle, else layout 8 (6 for
- * launches of fewer than three fields or where its shared memory does not fit, 5 where the right-hand side
- * is fused or FP32)),
- * 1 one lane per row, 2 chunked (each chain cut into chunks that run concurrently, joined by a short
- * sequential carried-state recurrence), 3 chunked with shorter chunks joined by a parallel carry
- * (precomputed products of the chunk maps, all applied at once), 4 split rows over 4 warps, 5 split rows
- * over 2 lanes in 2 warps (nr <= 32; 4 otherwise), 6 / 7 the chains in the reference's own order of
- * operations (Matrix_Operators.py:1139-1164, 1056-1083: per step D2 f_e, then Linv_j (g_j + b)), without the
- * h = Linv g pre-pass of the other layouts: 4 nr^2 multiply-adds per mode instead of 7, rows over 2 / 4
- * lanes; they need the full FP64 right-hand side, so launches with the fused or the FP32 right-hand side run
- * layout 5.  8: the same order of operations with the three chains of one (parity, shell) in one CTA, psi
- * rows over 2 lanes, T and S one lane per row, so every warp carries about the same work per step (launches
- * of fewer than three fields run layout 6).  9: the h pre-pass form (any right-hand side: fused, FP32) with
- * the three chains of one (parity, shell) in one CTA, psi rows over 2 lanes, T and S one lane per row
- * (launches of fewer than three fields, or whose three rings exceed a CTA's shared memory, run layout 5).
- * 10 / 11: the chunks of layouts 2 / 3 with each chunk in the reference's order of operations (no h
- * pre-pass; with the right-hand side fused into the split nonlinear term each chunk forms its own; FP32
- * right-hand sides run layouts 2 / 3).  The automatic choice runs its chunked layout as 10 / 11 where the
- * full FP64 right-hand side is there, and as 2 / 3 where it is fused (one shell: the pre-pass form is
- * faster there).  Set by the batch autotuner; no counterpart in the reference. */
+/* Chain layout of the implicit solves: 0 automatic (by the batch: 3 while its chunks and products fit the GPU,
+ * 2 for moderate batches, else whole chains), 1 and 4 to 9 whole chains (one kernel; the numbers are kept for
+ * callers and recorded tunings that select them), 2 / 10 chunked (each chain cut into chunks that run concurrently,
+ * joined by a short sequential carried-state recurrence), 3 / 11 chunked with shorter chunks joined by a parallel
+ * carry (precomputed products of the chunk maps, all applied at once).  h = Linv g of every mode
+ * (Matrix_Operators.py:1139-1164, 1056-1083) is formed ahead of the chains.  Layouts agree to rounding; within one, a
+ * shell's result does not depend on its batch.  The automatic choice reports its chunks as 10 / 11 where the full
+ * right-hand side is there, and as 2 / 3 where it is fused.  Set by the batch autotuner; no counterpart in the
+ * reference. */
 int sdd_plan_set_chain_layout(sdd_plan* plan, int layout);
 /* Chunk length (steps per chunk) of chunk set 0 (layouts 2 / 10, sequential carry) or 1 (layouts 3 / 11,
  * parallel carry): the set's tables are rebuilt for kc and the carry workspace regrown; kc = 0 restores the
- * plan's rule (round(sqrt(2 S)) / round(sqrt(S / 2)) steps, S = N_fm / 2).  2 <= kc <= S, at most 64 chunks
+ * plan's rule (round(sqrt(2 S)) / round(sqrt(S / 2)) steps, the latter round(sqrt(0.72 S)) with nr > 32; S = N_fm / 2).  2 <= kc <= S, at most 64 chunks
  * (32 for set 1, whose products grow as the square); otherwise SDD_ERR_ARG.  Synchronises the device.  Set
  * by the batch autotuner; no counterpart in the reference. */
 int sdd_plan_set_chunk_length(sdd_plan* plan, int set, int kc);

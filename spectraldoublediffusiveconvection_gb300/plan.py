@@ -132,12 +132,8 @@ class Plan:
             _lib.check(self._L.sdd_plan_reserve(self._h, int(batch)), "sdd_plan_reserve")
 
     def set_chain_layout(self, layout):
-        """0 automatic, 1 one lane per row, 2 chunked (sequential carry), 3 chunked (parallel carry), 4 rows
-        split over 4 warps, 5 rows split over 2 lanes in 2 warps, 6 / 7 the reference's order of operations
-        without the h pre-pass, rows over 2 / 4 lanes (full right-hand sides only; otherwise 5), 8 the same
-        with a (parity, shell)'s three chains in one CTA, 9 the pre-pass form with a (parity, shell)'s three
-        chains in one CTA, 10 / 11 the chunks of 2 / 3 in the reference's order (FP64 right-hand sides, full
-        or fused; otherwise 2 / 3) (sdd_plan_set_chain_layout); the results agree to rounding."""
+        """0 automatic (by the batch), 2 / 10 chunked chains with a sequential carry, 3 / 11 with a parallel
+        carry, 1 and 4 to 9 whole chains (sdd_plan_set_chain_layout); the results agree to rounding."""
         _lib.check(self._L.sdd_plan_set_chain_layout(self._h, int(layout)), "sdd_plan_set_chain_layout")
         self.chain_layout = int(layout)
 
