@@ -111,8 +111,9 @@ __device__ __forceinline__ i64 fx_rmul(i64 x, int h1, int h0) {
 // calling thread wrote the elements k = tid, tid + blockDim, ... (no barrier is needed before the call).
 // Afterwards the row holds round(x 2^(60 - E[t])) as 64-bit integers with sum |x| < 2^E[t]: the row's transform
 // and everything inside it stays below 2^61 (two rows of a pair).  E[t] = kFxBad marks a row with an infinity
-// or NaN (left as zeros); E of the row after an odd last one is a zero row's.  red: 2 nrows 32 words.  Ends with
-// a barrier.
+// or NaN (left as zeros); E of the row after an odd last one is a zero row's.  The sum is of whole numbers in units
+// of the row's largest exponent, so E does not depend on how many threads share the row.  red: 2 nrows 32 words.
+// Ends with a barrier.
 constexpr int kFxBad = 0x7fffffff;
 // (Out of line, with byte offsets into the dynamic shared memory, like the transforms' passes.)
 static __device__ __noinline__ void rows_to_fixed_at(int xv, int P, int nrows, int redo, int eo) {
@@ -124,30 +125,33 @@ static __device__ __noinline__ void rows_to_fixed_at(int xv, int P, int nrows, i
 #pragma unroll 1
   for (int t = 0; t < nrows; ++t) {
     const double* x = XV + t * P;
-    unsigned m = 0, s = 0;
+    unsigned m = 0;
 #pragma unroll 1
     for (int k = tid; k < P; k += bd) m = max(m, abs_hi(x[k]));
-    const int ew = (int)(__reduce_max_sync(0xffffffffu, m) >> 20);
+    m = __reduce_max_sync(0xffffffffu, m) >> 20;
+    if (lane == 0) red[t * 32 + warp] = m;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int t = 0; t < nrows; ++t) {
+    const double* x = XV + t * P;
+    const int em = (int)__reduce_max_sync(0xffffffffu, lane < nw ? red[t * 32 + lane] : 0u);
+    unsigned s = 0;                                    // (at most 2^18 an element)
 #pragma unroll 1
     for (int k = tid; k < P; k += bd) {
       const unsigned h = abs_hi(x[k]);
       const int e = (int)(h >> 20);
-      if (e) s += (((h & 0xfffffu) | 0x100000u) >> min(ew - e, 31)) + 1;
+      if (e) s += (((h & 0xfffffu) | 0x100000u) >> min(em - e + 3, 31)) + 1;
     }
     s = __reduce_add_sync(0xffffffffu, s);
-    if (lane == 0) {
-      red[t * 32 + warp] = (unsigned)ew;
-      red[(nrows + t) * 32 + warp] = s;
-    }
+    if (lane == 0) red[(nrows + t) * 32 + warp] = s;
   }
   __syncthreads();
 #pragma unroll 1
   for (int t = warp; t < ((nrows + 1) & ~1); t += nw) {
     const bool on = t < nrows && lane < nw;
-    const unsigned e = on ? red[t * 32 + lane] : 0u;
-    const unsigned s = on ? red[(nrows + t) * 32 + lane] : 0u;
-    const unsigned em = __reduce_max_sync(0xffffffffu, e);
-    const unsigned tot = __reduce_add_sync(0xffffffffu, s ? ((s >> 3) >> min(em - e, 31u)) + 1 : 0u);
+    const unsigned em = __reduce_max_sync(0xffffffffu, on ? red[t * 32 + lane] : 0u);
+    const unsigned tot = __reduce_add_sync(0xffffffffu, on ? red[(nrows + t) * 32 + lane] : 0u);
     if (lane == 0) E[t] = em >= 0x7ffu ? kFxBad : (int)em - 1040 + (32 - __clz((int)tot));
   }
   __syncthreads();

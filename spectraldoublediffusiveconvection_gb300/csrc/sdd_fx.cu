@@ -69,8 +69,8 @@ __device__ __forceinline__ void with_x(const FxArgs& a, int b, F&& body) {
 // The linear parts of the three right-hand sides (Main.py:262-280) at one row and mode, in the three kernels that form
 // them (k_fx_grid, k_rhs_lin, k_rhs), so that all give the same bits.  An FP64 instruction holds the pipe for 64 cycles
 // and a dependent one waits as long: fused multiply-adds, the row's scalars multiplied once, doublings in the exponent
-// and mode numbers without conversions leave 12 a mode of 22 (k_rhs_lin, 64 shells of 256 x 30: 38.9 -> 28.7 us, in a step 525 -> 516; mixed 315 -> 306;
-// one shell 41.5 -> 41.1).
+// and mode numbers without conversions leave 12 a mode of 22 (k_rhs_lin, 64 shells of 256 x 30: 38.9 -> 28.7 us, in a
+// step 525 -> 516; mixed 315 -> 306; one shell 41.5 -> 41.1).
 __device__ __forceinline__ double twice(double x) {
   const int hi = __double2hiint(x), lo = __double2loint(x), e = hi & 0x7ff00000, sgn = hi & (int)0x80000000;
   if (e == 0x7ff00000) return x;
