@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_rows(FxArgs a) {
 //   k_fx_prod (nr x 2 CTAs per shell): CTA (n, p) forms product pair p on the grid of row n (p = 0: the
 //     sine-type Q, R; p = 1: the cosine-type NT, NS) and runs their paired forward transform into out4.
 // Per element the operations and their order are those of k_fx_rows, so the results are identical.
-constexpr int kFxSplitThreads = 256;
+constexpr int kFxSplitThreads = 256;   // (up to kFxRowThreads: fx_split_threads)
 
 // FP32 grid kernels of the fused right-hand side keep FP64 copies of the row's psi, T, S and psi's parity
 // suffix sums (4 M doubles) for the linear parts, after the T-typed arrays.
@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, size_t grid_stride) {
+__global__ void __launch_bounds__(kFxRowThreads) k_fx_grid(FxArgs a, T* grid, size_t grid_stride) {
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
@@ -914,7 +914,7 @@ __global__ void __launch_bounds__(kFxSplitThreads) k_fx_grid(FxArgs a, T* grid, 
 }
 
 template <typename T, int MODE>
-__global__ void __launch_bounds__(kFxSplitThreads) k_fx_prod(FxArgs a, const T* grid, size_t grid_stride) {
+__global__ void __launch_bounds__(kFxRowThreads) k_fx_prod(FxArgs a, const T* grid, size_t grid_stride) {
   using C = typename Cplx<T>::type;
   using W = typename Cplx<T>::tw;
   using Tr = RowTr<T>;
@@ -1518,6 +1518,16 @@ static cudaError_t launch_fx_t(const FxArgs& a, int batch, cudaStream_t s) {
   return e;
 }
 
+// Threads of the split kernels' CTAs.  While every CTA has an SM of its own, what counts is the latency of the loops over
+// the row's P elements: as many threads as give each loop its fewest rounds (P = 384: one of 384 instead of two of 256;
+// us a step, 256 threads / this rule: 256 x 30 41.5 / 40.2, its residual 46.2 / 43.6, 540 x 65 138.5 / 136.8); with
+// more CTAs than SMs, 256, of which two share an SM.
+static int fx_split_threads(int P, long ctas) {
+  if (ctas > fx_sm_count()) return kFxSplitThreads;
+  const int passes = (P + kFxRowThreads - 1) / kFxRowThreads;
+  return std::max(128, ((P + passes - 1) / passes + 31) / 32 * 32);
+}
+
 template <typename T, int MODE>
 static cudaError_t launch_fx_split_t(const FxArgs& a, int batch, cudaStream_t s) {
   const int prec = sizeof(T) == 4 ? SDD_PREC_MIXED : SDD_PREC_FP64;
@@ -1531,16 +1541,16 @@ static cudaError_t launch_fx_split_t(const FxArgs& a, int batch, cudaStream_t s)
   {
     static unsigned long long done = 0;
     if ((e = ensure_smem_attr(k_fx_grid<T>, &done)) != cudaSuccess) return e;
-    e = launch_kernel(k_fx_grid<T>, dim3(a.nr, 5, batch), dim3(kFxSplitThreads), fx_grid_smem_bytes(a.M, a.P, prec),
-                   s, a, grid, gs);
+    e = launch_kernel(k_fx_grid<T>, dim3(a.nr, 5, batch), dim3(fx_split_threads(a.P, 5L * a.nr * batch)),
+                      fx_grid_smem_bytes(a.M, a.P, prec), s, a, grid, gs);
     ktimer_mark(SDD_K_FX_GRID, s);
     if (e != cudaSuccess || MODE == 2) return e;
   }
   constexpr int PM = MODE == 1 ? 1 : 0;
   static unsigned long long done = 0;
   if ((e = ensure_smem_attr(k_fx_prod<T, PM>, &done)) != cudaSuccess) return e;
-  e = launch_kernel(k_fx_prod<T, PM>, dim3(a.nr, 2, batch), dim3(kFxSplitThreads), fx_prod_smem_bytes(a.P, prec), s,
-                 a, (const T*)grid, gs);
+  e = launch_kernel(k_fx_prod<T, PM>, dim3(a.nr, 2, batch), dim3(fx_split_threads(a.P, 2L * a.nr * batch)),
+                    fx_prod_smem_bytes(a.P, prec), s, a, (const T*)grid, gs);
   ktimer_mark(SDD_K_FX_PROD, s);
   return e;
 }
