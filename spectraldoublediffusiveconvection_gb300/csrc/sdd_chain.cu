@@ -792,7 +792,8 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   // layout 9 needs all three fields and its three rings in one CTA
   if (layout == 9 && (nfields != 3 || a.field0 != 0 || layout_bytes(9, a.M, a.nr, a.ldl) > (size_t)optin))
     layout = 5;
-  // layouts 10 / 11 (chunks in the reference's order) need an FP64 right-hand side (full or fused): else 2 / 3
+  // (the numbers 4 to 11 are kept for callers that select or record them: 10 / 11 are the chunks of 2 / 3, reported as
+  // 2 / 3 with an FP32 right-hand side)
   if ((layout == 10 || layout == 11) && a.g32) layout -= 8;
   // Chunks shorten the chains' critical path and add a correction matvec per mode (nr > 32: two, or their columns
   // in halves), so what decides is the batch.  Parallel carry while its chunks and products fit the chip (us a
@@ -804,7 +805,7 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   const bool wide = a.nr > 32;
   if (layout == 0 && a.M > 16 && c3.nch > 1 && c3.GA4 && 4 * nfields * batch * c3.nch <= (wide ? 3 : 7) * sms) layout = 3;
   if (layout == 0 && a.M >= 40 && c2.nch > 1 && c2.GA4 && (wide ? 4 : 1) * nfields * batch <= sms) layout = 2;
-  // chosen chunks run in the reference's order where the full FP64 right-hand side is there (no pre-pass)
+  // (the same chunks; the number says that the full FP64 right-hand side is there)
   if (a.layout == 0 && (layout == 2 || layout == 3) && !a.split_fx && !a.g32) layout += 8;
   // layouts 6 / 7 need the full right-hand side in FP64: with the fused or the FP32 one, the pre-pass form
   if ((layout == 6 || layout == 7) && (a.split_fx || a.g32)) layout = 5;
