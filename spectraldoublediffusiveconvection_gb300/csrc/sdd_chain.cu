@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(128) k_mode_mv(ChainArgs a, int nfields, int b
           const double* o4 = a.out4 + (size_t)b * a.out_stride + ro;
           v.x[p] = o4[(size_t)(field + 1) * N + e];      // psi: R
           v.ln[p] = a.lin[(size_t)b * a.g_stride + foff + e];
-          if (a4) v.q[p] = a.q32 ? (double)__ldg(a.q32 + (size_t)b * N + ro + e) : o4[e];
+          if (a4) v.q[p] = a.q32 ? (double)a.q32[(size_t)b * N + ro + e] : o4[e];
         }
       }
       if (FIX && sg + 1 == nseg && r < nr) v.ln[0] = a.f[(size_t)b * a.f_stride + foff + r];

@@ -59,10 +59,10 @@ template <typename T, typename F>
 __device__ __forceinline__ void with_x(const FxArgs& a, int b, F&& body) {
   if (sizeof(T) == 4 && a.X32) {
     const float* x = a.X32 + (size_t)b * a.x32_stride;
-    body([x](size_t e) { return (T)__ldg(x + e); });
+    body([x](size_t e) { return (T)x[e]; });
   } else {
     const double* x = a.X + (size_t)b * a.x_stride;
-    body([x](size_t e) { return (T)__ldg(x + e); });
+    body([x](size_t e) { return (T)x[e]; });
   }
 }
 
@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(32 * deriv_warps(LD), LD <= 32 ? 2 : 1)
     if (a.X32 && !a.fix.on) {                          // the caller's FP32 copy (the same values)
       for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) {
         const int m = q / (3 * nr), e = q - m * 3 * nr, f = e / nr;
-        xv[q] = __ldg(a.X32 + (size_t)b * a.x32_stride + f * N + (size_t)(k0 + m) * nr + (e - f * nr));
+        xv[q] = a.X32[(size_t)b * a.x32_stride + f * N + (size_t)(k0 + m) * nr + (e - f * nr)];
       }
     } else {
       for (int q = threadIdx.x; q < kn * 3 * nr; q += blockDim.x) xv[q] = (float)xd[q];
@@ -844,9 +844,9 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_grid(FxArgs a, T* grid, si
     DTv[k] = dtv;
     DCv[k] = dcv;
     if (pv64) {
-      pv64[k] = psi_on ? __ldg(Xs + (size_t)k * nr + n) : 0.0;
-      pv64[2 * M + k] = ts_on ? __ldg(Xs + N + (size_t)k * nr + n) : 0.0;
-      pv64[3 * M + k] = ts_on ? __ldg(Xs + 2 * N + (size_t)k * nr + n) : 0.0;
+      pv64[k] = psi_on ? Xs[(size_t)k * nr + n] : 0.0;
+      pv64[2 * M + k] = ts_on ? Xs[N + (size_t)k * nr + n] : 0.0;
+      pv64[3 * M + k] = ts_on ? Xs[2 * N + (size_t)k * nr + n] : 0.0;
     }
   }
   });
@@ -1020,24 +1020,24 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
     const double* ps = Xs + (size_t)k * nr;
     double d2 = 0, pn = 0, q = 0;
     if (psi_on) {
-      for (int m = 0; m < nr; ++m) d2 = fma(opr[nr + m], __ldg(ps + m), d2);
-      pn = __ldg(ps + n);
+      for (int m = 0; m < nr; ++m) d2 = fma(opr[nr + m], ps[m], d2);
+      pn = ps[n];
     }
     if (O4 && a.q32) {         // FP32 nonlinear term: Dr Q in FP32 (the order of the chains' fused_g)
       const float* qs = a.q32 + (size_t)b * M * nr + (size_t)k * nr;
       const float* drn = a.Dr32 + (size_t)n * nr;
       float d = 0.0f;
-      for (int m = 0; m < nr; ++m) d = fmaf(__ldg(drn + m), __ldg(qs + m), d);
+      for (int m = 0; m < nr; ++m) d = fmaf(__ldg(drn + m), qs[m], d);
       q = (double)d;
     } else if (O4) {
       const double* qs = O4 + (size_t)k * nr;
-      for (int m = 0; m < nr; ++m) q = fma(opr[m], __ldg(qs + m), q);
+      for (int m = 0; m < nr; ++m) q = fma(opr[m], qs[m], q);
     }
     pv[k] = pn;
     D2p[k] = d2;
     DrQ[k] = q;
-    Tv[k] = ts_on ? __ldg(Xs + N + (size_t)k * nr + n) : 0.0;
-    Sv[k] = ts_on ? __ldg(Xs + 2 * N + (size_t)k * nr + n) : 0.0;
+    Tv[k] = ts_on ? Xs[N + (size_t)k * nr + n] : 0.0;
+    Sv[k] = ts_on ? Xs[2 * N + (size_t)k * nr + n] : 0.0;
   }
   __syncthreads();
   parity_suffix<double>(pv, Sc, M);
@@ -1112,10 +1112,10 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs_lin(RhsArgs a, const double*
     const bool psi_on = !(a.sym && (k % 2 == 0));
     const bool ts_on = !(a.sym && (k % 2 == 1));
     const size_t o = (size_t)k * nr + n;
-    pv[k] = psi_on ? __ldg(Xs + o) : 0.0;
-    D2p[k] = psi_on ? __ldg(d2 + o) : 0.0;
-    Tv[k] = ts_on ? __ldg(Xs + N + o) : 0.0;
-    Sv[k] = ts_on ? __ldg(Xs + 2 * N + o) : 0.0;
+    pv[k] = psi_on ? Xs[o] : 0.0;
+    D2p[k] = psi_on ? d2[o] : 0.0;
+    Tv[k] = ts_on ? Xs[N + o] : 0.0;
+    Sv[k] = ts_on ? Xs[2 * N + o] : 0.0;
   }
   const double Ra = a.Ra[b], Ras = a.Ra_s[b], ir2 = a.ir2s[n], rsq = a.rsq[n];
   const double gd = a.dt * a.Pr * a.gr[n], dd = a.dt * a.dT0[n];
@@ -1180,18 +1180,18 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs32(RhsArgs a) {
     const float* ps = Xs + (size_t)k * nr;
     float d2 = 0.0f, pn = 0.0f, q = 0.0f;
     if (psi_on) {
-      for (int m = 0; m < nr; ++m) d2 = fmaf(opr[nr + m], __ldg(ps + m), d2);
-      pn = __ldg(ps + n);
+      for (int m = 0; m < nr; ++m) d2 = fmaf(opr[nr + m], ps[m], d2);
+      pn = ps[n];
     }
     if (O4) {
       const float* qs = a.q32 + (size_t)b * M * nr + (size_t)k * nr;
-      for (int m = 0; m < nr; ++m) q = fmaf(opr[m], __ldg(qs + m), q);
+      for (int m = 0; m < nr; ++m) q = fmaf(opr[m], qs[m], q);
     }
     pv[k] = pn;
     D2p[k] = d2;
     DrQ[k] = q;
-    Tv[k] = ts_on ? __ldg(Xs + N + (size_t)k * nr + n) : 0.0f;
-    Sv[k] = ts_on ? __ldg(Xs + 2 * N + (size_t)k * nr + n) : 0.0f;
+    Tv[k] = ts_on ? Xs[N + (size_t)k * nr + n] : 0.0f;
+    Sv[k] = ts_on ? Xs[2 * N + (size_t)k * nr + n] : 0.0f;
   }
   __syncthreads();
   parity_suffix<float>(pv, Sc, M);
@@ -1252,8 +1252,8 @@ __global__ void __launch_bounds__(kFxThreads) k_theta_op(ThetaArgs a) {
     if (on) {
       const double* ps = g + (size_t)k * nr;
       if (a2)
-        for (int m = 0; m < nr; ++m) d2 = fma(opr[m], __ldg(ps + m), d2);
-      pn = __ldg(ps + n);
+        for (int m = 0; m < nr; ++m) d2 = fma(opr[m], ps[m], d2);
+      pn = ps[n];
     }
     pv[k] = pn;
     D2p[k] = d2;

@@ -23,7 +23,10 @@ void set_cuda_error(cudaError_t e);
 // EVERY kernel launched this way calls after_previous_kernel(), which waits for the completion (and the writes) of all
 // kernels before it, ahead of anything it reads that a kernel writes and of every write to global memory.  Before it
 // stand only loads of the plan's tables (operators, twiddles, blocks, chain scalars: written and synchronised when the
-// plan or its chunk tables are made).  Dependents hide most of a launch's latency: single steps of 64 x 20 47.5 -> 31
+// plan or its chunk tables are made).  The kernel is resident while the one before it still writes, so only those tables
+// go through __ldg: a read-only load promises that its data do not change during the whole kernel, and the compiler may
+// move it across the wait.  Everything that a kernel writes (states, derivatives, right-hand sides, products) is read by
+// plain loads after the wait.  Dependents hide most of a launch's latency: single steps of 64 x 20 47.5 -> 31
 // us, 256 x 30 62.8 -> 46.5, 64 shells 618 -> 606; inside the captured step graphs 44.6 -> 43.4.
 // next_kernel_may_start() stands where a kernel's last phase begins: the next kernel's CTAs come up and load their
 // tables beside it (us a step: 256 x 30 43.5 -> 41.5, 540 x 65 146 -> 139, 3 shells of 128 x 28 mixed 44.4 -> 41.7, 90 x

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_deriv_tc(TcArgs a) {
         for (int e = tid; e < cnt * nr; e += kTcThreads) cp_async4(dst + e, src + e);
       } else {
         const double* src = a.X + (size_t)b * a.x_stride + (size_t)fk * nr;
-        for (int e = tid; e < cnt * nr; e += kTcThreads) dst[e] = (float)__ldg(src + e);
+        for (int e = tid; e < cnt * nr; e += kTcThreads) dst[e] = (float)src[e];
       }
       r0 += cnt;
     }
