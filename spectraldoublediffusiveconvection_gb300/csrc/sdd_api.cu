@@ -630,6 +630,7 @@ int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
   if (fx_smem_bytes(M, P, SDD_PREC_FP64) > fx_rows_max_dynamic_smem(SDD_PREC_FP64)) return SDD_ERR_UNSUPPORTED;
   const FftPlan* fp = get_fft_plan(P);
   if (!fp) return SDD_ERR_UNSUPPORTED;
+  if (!d->D2_A4 || !d->ir2_A4 || !d->ir4_A4) return SDD_ERR_ARG;   // (read on the host alone: the psi step matrices)
   sdd_plan* p = new sdd_plan();
   std::memset(p, 0, sizeof(*p));
   p->M = M; p->nr = nr; p->P = P; p->ldl = fx_ld(nr); p->sym = d->symmetric ? 1 : 0;
