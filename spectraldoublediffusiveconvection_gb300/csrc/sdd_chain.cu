@@ -16,9 +16,10 @@
 // Arithmetic.  An FP64 warp instruction holds its SM sub-partition for 64 cycles on GB300, and a chain is one
 // dependent matvec after another, so with FP64 matvecs a chain step cost (columns per lane) x 64 cycles.  Every
 // block matvec here runs in 64-bit fixed point (sdd_fixed.cuh): blocks as digits scaled per row by its
-// 1-norm, the operand scaled by its largest entry to 57 bits, three IMAD.WIDE (13 to 15 cycles) a column instead
+// 1-norm, the operand scaled by its largest entry to 61 bits, three IMAD.WIDE (13 to 15 cycles) a column instead
 // of 64.  The carried states (f_e, bf_e, b) stay FP64; h, the matvec and its parts are summed in fixed point and
-// rounded once.  Error of a matvec against extended precision: 1e-18 to 1e-17 of the result, FP64's 1.5e-16.
+// rounded once.  Error of a matvec against extended precision: 1e-18 to 2e-17 of the result, FP64's 1e-16 to 5e-16
+// (row by row: sdd_fixed.cuh).
 // An operand with an infinity takes an FP64 path with the same blocks (fx_dot_slow); one with a NaN gives NaN.
 //
 // k_chain_fx: a CTA holds one parity's chains of psi (two groups of warps: one carries f_e and multiplies by
@@ -873,11 +874,11 @@ __global__ void __launch_bounds__(64) k_to_fixed(const double* src, size_t src_s
     double l1 = 0.0;
     if (r < nr)
       for (int c = 0; c < nr; ++c) l1 += fabs(ldexp(a[(size_t)c * ld + r], -cx[c]));
-    // 2^ea above the sum with room for its rounding
-    const unsigned h = abs_hi(l1 * (1.0 + 1e-13)) >> 20;
+    // 2^ea above the sum, with room for its rounding and for that of the high digits (31 bits and the sign)
+    const unsigned h = abs_hi(l1 * (1.0 + 1e-9)) >> 20;
     const int ea = h == 0x7ff ? kFxBad : (int)h - 1022;
     for (int c = 0; c < ldl; ++c) {
-      const i64 A = r < nr && c < nr && ea != kFxBad ? d2fx(a[(size_t)c * ld + r], 1027 + ea + cx[c]) : 0;
+      const i64 A = r < nr && c < nr && ea != kFxBad ? d2fx(a[(size_t)c * ld + r], 1084 - kMvA + ea + cx[c]) : 0;
       reinterpret_cast<int2*>(o)[(size_t)c * ldl + r] = mv_digits(A);
     }
     rexp[r] = ea;

@@ -5,12 +5,19 @@
 // the block matvecs of the implicit solves are sums of products with known operators over a row or a vector
 // whose largest entry is easy to find, so they run on integers: a vector is scaled by one power of two to a
 // 64-bit integer each, an operator by one per row and one per column, both are split into two signed digits
-// (transforms: value = hi 2^32 + lo; matvecs: hi 2^27 + lo with 30 bits of hi, so that no sum of products of 64
-// columns overflows), and a product keeps three of its four digit products in 64-bit accumulators (hi hi, hi lo
-// and lo hi; lo lo is below the last bit kept).  The sums are exact, so they do not depend on their order.  Rounding to 57-60 bits below a bound on the vector replaces FP64's 53
-// bits per operation: against extended precision the errors are below FP64's (transforms: the bound is the
-// row's 1-norm, which no intermediate value exceeds; matvecs: 1e-18 to 1e-17 of the result's norm against
-// 1.5e-16 to 1e-15 on states of the time step).
+// (transforms: value = hi 2^32 + lo; matvecs: see mv_digits), and a product keeps three of its four digit products in
+// 64-bit accumulators (hi hi, hi lo and lo hi; lo lo is below the last bit kept).  The sums are exact, so they do not
+// depend on their order.  Rounding to 59-61 bits below a bound on the vector replaces FP64's 53 bits per operation.
+// Transforms: the bound is the row's 1-norm, which no intermediate value exceeds; the errors are below FP64's.
+// Matvecs: operators keep 59 bits below a row's 1-norm, operands 61 below their largest entry, both after the
+// columns' scales 2^cx, so a row r of a product A x is off by at most
+//   2^-58 (n + 2) (sum_k |A_rk| 2^-cx_k) max_k |x_k 2^cx_k|      (n columns)
+// and in the norm by less than FP64: on smooth profiles Dr's products 0.03 to 0.4 of FP64's error (N_r 8 to 65; rows
+// against their own sum |A||x| 0.4 of a rounding at most, FP64 0.3 to 0.6), the solves' 1e-18 to 2e-17 of the result
+// against 1e-16 to 5e-16.  What FP64 has and this has not is the relative precision of single small entries: where the operand
+// falls off steeply (a layer of 1/60 of the gap), rows in its tail, whose own sum |A||x| is 1e-3 to 1e-12 of the largest,
+// keep 2e-15 to 4e-13 of that sum (N_r 20 to 65) where FP64 keeps 2e-16 and the inverse itself is good to 1e-15 to
+// 3e-14.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -174,7 +181,7 @@ __device__ __forceinline__ void rows_to_fixed(double* XV, int P, int nrows, void
 // ---- block matvecs -------------------------------------------------------------------------------
 // An nr x nr block A in global memory, padded with zeros to L x L (L = fx_ld(nr), so that the inner loops have
 // no remainder) and its columns scaled to a = A 2^-cx with |a| < 1: word [col][row] = the two digits of
-// round(a 2^(57 - ea)) (lo in the low half), then the L rows' exponents ea as ints, sum over a row of
+// round(a 2^(59 - ea)) (lo in the low half), then the L rows' exponents ea as ints, sum over a row of
 // |a| < 2^ea (kFxBad: a row with an infinity or NaN), and the L columns' exponents cx.  Operands are scaled by
 // 2^cx before their largest entry sets their fixed point: so the bits kept are relative to the largest product
 // A_kc x_c, not to the largest x_c (the Chebyshev operators' columns differ by N^2 to N^4, and so do a state's
@@ -186,11 +193,16 @@ __device__ __forceinline__ const int* fx_row_exp(const i64* blk, int ld) {
 }
 __device__ __forceinline__ const int* fx_col_exp(const i64* blk, int ld) { return fx_row_exp(blk, ld) + ld; }
 
-// A matvec's digits: v = hi 2^27 + lo, lo in [-2^26, 2^26), |v| <= 2^57.
-__device__ __forceinline__ int2 mv_digits(i64 v) {
-  return make_int2(((int)v << 5) >> 5, (int)((v + (1ll << 26)) >> 27));
+// A matvec's digits (lo, hi).  Operators: 59 bits, hi 2^28 + lo with lo in [-2^27, 2^27), hi 31 bits and its sign.
+// Operands: 61 bits, hi 2^32 + lo with lo in [-2^31, 2^31), |hi| <= 2^29.  So the sums of at most 64 columns stay in
+// 64 bits: a row's |a| add up to 2^59 at most (its scale), hence hi hi to 2^60, hi lo to 2^31 2^31, and lo hi, whose
+// operator digits have no such bound, to 64 2^27 2^29.  (27 and 27 bits of lo, 57 of both, cost the same three
+// multiplies and lost what FP64 keeps: Dr's products had 1.3 times FP64's error at N_r = 30, 3.2 times at 65.)
+constexpr int kMvA = 59, kMvALo = 28, kMvX = 61;
+__device__ __forceinline__ int2 mv_digits(i64 a) {
+  return make_int2(((int)a << (32 - kMvALo)) >> (32 - kMvALo), (int)((a + (1ll << (kMvALo - 1))) >> kMvALo));
 }
-__device__ __forceinline__ i64 mv_value(int2 d) { return ((i64)d.y << 27) + d.x; }
+__device__ __forceinline__ i64 mv_value(int2 a) { return ((i64)a.y << kMvALo) + a.x; }
 
 // An operand's exponent (biased, after its column scale): x = 0 counts below every number, an infinity above
 // (kFxInf), a NaN above that (kFxBad).
@@ -201,10 +213,10 @@ __device__ __forceinline__ int fx_key(double x, int cx) {
   if (e == 0x7ff) return ((h & 0xfffffu) | (unsigned)__double2loint(x)) ? kFxBad : kFxInf;
   return e ? e + cx : -0x10000;
 }
-// The operand's digits, 57 bits below the largest exponent em; with em = kFxInf its raw bits.
+// The operand's digits, kMvX bits below the largest exponent em; with em = kFxInf its raw bits.
 __device__ __forceinline__ int2 fx_digits(double x, int cx, int em) {
-  const i64 X = em >= kFxInf ? __double_as_longlong(x) : d2fx(x, 5 + em - cx);
-  return em >= kFxInf ? make_int2((int)X, (int)(X >> 32)) : mv_digits(X);
+  const i64 X = em >= kFxInf ? __double_as_longlong(x) : d2fx(x, 1084 - 1022 - kMvX + em - cx);
+  return make_int2(fx_lo(X), em >= kFxInf ? (int)(X >> 32) : fx_hi(X));
 }
 
 // A product's unit: fx_dot's integer is the product times 2^(kFxMvExp - ea - em).
@@ -237,12 +249,20 @@ __device__ __forceinline__ double fx_sum(double h, FxVal p, FxVal q) {
   return LAT ? fx2d_lat(v, -em) : fx2d(v, -em);
 }
 
-// Row A of a block in shared memory (column stride LD words) times NC operand digits xs, in units of 2^53 of the
-// operands' units.
+// The sums of hi hi, hi lo and lo hi (operator, operand) as one integer in units of 2^59 of the digits' units.
+struct FxPart {
+  i64 t2, t1, t0;
+  __device__ __forceinline__ i64 value() const {
+    return (t2 << 1) + (((t1 >> 4) + t0 + (1ll << (kMvALo - 2))) >> (kMvALo - 1));
+  }
+};
+static_assert(kMvA + kMvX - 61 == 59 && 32 - kMvALo == 4, "FxPart::value");
+
+// Row A of a block in shared memory (column stride LD words) times NC operand digits xs.
 template <int NC, int LD>
 __device__ __forceinline__ i64 fx_dot(const int2* A, const int2* xs) {
   const int4* x4 = reinterpret_cast<const int4*>(xs);
-  i64 t2 = 0, t1 = 1ll << 25, t0 = 0;
+  i64 t2 = 0, t1 = 0, t0 = 0;
 #pragma unroll
   for (int c = 0; c < NC; c += 2) {
     const int4 v = x4[c >> 1];
@@ -254,7 +274,7 @@ __device__ __forceinline__ i64 fx_dot(const int2* A, const int2* xs) {
     t1 = fx_mad(b.y, v.z, t1);
     t0 = fx_mad(b.x, v.w, t0);
   }
-  return (t2 << 1) + ((t1 + t0) >> 26);
+  return FxPart{t2, t1, t0}.value();
 }
 
 // The same product in FP64 over columns [c0, c1) of row r, for an operand with an infinity (em = kFxInf: raw
@@ -266,9 +286,9 @@ static __device__ __noinline__ double fx_dot_slow(const i64* blk, int ld, int r,
   double acc = 0.0;
   for (int c = c0; c < c1; ++c) {
     const int2 a = A[(size_t)c * ld], x = xs[c];
-    const double av = ea == kFxBad ? fx_nan() : ldexp(__ll2double_rn(mv_value(a)), ea - 57 + cx[c]);
+    const double av = ea == kFxBad ? fx_nan() : ldexp(__ll2double_rn(mv_value(a)), ea - kMvA + cx[c]);
     const double xv = em >= kFxInf ? __hiloint2double(x.y, x.x)
-                                   : ldexp(__ll2double_rn(mv_value(x)), em - (1022 + 57) - cx[c]);
+                                   : ldexp(__ll2double_rn(((i64)x.y << 32) + x.x), em - (1022 + kMvX) - cx[c]);
     acc = fma(av, xv, acc);
   }
   return acc;
@@ -305,9 +325,6 @@ __device__ __forceinline__ FxVal block_vec(const i64* blk, int nr, int r, const 
 
 // Columns [c0, c0 + NC) of a lane's row of a block in registers (its loads all in flight at once), and their
 // product with a published operand: the arithmetic of fx_dot.  LD <= 32 NP; sums of ranges add up to a row's.
-struct FxPart {
-  i64 t2, t1;                // the product is t2 2 + (t1 + 2^25 >> 26)
-};
 template <int LD, int NP, int NC = LD>
 struct FxRow {
   int2 m[NC];
@@ -333,11 +350,11 @@ struct FxRow {
       t1 = fx_mad(m[c + 1].y, v.z, t1);
       t0 = fx_mad(m[c + 1].x, v.w, t0);
     }
-    return {t2, t1 + t0};
+    return {t2, t1, t0};
   }
   __device__ __forceinline__ FxVal value(FxPart t, const i64* blk, int nr, int r, const int2* xs, int em) const {
     FxVal p;
-    p.v = (t.t2 << 1) + ((t.t1 + (1ll << 25)) >> 26);
+    p.v = t.value();
     p.e = ea + em - kFxMvExp;
     if (em >= kFxInf || ea == kFxBad) {                // (after the registers of the row are done with)
       p.v = __double_as_longlong(em == kFxInf ? fx_dot_slow(blk, LD, r, xs, 0, nr, em) : fx_nan());

@@ -584,6 +584,7 @@ __device__ void apply_pending_fix(const FxArgs& a, int b, int k0, int kn, double
         const FxPart u = s_p[task * NP + sl][lane];
         t.t2 += u.t2;
         t.t1 += u.t1;
+        t.t0 += u.t0;
       }
       const FxVal p = G.value(t, fx.block(a, k0 + m), nr, rr, s_x[warp], em);
       s_v[mg][task][r] = p.v;
@@ -626,9 +627,9 @@ static size_t fx_deriv_smem_bytes(int nr, bool d2s, bool fix, int km, bool f32) 
 // FP64 as a fifth block (per shell: 4 M nr T, [op][k][n], then M nr doubles).  FP64 contractions run in fixed
 // point (sdd_fixed.cuh), a warp per operator, 32 rows and mode, the operators in shared memory; FP32 ones
 // (contract: not already on the tensor cores) as sequential FP32 chains in the order of the fused kernel's.  Inside sdd_step a pending chain correction is applied to the rows first.
-// Dr takes two digits here: its products with psi, T and S go into pointwise products, which no operator
-// differentiates again on the way to the result (the h kernel's Dr Q and D2 psi meet the implicit solves, which
-// cancel their large parts, and take three).
+// Dr takes two digits here (0.03 to 0.4 of FP64's error in the norm, sdd_fixed.cuh): its products with psi, T and S go
+// into pointwise products, which no operator differentiates again on the way to the result (the h kernel's Dr Q and D2
+// psi meet the implicit solves, which cancel their large parts, and take three).
 // Bound: 64 shells of 256 x 30, the integer pipe (a D2 product is about 1500 warp cycles, a Dr product 800): 79 us,
 // 146 us with every operator in three digits.  One shell, the L2 round trips of the rows, the correction's blocks
 // and the operators: 14 us; 540 x 65: 37 us (64 us with the operators' rows in registers, loaded for every mode).
