@@ -42,17 +42,23 @@ inline void fx_split_host(i64 v, int* hi, int* lo) {
   *hi = (int)((v - l) >> 32);
 }
 
-// round(x 2^s), c = 1084 - s; the caller's scale keeps |x| 2^s < 2^62.  Subnormal x gives 0.
+// The high word of |x|'s significand, 53 bits in all, from |x|'s high word h (below the normal range without the leading
+// one); |x| = that 2^(e1 - 1075) with the exponent e1, the exponent field or 1.
+__device__ __forceinline__ unsigned fx_mant_hi(unsigned h, int& e1) {
+  e1 = max((int)(h >> 20), 1);
+  return h + 0x100000u - ((unsigned)e1 << 20);
+}
+
+// round(x 2^s), c = 1084 - s; the caller's scale keeps |x| 2^s < 2^62, and s <= 1083 where x is below the normal range.
 __device__ __forceinline__ i64 d2fx(double x, int c) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const int e = (int)((hi >> 20) & 0x7ffu);
-  const u64 m = (((u64)((hi & 0xfffffu) | 0x100000u) << 32) | lo) << 10;
-  const int r = e ? min(c - e, 63) : 63;
-  const i64 q = (i64)(((m >> r) + 1) >> 1);
+  int e1;
+  const u64 m = (((u64)fx_mant_hi(hi & 0x7fffffffu, e1) << 32) | lo) << 10;
+  const i64 q = (i64)(((m >> min((unsigned)(c - e1), 63u)) + 1) >> 1);
   return (int)hi < 0 ? -q : q;
 }
 
-// v 2^-s as a double (rounded to nearest; below the normal range 0)
+// v 2^-s as a double (rounded to nearest, also below the normal range)
 __device__ __forceinline__ double fx2d(i64 v, int s) {
   u64 a = (u64)(v < 0 ? -v : v);
   const int lz = __clzll((i64)a);
@@ -60,17 +66,21 @@ __device__ __forceinline__ double fx2d(i64 v, int s) {
   a <<= (lz & 63);
   u64 bits = ((u64)(unsigned)(e - 1) << 52) + (a >> 11) + ((a >> 10) & 1);
   if (e >= 2047) bits = 0x7ff0000000000000ull;
-  if (v == 0 || e <= 0) bits = 0;
+  if (e <= 0) bits = e > -53 ? ((a >> (11 - e)) + 1) >> 1 : 0;   // in units of 2^-1074
+  if (v == 0) bits = 0;
   return __longlong_as_double((i64)(bits | ((u64)v & 0x8000000000000000ull)));
 }
 
 // The same by the FP64 pipe's conversion: half the latency (66 against 107 cycles), as many cycles of issue;
-// for a lone dependent value.
+// for a lone dependent value.  Below the normal range out of line: inside, either form of it made the chains of 64
+// shells of 256 x 30 133 us instead of 125.
+static __device__ __noinline__ double fx2d_small(i64 v, int s) { return fx2d(v, s); }
 __device__ __forceinline__ double fx2d_lat(i64 v, int s) {
   const double d = __ll2double_rn(v);
   const int hi = __double2hiint(d), e = ((hi >> 20) & 0x7ff) - s;
   const double r = __hiloint2double(hi - (s << 20), __double2loint(d));
-  if (v == 0 || e <= 0) return 0.0;
+  if (v == 0) return 0.0;
+  if (e <= 0) return fx2d_small(v, s);
   return e >= 2047 ? __longlong_as_double((v < 0 ? 0xfff0000000000000ll : 0x7ff0000000000000ll)) : r;
 }
 
@@ -117,7 +127,8 @@ __device__ __forceinline__ i64 fx_rmul(i64 x, int h1, int h0) {
 // Scales of rows by their 1-norms and their conversion in place.  Row t holds P doubles at XV + t P, of which the
 // calling thread wrote the elements k = tid, tid + blockDim, ... (no barrier is needed before the call).
 // Afterwards the row holds round(x 2^(60 - E[t])) as 64-bit integers with sum |x| < 2^E[t]: the row's transform
-// and everything inside it stays below 2^61 (two rows of a pair).  E[t] = kFxBad marks a row with an infinity
+// and everything inside it stays below 2^61 (two rows of a pair).  E is -1022 at least (2^-1082 a unit: all of a
+// number below the normal range, which has no leading bit to shift up).  E[t] = kFxBad marks a row with an infinity
 // or NaN (left as zeros); E of the row after an odd last one is a zero row's.  The sum is of whole numbers in units
 // of the row's largest exponent, so E does not depend on how many threads share the row.  red: 2 nrows 32 words.
 // Ends with a barrier.
@@ -142,13 +153,14 @@ static __device__ __noinline__ void rows_to_fixed_at(int xv, int P, int nrows, i
 #pragma unroll 1
   for (int t = 0; t < nrows; ++t) {
     const double* x = XV + t * P;
-    const int em = (int)__reduce_max_sync(0xffffffffu, lane < nw ? red[t * 32 + lane] : 0u);
+    const int em = max((int)__reduce_max_sync(0xffffffffu, lane < nw ? red[t * 32 + lane] : 0u), 1);
     unsigned s = 0;                                    // (at most 2^18 an element)
 #pragma unroll 1
     for (int k = tid; k < P; k += bd) {
-      const unsigned h = abs_hi(x[k]);
-      const int e = (int)(h >> 20);
-      if (e) s += (((h & 0xfffffu) | 0x100000u) >> min(em - e + 3, 31)) + 1;
+      const unsigned h = abs_hi(x[k]);                 // (numbers below 2^-1042 do not count: E is -1022 at least)
+      int e1;
+      const unsigned m = fx_mant_hi(h, e1);
+      if (h) s += (m >> min(em - e1 + 3, 31)) + 1;
     }
     s = __reduce_add_sync(0xffffffffu, s);
     if (lane == 0) red[(nrows + t) * 32 + warp] = s;
@@ -157,9 +169,9 @@ static __device__ __noinline__ void rows_to_fixed_at(int xv, int P, int nrows, i
 #pragma unroll 1
   for (int t = warp; t < ((nrows + 1) & ~1); t += nw) {
     const bool on = t < nrows && lane < nw;
-    const unsigned em = __reduce_max_sync(0xffffffffu, on ? red[t * 32 + lane] : 0u);
+    const unsigned em = max(__reduce_max_sync(0xffffffffu, on ? red[t * 32 + lane] : 0u), 1u);
     const unsigned tot = __reduce_add_sync(0xffffffffu, on ? red[(nrows + t) * 32 + lane] : 0u);
-    if (lane == 0) E[t] = em >= 0x7ffu ? kFxBad : (int)em - 1040 + (32 - __clz((int)tot));
+    if (lane == 0) E[t] = em >= 0x7ffu ? kFxBad : max((int)em - 1040 + (32 - __clz((int)tot)), -1022);
   }
   __syncthreads();
 #pragma unroll 1
@@ -211,7 +223,7 @@ __device__ __forceinline__ int fx_key(double x, int cx) {
   const unsigned h = abs_hi(x);
   const int e = (int)(h >> 20);
   if (e == 0x7ff) return ((h & 0xfffffu) | (unsigned)__double2loint(x)) ? kFxBad : kFxInf;
-  return e ? e + cx : -0x10000;
+  return h | (unsigned)__double2loint(x) ? e + cx : -0x10000;   // |x| < 2^(e - 1022), also with e = 0
 }
 // The operand's digits, kMvX bits below the largest exponent em; with em = kFxInf its raw bits.
 __device__ __forceinline__ int2 fx_digits(double x, int cx, int em) {
@@ -228,14 +240,17 @@ struct FxVal {
   int e;
 };
 __device__ __forceinline__ i64 fx_shr(i64 v, int n) { return v >> min(n, 63); }
-__device__ __forceinline__ double fx_val(FxVal p) { return p.e == kFxBad ? __longlong_as_double(p.v) : fx2d(p.v, -p.e); }
+template <bool LAT = false>
+__device__ __forceinline__ double fx_val(FxVal p) {
+  return p.e == kFxBad ? __longlong_as_double(p.v) : LAT ? fx2d_lat(p.v, -p.e) : fx2d(p.v, -p.e);
+}
 
 // h + p and h + p + q, summed in fixed point 59 bits below the largest and rounded once (LAT: the conversion
 // with the lower latency, for the chains).
 template <bool LAT = false>
 __device__ __forceinline__ double fx_sum(double h, FxVal p) {
   const int eh = (int)(abs_hi(h) >> 20);
-  if (p.e == kFxBad || eh == 0x7ff) return h + fx_val(p);
+  if (p.e == kFxBad || eh == 0x7ff) return h + fx_val<LAT>(p);
   const int em = max(eh - 1081, p.e);
   const i64 v = fx_shr(p.v, em - p.e) + d2fx(h, 1084 + em);
   return LAT ? fx2d_lat(v, -em) : fx2d(v, -em);
@@ -243,7 +258,7 @@ __device__ __forceinline__ double fx_sum(double h, FxVal p) {
 template <bool LAT = false>
 __device__ __forceinline__ double fx_sum(double h, FxVal p, FxVal q) {
   const int eh = (int)(abs_hi(h) >> 20);
-  if (p.e == kFxBad || q.e == kFxBad || eh == 0x7ff) return (h + fx_val(p)) + fx_val(q);
+  if (p.e == kFxBad || q.e == kFxBad || eh == 0x7ff) return (h + fx_val<LAT>(p)) + fx_val<LAT>(q);
   const int em = max(max(eh - 1081, p.e), q.e);
   const i64 v = fx_shr(p.v, em - p.e) + fx_shr(q.v, em - q.e) + d2fx(h, 1084 + em);
   return LAT ? fx2d_lat(v, -em) : fx2d(v, -em);
@@ -376,10 +391,11 @@ struct FxRow {
 // columns' exponents (as in the two-digit blocks).
 __host__ __device__ constexpr size_t wx_block_ints(int ld) { return (size_t)(3 * ld + 2) * ld; }
 
-// The digits of m 2^27 >> sh (m the 53-bit significand of x), with x's sign; x = 0 (or subnormal) gives 0.
+// The digits of m 2^27 >> sh, with x's sign; x = m 2^(e - 1075) in magnitude with its exponent field e.
 __device__ __forceinline__ void wx_split(double x, int sh, int& d2, int& d1, int& d0) {
   const unsigned hi = (unsigned)__double2hiint(x), mask = 0x7ffffffu;
-  const u64 m = ((hi >> 20) & 0x7ffu) ? ((u64)((hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x) : 0;
+  u64 m = ((u64)(hi & 0xfffffu) << 32) | (unsigned)__double2loint(x);
+  m = (hi & 0x7ff00000u) ? m | 0x10000000000000ull : m << 1;
   const unsigned a2 = (unsigned)(m >> min(27 + sh, 63)), a1 = (unsigned)(m >> min(sh, 63)) & mask;
   const unsigned a0 = (unsigned)(sh <= 27 ? m << (27 - sh) : m >> min(sh - 27, 63)) & mask;
   const int s = (int)hi >> 31;
