@@ -368,7 +368,9 @@ struct ArnoldiColumn {
 __device__ __forceinline__ ArnoldiColumn new_rotation(double a, double nrm2, double gj, double beta, double target, int j,
                                                       int m, int lane) {
   ArnoldiColumn o;
-  const double root = sqrt(lane == 0 ? nrm2 : fma(a, a, nrm2));
+  const double r2 = fma(a, a, nrm2);
+  double root = sqrt(lane == 0 ? nrm2 : r2);
+  if (!(r2 > 1e-280 && r2 < 1e290) && lane != 0) root = hypot(a, sqrt(nrm2));   // (a a out of range, or zero)
   const double hnext = __shfl_sync(0xffffffffu, root, 0);
   o.r = __shfl_sync(0xffffffffu, root, 1);
   const double q = (lane == 0 ? a : (lane == 1 ? hnext : 1.0)) / (lane < 2 ? o.r : hnext);
@@ -629,8 +631,9 @@ __global__ void __launch_bounds__(kDotThreads + 32) k_orth(const VT* __restrict_
 }
 
 // Back substitution R y = g over the first kb[b] columns, one warp per shell: R in shared memory, lane l the rows l
-// and l + 32; y_i = t_i (1 / R_ii) goes to all lanes, which take its column off their rows (one thread for a whole
-// shell, a division a row: 37 us at 50 columns; now 9 us).
+// and l + 32; y_i = t_i / R_ii goes to all lanes, which take its column off their rows (one thread for a whole
+// shell: 37 us at 50 columns, now about 20; the rows' divisions are 10 of them, which reciprocals formed ahead would save
+// at the price of one more rounding an entry).
 __global__ void __launch_bounds__(32) k_solve_y(GmresState s) {
   extern __shared__ __align__(16) double R[];
   const int b = blockIdx.x, lane = threadIdx.x;
@@ -641,17 +644,17 @@ __global__ void __launch_bounds__(32) k_solve_y(GmresState s) {
 #pragma unroll 8
   for (int q = lane; q < k * m; q += 32) R[q] = H[q];
   __syncwarp();
-  double t[2], inv[2];
+  double t[2], d[2];
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int r = lane + 32 * u;
     t[u] = r < k ? g[r] : 0.0;
-    const double d = r < k ? R[r * m + r] : 0.0;
-    inv[u] = d != 0.0 ? 1.0 / d : 0.0;
+    d[u] = r < k ? R[r * m + r] : 0.0;
   }
   for (int i = k - 1; i >= 0; --i) {
     const int u = i >> 5;
-    const double yi = __shfl_sync(0xffffffffu, u ? t[1] * inv[1] : t[0] * inv[0], i & 31);
+    const double di = u ? d[1] : d[0];
+    const double yi = __shfl_sync(0xffffffffu, di != 0.0 ? (u ? t[1] : t[0]) / di : 0.0, i & 31);
     if (lane == 0) y[i] = yi;
 #pragma unroll
     for (int v = 0; v < 2; ++v)
