@@ -141,9 +141,9 @@ struct sdd_plan {
   // chunked chains: cs[0] the chunking of layout 2 (sequential carry), cs[1] of layout 3 (parallel
   // carry); leading dimensions; workspaces sized for the larger chunk and product counts
   ChunkSet cs[2];
-  int ldmA, ldmT, ldd, nch_alloc, np_alloc;
+  int ldd, nch_alloc, np_alloc;
   // host copies of what the chunk tables are built from, for sdd_plan_set_chunk_length: the psi step
-  // matrices [A B] (M x 2nr x ldl), Linv_T, Linv_S (M nr nr), the per-step scalars (4 M each)
+  // matrices [A B] (M x 2nr x nr), Linv_T, Linv_S (M nr nr), the per-step scalars (4 M each)
   double *h_AB, *h_LinvT, *h_LinvS, *h_cA, *h_cT, *h_cS;
   double *dbuf, *cbuf;              // [B][3][2][nch_alloc][ldd] chunk end states / carried states
   int* dcnt;                        // [B][6] chunk counters of the sequential carry
@@ -268,58 +268,86 @@ static int upload32(float** dst, const double* src, size_t n) {
   SDD_CUDA(cudaMemcpy(*dst, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
   return SDD_OK;
 }
-// Matrices as fixed-point blocks (sdd_fixed.cuh): nmat host matrices of nrg nr x nseg nr, column-major with
-// leading dimension ld (stride cols ld), become nrg nseg blocks each, row halves outermost.
-// On the plan's private non-blocking stream: another host thread may be capturing a graph meanwhile, which
-// rules out the default stream's launches and device-wide waits.
-static int upload_fixed(sdd_plan* p, const i64** dst, const double* src, int nmat, int cols, int ld, int nr, int ldl,
-                        int nrg, int nseg) {
-  if (!p->cap_stream) SDD_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
-  cudaStream_t s = p->cap_stream;
-  const size_t n = (size_t)nmat * cols * ld, bw = fx_block_words(ldl), per = (size_t)nrg * nseg * bw;
-  double* tmp = nullptr;
+// Host tables on their way to fixed-point blocks: copied to a device buffer and converted there, on the plan's private
+// non-blocking stream (another host thread may be capturing a graph meanwhile, which rules out the default stream's
+// launches and device-wide waits).  A copy from pageable memory may still be reading its source when it returns, so
+// whoever owns a source keeps it (or gives it to keep()) until the next wait(); the tables are there after it.  With a
+// buffer and a wait for each of a plan's 25 tables (and slower conversions) a plan of 64 x 20 took 3.0 ms instead of
+// 2.6, 128 x 28 mixed 12.3 instead of 11.3, 256 x 30 28.2 instead of 26.4.
+struct TableUpload {
+  sdd_plan* p;
+  double* buf = nullptr;
+  size_t cap = 0, used = 0;
+  std::vector<std::vector<double>> kept;
+  explicit TableUpload(sdd_plan* plan) : p(plan) {}
+  TableUpload(const TableUpload&) = delete;
+  ~TableUpload() {
+    wait();
+    cudaFree(buf);
+  }
+  cudaError_t wait() {
+    const cudaError_t e = p->cap_stream ? cudaStreamSynchronize(p->cap_stream) : cudaSuccess;
+    used = 0;
+    kept.clear();
+    return e;
+  }
+  const double* keep(std::vector<double>&& v) {
+    kept.push_back(std::move(v));
+    return kept.back().data();
+  }
+  // n doubles of the buffer holding src's (nullptr and e: an error)
+  const double* put(const double* src, size_t n, cudaError_t* e) {
+    *e = cudaSuccess;
+    if (!p->cap_stream) *e = cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking);
+    if (*e == cudaSuccess && used + n > cap) {
+      if (used) {
+        // the sources copied so far may go; the one at hand may be among the kept
+        *e = cudaStreamSynchronize(p->cap_stream);
+        used = 0;
+      }
+      if (*e == cudaSuccess && n > cap) {
+        cudaFree(buf);
+        buf = nullptr;
+        cap = std::max(n, std::min((size_t)1 << 21, (size_t)16 * p->M * p->nr * p->nr));   // 16 MB, small plans less
+        *e = cudaMalloc(&buf, cap * sizeof(double));
+        if (*e != cudaSuccess) cap = 0;
+      }
+    }
+    double* at = buf + used;
+    if (*e == cudaSuccess) *e = cudaMemcpyAsync(at, src, n * sizeof(double), cudaMemcpyHostToDevice, p->cap_stream);
+    used += n;
+    return *e == cudaSuccess ? at : nullptr;
+  }
+};
+
+// nmat host matrices of nrg nr x nseg nr (element (r, c) at r rs + c cs) become nrg nseg blocks each, row halves
+// outermost.
+static int upload_fixed(TableUpload& up, const i64** dst, const double* src, int nmat, int rs, int cs, int nrg = 1,
+                        int nseg = 1) {
+  if (!src) return SDD_ERR_ARG;
+  const int nr = up.p->nr, ldl = up.p->ldl;
+  const size_t one = (size_t)nrg * nseg * nr * nr, bw = fx_block_words(ldl), per = (size_t)nrg * nseg * bw;
+  cudaError_t e;
+  const double* tmp = up.put(src, nmat * one, &e);
   i64* out = nullptr;
-  cudaError_t e = cudaMalloc(&tmp, n * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&out, nmat * per * sizeof(i64));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, src, n * sizeof(double), cudaMemcpyHostToDevice, s);
   for (int q = 0; q < nrg * nseg && e == cudaSuccess; ++q)
-    e = launch_to_fixed(tmp, (size_t)cols * ld, ld, nrg * nr, q / nseg * nr, q % nseg * nr, nr, ldl, out + q * bw, per,
-                        nmat, s);
-  const cudaError_t ew = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) e = ew;
-  cudaFree(tmp);
-  if (e != cudaSuccess) cudaFree(out);
+    e = launch_to_fixed(tmp, one, rs, cs, nrg * nr, q / nseg * nr, q % nseg * nr, nr, ldl, out + q * bw, per, nmat,
+                        up.p->cap_stream);
+  *dst = out;                                          // (freed with the plan or the chunk set, also after an error)
   SDD_CUDA(e);
-  *dst = out;
   return SDD_OK;
 }
 // A radial operator (row-major on the host) as a three-digit block.
-static int upload_wide(sdd_plan* p, int** dst, const double* src, int nr, int ld) {
+static int upload_wide(TableUpload& up, int** dst, const double* src) {
   if (!src) return SDD_ERR_ARG;
-  if (!p->cap_stream) SDD_CUDA(cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking));
-  const size_t n = (size_t)nr * nr * sizeof(double);
-  double* tmp = nullptr;
-  int* out = nullptr;
-  cudaError_t e = cudaMalloc(&tmp, n);
-  if (e == cudaSuccess) e = cudaMalloc(&out, wx_block_ints(ld) * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(tmp, src, n, cudaMemcpyHostToDevice, p->cap_stream);
-  if (e == cudaSuccess) e = launch_to_wide(tmp, nr, ld, out, p->cap_stream);
-  const cudaError_t ew = cudaStreamSynchronize(p->cap_stream);
-  if (e == cudaSuccess) e = ew;
-  cudaFree(tmp);
-  if (e != cudaSuccess) cudaFree(out);
+  const int nr = up.p->nr, ld = up.p->ldl;
+  cudaError_t e;
+  const double* tmp = up.put(src, (size_t)nr * nr, &e);
+  if (e == cudaSuccess) e = cudaMalloc(dst, wx_block_ints(ld) * sizeof(int));
+  if (e == cudaSuccess) e = launch_to_wide(tmp, nr, ld, *dst, up.p->cap_stream);
   SDD_CUDA(e);
-  *dst = out;
   return SDD_OK;
-}
-// Linv blocks and Dr (row-major on the host).
-static int upload_linv(sdd_plan* p, const i64** dst, const double* src, int M, int nr, int ldl) {
-  if (!src) return SDD_ERR_ARG;
-  std::vector<double> h((size_t)M * nr * nr);
-  for (int m = 0; m < M; ++m)
-    for (int i = 0; i < nr; ++i)
-      for (int c = 0; c < nr; ++c) h[((size_t)m * nr + c) * nr + i] = src[((size_t)m * nr + i) * nr + c];
-  return upload_fixed(p, dst, h.data(), M, nr, nr, nr, ldl, 1, 1);
 }
 // Linv blocks transposed (column c contiguous, leading dimension ldl) and rounded to FP32.
 static int upload_linv32(float** dst, const double* src, int M, int nr, int ldl) {
@@ -423,7 +451,7 @@ static void free_plan(sdd_plan* p) {
 //   T/S (s = b, m = nr):  G_k = -w_k Linv_k Psi_k,  Psi_{k+1} = Psi_k + k_{k+1} G_k   (b += k f before
 //     the next step, k = 2 dt (j+2) of that step, w = 0.5 for j = 0 else 1)
 // with Psi = I at the chunk start, and Phi_c = Psi after the chunk's last step.  Formed in FP64 (transposed, G
-// per mode [jj][m cols][ldl], Phi per (parity, chunk) [m cols][ldm]), uploaded as fixed-point blocks.
+// per mode [jj][m cols][nr], Phi per (parity, chunk) [m cols][m]), uploaded as fixed-point blocks.
 static void matmul_rows(const double* A, const double* B, double* C, int n, int k, int m) {  // C = A B
   for (int i = 0; i < n; ++i) {
     double* c = C + (size_t)i * m;
@@ -438,10 +466,10 @@ static void matmul_rows(const double* A, const double* B, double* C, int n, int 
 
 // Products of the parallel carry: P_{j,i} = Phi_{j-1} ... Phi_{i+1} for 2 <= j < nch, 0 <= i <= j-2,
 // built as P_{j,j-2} = Phi_{j-1}, P_{j,i} = Phi_{j-1} P_{j-1,i}; stored transposed like Phi, row j after
-// row j-1.  PhiT holds the Phi_c of both parities ([par][c][m cols][ldm]).
-static void carry_products(const std::vector<double>& PhiT, int nch, int m, int ldm, std::vector<double>& out) {
+// row j-1.  PhiT holds the Phi_c of both parities ([par][c][m cols][m]).
+static void carry_products(const std::vector<double>& PhiT, int nch, int m, std::vector<double>& out) {
   const int np = (nch - 1) * (nch - 2) / 2;
-  const size_t blk = (size_t)m * ldm;
+  const size_t blk = (size_t)m * m;
   out.assign((size_t)2 * std::max(np, 1) * blk, 0.0);
   std::vector<double> Phi((size_t)m * m), Q((size_t)m * m), R((size_t)m * m);
   std::vector<std::vector<double>> prev, cur;   // row-major P_{j-1,i}, P_{j,i}
@@ -450,7 +478,7 @@ static void carry_products(const std::vector<double>& PhiT, int nch, int m, int 
     for (int j = 2; j < nch; ++j) {
       const double* src = PhiT.data() + ((size_t)par * nch + (j - 1)) * blk;   // Phi_{j-1}, transposed
       for (int i = 0; i < m; ++i)
-        for (int col = 0; col < m; ++col) Phi[(size_t)i * m + col] = src[(size_t)col * ldm + i];
+        for (int col = 0; col < m; ++col) Phi[(size_t)i * m + col] = src[(size_t)col * m + i];
       cur.assign(j - 1, std::vector<double>());
       for (int i = 0; i <= j - 2; ++i) {
         if (i == j - 2) {
@@ -461,7 +489,7 @@ static void carry_products(const std::vector<double>& PhiT, int nch, int m, int 
         }
         double* dst = out.data() + ((size_t)par * np + (size_t)(j - 1) * (j - 2) / 2 + i) * blk;
         for (int r = 0; r < m; ++r)
-          for (int col = 0; col < m; ++col) dst[(size_t)col * ldm + r] = cur[i][(size_t)r * m + col];
+          for (int col = 0; col < m; ++col) dst[(size_t)col * m + r] = cur[i][(size_t)r * m + col];
       }
       prev.swap(cur);
     }
@@ -470,18 +498,17 @@ static void carry_products(const std::vector<double>& PhiT, int nch, int m, int 
 
 // One chunking of the three chains' tables (see matmul_rows above for G and Phi): products for the
 // parallel carry (layout 3), else the per-chunk maps Phi_c (layout 2).
-static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB, const double* LinvT,
+static int build_chunk_set(TableUpload& up, int kc, bool products, const double* AB, const double* LinvT,
                            const double* LinvS, const double* cA, const double* cT, const double* cS,
                            ChunkSet* cs) {
-  const int M = p->M, nr = p->nr, ldl = p->ldl, S = M / 2;
+  const int M = up.p->M, nr = up.p->nr, S = M / 2;
   const int nch = (S + kc - 1) / kc;
   cs->kc = kc;
   cs->nch = nch;
   cs->np = products ? (nch - 1) * (nch - 2) / 2 : 0;
-  std::vector<double> Pr;
   {  // psi
-    const int m = 2 * nr, ldm = p->ldmA;
-    std::vector<double> G((size_t)M * m * ldl, 0.0), Phi((size_t)2 * nch * m * ldm, 0.0);
+    const int m = 2 * nr;
+    std::vector<double> G((size_t)M * m * nr, 0.0), Phi((size_t)2 * nch * m * m, 0.0), Pr;
     std::vector<double> Psi((size_t)m * m), Gs((size_t)nr * m), C((size_t)nr * m);
     for (int par = 0; par < 2; ++par)
       for (int c = 0; c < nch; ++c) {
@@ -489,12 +516,12 @@ static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB,
         for (int i = 0; i < m; ++i) Psi[(size_t)i * m + i] = 1.0;
         for (int s = c * kc; s < std::min(S, (c + 1) * kc); ++s) {
           const int jj = par + 2 * s;
-          const double* blk = AB + (size_t)jj * 2 * nr * ldl;
+          const double* blk = AB + (size_t)jj * 2 * nr * nr;
           for (int i = 0; i < nr; ++i)
-            for (int col = 0; col < m; ++col) C[(size_t)i * m + col] = blk[(size_t)col * ldl + i];
+            for (int col = 0; col < m; ++col) C[(size_t)i * m + col] = blk[(size_t)col * nr + i];
           matmul_rows(C.data(), Psi.data(), Gs.data(), nr, m, m);
           for (int i = 0; i < nr; ++i)
-            for (int col = 0; col < m; ++col) G[((size_t)jj * m + col) * ldl + i] = Gs[(size_t)i * m + col];
+            for (int col = 0; col < m; ++col) G[((size_t)jj * m + col) * nr + i] = Gs[(size_t)i * m + col];
           const double bj = cA[4 * jj + 2], bjt = cA[4 * jj + 3];
           for (int i = 0; i < nr; ++i)
             for (int col = 0; col < m; ++col) {
@@ -506,19 +533,19 @@ static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB,
         if (c + 1 < nch)
           for (int i = 0; i < m; ++i)
             for (int col = 0; col < m; ++col)
-              Phi[(((size_t)par * nch + c) * m + col) * ldm + i] = Psi[(size_t)i * m + col];
+              Phi[(((size_t)par * nch + c) * m + col) * m + i] = Psi[(size_t)i * m + col];
       }
     int st;
-    if ((st = upload_fixed(p, &cs->GA4, G.data(), M, m, ldl, nr, ldl, 1, 2))) return st;
-    if (products) carry_products(Phi, nch, m, ldm, Pr);
-    if (products && cs->np > 0 && (st = upload_fixed(p, &cs->PA4, Pr.data(), 2 * cs->np, m, ldm, nr, ldl, 2, 2))) return st;
-    if (!products && (st = upload_fixed(p, &cs->PhiA4, Phi.data(), 2 * nch, m, ldm, nr, ldl, 2, 2))) return st;
+    if ((st = upload_fixed(up, &cs->GA4, up.keep(std::move(G)), M, 1, nr, 1, 2))) return st;
+    if (products) carry_products(Phi, nch, m, Pr);
+    if (products && cs->np > 0 && (st = upload_fixed(up, &cs->PA4, up.keep(std::move(Pr)), 2 * cs->np, 1, m, 2, 2))) return st;
+    if (!products && (st = upload_fixed(up, &cs->PhiA4, up.keep(std::move(Phi)), 2 * nch, 1, m, 2, 2))) return st;
   }
   for (int fld = 1; fld <= 2; ++fld) {  // T, S
-    const int m = nr, ldm = p->ldmT;
+    const int m = nr;
     const double* Linv = fld == 1 ? LinvT : LinvS;
     const double* cf = fld == 1 ? cT : cS;
-    std::vector<double> G((size_t)M * m * ldl, 0.0), Phi((size_t)2 * nch * m * ldm, 0.0);
+    std::vector<double> G((size_t)M * m * nr, 0.0), Phi((size_t)2 * nch * m * m, 0.0), Pr;
     std::vector<double> Psi((size_t)m * m), Gs((size_t)nr * m);
     for (int par = 0; par < 2; ++par)
       for (int c = 0; c < nch; ++c) {
@@ -530,22 +557,22 @@ static int build_chunk_set(sdd_plan* p, int kc, bool products, const double* AB,
           const double w = cf[4 * jj + 1];
           for (double& x : Gs) x *= -w;
           for (int i = 0; i < nr; ++i)
-            for (int col = 0; col < m; ++col) G[((size_t)jj * m + col) * ldl + i] = Gs[(size_t)i * m + col];
+            for (int col = 0; col < m; ++col) G[((size_t)jj * m + col) * nr + i] = Gs[(size_t)i * m + col];
           const double knext = (s + 1 < S) ? cf[4 * (jj + 2)] : 0.0;
           for (size_t e = 0; e < Psi.size(); ++e) Psi[e] += knext * Gs[e];
         }
         if (c + 1 < nch)
           for (int i = 0; i < m; ++i)
             for (int col = 0; col < m; ++col)
-              Phi[(((size_t)par * nch + c) * m + col) * ldm + i] = Psi[(size_t)i * m + col];
+              Phi[(((size_t)par * nch + c) * m + col) * m + i] = Psi[(size_t)i * m + col];
       }
     int st;
-    if ((st = upload_fixed(p, fld == 1 ? &cs->GT : &cs->GS, G.data(), M, m, ldl, nr, ldl, 1, 1))) return st;
-    if (products) carry_products(Phi, nch, m, ldm, Pr);
+    if ((st = upload_fixed(up, fld == 1 ? &cs->GT : &cs->GS, up.keep(std::move(G)), M, 1, nr))) return st;
+    if (products) carry_products(Phi, nch, m, Pr);
     if (products && cs->np > 0 &&
-        (st = upload_fixed(p, fld == 1 ? &cs->PT : &cs->PS, Pr.data(), 2 * cs->np, m, ldm, nr, ldl, 1, 1)))
+        (st = upload_fixed(up, fld == 1 ? &cs->PT : &cs->PS, up.keep(std::move(Pr)), 2 * cs->np, 1, m)))
       return st;
-    if (!products && (st = upload_fixed(p, fld == 1 ? &cs->PhiT : &cs->PhiS, Phi.data(), 2 * nch, m, ldm, nr, ldl, 1, 1)))
+    if (!products && (st = upload_fixed(up, fld == 1 ? &cs->PhiT : &cs->PhiS, up.keep(std::move(Phi)), 2 * nch, 1, m)))
       return st;
   }
   return SDD_OK;
@@ -562,15 +589,14 @@ static int chunk_len(int S, int layout, int nr) {
   return std::max(layout == 3 ? 2 : 4, std::min(layout == 3 ? 16 : 32, (int)std::lround(k)));
 }
 
-static int build_chunk_tables(sdd_plan* p, const double* AB, const double* LinvT, const double* LinvS,
+static int build_chunk_tables(TableUpload& up, const double* AB, const double* LinvT, const double* LinvS,
                               const double* cA, const double* cT, const double* cS) {
+  sdd_plan* p = up.p;
   const int S = p->M / 2, nr = p->nr;
-  p->ldmA = 2 * nr;
-  p->ldmT = nr + (nr & 1);
   p->ldd = 2 * nr;
   int st;
-  if ((st = build_chunk_set(p, chunk_len(S, 2, nr), false, AB, LinvT, LinvS, cA, cT, cS, &p->cs[0])) ||
-      (st = build_chunk_set(p, chunk_len(S, 3, nr), true, AB, LinvT, LinvS, cA, cT, cS, &p->cs[1])))
+  if ((st = build_chunk_set(up, chunk_len(S, 2, nr), false, AB, LinvT, LinvS, cA, cT, cS, &p->cs[0])) ||
+      (st = build_chunk_set(up, chunk_len(S, 3, nr), true, AB, LinvT, LinvS, cA, cT, cS, &p->cs[1])))
     return st;
   p->nch_alloc = std::max(p->cs[0].nch, p->cs[1].nch);
   p->np_alloc = std::max(p->cs[1].np, 1);
@@ -614,6 +640,109 @@ static int build_diag_tables(sdd_plan* p, const sdd_plan_desc* d) {
   return SDD_OK;
 }
 
+// The plan's tables (p: sizes, precision and scalars set).  What is built before an error is freed with the plan.
+static int fill_plan(sdd_plan* p, const sdd_plan_desc* d, TableUpload& up) {
+  const int M = p->M, nr = p->nr;
+  const size_t nn = (size_t)nr * nr, nm = (size_t)M * nr * nr;
+  int st = SDD_OK;
+  if ((st = upload(&p->Dr, d->Dr, nn)) || (st = upload(&p->D2r2, d->D2_r2, nn)) ||
+      (st = upload(&p->ir4r2, d->ir4_r2, nr)) || (st = upload(&p->D2s, d->D2_sine, nn)) ||
+      (st = upload(&p->ir2s, d->ir2_sine, nr)) || (st = upload(&p->rsq, d->rsq, nr)) || (st = upload(&p->dT0, d->dT0, nr)) ||
+      (st = upload(&p->gr, d->gr, nr)) || (st = upload_fixed(up, &p->LinvA4, d->Linv_A4, M, nr, 1)) ||
+      (st = upload_fixed(up, &p->LinvT, d->Linv_T, M, nr, 1)) ||
+      (st = upload_fixed(up, &p->fxDr, d->Dr, 1, nr, 1)) ||
+      (st = upload_wide(up, &p->opwx[0], d->D2_r2)) ||
+      (st = upload_wide(up, &p->opwx[1], d->D2_sine)) ||
+      (st = upload_wide(up, &p->opwx[2], d->Dr)) ||
+      (st = upload_fixed(up, &p->LinvS, d->Linv_S, M, nr, 1)) ||
+      (st = upload32(&p->Dr32, d->Dr, nn)) || (st = upload32(&p->D2r232, d->D2_r2, nn)) ||
+      (st = upload32(&p->ir4r232, d->ir4_r2, nr))) {
+    return st;
+  }
+  if (p->prec == SDD_PREC_MIXED &&
+      ((st = upload32(&p->D2s32, d->D2_sine, nn)) ||
+       (st = upload_linv32(&p->Linv32[0], d->Linv_A4, M, nr, p->ldl)) ||
+       (st = upload_linv32(&p->Linv32[1], d->Linv_T, M, nr, p->ldl)) ||
+       (st = upload_linv32(&p->Linv32[2], d->Linv_S, M, nr, p->ldl)))) {
+    return st;
+  }
+  if (p->prec == SDD_PREC_MIXED) {   // 3xTF32 operator tiles of the tensor-core contractions
+    p->tcKP = p->tcNP = (nr + 7) / 8 * 8;
+    std::vector<float> tb((size_t)2 * 2 * p->tcNP * p->tcKP);
+    build_tc_operator(d->Dr, d->D2_r2, nr, p->tcKP, p->tcNP, tb.data());
+    cudaError_t e = cudaMalloc(&p->tcB, tb.size() * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemcpy(p->tcB, tb.data(), tb.size() * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&p->tc_err, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(p->tc_err, 0, sizeof(int));
+    if (e != cudaSuccess) {
+      set_cuda_error(e);
+      cudaGetLastError();
+      return e == cudaErrorMemoryAllocation ? SDD_ERR_NOMEM : SDD_ERR_CUDA;
+    }
+    p->use_tc = 1;
+  }
+  {  // per-step scalars of the chains (Matrix_Operators.py:1143-1159 and 1056-1083)
+    std::vector<double> cA((size_t)M * 4), cT((size_t)M * 4), cS((size_t)M * 4);
+    const double dA = d->Pr * d->dt, dT = d->dt, dS = d->Tau * d->dt;
+    for (int jj = 0; jj < M; ++jj) {
+      const double j = (double)(M - jj);
+      const double bj = -j * (j + 1.0), bjt = -2.0 * j;
+      cA[4 * jj] = dA * bjt;
+      cA[4 * jj + 1] = dA * bjt * bj;
+      cA[4 * jj + 2] = bj;
+      cA[4 * jj + 3] = bjt;
+      const double jc = (double)(M - 1 - jj);
+      cT[4 * jj] = -dT * (-2.0 * (jc + 2.0));
+      cS[4 * jj] = -dS * (-2.0 * (jc + 2.0));
+      cT[4 * jj + 1] = cS[4 * jj + 1] = (M - 1 - jj == 0) ? 0.5 : 1.0;
+      cT[4 * jj + 2] = cT[4 * jj + 3] = cS[4 * jj + 2] = cS[4 * jj + 3] = 0.0;
+    }
+    if ((st = upload(&p->coefA4, cA.data(), cA.size())) || (st = upload(&p->coefT, cT.data(), cT.size())) ||
+        (st = upload(&p->coefS, cS.data(), cS.size()))) {
+      return st;
+    }
+    // psi chain step matrices (exact algebra of b_test, Matrix_Operators.py:1149-1157):
+    //   A_j = Linv_j (c1 D2 + diag(alpha)), B_j = Linv_j diag(beta),
+    //   c1 = dt bjt, alpha = c1 bj IR4 - bjt IR2, beta = c1 IR4;  stored transposed, [A B] per mode.
+    p->h_AB = new double[(size_t)M * 2 * nr * nr];
+    std::vector<double> LD((size_t)nr * nr);
+    for (int jj = 0; jj < M; ++jj) {
+      const double c1 = cA[4 * jj], bj = cA[4 * jj + 2], bjt = cA[4 * jj + 3];
+      const double* L = d->Linv_A4 + (size_t)jj * nr * nr;
+      for (int i = 0; i < nr; ++i)
+        for (int c = 0; c < nr; ++c) {
+          double acc = 0.0;
+          for (int k = 0; k < nr; ++k) acc += L[i * nr + k] * d->D2_A4[k * nr + c];
+          LD[(size_t)i * nr + c] = acc;
+        }
+      double* blk = p->h_AB + (size_t)jj * 2 * nr * nr;
+      for (int c = 0; c < nr; ++c) {
+        const double alpha = c1 * bj * d->ir4_A4[c] - bjt * d->ir2_A4[c];
+        const double beta = c1 * d->ir4_A4[c];
+        for (int i = 0; i < nr; ++i) {
+          blk[(size_t)c * nr + i] = c1 * LD[(size_t)i * nr + c] + L[i * nr + c] * alpha;
+          blk[(size_t)(nr + c) * nr + i] = L[i * nr + c] * beta;
+        }
+      }
+    }
+    auto keep = [](const double* src, size_t n) {
+      double* h = new double[n];
+      std::memcpy(h, src, n * sizeof(double));
+      return h;
+    };
+    p->h_LinvT = keep(d->Linv_T, nm);
+    p->h_LinvS = keep(d->Linv_S, nm);
+    p->h_cA = keep(cA.data(), cA.size());
+    p->h_cT = keep(cT.data(), cT.size());
+    p->h_cS = keep(cS.data(), cS.size());
+    if ((st = upload_fixed(up, &p->ABA4, p->h_AB, M, 1, nr, 1, 2)) ||
+        (st = build_chunk_tables(up, p->h_AB, d->Linv_T, d->Linv_S, cA.data(), cT.data(), cS.data())) ||
+        (st = build_diag_tables(p, d)))
+      return st;
+  }
+  return SDD_OK;
+}
+
 int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
   if (!d || !out) return SDD_ERR_ARG;
   *out = nullptr;
@@ -638,110 +767,19 @@ int sdd_plan_create(const sdd_plan_desc* d, sdd_plan** out) {
   p->reorth_eta = kReorthEta;
   p->dt = d->dt; p->Pr = d->Pr; p->Tau = d->Tau;
   p->fft = fp;
-  const size_t nn = (size_t)nr * nr, nm = (size_t)M * nr * nr;
-  int st = SDD_OK;
-  if ((st = upload(&p->Dr, d->Dr, nn)) || (st = upload(&p->D2r2, d->D2_r2, nn)) ||
-      (st = upload(&p->ir4r2, d->ir4_r2, nr)) || (st = upload(&p->D2s, d->D2_sine, nn)) ||
-      (st = upload(&p->ir2s, d->ir2_sine, nr)) || (st = upload(&p->rsq, d->rsq, nr)) || (st = upload(&p->dT0, d->dT0, nr)) ||
-      (st = upload(&p->gr, d->gr, nr)) || (st = upload_linv(p, &p->LinvA4, d->Linv_A4, M, nr, p->ldl)) ||
-      (st = upload_linv(p, &p->LinvT, d->Linv_T, M, nr, p->ldl)) ||
-      (st = upload_linv(p, &p->fxDr, d->Dr, 1, nr, p->ldl)) ||
-      (st = upload_wide(p, &p->opwx[0], d->D2_r2, nr, p->ldl)) ||
-      (st = upload_wide(p, &p->opwx[1], d->D2_sine, nr, p->ldl)) ||
-      (st = upload_wide(p, &p->opwx[2], d->Dr, nr, p->ldl)) ||
-      (st = upload_linv(p, &p->LinvS, d->Linv_S, M, nr, p->ldl)) ||
-      (st = upload32(&p->Dr32, d->Dr, nn)) || (st = upload32(&p->D2r232, d->D2_r2, nn)) ||
-      (st = upload32(&p->ir4r232, d->ir4_r2, nr))) {
-    free_plan(p);
-    return st;
-  }
-  if (p->prec == SDD_PREC_MIXED &&
-      ((st = upload32(&p->D2s32, d->D2_sine, nn)) ||
-       (st = upload_linv32(&p->Linv32[0], d->Linv_A4, M, nr, p->ldl)) ||
-       (st = upload_linv32(&p->Linv32[1], d->Linv_T, M, nr, p->ldl)) ||
-       (st = upload_linv32(&p->Linv32[2], d->Linv_S, M, nr, p->ldl)))) {
-    free_plan(p);
-    return st;
-  }
-  if (p->prec == SDD_PREC_MIXED) {   // 3xTF32 operator tiles of the tensor-core contractions
-    p->tcKP = p->tcNP = (nr + 7) / 8 * 8;
-    std::vector<float> tb((size_t)2 * 2 * p->tcNP * p->tcKP);
-    build_tc_operator(d->Dr, d->D2_r2, nr, p->tcKP, p->tcNP, tb.data());
-    cudaError_t e = cudaMalloc(&p->tcB, tb.size() * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemcpy(p->tcB, tb.data(), tb.size() * sizeof(float), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&p->tc_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(p->tc_err, 0, sizeof(int));
-    if (e != cudaSuccess) {
+  int st;
+  {
+    TableUpload up(p);
+    st = fill_plan(p, d, up);
+    const cudaError_t e = up.wait();
+    if (st == SDD_OK && e != cudaSuccess) {
       set_cuda_error(e);
-      cudaGetLastError();
-      free_plan(p);
-      return e == cudaErrorMemoryAllocation ? SDD_ERR_NOMEM : SDD_ERR_CUDA;
+      st = SDD_ERR_CUDA;
     }
-    p->use_tc = 1;
   }
-  {  // per-step scalars of the chains (Matrix_Operators.py:1143-1159 and 1056-1083)
-    std::vector<double> cA((size_t)M * 4), cT((size_t)M * 4), cS((size_t)M * 4);
-    const double dA = d->Pr * d->dt, dT = d->dt, dS = d->Tau * d->dt;
-    for (int jj = 0; jj < M; ++jj) {
-      const double j = (double)(M - jj);
-      const double bj = -j * (j + 1.0), bjt = -2.0 * j;
-      cA[4 * jj] = dA * bjt;
-      cA[4 * jj + 1] = dA * bjt * bj;
-      cA[4 * jj + 2] = bj;
-      cA[4 * jj + 3] = bjt;
-      const double jc = (double)(M - 1 - jj);
-      cT[4 * jj] = -dT * (-2.0 * (jc + 2.0));
-      cS[4 * jj] = -dS * (-2.0 * (jc + 2.0));
-      cT[4 * jj + 1] = cS[4 * jj + 1] = (M - 1 - jj == 0) ? 0.5 : 1.0;
-      cT[4 * jj + 2] = cT[4 * jj + 3] = cS[4 * jj + 2] = cS[4 * jj + 3] = 0.0;
-    }
-    if ((st = upload(&p->coefA4, cA.data(), cA.size())) || (st = upload(&p->coefT, cT.data(), cT.size())) ||
-        (st = upload(&p->coefS, cS.data(), cS.size()))) {
-      free_plan(p);
-      return st;
-    }
-    // psi chain step matrices (exact algebra of b_test, Matrix_Operators.py:1149-1157):
-    //   A_j = Linv_j (c1 D2 + diag(alpha)), B_j = Linv_j diag(beta),
-    //   c1 = dt bjt, alpha = c1 bj IR4 - bjt IR2, beta = c1 IR4;  stored transposed, [A B] per mode.
-    const int ldl = p->ldl;
-    std::vector<double> AB((size_t)M * 2 * nr * ldl, 0.0);
-    std::vector<double> LD((size_t)nr * nr);
-    for (int jj = 0; jj < M; ++jj) {
-      const double c1 = cA[4 * jj], bj = cA[4 * jj + 2], bjt = cA[4 * jj + 3];
-      const double* L = d->Linv_A4 + (size_t)jj * nr * nr;
-      for (int i = 0; i < nr; ++i)
-        for (int c = 0; c < nr; ++c) {
-          double acc = 0.0;
-          for (int k = 0; k < nr; ++k) acc += L[i * nr + k] * d->D2_A4[k * nr + c];
-          LD[(size_t)i * nr + c] = acc;
-        }
-      double* blk = AB.data() + (size_t)jj * 2 * nr * ldl;
-      for (int c = 0; c < nr; ++c) {
-        const double alpha = c1 * bj * d->ir4_A4[c] - bjt * d->ir2_A4[c];
-        const double beta = c1 * d->ir4_A4[c];
-        for (int i = 0; i < nr; ++i) {
-          blk[(size_t)c * ldl + i] = c1 * LD[(size_t)i * nr + c] + L[i * nr + c] * alpha;
-          blk[(size_t)(nr + c) * ldl + i] = L[i * nr + c] * beta;
-        }
-      }
-    }
-    if ((st = upload_fixed(p, &p->ABA4, AB.data(), M, 2 * nr, ldl, nr, ldl, 1, 2)) ||
-        (st = build_chunk_tables(p, AB.data(), d->Linv_T, d->Linv_S, cA.data(), cT.data(), cS.data())) ||
-        (st = build_diag_tables(p, d))) {
-      free_plan(p);
-      return st;
-    }
-    auto keep = [](const double* src, size_t n) {
-      double* h = new double[n];
-      std::memcpy(h, src, n * sizeof(double));
-      return h;
-    };
-    p->h_AB = keep(AB.data(), AB.size());
-    p->h_LinvT = keep(d->Linv_T, nm);
-    p->h_LinvS = keep(d->Linv_S, nm);
-    p->h_cA = keep(cA.data(), cA.size());
-    p->h_cT = keep(cT.data(), cT.size());
-    p->h_cS = keep(cS.data(), cS.size());
+  if (st) {
+    free_plan(p);
+    return st;
   }
   *out = p;
   return SDD_OK;
@@ -767,7 +805,16 @@ int sdd_plan_set_chunk_length(sdd_plan* p, int set, int kc) {
   clear_step_graphs(p);                    // the graphs bake in the tables' pointers
   SDD_CUDA(cudaDeviceSynchronize());      // no launch may still read the old tables
   ChunkSet c{};
-  int st = build_chunk_set(p, kc, set == 1, p->h_AB, p->h_LinvT, p->h_LinvS, p->h_cA, p->h_cT, p->h_cS, &c);
+  int st;
+  {
+    TableUpload up(p);
+    st = build_chunk_set(up, kc, set == 1, p->h_AB, p->h_LinvT, p->h_LinvS, p->h_cA, p->h_cT, p->h_cS, &c);
+    const cudaError_t e = up.wait();
+    if (st == SDD_OK && e != cudaSuccess) {
+      set_cuda_error(e);
+      st = SDD_ERR_CUDA;
+    }
+  }
   if (st) {
     free_chunk_set(c);
     return st;

@@ -848,84 +848,104 @@ cudaError_t launch_chain(const ChainArgs& a_in, int batch, int nfields, cudaStre
 }
 
 // ---- blocks to fixed point ------------------------------------------------------------------------
-// Block m of `out` (stride out_stride words) from rows [r0, r0 + nr) and columns [c0, c0 + nr) of the m-th
-// source matrix (column-major, leading dimension ld, stride src_stride, nrows rows: the column exponents are
-// those of whole columns, so that the row halves of a column share them); one thread per column, then per row.
-__global__ void __launch_bounds__(64) k_to_fixed(const double* src, size_t src_stride, int ld, int nrows, int r0, int c0,
-                                                 int nr, int ldl, i64* out, size_t out_stride) {
-  __shared__ int cx[kMaxNr];
-  const double* col = src + (size_t)blockIdx.x * src_stride + (size_t)c0 * ld;
-  i64* o = out + (size_t)blockIdx.x * out_stride;
-  int* rexp = reinterpret_cast<int*>(o + (size_t)ldl * ldl);
-  for (int c = threadIdx.x; c < ldl; c += blockDim.x) {
-    unsigned m = 0;
-    if (c < nr)
-      for (int r = 0; r < nrows; ++r) {
-        const unsigned h = abs_hi(col[(size_t)c * ld + r]);
-        if (h < 0x7ff00000u) m = max(m, h);
-      }
-    const int e = m >> 20 ? (int)(m >> 20) - 1022 : 0; // |A| < 2^e down the column
-    if (c < nr) cx[c] = e;
-    rexp[ldl + c] = e;
-  }
-  __syncthreads();
-  const double* a = col + r0;
-  for (int r = threadIdx.x; r < ldl; r += blockDim.x) {
-    double l1 = 0.0;
-    if (r < nr)
-      for (int c = 0; c < nr; ++c) l1 += fabs(ldexp(a[(size_t)c * ld + r], -cx[c]));
-    // 2^ea above the sum, with room for its rounding and for that of the high digits (31 bits and the sign)
-    const unsigned h = abs_hi(l1 * (1.0 + 1e-9)) >> 20;
-    const int ea = h == 0x7ff ? kFxBad : (int)h - 1022;
-    for (int c = 0; c < ldl; ++c) {
-      const i64 A = r < nr && c < nr && ea != kFxBad ? d2fx(a[(size_t)c * ld + r], 1084 - kMvA + ea + cx[c]) : 0;
-      reinterpret_cast<int2*>(o)[(size_t)c * ldl + r] = mv_digits(A);
-    }
-    rexp[r] = ea;
-  }
-}
-
-// A radial operator (row-major nr x nr on the device) as a three-digit block; one thread per column, then row.
-__global__ void __launch_bounds__(64) k_to_wide(const double* src, int nr, int ld, int* out) {
-  __shared__ int cx[kMaxNr];
-  int* rexp = out + 3 * ld * ld;
+// The scales of an nr x nr block at a (element (r, c) at a[r rs + c cs]), padded to ld: cx[c] with |A_rc| < 2^cx down
+// the column (over nrows rows from r = -r0 on, which share it), ea[r] with sum_c |A_rc| 2^-cx < 2^ea along the row
+// (kFxBad: a row with an infinity or NaN).  A row's sum is of whole numbers, 18 bits of its largest entry, each rounded
+// up: so a single entry stays 2^-24 below 2^ea, which the high digits (31 bits and the sign) need.  One thread a column,
+// then a row (with FP64 sums and scalings the conversions of a plan of 64 x 20 took 0.35 ms).
+// Ends with a barrier.
+__device__ __forceinline__ void block_scales(const double* a, int rs, int cs, int nrows, int r0, int nr, int ld, int* cx,
+                                             int* ea) {
   for (int c = threadIdx.x; c < ld; c += blockDim.x) {
     unsigned m = 0;
-    if (c < nr)
-      for (int r = 0; r < nr; ++r) m = max(m, abs_hi(src[r * nr + c]));
-    const int e = m >> 20 && m < 0x7ff00000u ? (int)(m >> 20) - 1022 : 0;
-    cx[c] = e;
-    rexp[ld + c] = e;
+    if (c < nr) {
+      const double* col = a + (ptrdiff_t)c * cs - (ptrdiff_t)r0 * rs;
+#pragma unroll 8
+      for (int r = 0; r < nrows; ++r) {
+        const unsigned h = abs_hi(col[(size_t)r * rs]);
+        if (h < 0x7ff00000u) m = max(m, h);
+      }
+    }
+    cx[c] = m >> 20 ? (int)(m >> 20) - 1022 : 0;
   }
   __syncthreads();
   for (int r = threadIdx.x; r < ld; r += blockDim.x) {
-    double l1 = 0.0;
-    if (r < nr)
-      for (int c = 0; c < nr; ++c) l1 += fabs(ldexp(src[r * nr + c], -cx[c]));
-    const unsigned h = abs_hi(l1 * (1.0 + 1e-13)) >> 20;
-    const int ea = h == 0x7ff ? kFxBad : (int)h - 1022;
-    for (int c = 0; c < ld; ++c) {
-      int d2 = 0, d1 = 0, d0 = 0;
-      if (r < nr && c < nr && ea != kFxBad) {
-        const double x = src[r * nr + c];
-        wx_split(x, 1022 + cx[c] + ea - (int)(abs_hi(x) >> 20), d2, d1, d0);
-      }
-      out[c * ld + r] = d2;
-      out[(ld + c) * ld + r] = d1;
-      out[(2 * ld + c) * ld + r] = d0;
+    const double* row = a + (size_t)r * rs;
+    const int n = r < nr ? nr : 0;
+    int em = -0x10000, bad = 0;
+#pragma unroll 8
+    for (int c = 0; c < n; ++c) {
+      const unsigned h = abs_hi(row[(size_t)c * cs]);
+      bad |= h >= 0x7ff00000u;
+      em = max(em, max((int)(h >> 20), 1) - cx[c]);
     }
-    rexp[r] = ea;
+    unsigned tot = 0;
+#pragma unroll 8
+    for (int c = 0; c < n; ++c) {
+      const unsigned h = abs_hi(row[(size_t)c * cs]);
+      int e1;
+      const unsigned m = fx_mant_hi(h, e1);
+      if (h) tot += (m >> min(em - (e1 - cx[c]) + 3, 31)) + 1;
+    }
+    ea[r] = bad ? kFxBad : max(tot ? em - 1040 + (32 - __clz((int)tot)) : -1022, -1022);
+  }
+  __syncthreads();
+}
+
+constexpr int kConvThreads = 256;
+
+// Block m of `out` (stride out_stride words) from rows [r0, r0 + nr) and columns [c0, c0 + nr) of the m-th
+// source matrix (element (r, c) at r rs + c cs, stride src_stride, nrows rows: the column exponents are those of whole
+// columns, so that the row halves of a column share them).
+__global__ void __launch_bounds__(kConvThreads) k_to_fixed(const double* src, size_t src_stride, int rs, int cs, int nrows,
+                                                           int r0, int c0, int nr, int ldl, i64* out, size_t out_stride) {
+  __shared__ int cx[kMaxNr], ea[kMaxNr];
+  const double* a = src + (size_t)blockIdx.x * src_stride + (size_t)r0 * rs + (size_t)c0 * cs;
+  i64* o = out + (size_t)blockIdx.x * out_stride;
+  block_scales(a, rs, cs, nrows, r0, nr, ldl, cx, ea);
+  for (int q = threadIdx.x; q < ldl * ldl; q += blockDim.x) {
+    const int c = q / ldl, r = q - c * ldl;
+    const bool in = r < nr && c < nr && ea[r] != kFxBad;
+    const i64 A = in ? d2fx(a[(size_t)r * rs + (size_t)c * cs], 1084 - kMvA + ea[r] + cx[c]) : 0;
+    reinterpret_cast<int2*>(o)[q] = mv_digits(A);
+  }
+  int* rexp = reinterpret_cast<int*>(o + (size_t)ldl * ldl);
+  for (int q = threadIdx.x; q < ldl; q += blockDim.x) {
+    rexp[q] = ea[q];
+    rexp[ldl + q] = cx[q];
+  }
+}
+
+// A radial operator (row-major nr x nr on the device) as a three-digit block.
+__global__ void __launch_bounds__(kConvThreads) k_to_wide(const double* src, int nr, int ld, int* out) {
+  __shared__ int cx[kMaxNr], ea[kMaxNr];
+  block_scales(src, nr, 1, nr, 0, nr, ld, cx, ea);
+  for (int q = threadIdx.x; q < ld * ld; q += blockDim.x) {
+    const int c = q / ld, r = q - c * ld;
+    int d2 = 0, d1 = 0, d0 = 0;
+    if (r < nr && c < nr && ea[r] != kFxBad) {
+      const double x = src[r * nr + c];
+      wx_split(x, 1022 + cx[c] + ea[r] - (int)(abs_hi(x) >> 20), d2, d1, d0);
+    }
+    out[q] = d2;
+    out[ld * ld + q] = d1;
+    out[2 * ld * ld + q] = d0;
+  }
+  int* rexp = out + 3 * ld * ld;
+  for (int q = threadIdx.x; q < ld; q += blockDim.x) {
+    rexp[q] = ea[q];
+    rexp[ld + q] = cx[q];
   }
 }
 
 cudaError_t launch_to_wide(const double* src, int nr, int ld, int* out, cudaStream_t s) {
-  k_to_wide<<<1, 64, 0, s>>>(src, nr, ld, out);
+  k_to_wide<<<1, kConvThreads, 0, s>>>(src, nr, ld, out);
   return cudaGetLastError();
 }
 
-cudaError_t launch_to_fixed(const double* src, size_t src_stride, int ld, int nrows, int r0, int c0, int nr, int ldl,
-                            i64* out, size_t out_stride, int nblk, cudaStream_t s) {
-  k_to_fixed<<<nblk, 64, 0, s>>>(src, src_stride, ld, nrows, r0, c0, nr, ldl, out, out_stride);
+cudaError_t launch_to_fixed(const double* src, size_t src_stride, int rs, int cs, int nrows, int r0, int c0, int nr,
+                            int ldl, i64* out, size_t out_stride, int nblk, cudaStream_t s) {
+  k_to_fixed<<<nblk, kConvThreads, 0, s>>>(src, src_stride, rs, cs, nrows, r0, c0, nr, ldl, out, out_stride);
   return cudaGetLastError();
 }
 

@@ -381,8 +381,8 @@ cudaError_t launch_chain(const ChainArgs& a, int batch, int nfields, cudaStream_
 // the chain layout launch_chain runs for a.layout (0 = automatic) and this launch size
 int resolve_chain_layout(const ChainArgs& a, int batch, int nfields);
 // fixed-point blocks from FP64 matrices on the device (setup)
-cudaError_t launch_to_fixed(const double* src, size_t src_stride, int ld, int nrows, int r0, int c0, int nr, int ldl,
-                            i64* out, size_t out_stride, int nblk, cudaStream_t s);
+cudaError_t launch_to_fixed(const double* src, size_t src_stride, int rs, int cs, int nrows, int r0, int c0, int nr,
+                            int ldl, i64* out, size_t out_stride, int nblk, cudaStream_t s);
 cudaError_t launch_to_wide(const double* src, int nr, int ld, int* out, cudaStream_t s);
 cudaError_t launch_chunk_fix(const ChainArgs& a, int batch, int nfields, cudaStream_t s);
 cudaError_t launch_theta_op(int op, int M, int nr, int sym, const double* D2, const double* ir,
