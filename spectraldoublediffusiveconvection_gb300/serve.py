@@ -28,6 +28,7 @@ its next quantum boundary (integrations) or when its batched call returns (conti
 """
 import collections
 import itertools
+import math
 import threading
 import time
 
@@ -128,6 +129,25 @@ class _IntGroup:
         self.left.pop()
 
 
+def table_bytes(M, nr, mixed):
+    """Device bytes of a plan's tables as the library allocates them (csrc/sdd_api.cu): per mode the blocks of the three
+    inverses, of the psi step matrices (two) and of the corrections of two chunkings (four each), the chunkings' carry
+    maps and products, each block padded to ld x ld 64-bit words and its exponents; the radial operators; mixed plans
+    also FP32 inverses.  Allocations above 1 MB take whole pages of 2 MB."""
+    ld = (nr + 7) // 8 * 8 if nr <= 32 else (nr + 15) // 16 * 16
+    S = M // 2
+    nch = [-(-S // max(lo, min(hi, int(math.floor(math.sqrt(f * S) + 0.5)))))
+           for lo, hi, f in ((4, 32, 2.0), (2, 16, 0.72 if nr > 32 else 0.5))]
+    products = (nch[1] - 1) * (nch[1] - 2) // 2
+    blocks = [M] * 3 + [2 * M] + 2 * [2 * M, M, M] + [8 * nch[0]] + 2 * [2 * nch[0]] + [8 * products] + 2 * [2 * products]
+    sizes = [8 * (ld + 1) * ld * n for n in blocks + [1]] + 3 * [4 * (3 * ld + 2) * ld]
+    sizes += [8 * nr * nr] * 3 + [4 * nr * nr] * 2 + [32 * M] * 3 + [8 * ((M + 1) // 2) * nr, 24 * M]
+    if mixed:
+        sizes += 3 * [4 * M * nr * ld] + [4 * nr * nr, 16 * ((nr + 7) // 8 * 8) ** 2]
+    page = 1 << 21
+    return sum(-(-n // page) * page if 2 * n > page else n for n in sizes)
+
+
 class Server:
     """Request server over one GPU.  Integrations use plans with step dt and nonlinear-term precision
     ``int_precision``; continuation steps use plans with dt = 1 (Main.py:430, PFX over one unit of time),
@@ -204,11 +224,10 @@ class Server:
             per += 8 * ((self.restart + 12) * (n + 1) + 2 * 9 * nr * (3 * M // 2 + 1))
         return per
 
-    @staticmethod
-    def plan_bytes(req):
-        """Device bytes of a plan's operators (dense radial inverses and fused chain tables per mode)."""
-        M, nr = req.N_theta, req.N_r - 1
-        return 8 * (7 * M * nr * nr + 16 * nr * nr)
+    def plan_bytes(self, req):
+        """Device bytes of the plan a request runs on (table_bytes)."""
+        mixed = self.int_precision == "mixed" if req.kind == "integrate" else bool(self.con_mixed)
+        return table_bytes(req.N_theta, req.N_r - 1, mixed)
 
     def _try_admit(self, req):
         """True when admitted, False to wait for memory, "reject" when the request can never fit (the
