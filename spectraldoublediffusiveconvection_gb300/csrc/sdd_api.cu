@@ -1025,7 +1025,6 @@ static ChainArgs chain_args(const sdd_plan* p, const double* g, double* f, const
   a.h = p->hbuf;
   a.h_stride = shell_elems(p);
   a.coefA4 = p->coefA4; a.coefT = p->coefT; a.coefS = p->coefS;
-  a.dtA4 = p->Pr * p->dt; a.dtT = p->dt; a.dtS = p->Tau * p->dt;
   a.ldd = p->ldd;
   a.cset[0] = p->cs[0];
   a.cset[1] = p->cs[1];
@@ -1047,9 +1046,9 @@ static int check_plan(sdd_plan* p, int batch) {
 // One application of Phi (the step map) or its Jacobian to X (or dv), into out.
 // mode 0: FX (nonlinear term of X); 1: DFX about the base in `base`; 2: linear only.
 // Same as apply_step with explicit strides (doubles between shells) of the input X, the output and sub.
-// The right-hand sides are not assembled by k_rhs: the grid kernel (split nonlinear term) or k_rhs_lin writes
-// their linear parts (FP64 in both precisions) and the chains' h kernel adds the nonlinear parts (the roundings
-// of k_rhs).
+// The right-hand sides of a step are not assembled by k_rhs: the grid kernel (split nonlinear term) or k_rhs_lin
+// writes their linear parts (FP64 in both precisions) and the chains' h kernel adds the nonlinear parts, with Dr Q as a
+// three-digit product (k_rhs sums it in FP64: the two agree to rounding).
 // ev (nullable): four events recorded around the nonlinear term, the rhs and the chains.
 // The pending correction of layouts 3 / 11 (chunk set 1) of a state X (and its FP32 copy x32, nullable),
 // for FixArgs.

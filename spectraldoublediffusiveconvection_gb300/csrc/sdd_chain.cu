@@ -447,7 +447,7 @@ __device__ __forceinline__ double carried_state(const ChainArgs& a, int b, size_
 //   FIX = true:   f_jj += G_jj s_c(jj) for the modes of chunks c >= 1   (chunked chains' correction)
 constexpr int kMvShells = 4;
 
-// The right-hand side of FIX = false is a.g, or (fuse_rhs) formed here with the roundings of k_rhs:
+// The right-hand side of FIX = false is a.g, or (fuse_rhs) formed here, each operation rounded by itself:
 //   psi: (-dt (Dr Q - R)) + lin,  T: (-dt NT) + lin,  S: (-dt NS) + lin,
 // Dr Q in fixed point like the other matvecs, or (mixed plans' FP32 nonlinear term) in FP32.
 template <bool FIX, int LD>
@@ -765,14 +765,11 @@ cudaError_t launch_chunk_fix(const ChainArgs& a_in, int batch, int nfields, cuda
 }
 
 // The number a layout request resolves to (sdd_plan_chain_choice).  The whole-chain layouts run one kernel
-// (k_chain_fx); which of their numbers is reported follows the shared memory that a step-matrix ring of that
-// layout takes at this shape, so that callers keep the numbers they have stored.
+// (k_chain_fx); whether 8 and 9 are reported as such follows the shared memory that three step-matrix rings in one CTA
+// would take at this shape, so that callers keep the numbers they have stored.
 static size_t layout_bytes(int layout, int M, int nr, int ldl) {
   const size_t blk = (size_t)nr * ldl, ns = 4 * ((size_t)(M + 1) / 2 + 1), v = nr;
-  if (layout == 8) return ((4 * blk + ns + 4 * v) + 2 * (3 * blk + ns + 2 * v)) * sizeof(double);
-  if (layout == 9) return ((6 * blk + ns + 4 * v) + 2 * (3 * blk + ns + 4 * v)) * sizeof(double);
-  if (layout == 6) return (4 * blk + ns + 4 * v) * sizeof(double);
-  return (6 * blk + ns + 4 * v) * sizeof(double);
+  return ((layout == 8 ? 4 : 6) * blk + ns + 4 * v + 2 * (3 * blk + ns + (layout == 8 ? 2 : 4) * v)) * sizeof(double);
 }
 
 int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
@@ -810,9 +807,6 @@ int resolve_chain_layout(const ChainArgs& a, int batch, int nfields) {
   if (a.layout == 0 && (layout == 2 || layout == 3) && !a.split_fx && !a.g32) layout += 8;
   // layouts 6 / 7 need the full right-hand side in FP64: with the fused or the FP32 one, the pre-pass form
   if ((layout == 6 || layout == 7) && (a.split_fx || a.g32)) layout = 5;
-  if ((layout == 6 || layout == 7) && layout_bytes(6, a.M, a.nr, a.ldl) > (size_t)optin) layout = 2;
-  if (layout != 2 && layout != 3 && layout < 6 && layout_bytes(4, a.M, a.nr, a.ldl) > (size_t)optin)
-    layout = 2;   // whole chain too long for shared memory
   // a launch that fills the SMs (one kernel; the number as in layout_bytes)
   if (layout == 0) {
     if (2 * nfields * batch <= sms) layout = 4;

@@ -17,10 +17,11 @@
 // ping-ponging between two shared-memory buffers; twiddles come from a table exp(-2 pi i k/L) built on
 // the host.
 //
-// FP32 transforms run in FP32.  FP64 transforms run in 64-bit fixed point on the integer pipe (sdd_fixed.cuh):
-// each row scaled by a power of two above its 1-norm, which bounds every value inside its transform, 36 wide multiply-adds (4.5 to 5
-// cycles each)  N_r=30, N_theta=256: grid kernel
-// 18.9 -> 14.6 us, product kernel 14.4 -> 10.2 us, row kernel of 64 shells 712 -> 492 us.
+// FP32 transforms run in FP32.  FP64 transforms run in 64-bit fixed point on the integer pipe (sdd_fixed.cuh): each row
+// scaled by a power of two above its 1-norm, which bounds every value inside its transform; a complex product is 12 wide
+// multiply-adds, a radix-4 butterfly with its twiddles 36, of 4.5 to 5 cycles each.
+// N_r=30, N_theta=256, FP64 / fixed point: grid kernel 18.9 / 14.6 us, product kernel 14.4 / 10.2 us, row kernel of 64
+// shells 712 / 492 us.
 #pragma once
 #include <cuda_runtime.h>
 #include "sdd_fixed.cuh"

@@ -988,6 +988,8 @@ __global__ void __launch_bounds__(kFxRowThreads) k_fx_prod(FxArgs a, const T* gr
 }
 
 // ---- right-hand sides of the three implicit solves (Main.py:262-280) ---------------------------
+// Linear steps, and (cnab2) the second-order step with the nonlinear term's outputs and the history; other steps form
+// theirs in k_fx_grid or k_rhs_lin and the h kernel.
 __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr;
@@ -1024,7 +1026,7 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
       for (int m = 0; m < nr; ++m) d2 = fma(opr[nr + m], ps[m], d2);
       pn = ps[n];
     }
-    if (O4 && a.q32) {         // FP32 nonlinear term: Dr Q in FP32 (the order of the chains' fused_g)
+    if (O4 && a.q32) {         // FP32 nonlinear term: Dr Q in FP32 (the h kernel's order of sums)
       const float* qs = a.q32 + (size_t)b * M * nr + (size_t)k * nr;
       const float* drn = a.Dr32 + (size_t)n * nr;
       float d = 0.0f;
@@ -1053,22 +1055,14 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
     const double k1 = kd[k + 1], k2 = kd[k + 2];
     const double JP = lin_jt(k, k1, k > 0 ? pv[k - 1] : 0.0, (k + 1 < M) ? Sc[k + 1] : 0.0);    // J_theta_RT
     const double Om = lin_a2(D2p[k], k1, k2, ir2, pv[k], (k + 2 < M) ? Sc[k + 2] : 0.0);          // A2_SINE
-    double nxp = 0, nxt = 0, nxs = 0;
-    if (O4) {
-      const size_t o = (size_t)k * nr + n;
-      nxp = -dt * (DrQ[k] - O4[N + o]);
-      nxt = -dt * O4[2 * N + o];
-      nxs = -dt * O4[3 * N + o];
-    }
     const size_t o = (size_t)k * nr + n;
     if (a.cnab2) {
       const double grv = (k < M - 1) ? (-k1 * gr) * (Ra * Tv[k + 1] - Ras * Sv[k + 1]) : 0.0;
       const double psiT0 = dT0 * JP;                                            // DT0_theta
       // explicit terms per unit time at this step, and the Adams-Bashforth 2 extrapolation
-      const size_t ko = (size_t)k * nr + n;
-      const double ep = (O4 ? -(DrQ[k] - O4[N + ko]) : 0.0) + a.Pr * grv;
-      const double et = (O4 ? -O4[2 * N + ko] : 0.0) - psiT0;
-      const double es = (O4 ? -O4[3 * N + ko] : 0.0) - psiT0;
+      const double ep = -(DrQ[k] - O4[N + o]) + a.Pr * grv;
+      const double et = -O4[2 * N + o] - psiT0;
+      const double es = -O4[3 * N + o] - psiT0;
       double* H = a.hist + (size_t)b * a.rhs_stride;
       double xp = ep, xt = et, xs = es;
       if (a.hist_valid) {
@@ -1084,9 +1078,9 @@ __global__ void __launch_bounds__(kFxThreads) k_rhs(RhsArgs a) {
       R[2 * N + o] = fma(dt, xs, 2.0 * (rsq * Sv[k]));
       continue;
     }
-    R[o] = nxp + (k < M - 1 ? lin_psi_rhs(Om, k1, gd, Ra, Ras, Tv[k + 1], Sv[k + 1]) : Om);
-    R[N + o] = nxt + lin_ts_rhs(rsq, Tv[k], dd, JP);
-    R[2 * N + o] = nxs + lin_ts_rhs(rsq, Sv[k], dd, JP);
+    R[o] = k < M - 1 ? lin_psi_rhs(Om, k1, gd, Ra, Ras, Tv[k + 1], Sv[k + 1]) : Om;
+    R[N + o] = lin_ts_rhs(rsq, Tv[k], dd, JP);
+    R[2 * N + o] = lin_ts_rhs(rsq, Sv[k], dd, JP);
   }
 }
 

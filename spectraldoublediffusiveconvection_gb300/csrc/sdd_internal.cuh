@@ -227,7 +227,6 @@ struct FxArgs {
   size_t base_stride;        // elements between shells in base
   double* out4;              // [shell][4][M][nr] : Qhat, Rhat, NJ_T hat, NJ_S hat
   size_t out_stride;         // doubles between shells in out4
-  double* fx_out;            // optional: write F directly in state layout [shell][3][M][nr]
   size_t fx_stride;
   void* grid;                // nullable: grid-field scratch [shell][nr][9][P] (T precision) of the split path
   size_t grid_stride;        // elements between shells in grid
@@ -235,7 +234,7 @@ struct FxArgs {
   void* deriv;               // split path: radial derivatives [shell][5][M][nr] (T): Dr psi, D2r2 psi, Dr T, Dr S
                              // (and, with fuse_rhs, D2s psi in FP64 as the fifth block)
   size_t deriv_stride;       // elements between shells in deriv
-  // fuse_rhs: the right-hand sides' linear parts (the terms of k_rhs that do not involve the nonlinear term)
+  // fuse_rhs: the right-hand sides' linear parts (the terms of Main.py:262-280 that do not involve the nonlinear term)
   // are written into rl.rhs, by k_fx_grid (split path) or k_rhs_lin; the chains' h kernel adds the nonlinear
   // parts from out4.  rl carries the operators, parameters and the rhs buffer; deriv's fifth block the FP64
   // D2 psi that they need.
@@ -270,7 +269,7 @@ struct TcArgs {
 
 
 
-// Tables of one chunking of the chains (see k_chain): chunk length kc, nch chunks per chain, the
+// Tables of one chunking of the chains (see k_chain_fx): chunk length kc, nch chunks per chain, the
 // corrections G_jj of every mode and the carried-state maps, either per chunk (Phi_c, the sequential
 // carry of layout 2) or as the products P_{j,i} = Phi_{j-1} ... Phi_{i+1}, i <= j - 2 (np per chain,
 // row j after row j-1; the parallel carry of layout 3).
@@ -301,9 +300,8 @@ struct ChainArgs {
   size_t h_stride;           // doubles between shells in h
   const double* coefA4;      // [M][4] per jj: (dt bjt, dt bjt bj, bj, bjt), dt = Pr*dt, j = M - jj
   const double* coefT, *coefS;  // [M][4] per jj: (2 dt (j+2), 0.5 if j == 0 else 1, 0, 0), j = M-1-jj
-  double dtA4, dtT, dtS;     // Pr*dt, dt, Tau*dt
   // fuse_rhs: g is not read; the h kernel forms g from the linear parts in `lin` and the nonlinear-term
-  // outputs in out4 (psi: -dt (Dr Q - R) + lin; T, S: -dt N + lin), exactly as k_rhs would
+  // outputs in out4 (psi: -dt (Dr Q - R) + lin; T, S: -dt N + lin)
   int fuse_rhs;
   const double* lin;         // [shell][3][M][nr] linear parts (k_fx_grid), stride g_stride
   const double* out4;        // [shell][4][M][nr]

@@ -64,19 +64,13 @@ __device__ __forceinline__ double warp_sum4(const double (&sv)[4], int lane) {
   return k;
 }
 
-// Exact power-of-two balancing of the rows that share one complex FFT.  The two rows of a pair ride in
+// Exact power-of-two balancing of the FP32 rows that share one complex FFT (FP64 rows: rows_to_fixed).  The two rows of a pair ride in
 // the real and imaginary parts, and the FFT's rounding error scales with the larger of the two: an
 // unbalanced pair (|komega| ~ 1e3 next to |JT_psi| ~ 1e-2) would leave the small row with an error of
 // eps*1e3.  Each row is therefore scaled by 2^-e, e = exponent of its max |value| (exact), before the
 // transform and scaled back after it.  The maxima are taken on the IEEE bit patterns (for non-negative
-// values the unsigned order is the numeric order), i.e. with integer instructions: on GB300 the FP64
-// pipe is the scarce resource of these kernels.
+// values the unsigned order is the numeric order), i.e. with integer instructions.
 template <typename T> struct Bits;
-template <> struct Bits<double> {
-  using U = unsigned long long;
-  static __device__ __forceinline__ U absbits(double x) { return (U)__double_as_longlong(x) & 0x7fffffffffffffffull; }
-  static __device__ __forceinline__ double val(U u) { return __longlong_as_double((long long)u); }
-};
 template <> struct Bits<float> {
   using U = unsigned int;
   static __device__ __forceinline__ U absbits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
