@@ -176,6 +176,12 @@ class ShellBatch:
             best = min(best, e0.elapsed_time(e1) * 1e-3 / reps)
         return best
 
+    @staticmethod
+    def _chain_form(g):
+        """The chains that a step of the group runs: "whole", or 0 / 1 (chunk set: sequential / parallel carry)."""
+        lay = g.plan.chain_choice(len(g.idx))[0]
+        return {2: 0, 10: 0, 3: 1, 11: 1}.get(lay, "whole")
+
     def autotune(self, steps_per_launch=5, reps=3, layouts=(1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11), fx_modes=(1, 2),
                  chunk_scales=(0.6, 1.6), min_gain=0.015):
         """Greedy per-group choice of the chain layout, then of the nonlinear-term kernel (fused or split),
@@ -189,11 +195,15 @@ class ShellBatch:
         start = [(g.plan.chain_layout, g.plan.fx_split, list(g.plan.chunk_length)) for g in self.groups]
         t_start = best = self._time_graph(reps)
         for g in self.groups:
+            # layouts that run the same chains as one already timed (whole chains; chunks with a sequential or a
+            # parallel carry) are the same launches: another timing of them would only add noise to the choice
             choice = g.plan.chain_layout
+            timed = {self._chain_form(g)}
             for lay in layouts:
-                if lay == choice:
-                    continue
                 g.plan.set_chain_layout(lay)
+                if self._chain_form(g) in timed:
+                    continue
+                timed.add(self._chain_form(g))
                 t = self._time_graph(reps)
                 if t < best * (1.0 - min_gain):
                     best, choice = t, lay
