@@ -68,11 +68,28 @@ const FftPlan* get_fft_plan(int L) {
     fx_split_host(llroundl(ldexpl(sn, 62)), &d.z, &d.w);
     return d;
   };
+  // pi j / 2L for j <= L/2 (the first eighth of the circle) gives every angle by reflection: long double sines and
+  // cosines are formed in software on some hosts (the first transform of 2000 points takes 1.0 ms, 2.8 with one of them
+  // for each entry), and the large arguments' rounding cost bits where long doubles have 64 (2^-60.5, now 2^-63.4)
+  std::vector<long double> c8(L / 2 + 1), s8(L / 2 + 1);
+  for (int j = 0; j <= L / 2; ++j) {
+    const long double t = pi * (long double)j / (2.0L * (long double)L);
+    c8[j] = cosl(t);
+    s8[j] = sinl(t);
+  }
+  auto at = [&](int m, long double* c, long double* sn) {   // angle 2 pi m / 4L, 0 <= m < 4L
+    const int q = m / L, r = m % L;
+    const bool low = 2 * r <= L;
+    const long double x = low ? c8[r] : s8[L - r], y = low ? s8[r] : c8[L - r];
+    *c = q == 0 ? x : q == 1 ? -y : q == 2 ? -x : y;
+    *sn = q == 0 ? y : q == 1 ? x : q == 2 ? -y : -x;
+  };
   for (int k = 0; k < L; ++k) {
-    const long double a = 2.0L * pi * (long double)k / (long double)L;
-    const long double b = pi * (long double)k / (2.0L * (long double)L);
-    w[k] = digits(cosl(a), -sinl(a));
-    e[k] = digits(0.5L * cosl(b), 0.5L * sinl(b));
+    long double c, sn;
+    at(4 * k, &c, &sn);
+    w[k] = digits(c, -sn);
+    at(k, &c, &sn);
+    e[k] = digits(0.5L * c, 0.5L * sn);
     const double ad = 2.0 * (double)pi * (double)k / (double)L, bd = (double)pi * (double)k / (2.0 * (double)L);
     wf[k] = make_float2((float)std::cos(ad), (float)-std::sin(ad));
     ef[k] = make_float2((float)(0.5 * std::cos(bd)), (float)(0.5 * std::sin(bd)));
