@@ -28,7 +28,10 @@ size_t diag_rows_smem_bytes(int M, int L) {
 // state (|X|^2, Nu_T, Nu_S); the shell's last CTA adds the partial sums in order.  (As a kernel of one CTA a shell
 // the outer sums took longer than the rows: 12.0 + 17.5 us at 90 x 23, now 15 us, most of it the latency of the
 // transform's passes and of a few dozen dependent FP64 operations.)
-__global__ void __launch_bounds__(256) k_diag(DiagArgs a) {
+// Two CTAs an SM (128 registers): of the 196 that the widest pass takes unbounded one CTA fits, and batches, whose small
+// CTAs wait at their barriers, took longer than with FP64 transforms.  us a call, FP64 / 196 / 128 registers: 12 x 65, 64
+// shells 152 / 234 / 129, 24 x 34 78 / 118 / 65, 64 x 20 56 / 72 / 42, one shell 21 / 12 / 11; 90 x 23 29 / 13.3 / 13.0.
+__global__ void __launch_bounds__(256, 2) k_diag(DiagArgs a) {
   using C = longlong2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int M = a.M, nr = a.nr, L = a.L;
