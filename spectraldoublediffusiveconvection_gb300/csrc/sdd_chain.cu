@@ -709,17 +709,30 @@ static cudaError_t launch_mode_mv(const ChainArgs& a, int batch, int nfields, cu
 }
 
 // The chains themselves: whole (nch = 1 CTA per pair of chains) or chunked.  Two shells share a CTA (and the
-// blocks' way through shared memory) once a CTA per shell would give every SM more than one.
+// blocks' way through shared memory) once a CTA per shell would give every SM more than one.  Blocks of 48 rows: a ring of
+// four slots while every CTA has an SM of its own, of two slots beyond, of which three CTAs share an SM and hide each
+// other's waits (a ring of four takes 150 KB; FP64 chains before ran two an SM).  us a linear step, four / two slots (and
+// FP64 chains): 24 x 34, 64 shells 62 / 51 (58), 128 shells 114 / 91 (96); 96 x 36, 128 shells 339 / 266 (305), 8 shells
+// in chunks (160 CTAs) 58 / 55; one CTA an SM: 24 x 34, 32 shells 34 / 37, 192 x 36, 4 shells in chunks 59 / 67.
+template <int LD, bool CHUNK, int D>
+static cudaError_t launch_chains_ring(const ChainArgs& a, int batch, int ntypes, int nch, int nsteps, int spc,
+                                      cudaStream_t s) {
+  constexpr int W = (LD + 31) / 32;
+  static unsigned long long done = 0;
+  const cudaError_t e = ensure_smem_attr(k_chain_fx<LD, CHUNK, D>, &done);
+  if (e != cudaSuccess) return e;
+  return launch_kernel(k_chain_fx<LD, CHUNK, D>, dim3(2 * ntypes, (batch + spc - 1) / spc, nch), dim3(64 * W * spc + 32),
+                       chain_fx_smem_bytes(nsteps, LD, D), s, a, spc, batch);
+}
 template <bool CHUNK>
 static cudaError_t launch_chains(const ChainArgs& a, int batch, int ntypes, int nch, int nsteps, cudaStream_t s) {
+  const bool many = 2l * ntypes * batch * nch > sm_count();
   const cudaError_t e = with_ld(a.ldl, [&](auto ld) {
-    constexpr int LD = decltype(ld)::value, W = (LD + 31) / 32, D = LD > 48 ? 3 : 4;
-    static unsigned long long done = 0;
-    const cudaError_t er = ensure_smem_attr(k_chain_fx<LD, CHUNK, D>, &done);
-    if (er != cudaSuccess) return er;
-    const int spc = W == 1 && 2l * ntypes * batch * nch > sm_count() ? 2 : 1;
-    return launch_kernel(k_chain_fx<LD, CHUNK, D>, dim3(2 * ntypes, (batch + spc - 1) / spc, nch),
-                         dim3(64 * W * spc + 32), chain_fx_smem_bytes(nsteps, LD, D), s, a, spc, batch);
+    constexpr int LD = decltype(ld)::value;
+    if constexpr (LD == 48) {
+      if (many) return launch_chains_ring<LD, CHUNK, 2>(a, batch, ntypes, nch, nsteps, 1, s);
+    }
+    return launch_chains_ring<LD, CHUNK, (LD > 48 ? 3 : 4)>(a, batch, ntypes, nch, nsteps, LD <= 32 && many ? 2 : 1, s);
   });
   ktimer_mark(SDD_K_CHAIN, s);
   return e;
