@@ -452,6 +452,11 @@ __device__ __forceinline__ void cp_async_one(E* smem, const E* gmem) {
 // multiply-adds, which run on kOrthCtas SMs a shell only: longer vectors keep the launches.  us a column with its
 // product, launches / one launch: FP64, n = 3648 104 / 67, 7488 114 / 83, 11808 120 / 109, 15744 128 / 132; FP32 basis,
 // 8 shells, n = 4416 113 / 80, 15744 182 / 180.
+// The rule goes by the vector's length alone, so that a shell's solve has the same bits alone and in any batch (the two
+// forms sum in different orders).  Large batches pay for that: a cluster takes 16 SMs, nine run at a time.  Launches /
+// one launch, 64 shells: FP64 n = 336 128 / 103, 3648 241 / 252, 6624 378 / 409, 11808 697 / 768; FP32 basis 336 110 / 112,
+// 3648 155 / 164, 8832 268 / 277, 15744 507 / 598.  With 12 shells or fewer one launch is the faster one at every length
+// it takes (the closest: FP64 n = 11808, 12 shells, 218 / 209).
 // Projections: a warp takes four vectors and (few vectors) a quarter or a half of the slice; FP64 sums, or with an
 // FP32 basis FP32 sums of at most 256 products, as in k_dot_partials.
 // STAGE: the slice's part of V_0 .. V_j waits in shared memory (both passes read it twice), where it fits.
