@@ -884,7 +884,7 @@ __device__ __forceinline__ void block_scales(const double* a, int rs, int cs, in
     for (int c = 0; c < n; ++c) {
       const unsigned h = abs_hi(row[(size_t)c * cs]);
       bad |= h >= 0x7ff00000u;
-      em = max(em, max((int)(h >> 20), 1) - cx[c]);
+      if (h) em = max(em, max((int)(h >> 20), 1) - cx[c]);
     }
     unsigned tot = 0;
 #pragma unroll 8

@@ -64,3 +64,27 @@ def test_rows_of_the_solves_keep_to_their_bound(cuda, nr):
                 bound = 2.0 ** -58 * (nr + 2) * np.ldexp(np.abs(A), -cx).sum(axis=1) * np.abs(np.ldexp(v, cx)).max()
                 ref = A.astype(LD) @ v.astype(LD)
                 assert np.all(np.abs((y[M - 1 - jj] - ref).astype(float)) <= bound + 2.0 ** -53 * np.abs(ref.astype(float)))
+
+
+def test_zeros_of_a_tiny_column_do_not_set_a_rows_scale(cuda):
+    """A column of numbers near 2^-1010 with zeros in it, and a row whose other entries lie 2^-40 below their columns'
+    largest: the row keeps to its own bound (test_rows_of_the_solves_keep_to_their_bound)."""
+    from spectraldoublediffusiveconvection_gb300.operators import plan_arrays
+    from spectraldoublediffusiveconvection_gb300.plan import Plan
+    M, N_r = 4, 12
+    nr = N_r - 1
+    arrays = plan_arrays(M, N_r, 2.0, 1e-3, 1.0, 0.01)
+    A = np.random.default_rng(5).standard_normal((nr, nr))
+    A[1] *= 2.0 ** -40
+    A[:, 0] = 0.0
+    A[0, 0] = 2.0 ** -1010
+    arrays["Linv_T"] = np.repeat(A[None], M, axis=0)
+    p = Plan(M, N_r, 2.0, 1e-3, 1.0, 0.01, arrays=arrays)
+    G = np.zeros((M, nr))
+    G[M - 1] = np.random.default_rng(6).standard_normal(nr)
+    y = p.nab2_bsub(1, cuda.from_numpy(G.ravel()).cuda()).cpu().numpy().reshape(M, nr)[M - 1]
+    v = G[M - 1]
+    cx = np.frexp(np.abs(A).max(axis=0))[1]
+    bound = 2.0 ** -58 * (nr + 2) * np.ldexp(np.abs(A), -cx).sum(axis=1) * np.abs(np.ldexp(v, cx)).max()
+    ref = A.astype(LD) @ v.astype(LD)
+    assert np.all(np.abs((y - ref).astype(float)) <= bound + 2.0 ** -53 * np.abs(ref.astype(float)))
